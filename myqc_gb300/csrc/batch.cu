@@ -38,42 +38,21 @@ constexpr int BATCH_MAX_N = 116;  // 2 n^2 doubles of shared memory per CTA
 
 __device__ __forceinline__ double bsum(double v, double *red) { return jac_block_sum(v, red); }
 
-__device__ __forceinline__ double bmax(double v, double *red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t = fmax(t, red[w]);
-  return t;
-}
-
-// C = A B for n x n column-major matrices (any of them shared or global)
-__device__ __forceinline__ void cta_matmul(int n, const double *A, const double *B, double *C) {
-  const size_t n2 = (size_t)n * n;
-  for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) {
-    const int i = (int)(idx % n), j = (int)(idx / n);
-    double s = 0.0;
-    for (int k = 0; k < n; ++k) s += A[i + (size_t)n * k] * B[k + (size_t)n * j];
-    C[idx] = s;
-  }
-}
+__device__ __forceinline__ double bmax(double v, double *red) { return jac_block_max(v, red); }
 
 // X = S^-1/2 = U s^-1/2 U^T per molecule; status bit 1 if S is not positive definite
 __global__ void __launch_bounds__(BT) batch_orth_kernel(const MolDesc *__restrict__ mols,
                                                         const double *__restrict__ S, double *__restrict__ X,
-                                                        int *__restrict__ status) {
+                                                        double *__restrict__ work, int *__restrict__ status) {
   extern __shared__ double sm[];
   __shared__ double red[BT / 32];
-  __shared__ int flag;
   const MolDesc md = mols[blockIdx.x];
   const int n = md.n;
   const size_t n2 = (size_t)n * n;
   double *A = sm, *V = sm + n2, *cs = V + n2;
   for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) A[idx] = S[md.mat + idx];
   __syncthreads();
-  const bool ok = jacobi_block(n, A, V, cs, red, &flag, 60, 1e-14);
+  const bool ok = jacobi_block(n, A, V, cs, red, work + 2 * md.mat, 60, 1e-14);
   // s^-1/2 on the diagonal of A
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double s = A[i + (size_t)n * i];
@@ -82,12 +61,9 @@ __global__ void __launch_bounds__(BT) batch_orth_kernel(const MolDesc *__restric
   }
   __syncthreads();
   if (threadIdx.x == 0 && !ok) atomicOr(status + blockIdx.x, 2);
-  for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) {
-    const int k = (int)(idx % n), l = (int)(idx / n);
-    double x = 0.0;
-    for (int i = 0; i < n; ++i) x += V[k + (size_t)n * i] * cs[i] * V[l + (size_t)n * i];
-    X[md.mat + idx] = x;
-  }
+  for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) A[idx] = V[idx] * cs[idx / n];
+  __syncthreads();
+  cta_mm<true>(n, n, n, A, V, X + md.mat);
 }
 
 // F = H + G and E_k = 1/2 sum D (F + H) + E_nuc (getEnr, scf.f90:1122-1152;
@@ -135,9 +111,9 @@ __global__ void __launch_bounds__(BT) batch_diis_kernel(const MolDesc *__restric
   double *T = sm, *U = sm + n2;
   const int2 st = state[m];
   const int h = st.x, nh = min(st.y + 1, ndiis);
-  cta_matmul(n, F + md.mat, D + md.mat, T);
+  cta_mm(n, n, n, F + md.mat, D + md.mat, T);
   __syncthreads();
-  cta_matmul(n, T, S + md.mat, U);
+  cta_mm(n, n, n, T, S + md.mat, U);
   __syncthreads();
   double *Fs = Fh + mat_total * h + md.mat, *Es = Eh + mat_total * h + md.mat;
   for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) {
@@ -219,10 +195,10 @@ __global__ void __launch_bounds__(BT) batch_density_kernel(
     int guess, const MolDesc *__restrict__ mols, int *__restrict__ active, const double *__restrict__ X,
     const double *__restrict__ Fx, double *__restrict__ D, double *__restrict__ Dn, double *__restrict__ eps,
     int *__restrict__ iters, int *__restrict__ conv, const double *__restrict__ Ek, double *__restrict__ Efin,
-    double thr, int conv_rms, int max_iter, int *__restrict__ status) {
+    double thr, int conv_rms, int max_iter, double *__restrict__ work, int *__restrict__ status) {
   extern __shared__ double sm[];
   __shared__ double red[BT / 32];
-  __shared__ int flag, decision;
+  __shared__ int decision;
   const int m = blockIdx.x;
   if (!guess && !active[m]) return;
   const MolDesc md = mols[m];
@@ -231,11 +207,11 @@ __global__ void __launch_bounds__(BT) batch_density_kernel(
   double *A = sm, *V = sm + n2, *cs = V + n2;
   int *perm = (int *)(cs + n + 2);
   const double *Xm = X + md.mat;
-  cta_matmul(n, Fx + md.mat, Xm, V);  // T = Fx X
+  cta_mm(n, n, n, Fx + md.mat, Xm, V);  // T = Fx X
   __syncthreads();
-  cta_matmul(n, Xm, V, A);  // X T (X symmetric)
+  cta_mm(n, n, n, Xm, V, A);  // X T (X symmetric)
   __syncthreads();
-  const bool ok = jacobi_block(n, A, V, cs, red, &flag, 60, 1e-14);
+  const bool ok = jacobi_block(n, A, V, cs, red, work + 2 * md.mat, 60, 1e-14);
   if (threadIdx.x == 0 && !ok) atomicOr(status + m, 2);
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const int r = jacobi_rank(n, A, i);
@@ -243,25 +219,16 @@ __global__ void __launch_bounds__(BT) batch_density_kernel(
     eps[md.vec + r] = A[i + (size_t)n * i];
   }
   __syncthreads();
-  // C_occ (n x nocc) into A
-  for (size_t idx = threadIdx.x; idx < (size_t)n * nocc; idx += blockDim.x) {
-    const int k = (int)(idx % n), r = (int)(idx / n);
-    const double *v = V + (size_t)n * perm[r];
-    double s = 0.0;
-    for (int l = 0; l < n; ++l) s += Xm[k + (size_t)n * l] * v[l];
-    A[idx] = s;
-  }
+  // C_occ (n x nocc) into A, D_new
+  cta_mm(n, nocc, n, Xm, V, A, 1.0, perm);
+  __syncthreads();
+  cta_mm<true>(n, n, nocc, A, A, Dn + md.mat, 2.0);
   __syncthreads();
   double dmax = 0.0, dss = 0.0;
   for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) {
-    const int k = (int)(idx % n), l = (int)(idx / n);
-    double s = 0.0;
-    for (int r = 0; r < nocc; ++r) s += A[k + (size_t)n * r] * A[l + (size_t)n * r];
-    s *= 2.0;
-    const double d = s - D[md.mat + idx];
+    const double d = Dn[md.mat + idx] - D[md.mat + idx];
     dmax = fmax(dmax, fabs(d));
     dss += d * d;
-    Dn[md.mat + idx] = s;
   }
   dmax = bmax(dmax, red);
   dss = bsum(dss, red);
@@ -509,7 +476,8 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
   float2 *d_DJ = (float2 *)buf(c, "batch_dsplit", mat * sizeof(float2));
   double *d_Kp = (double *)buf(c, "batch_kslices", tl.size() * (size_t)nmax * sizeof(double));
   double *d_Q = (double *)buf(c, "batch_Q", std::max<size_t>(q, 1) * sizeof(double));
-  if (!d_XX || !d_mats || !d_vecs || !d_B || !d_ints || !d_DJ || !d_Kp || !d_Q) return MQ_ENOMEM;
+  double *d_eig = (double *)buf(c, "batch_eig", mat * sizeof(double) * 2);  // the eigensolver's scratch
+  if (!d_eig || !d_XX || !d_mats || !d_vecs || !d_B || !d_ints || !d_DJ || !d_Kp || !d_Q) return MQ_ENOMEM;
   double *dS = d_mats, *dH = dS + mat, *dX = dH + mat, *dD = dX + mat, *dDn = dD + mat, *dF = dDn + mat,
          *dG = dF + mat, *dFx = dG + mat, *dJ = dFx + mat, *dK = dJ + mat, *dFh = dK + mat,
          *dEh = dFh + mat * (size_t)nd;
@@ -537,9 +505,9 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
   MQ_CUDA(c, cudaFuncSetAttribute(batch_orth_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   MQ_CUDA(c, cudaFuncSetAttribute(batch_density_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   MQ_CUDA(c, cudaFuncSetAttribute(batch_diis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_diis));
-  batch_orth_kernel<<<M, BT, smem, c->stream>>>(d_md, dS, dX, d_status);
+  batch_orth_kernel<<<M, BT, smem, c->stream>>>(d_md, dS, dX, d_eig, d_status);
   batch_density_kernel<<<M, BT, smem, c->stream>>>(1, d_md, d_active, dX, dH, dD, dDn, d_eps, d_it, d_conv, d_Ek,
-                                                   d_Ef, thr, o->conv_rms, max_iter, d_status);
+                                                   d_Ef, thr, o->conv_rms, max_iter, d_eig, d_status);
   c->stats.launches += 2;
   c->stats.guesses_taken = 0;
   if (o->D_in) {
@@ -585,7 +553,7 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
       Fuse = dFx;
     }
     batch_density_kernel<<<M, BT, smem, c->stream>>>(0, d_md, d_active, dX, Fuse, dD, dDn, d_eps, d_it, d_conv,
-                                                     d_Ek, d_Ef, thr, o->conv_rms, max_iter, d_status);
+                                                     d_Ek, d_Ef, thr, o->conv_rms, max_iter, d_eig, d_status);
     MQ_CUDA(c, cudaGetLastError());
     return MQ_OK;
   };

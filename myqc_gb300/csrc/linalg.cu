@@ -28,21 +28,13 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(int n, double *__re
   extern __shared__ double sm[];
   const int b = blockIdx.x;
   const size_t n2 = (size_t)n * n;
-  double *Ain = Ag + n2 * b;
-  double *A, *V;
-  if (SMEM) {
-    A = sm;
-    V = sm + n2;
-  } else {
-    A = work + 2 * n2 * b;
-    V = A + n2;
-  }
+  double *Ain = Ag + n2 * b, *A = sm, *V = sm + n2;
+  double *W = SMEM ? sm + 2 * n2 : work + 2 * n2 * b;  // 2 n^2 doubles of scratch
   __shared__ double cs[2 * 512];  // (c, s) per pair of a round, n <= 1024
   __shared__ double red[JAC_THREADS / 32];
-  __shared__ int flag;
   for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) A[idx] = Ain[idx];
   __syncthreads();
-  const bool ok = jacobi_block(n, A, V, cs, red, &flag, max_sweeps, tol);
+  const bool ok = jacobi_block(n, A, V, cs, red, W, max_sweeps, tol);
   if (threadIdx.x == 0 && !ok) atomicExch(status, 1);
   jacobi_sorted_out(n, A, V, wg + (size_t)n * b, Vg + n2 * b);
 }
@@ -279,19 +271,22 @@ int syev_batched_device(mq_ctx *c, int n, int batch, double *d_A, double *d_w, d
     for (int b = 0; b < batch; ++b) MQ_TRY(syev_large_cold(c, n, d_A + n2 * b, d_w + (size_t)n * b, d_V + n2 * b));
     return MQ_OK;
   }
-  const size_t smem = 2 * n2 * sizeof(double);
-  int *status = (int *)buf(c, "jacobi_work", 64 + (smem > 200 * 1024 ? 2 * n2 * sizeof(double) * batch : 0));
+  // A, V and the scratch in shared memory while 4 n^2 doubles fit (n <= 80);
+  // above, the scratch in global memory
+  const size_t mat2 = 2 * n2 * sizeof(double);
+  const bool smem_work = 2 * mat2 <= 205 * 1024;
+  const size_t smem = smem_work ? 2 * mat2 : mat2;
+  int *status = (int *)buf(c, "jacobi_work", 64 + (smem_work ? 0 : mat2 * batch));
   if (!status) return MQ_ENOMEM;
   MQ_CUDA(c, cudaMemsetAsync(status, 0, sizeof(int), c->stream));
   const int max_sweeps = 60;
   const double tol = 1e-14;  // ||offdiag||_F / ||A||_F at stop; eigenvalue error ~ tol^2 ||A|| / gap
-  if (smem <= 200 * 1024) {
-    MQ_CUDA(c, cudaFuncSetAttribute(jacobi_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    jacobi_kernel<true><<<batch, JAC_THREADS, smem, c->stream>>>(n, d_A, d_w, d_V, nullptr, max_sweeps, tol, status);
-  } else {
-    double *work = (double *)((char *)status + 64);
-    jacobi_kernel<false><<<batch, JAC_THREADS, 0, c->stream>>>(n, d_A, d_w, d_V, work, max_sweeps, tol, status);
-  }
+  auto kern = smem_work ? jacobi_kernel<true> : jacobi_kernel<false>;
+  MQ_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // small orders: fewer warps to wait for at a round's two barriers
+  const int threads = n <= 16 ? 128 : (n <= 32 ? 256 : JAC_THREADS);
+  kern<<<batch, threads, smem, c->stream>>>(n, d_A, d_w, d_V, (double *)((char *)status + 64), max_sweeps, tol,
+                                                status);
   c->stats.launches += 1;
   MQ_CUDA(c, cudaGetLastError());
   int h = 0;
