@@ -167,6 +167,8 @@ void pairs_host(const std::vector<HostShell> &shells, const std::vector<double> 
       h.aoA.push_back(A.ao0);
       h.aoB.push_back(B.ao0);
       h.mol.push_back(0);
+      for (int k = 0; k < 3; ++k) h.geom.push_back(xa[k]);
+      for (int k = 0; k < 3; ++k) h.geom.push_back(xb[k] - xa[k]);
       h.off.push_back((int)h.p.size());
       // the surviving primitive pairs, K descending (stable: ties keep the
       // (i, j) order): the pairs of a ket passing the screen against one bra
@@ -222,6 +224,7 @@ void append_pairs_class(HostPairs &dst, const HostPairs &src, int cl, int mol) {
     dst.aoA.push_back(src.aoA[P]);
     dst.aoB.push_back(src.aoB[P]);
     dst.mol.push_back(mol);
+    dst.geom.insert(dst.geom.end(), src.geom.begin() + 6 * (size_t)P, src.geom.begin() + 6 * (size_t)P + 6);
     for (int q = src.off[P]; q < src.off[P + 1]; ++q) {
       dst.p.push_back(src.p[q]);
       dst.inv2p.push_back(src.inv2p[q]);
@@ -236,12 +239,116 @@ void append_pairs_class(HostPairs &dst, const HostPairs &src, int cl, int mol) {
   }
 }
 
+// ---- The exponent sums p of a table take few distinct values (shells of one
+// element share their exponents), and alpha = pq/(p+q) and the prefactor
+// 2 pi^5/2 / (p q sqrt(p+q)) of a primitive quartet depend on its two sums
+// alone: the distinct sums are numbered with a hash table, and both quantities
+// are tabulated once for all pairs of them.
+constexpr int PQ_SLOTS = 4096, PQ_PROBES = 64;
+struct PqHash {
+  unsigned long long key[PQ_SLOTS];  // bit patterns of p (0: free; p > 0)
+  int id[PQ_SLOTS];
+  double p[PQ_MAX];
+  int overflow;
+};
+
+__global__ void pq_insert_kernel(int npp, const double *__restrict__ p, PqHash *__restrict__ h, int *__restrict__ slot) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= npp) return;
+  const unsigned long long k = (unsigned long long)__double_as_longlong(p[i]);
+  unsigned s = (unsigned)((k * 0x9E3779B97F4A7C15ull) >> 52);
+  int found = -1;
+  for (int t = 0; t < PQ_PROBES && found < 0; ++t, s = (s + 1) % PQ_SLOTS) {
+    unsigned long long o = *(volatile unsigned long long *)&h->key[s];
+    if (o == 0) o = atomicCAS(&h->key[s], 0ull, k);
+    if (o == 0 || o == k) found = (int)s;
+  }
+  if (found < 0) h->overflow = 1;
+  slot[i] = found;
+}
+
+// the slots in use numbered in slot order (one CTA); more than PQ_MAX, or a sum without a slot: none
+__global__ void __launch_bounds__(1024) pq_number_kernel(PqHash *__restrict__ h, int *__restrict__ pq_n) {
+  __shared__ int cnt[1024];
+  constexpr int PER = PQ_SLOTS / 1024;
+  int c = 0;
+  for (int k = 0; k < PER; ++k) c += h->key[threadIdx.x * PER + k] != 0;
+  cnt[threadIdx.x] = c;
+  __syncthreads();
+  for (int o = 1; o < 1024; o <<= 1) {
+    const int v = threadIdx.x >= o ? cnt[threadIdx.x - o] : 0;
+    __syncthreads();
+    cnt[threadIdx.x] += v;
+    __syncthreads();
+  }
+  int id = cnt[threadIdx.x] - c;
+  for (int k = 0; k < PER; ++k) {
+    const int s = threadIdx.x * PER + k;
+    if (h->key[s] == 0) continue;
+    h->id[s] = id;
+    if (id < PQ_MAX) h->p[id] = __longlong_as_double((long long)h->key[s]);
+    ++id;
+  }
+  if (threadIdx.x == 1023) *pq_n = h->overflow || cnt[1023] > PQ_MAX ? 0 : cnt[1023];
+}
+
+__global__ void pq_table_kernel(const PqHash *__restrict__ h, const int *__restrict__ pq_n, double pref0,
+                                double2 *__restrict__ pq) {
+  const int n = *pq_n;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n * n; i += gridDim.x * blockDim.x) {
+    const double p = h->p[i / n], q = h->p[i % n], s = p + q;
+    pq[i] = make_double2(p * q / s, pref0 / (p * q * sqrt(s)));
+  }
+}
+
+// the record of each primitive pair (layout in eri_low.cuh)
+__global__ void pp_record_kernel(PairTable t, const PqHash *__restrict__ h, const int *__restrict__ slot) {
+  const int P = blockIdx.x;
+  for (int i = t.pp_off[P] + threadIdx.x; i < t.pp_off[P + 1]; i += blockDim.x) {
+    const double *c = t.c4 + 4 * (size_t)i;
+    const double be = t.beta[i] / t.p[i], H = -1.0 / t.p[i];
+    double *r = t.rec + (size_t)PP_REC * i;
+    r[0] = t.Px[i];
+    r[1] = t.Py[i];
+    r[2] = t.Pz[i];
+    r[3] = be;
+    r[4] = t.K[i];
+    r[5] = 1.0e-14 / t.K[i];
+    r[6] = c[0];
+    r[7] = c[2] * be;
+    r[8] = c[2] * H;
+    r[9] = c[1] * (be - 1.0);
+    r[10] = c[1] * H;
+    r[11] = c[3] * be * (be - 1.0);
+    r[12] = c[3] * H;
+    r[13] = H;
+    t.pid[i] = *t.pq_n > 0 ? h->id[slot[i]] : 0;
+  }
+}
+
+static int pair_records(mq_ctx *c, PairTable &t, int mode) {
+  if (t.npp == 0) return MQ_OK;
+  char *w = (char *)buf(c, "pair_hash", sizeof(PqHash) + sizeof(int) * (size_t)t.npp);
+  if (!w) return MQ_ENOMEM;
+  PqHash *h = (PqHash *)w;
+  int *slot = (int *)(w + sizeof(PqHash));
+  const double pref0 = mode == MQ_MODE_REFERENCE ? 2.0 * 17.493419544621675 : 2.0 * 17.493418327624862;  // 2 pi^2.5
+  MQ_CUDA(c, cudaMemsetAsync(h, 0, sizeof(PqHash), c->stream));
+  pq_insert_kernel<<<(t.npp + 255) / 256, 256, 0, c->stream>>>(t.npp, t.p, h, slot);
+  pq_number_kernel<<<1, 1024, 0, c->stream>>>(h, t.pq_n);
+  pq_table_kernel<<<64, 256, 0, c->stream>>>(h, t.pq_n, pref0, t.pq);
+  pp_record_kernel<<<t.npairs, 32, 0, c->stream>>>(t, h, slot);
+  c->stats.launches += 4;
+  MQ_CUDA(c, cudaGetLastError());
+  return MQ_OK;
+}
+
 // All arrays of the table in one device block (256-byte aligned pieces),
 // staged through one pinned host buffer and one copy.  allocs != null: a new
 // block recorded there (batches); null: the context's reusable "pair_table"
 // buffer, after the work queued on the stream (which may read the previous
 // table) has finished.
-int upload_pairs(mq_ctx *c, const HostPairs &h, std::vector<void *> *allocs, PairTable &t) {
+int upload_pairs(mq_ctx *c, const HostPairs &h, std::vector<void *> *allocs, PairTable &t, int mode) {
   t = PairTable{};
   for (int k = 0; k < 4; ++k) t.class_off[k] = h.class_off[k];
   t.npairs = (int)h.shA.size();
@@ -284,6 +391,16 @@ int upload_pairs(mq_ctx *c, const HostPairs &h, std::vector<void *> *allocs, Pai
   add(t.K, h.K);
   add(t.c4, h.c4);
   add(t.pf, pf);
+  add(t.geom, h.geom);
+  const size_t copied = total;  // behind it: what the device forms itself
+  auto room = [&](auto *&dst, size_t bytes) {
+    items.push_back({(void **)&dst, nullptr, 0, total});
+    total += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+  };
+  room(t.rec, sizeof(double) * PP_REC * h.p.size());
+  room(t.pid, sizeof(int) * h.p.size());
+  room(t.pq, sizeof(double2) * PQ_MAX * PQ_MAX);
+  room(t.pq_n, sizeof(int));
   char *dev = nullptr;
   MQ_CUDA(c, cudaStreamSynchronize(c->stream));
   if (allocs) {
@@ -293,28 +410,28 @@ int upload_pairs(mq_ctx *c, const HostPairs &h, std::vector<void *> *allocs, Pai
     dev = (char *)buf(c, "pair_table", total);
     if (!dev) return MQ_ENOMEM;
   }
-  if (c->pin_bytes < total) {
+  if (c->pin_bytes < copied) {
     if (c->pin) cudaFreeHost(c->pin);
     c->pin = nullptr;
     c->pin_bytes = 0;
-    MQ_CUDA(c, cudaHostAlloc(&c->pin, total, cudaHostAllocDefault));
-    c->pin_bytes = total;
+    MQ_CUDA(c, cudaHostAlloc(&c->pin, copied, cudaHostAllocDefault));
+    c->pin_bytes = copied;
   }
   char *st = (char *)c->pin;
   for (const Item &it : items) {
     if (it.bytes) memcpy(st + it.off, it.src, it.bytes);
     *it.dst = dev + it.off;
   }
-  MQ_CUDA(c, cudaMemcpyAsync(dev, st, total, cudaMemcpyHostToDevice, c->stream));
+  MQ_CUDA(c, cudaMemcpyAsync(dev, st, copied, cudaMemcpyHostToDevice, c->stream));
   MQ_CUDA(c, cudaStreamSynchronize(c->stream));  // the staging buffer is reused by the next upload
-  return MQ_OK;
+  return pair_records(c, t, mode);
 }
 
 int build_pairs(mq_ctx *c) {
   free_pairs(c);
   HostPairs h;
   pairs_host(c->shells, c->xyz, h);
-  MQ_TRY(upload_pairs(c, h, nullptr, c->pt));
+  MQ_TRY(upload_pairs(c, h, nullptr, c->pt, c->mode));
   c->pair_class_count = {h.class_off[1] - h.class_off[0], h.class_off[2] - h.class_off[1],
                          h.class_off[3] - h.class_off[2]};
   c->hp_shA = h.shA;
@@ -333,6 +450,7 @@ int build_pairs(mq_ctx *c) {
 // The table is a constant: computed once per process (the long-double series
 // is slow where long double is a software type, as on aarch64).
 static void tight_boys_compute(std::vector<double> &tab);
+static void fine_boys_compute(std::vector<double> &tab);
 void tight_boys_table(std::vector<double> &tab) {
   static std::once_flag once;
   static std::vector<double> cached;
@@ -356,23 +474,60 @@ void tight_boys_device_table(std::vector<double> &tab) {
         tab.push_back(f[(size_t)t * TIGHT_NM + m + k] / fact);
       }
     }
+  static std::once_flag once;
+  static std::vector<double> fine;
+  std::call_once(once, [] { fine_boys_compute(fine); });
+  while (tab.size() < BOYS_FINE_OFF) tab.push_back(0.0);
+  tab.insert(tab.end(), fine.begin(), fine.end());
+}
+
+// Values F_0 .. F_{nm-1} at T, the series at the top order and downward recursion.
+static void boys_series(long double T, int nm, long double *F) {
+  const int m = nm - 1;
+  long double term = 1.0L / (2 * m + 1), sum = term;
+  for (int k = 1; k < 2000; ++k) {
+    term *= 2.0L * T / (2 * m + 2 * k + 1);
+    sum += term;
+    if (term < 1e-22L * sum) break;
+  }
+  const long double e = expl(-T);
+  F[m] = e * sum;
+  for (int j = m - 1; j >= 0; --j) F[j] = (2.0L * T * F[j + 1] + e) / (2.0L * j + 1.0L);
+}
+
+// [m < 3][577 rows, T step 1/16][8]: F_m(T) as a polynomial of degree 6 in
+// d = Tk - T, |d| <= 1/32, and Tk.  The Taylor polynomial of degree 8 with its
+// two highest terms economised over the interval: x^8 and x^7 (x = 32 d)
+// replaced through the Chebyshev polynomials T8 = 128 x^8 - 256 x^6 + 160 x^4
+// - 32 x^2 + 1 and T7 = 64 x^7 - 112 x^5 + 56 x^3 - 7 x, which leaves at most
+// F_{m+7} / (7! 64 32^7) = 9e-17 F_{m+7}.
+static void fine_boys_compute(std::vector<double> &tab) {
+  constexpr int NM = BOYS_FINE_M + 8;
+  tab.assign((size_t)BOYS_FINE_M * BOYS_FINE_NT * 8, 0.0);
+  for (int t = 0; t < BOYS_FINE_NT; ++t) {
+    long double F[NM];
+    boys_series(t / 16.0L, NM, F);
+    for (int m = 0; m < BOYS_FINE_M; ++m) {
+      long double a[9], fact = 1.0L, h = 1.0L;  // coefficients of x^k
+      for (int k = 0; k < 9; ++k) {
+        if (k) fact *= k, h /= 32.0L;
+        a[k] = F[m + k] / fact * h;
+      }
+      a[6] += 2.0L * a[8], a[4] -= 1.25L * a[8], a[2] += 0.25L * a[8], a[0] -= a[8] / 128.0L;
+      a[5] += 1.75L * a[7], a[3] -= 0.875L * a[7], a[1] += 7.0L / 64.0L * a[7];
+      double *row = tab.data() + ((size_t)m * BOYS_FINE_NT + t) * 8;
+      long double s = 1.0L;
+      for (int k = 0; k < 7; ++k, s *= 32.0L) row[k] = (double)(a[k] * s);
+      row[7] = t / 16.0;
+    }
+  }
 }
 
 static void tight_boys_compute(std::vector<double> &tab) {
   tab.assign((size_t)TIGHT_NT * TIGHT_NM, 0.0);
   for (int it = 0; it < TIGHT_NT; ++it) {
-    long double T = it / 10.0L;
-    const int m = TIGHT_NM - 1;
-    long double term = 1.0L / (2 * m + 1), sum = term;
-    for (int k = 1; k < 2000; ++k) {
-      term *= 2.0L * T / (2 * m + 2 * k + 1);
-      sum += term;
-      if (term < 1e-22L * sum) break;
-    }
-    long double e = expl(-T);
     long double F[TIGHT_NM];
-    F[m] = e * sum;
-    for (int j = m - 1; j >= 0; --j) F[j] = (2.0L * T * F[j + 1] + e) / (2.0L * j + 1.0L);
+    boys_series(it / 10.0L, TIGHT_NM, F);
     for (int j = 0; j < TIGHT_NM; ++j) tab[(size_t)it * TIGHT_NM + j] = (double)F[j];
   }
 }

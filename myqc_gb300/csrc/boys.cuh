@@ -22,7 +22,8 @@
 // Table layout in device memory (one buffer, see set_system):
 //   parity: Ft(0:120,0:22) column-major (2783 doubles), then Tk/10 (121)
 //   tight : tab[Tk][m], 361 x 13 row-major (4693 doubles), then Tk/10 (361),
-//           then F_{m+k}(Tk)/k! [m < 5][Tk][k < 9]
+//           then F_{m+k}(Tk)/k! [m < 5][Tk][k < 9], then the degree-6 rows of
+//           boys_fine [m < 3][577][8]
 #pragma once
 #include "internal.h"
 
@@ -111,6 +112,39 @@ __device__ __forceinline__ void boys_tight(double T, const double *__restrict__ 
     F[0] = 0.8862269254527579 * rT;  // sqrt(pi)/2
 #pragma unroll
     for (int j = 1; j <= L; ++j) F[j] = i2T * (2 * j - 1) * F[j - 1];
+  }
+}
+
+// F_0 .. F_L, L <= 2, for the low-order integral kernels: below 36 each order
+// by its own polynomial of degree 6 about the nearest multiple of 1/16 (one row
+// of 64 bytes per order, whose last entry is that multiple).  The row number
+// comes from the low word of T + 1.5 2^48 (whose unit in the last place is
+// 1/16) and the range test from T's high word, so that neither takes an FP64
+// conversion or comparison.
+template <int L>
+__device__ __forceinline__ void boys_fine(double T, const double *__restrict__ tab, double (&F)[L + 1]) {
+  static_assert(L < BOYS_FINE_M, "Boys order");
+  if (__double2hiint(T) < 0x40420000) {  // T < 36
+    const int t = __double2loint(T + 0x1.8p48);
+    const double2 *row = reinterpret_cast<const double2 *>(tab + BOYS_FINE_OFF) + 4 * t;
+    double d = 0.0;
+#pragma unroll
+    for (int m = 0; m <= L; ++m) {
+      const double2 *r = row + 4 * BOYS_FINE_NT * m;
+      const double2 c6 = __ldg(r + 3), c4 = __ldg(r + 2), c2 = __ldg(r + 1), c0 = __ldg(r);
+      if (m == 0) d = c6.y - T;
+      double f = fma(c6.x, d, c4.y);
+      f = fma(f, d, c4.x);
+      f = fma(f, d, c2.y);
+      f = fma(f, d, c2.x);
+      f = fma(f, d, c0.y);
+      F[m] = fma(f, d, c0.x);
+    }
+  } else {
+    const double rT = rsqrt(T), i2T = 0.5 * rT * rT;
+    F[0] = 0.8862269254527579 * rT;  // sqrt(pi)/2
+#pragma unroll
+    for (int j = 1; j <= L; ++j) F[j] = (j == 1 ? i2T : i2T * (2 * j - 1)) * F[j - 1];
   }
 }
 

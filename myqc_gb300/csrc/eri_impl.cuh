@@ -249,6 +249,101 @@ __device__ __forceinline__ void boys_any(const EriArgs &g, float T, float (&F)[L
   boys_f32<L>(T, g.boys_f, F);
 }
 
+// What becomes of a quartet's integrals (this thread's share of them).
+template <int LA, int LB, int LC, int LD, int A0, int A1, int B0, int B1, int C0, int C1, int D0, int D1, int EPI,
+          class RT>
+__device__ __forceinline__ void eri_epilogue(const EriArgs &g, int P, int Q, size_t n, double *XXout,
+                                             const RT (&acc)[A1 - A0][B1 - B0][C1 - C0][D1 - D0], unsigned nprim) {
+  const PairTable &t = g.t;
+  const int A = t.shA[P], B = t.shB[P], C = t.shA[Q], D = t.shB[Q];
+  const int i0 = t.aoA[P], j0 = t.aoB[P], k0 = t.aoA[Q], l0 = t.aoB[Q];
+  if (EPI == EPI_SCHWARZ) {
+    double m = 0.0;
+#pragma unroll
+    for (int a = A0; a < A1; ++a)
+#pragma unroll
+      for (int b = B0; b < B1; ++b)
+        if (a >= C0 && a < C1 && b >= D0 && b < D1) m = fmax(m, fabs((double)acc[a - A0][b - B0][a - C0][b - D0]));
+    atomicMax(g.sch + P, (unsigned long long)__double_as_longlong(sqrt(m)));
+    return;
+  }
+  if (g.counters && A0 == 0 && B0 == 0 && C0 == 0 && D0 == 0) {  // one atomic pair per warp, not per quartet
+    const unsigned act = __activemask();
+    const unsigned nq_w = __popc(act), np_w = __reduce_add_sync(act, nprim);
+    if ((threadIdx.x & 31) == __ffs(act) - 1) {
+      atomicAdd(g.counters, (unsigned long long)nq_w);
+      atomicAdd(g.counters + 1, (unsigned long long)np_w);
+    }
+  }
+  if constexpr (EPI == EPI_STORE) {  // the whole block (this thread's share), layout ((a NB + b) NC + c) ND + d
+    constexpr int NB_ = nfun(LB), NC_ = nfun(LC), ND_ = nfun(LD);
+#pragma unroll
+    for (int a = A0; a < A1; ++a)
+#pragma unroll
+      for (int b = B0; b < B1; ++b)
+#pragma unroll
+        for (int c = C0; c < C1; ++c)
+#pragma unroll
+          for (int d = D0; d < D1; ++d)
+            XXout[((a * NB_ + b) * NC_ + c) * ND_ + d] = (double)acc[a - A0][b - B0][c - C0][d - D0];
+    return;
+  }
+#pragma unroll
+  for (int a = A0; a < A1; ++a)
+#pragma unroll
+    for (int b = B0; b < B1; ++b)
+#pragma unroll
+      for (int c = C0; c < C1; ++c)
+#pragma unroll
+        for (int d = D0; d < D1; ++d) {
+          const int i = i0 + a, j = j0 + b, k = k0 + c, l = l0 + d;
+          if (A == B && i < j) continue;
+          if (C == D && k < l) continue;
+          if (P == Q && (size_t)i * n + j < (size_t)k * n + l) continue;
+          const double x = (double)acc[a - A0][b - B0][c - C0][d - D0];
+          if (EPI == EPI_XX) {
+            double *XX = XXout;
+            const size_t ij = (size_t)i + n * j, ji = (size_t)j + n * i, kl = (size_t)k + n * l,
+                         lk = (size_t)l + n * k, n2 = n * n;
+            XX[ij + n2 * kl] = x;
+            XX[ji + n2 * kl] = x;
+            XX[ij + n2 * lk] = x;
+            XX[ji + n2 * lk] = x;
+            XX[kl + n2 * ij] = x;
+            XX[lk + n2 * ij] = x;
+            XX[kl + n2 * ji] = x;
+            XX[lk + n2 * ji] = x;
+          } else {  // EPI_FOCK: half-sums, symmetrised afterwards
+            double deg = 1.0;
+            if (i == j) deg *= 0.5;
+            if (k == l) deg *= 0.5;
+            if (i == k && j == l) deg *= 0.5;
+            const double x2 = 2.0 * deg * x, x4 = 2.0 * x2;
+            const double *Da = g.Da;
+            if (!g.uhf) {
+              atomicAdd(g.J + i + n * j, x4 * Da[k + n * l]);
+              atomicAdd(g.J + k + n * l, x4 * Da[i + n * j]);
+              atomicAdd(g.Ka + i + n * k, x2 * Da[j + n * l]);
+              atomicAdd(g.Ka + j + n * k, x2 * Da[i + n * l]);
+              atomicAdd(g.Ka + i + n * l, x2 * Da[j + n * k]);
+              atomicAdd(g.Ka + j + n * l, x2 * Da[i + n * k]);
+            } else {
+              const double *Db = g.Db;
+              atomicAdd(g.J + i + n * j, x4 * (Da[k + n * l] + Db[k + n * l]));
+              atomicAdd(g.J + k + n * l, x4 * (Da[i + n * j] + Db[i + n * j]));
+              atomicAdd(g.Ka + i + n * k, x2 * Da[j + n * l]);
+              atomicAdd(g.Ka + j + n * k, x2 * Da[i + n * l]);
+              atomicAdd(g.Ka + i + n * l, x2 * Da[j + n * k]);
+              atomicAdd(g.Ka + j + n * l, x2 * Da[i + n * k]);
+              atomicAdd(g.Kb + i + n * k, x2 * Db[j + n * l]);
+              atomicAdd(g.Kb + j + n * k, x2 * Db[i + n * l]);
+              atomicAdd(g.Kb + i + n * l, x2 * Db[j + n * k]);
+              atomicAdd(g.Kb + j + n * l, x2 * Db[i + n * k]);
+            }
+          }
+        }
+}
+
 // One contracted quartet (P, Q), the bra functions a in [A0, A1), b in [B0, B1)
 // and ket functions c in [C0, C1), d in [D0, D1) of it (a thread's share when a
 // quartet is split over threads).  With the whole bra in one thread (ONFLY)
@@ -406,94 +501,7 @@ __device__ __forceinline__ void quartet(const EriArgs &g, int P, int Q, size_t n
         }
     }
   }
-  // ---------------- epilogues ----------------
-  const int A = t.shA[P], B = t.shB[P], C = t.shA[Q], D = t.shB[Q];
-  const int i0 = t.aoA[P], j0 = t.aoB[P], k0 = t.aoA[Q], l0 = t.aoB[Q];
-  if (EPI == EPI_SCHWARZ) {
-    double m = 0.0;
-#pragma unroll
-    for (int a = A0; a < A1; ++a)
-#pragma unroll
-      for (int b = B0; b < B1; ++b)
-        if (a >= C0 && a < C1 && b >= D0 && b < D1) m = fmax(m, fabs((double)acc[a - A0][b - B0][a - C0][b - D0]));
-    atomicMax(g.sch + P, (unsigned long long)__double_as_longlong(sqrt(m)));
-    return;
-  }
-  if (g.counters && A0 == 0 && B0 == 0 && C0 == 0 && D0 == 0) {  // one atomic pair per warp, not per quartet
-    const unsigned act = __activemask();
-    const unsigned nq_w = __popc(act), np_w = __reduce_add_sync(act, nprim);
-    if ((threadIdx.x & 31) == __ffs(act) - 1) {
-      atomicAdd(g.counters, (unsigned long long)nq_w);
-      atomicAdd(g.counters + 1, (unsigned long long)np_w);
-    }
-  }
-  if constexpr (EPI == EPI_STORE) {  // the whole block (this thread's share), layout ((a NB + b) NC + c) ND + d
-    constexpr int NB_ = nfun(LB), NC_ = nfun(LC), ND_ = nfun(LD);
-#pragma unroll
-    for (int a = A0; a < A1; ++a)
-#pragma unroll
-      for (int b = B0; b < B1; ++b)
-#pragma unroll
-        for (int c = C0; c < C1; ++c)
-#pragma unroll
-          for (int d = D0; d < D1; ++d)
-            XXout[((a * NB_ + b) * NC_ + c) * ND_ + d] = (double)acc[a - A0][b - B0][c - C0][d - D0];
-    return;
-  }
-#pragma unroll
-  for (int a = A0; a < A1; ++a)
-#pragma unroll
-    for (int b = B0; b < B1; ++b)
-#pragma unroll
-      for (int c = C0; c < C1; ++c)
-#pragma unroll
-        for (int d = D0; d < D1; ++d) {
-          const int i = i0 + a, j = j0 + b, k = k0 + c, l = l0 + d;
-          if (A == B && i < j) continue;
-          if (C == D && k < l) continue;
-          if (P == Q && (size_t)i * n + j < (size_t)k * n + l) continue;
-          const double x = (double)acc[a - A0][b - B0][c - C0][d - D0];
-          if (EPI == EPI_XX) {
-            double *XX = XXout;
-            const size_t ij = (size_t)i + n * j, ji = (size_t)j + n * i, kl = (size_t)k + n * l,
-                         lk = (size_t)l + n * k, n2 = n * n;
-            XX[ij + n2 * kl] = x;
-            XX[ji + n2 * kl] = x;
-            XX[ij + n2 * lk] = x;
-            XX[ji + n2 * lk] = x;
-            XX[kl + n2 * ij] = x;
-            XX[lk + n2 * ij] = x;
-            XX[kl + n2 * ji] = x;
-            XX[lk + n2 * ji] = x;
-          } else {  // EPI_FOCK: half-sums, symmetrised afterwards
-            double deg = 1.0;
-            if (i == j) deg *= 0.5;
-            if (k == l) deg *= 0.5;
-            if (i == k && j == l) deg *= 0.5;
-            const double x2 = 2.0 * deg * x, x4 = 2.0 * x2;
-            const double *Da = g.Da;
-            if (!g.uhf) {
-              atomicAdd(g.J + i + n * j, x4 * Da[k + n * l]);
-              atomicAdd(g.J + k + n * l, x4 * Da[i + n * j]);
-              atomicAdd(g.Ka + i + n * k, x2 * Da[j + n * l]);
-              atomicAdd(g.Ka + j + n * k, x2 * Da[i + n * l]);
-              atomicAdd(g.Ka + i + n * l, x2 * Da[j + n * k]);
-              atomicAdd(g.Ka + j + n * l, x2 * Da[i + n * k]);
-            } else {
-              const double *Db = g.Db;
-              atomicAdd(g.J + i + n * j, x4 * (Da[k + n * l] + Db[k + n * l]));
-              atomicAdd(g.J + k + n * l, x4 * (Da[i + n * j] + Db[i + n * j]));
-              atomicAdd(g.Ka + i + n * k, x2 * Da[j + n * l]);
-              atomicAdd(g.Ka + j + n * k, x2 * Da[i + n * l]);
-              atomicAdd(g.Ka + i + n * l, x2 * Da[j + n * k]);
-              atomicAdd(g.Ka + j + n * l, x2 * Da[i + n * k]);
-              atomicAdd(g.Kb + i + n * k, x2 * Db[j + n * l]);
-              atomicAdd(g.Kb + j + n * k, x2 * Db[i + n * l]);
-              atomicAdd(g.Kb + i + n * l, x2 * Db[j + n * k]);
-              atomicAdd(g.Kb + j + n * l, x2 * Db[i + n * k]);
-            }
-          }
-        }
+  eri_epilogue<LA, LB, LC, LD, A0, A1, B0, B1, C0, C1, D0, D1, EPI>(g, P, Q, n, XXout, acc, nprim);
 }
 
 // decode (P, Q) of the launch's q-th quartet, and the molecule m (0 for one
@@ -579,7 +587,7 @@ __device__ __forceinline__ bool next_survivor(const PairTable &t, int p1, int q0
   return false;
 }
 
-// Quartet-store pass of the split classes ((sp sp|sp s): 4 warps, one ket
+// FP64 pass of the split classes ((sp sp|sp s): 4 warps, one ket
 // function c each; (sp sp|sp sp): 16 warps, one ket pair (c, d) each), with
 // the per-primitive-quartet work shared.  The CTA's warps serve the same 32
 // quartets (lane = quartet), so every one of them needs the same Boys values
@@ -593,9 +601,9 @@ __device__ __forceinline__ bool next_survivor(const PairTable &t, int p1, int q0
 // outputs.  The round count is the warp's largest S (every warp of the CTA
 // computes the same S per lane), so the barriers are reached by every thread,
 // and a round has idle producers only at the end of a lane's list.
-template <int LA, int LB, int LC, int LD, int NSPLIT, int C0, int C1, int D0, int D1>
-__device__ __forceinline__ void quartet_store_shared(const EriArgs &g, bool valid, int P, int Q, double *XXout,
-                                                     double *smR, int2 *smI) {
+template <int LA, int LB, int LC, int LD, int NSPLIT, int C0, int C1, int D0, int D1, int EPI>
+__device__ __forceinline__ void quartet_shared(const EriArgs &g, bool valid, int P, int Q, size_t n, double *XXout,
+                                               double *smR, int2 *smI) {
   constexpr int LAB = LA + LB, LT = LA + LB + LC + LD, NR = nherm(LT);
   constexpr int QREF = 3 * LT;
   constexpr int NA = nfun(LA), NB = nfun(LB), NC = nfun(LC), ND = nfun(LD);
@@ -742,19 +750,14 @@ __device__ __forceinline__ void quartet_store_shared(const EriArgs &g, bool vali
     }
   }
   if (!valid) return;
-#pragma unroll
-  for (int a = 0; a < NA; ++a)
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-      for (int c = C0; c < C1; ++c)
-#pragma unroll
-        for (int d = D0; d < D1; ++d) XXout[((a * NB + b) * NC + c) * ND + d] = acc[a][b][c - C0][d - D0];
+  EriArgs h = g;
+  h.counters = nullptr;  // counted above
+  eri_epilogue<LA, LB, LC, LD, 0, NA, 0, NB, C0, C1, D0, D1, EPI>(h, P, Q, n, XXout, acc, 0u);
 }
 
-// Store pass of a split class: one CTA of NSPLIT warps per 32 quartets.
-template <int LA, int LB, int LC, int LD>
-__global__ void __launch_bounds__(512) eri_store_shared_kernel(EriArgs g) {
+// A split class: one CTA of NSPLIT warps per 32 quartets.
+template <int LA, int LB, int LC, int LD, int EPI>
+__global__ void __launch_bounds__(512) eri_shared_kernel(EriArgs g) {
   constexpr int NOUT = nfun(LA) * nfun(LB) * nfun(LC) * nfun(LD);
   constexpr int NSPLIT = NOUT <= 64 ? 4 : 16;
   constexpr int NR = nherm(LA + LB + LC + LD);
@@ -765,28 +768,42 @@ __global__ void __launch_bounds__(512) eri_store_shared_kernel(EriArgs g) {
   long long q = (long long)blockIdx.x * 32 + lane;
   int P = 0, Q = 0, m = 0;
   const bool valid = decode(g, q, P, Q, m);
-  double *out = valid ? g.store + q * NOUT : nullptr;
+  size_t n = (size_t)g.n;
+  double *out = nullptr;
+  if constexpr (EPI == EPI_STORE) {
+    if (valid) out = g.store + q * NOUT;
+  } else {
+    out = g.XX;
+    if (valid && g.nmol) {
+      n = (size_t)g.mols[m].n;
+      out += g.mols[m].xx;
+    }
+  }
   if constexpr (NSPLIT == 4) {
     switch (w) {
-      case 0: quartet_store_shared<LA, LB, LC, LD, 4, 0, 1, 0, 1>(g, valid, P, Q, out, smR, smI); break;
-      case 1: quartet_store_shared<LA, LB, LC, LD, 4, 1, 2, 0, 1>(g, valid, P, Q, out, smR, smI); break;
-      case 2: quartet_store_shared<LA, LB, LC, LD, 4, 2, 3, 0, 1>(g, valid, P, Q, out, smR, smI); break;
-      default: quartet_store_shared<LA, LB, LC, LD, 4, 3, 4, 0, 1>(g, valid, P, Q, out, smR, smI); break;
+      case 0: quartet_shared<LA, LB, LC, LD, 4, 0, 1, 0, 1, EPI>(g, valid, P, Q, n, out, smR, smI); break;
+      case 1: quartet_shared<LA, LB, LC, LD, 4, 1, 2, 0, 1, EPI>(g, valid, P, Q, n, out, smR, smI); break;
+      case 2: quartet_shared<LA, LB, LC, LD, 4, 2, 3, 0, 1, EPI>(g, valid, P, Q, n, out, smR, smI); break;
+      default: quartet_shared<LA, LB, LC, LD, 4, 3, 4, 0, 1, EPI>(g, valid, P, Q, n, out, smR, smI); break;
     }
   } else {
-#define MQ_SH16(s)                                                                                             \
-  case s:                                                                                                      \
-    quartet_store_shared<LA, LB, LC, LD, 16, (s) / 4, (s) / 4 + 1, (s) % 4, (s) % 4 + 1>(g, valid, P, Q, out, smR, \
-                                                                                       smI);                   \
+#define MQ_SH16(s)                                                                                            \
+  case s:                                                                                                     \
+    quartet_shared<LA, LB, LC, LD, 16, (s) / 4, (s) / 4 + 1, (s) % 4, (s) % 4 + 1, EPI>(g, valid, P, Q, n, out, smR, \
+                                                                                        smI);                 \
     break;
     switch (w) {
       MQ_SH16(0) MQ_SH16(1) MQ_SH16(2) MQ_SH16(3) MQ_SH16(4) MQ_SH16(5) MQ_SH16(6) MQ_SH16(7) MQ_SH16(8)
       MQ_SH16(9) MQ_SH16(10) MQ_SH16(11) MQ_SH16(12) MQ_SH16(13) MQ_SH16(14)
-      default: quartet_store_shared<LA, LB, LC, LD, 16, 3, 4, 3, 4>(g, valid, P, Q, out, smR, smI); break;
+      default: quartet_shared<LA, LB, LC, LD, 16, 3, 4, 3, 4, EPI>(g, valid, P, Q, n, out, smR, smI); break;
     }
 #undef MQ_SH16
   }
 }
+
+}  // namespace mq
+#include "eri_low.cuh"
+namespace mq {
 
 // Schwarz bounds need only the diagonal integrals (ab|ab) of a shell pair: one
 // thread per pair and diagonal function pair S = (a, b), a single integral each
@@ -856,7 +873,9 @@ __device__ __forceinline__ void eri_unit(const EriArgs &g, long long warp, int l
   }
   if constexpr (EPI == EPI_STORE) XX = g.store + q * NOUT;
   constexpr int NC = nfun(LC), ND = nfun(LD);
-  if (NSPLIT == 1) {
+  if constexpr (NSPLIT == 1 && std::is_same<RT, double>::value && (EPI == EPI_XX || EPI == EPI_STORE)) {
+    quartet_low<LA, LB, LC, LD, EPI>(g, P, Q, n, XX);
+  } else if (NSPLIT == 1) {
     quartet<LA, LB, LC, LD, 0, NA, 0, NB, 0, NC, 0, ND, EPI, RT>(g, P, Q, n, XX);
   } else if (NSPLIT == 4) {  // (sp sp|sp s): one ket function c per thread, the whole bra
     switch (split) {
@@ -914,20 +933,21 @@ static int launch_class(mq_ctx *c, EriArgs g, int cP, int cQ, int block = 128, b
   }
   if (grid > 2147483647LL) return set_err(c, MQ_EINVAL, "integral launch too large");
   dim3 gd((unsigned)grid);
-  if constexpr (EPI == EPI_STORE && std::is_same<RT, double>::value) {
+  constexpr bool shared = (EPI == EPI_STORE || EPI == EPI_XX) && std::is_same<RT, double>::value;
+  if constexpr (shared) {
     if (nsplit > 1) {  // the split classes: per-primitive work shared by the CTA's warps
       const long long ctas = (g.nq + 31) / 32;
       if (ctas > 2147483647LL) return set_err(c, MQ_EINVAL, "integral launch too large");
       if (cP == 2 && cQ == 1) {
         const size_t sm = sizeof(double) * 4 * 32 * nherm(3) + sizeof(int2) * 4 * 32;
-        MQ_CUDA(c, cudaFuncSetAttribute(eri_store_shared_kernel<1, 1, 1, 0>,
+        MQ_CUDA(c, cudaFuncSetAttribute(eri_shared_kernel<1, 1, 1, 0, EPI>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        eri_store_shared_kernel<1, 1, 1, 0><<<(unsigned)ctas, 128, sm, c->stream>>>(g);
+        eri_shared_kernel<1, 1, 1, 0, EPI><<<(unsigned)ctas, 128, sm, c->stream>>>(g);
       } else {
         const size_t sm = sizeof(double) * 16 * 32 * nherm(4) + sizeof(int2) * 16 * 32;
-        MQ_CUDA(c, cudaFuncSetAttribute(eri_store_shared_kernel<1, 1, 1, 1>,
+        MQ_CUDA(c, cudaFuncSetAttribute(eri_shared_kernel<1, 1, 1, 1, EPI>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        eri_store_shared_kernel<1, 1, 1, 1><<<(unsigned)ctas, 512, sm, c->stream>>>(g);
+        eri_shared_kernel<1, 1, 1, 1, EPI><<<(unsigned)ctas, 512, sm, c->stream>>>(g);
       }
       c->stats.launches += 1;
       MQ_CUDA(c, cudaGetLastError());
@@ -939,8 +959,10 @@ static int launch_class(mq_ctx *c, EriArgs g, int cP, int cQ, int block = 128, b
   else if (cP == 1 && cQ == 0) MQ_LAUNCH(1, 0, 0, 0);
   else if (cP == 1 && cQ == 1) MQ_LAUNCH(1, 0, 1, 0);
   else if (cP == 2 && cQ == 0) MQ_LAUNCH(1, 1, 0, 0);
-  else if (cP == 2 && cQ == 1) MQ_LAUNCH(1, 1, 1, 0);
-  else MQ_LAUNCH(1, 1, 1, 1);
+  if constexpr (!shared) {
+    if (cP == 2 && cQ == 1) MQ_LAUNCH(1, 1, 1, 0);
+    else if (cP == 2 && cQ == 2) MQ_LAUNCH(1, 1, 1, 1);
+  }
 #undef MQ_LAUNCH
   c->stats.launches += 1;
   MQ_CUDA(c, cudaGetLastError());

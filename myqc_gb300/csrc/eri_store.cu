@@ -145,9 +145,9 @@ static int run_candidate(mq_ctx *c, const EriArgs &h0, int cP, int cQ, int slot,
 // ran last.
 template <int EPI>
 static int tuned_launch(mq_ctx *c, const EriArgs &h, int cP, int cQ, int combo, int slot) {
-  // the split classes of the quartet store run their CTA-shared kernel: its
-  // shape is fixed by the warp count, only the order is a choice
-  const bool fixed_shape = EPI == EPI_STORE && nsplit_of(cP, cQ) > 1;
+  // the split classes run their CTA-shared kernel: its shape is fixed by the
+  // warp count, only the order is a choice
+  const bool fixed_shape = nsplit_of(cP, cQ) > 1;
   EriTune def;
   if (c->eri_tune_mode == 0 || h.nq < TUNE_MIN_QUARTETS) return run_candidate<EPI>(c, h, cP, cQ, slot, def);
   const unsigned long long key = tune_key(EPI, combo, h.nq);
@@ -157,7 +157,7 @@ static int tuned_launch(mq_ctx *c, const EriArgs &h, int cP, int cQ, int combo, 
   for (int binned = 1; binned >= 0; --binned)
     for (int persistent = 0; persistent <= (fixed_shape ? 0 : 1); ++persistent)
       for (int block : {64, 128, 256}) {
-        if ((fixed_shape || nsplit_of(cP, cQ) > 1) && block != 128) continue;
+        if (fixed_shape && block != 128) continue;
         EriTune t;
         t.binned = binned;
         t.block = block;

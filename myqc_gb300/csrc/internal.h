@@ -47,7 +47,19 @@ struct PairTable {
   // single-precision copy, 4 float4 per primitive pair:
   // p 1/2p K Px | Py Pz PAx PAy | PAz PBx PBy PBz | c4
   float4 *pf;
+  // what the low-order integral kernels read (eri_low.cuh), formed on the
+  // device at upload: per pair its first centre and AB = B - A; per primitive
+  // pair PP_REC doubles and the number of its exponent sum among the distinct
+  // ones; for two such numbers alpha = pq/(p+q) and the integral prefactor
+  // (*pq_n = 0: more than PQ_MAX distinct sums, no table)
+  double *geom;  // 6 per pair
+  double *rec;
+  int *pid;
+  double2 *pq;
+  int *pq_n;
 };
+constexpr int PP_REC = 14;
+constexpr int PQ_MAX = 512;
 
 // Host copy of a pair table (same fields as PairTable), built per molecule
 // and concatenated for batches.
@@ -55,6 +67,7 @@ struct HostPairs {
   int class_off[4] = {0, 0, 0, 0};
   std::vector<int> shA, shB, off, aoA, aoB, mol;
   std::vector<double> p, inv2p, beta, Px, Py, Pz, PAx, PAy, PAz, PBx, PBy, PBz, K, c4;
+  std::vector<double> geom;  // 6 per pair: A, B - A
 };
 
 // One molecule added to a batch: host pair table, nuclei (x, y, z, Z) and
@@ -374,10 +387,13 @@ int build_shells(mq_ctx *c, int nnuc, const int *Z, const double *xyz, const dou
 int build_pairs(mq_ctx *c);
 void pairs_host(const std::vector<HostShell> &shells, const std::vector<double> &xyz, HostPairs &h);
 void append_pairs_class(HostPairs &dst, const HostPairs &src, int cl, int mol);
-int upload_pairs(mq_ctx *c, const HostPairs &h, std::vector<void *> *allocs, PairTable &t);
+int upload_pairs(mq_ctx *c, const HostPairs &h, std::vector<void *> *allocs, PairTable &t, int mode);
 void free_pairs(mq_ctx *c);
 void tight_boys_table(std::vector<double> &tab);  // TIGHT_NT x TIGHT_NM, row-major [T][m]
 constexpr int BOYS_SCALED_M = 5;                  // orders with their own Taylor-coefficient table
+constexpr int BOYS_FINE_M = 3, BOYS_FINE_NT = 577;  // orders and rows (T step 1/16) of the degree-6 tables
+// their offset in the device table: behind the values, grid and Taylor tables, on a 64-byte boundary
+constexpr size_t BOYS_FINE_OFF = ((size_t)TIGHT_NT * (TIGHT_NM + 1 + 9 * BOYS_SCALED_M) + 7) / 8 * 8;
 void tight_boys_device_table(std::vector<double> &tab);  // the table, its grid, the scaled tables
 
 // eri.cu
