@@ -43,16 +43,18 @@ __device__ __forceinline__ double bmax(double v, double *red) { return jac_block
 // X = S^-1/2 = U s^-1/2 U^T per molecule; status bit 1 if S is not positive definite
 __global__ void __launch_bounds__(BT) batch_orth_kernel(const MolDesc *__restrict__ mols,
                                                         const double *__restrict__ S, double *__restrict__ X,
-                                                        double *__restrict__ work, int *__restrict__ status) {
+                                                        double *__restrict__ work, size_t wstride, int *__restrict__ status) {
   extern __shared__ double sm[];
-  __shared__ double red[BT / 32];
+  __shared__ double red[32];
   const MolDesc md = mols[blockIdx.x];
   const int n = md.n;
   const size_t n2 = (size_t)n * n;
-  double *A = sm, *V = sm + n2, *cs = V + n2;
+  double *A = sm, *V = sm + n2;
   for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) A[idx] = S[md.mat + idx];
   __syncthreads();
-  const bool ok = jacobi_block(n, A, V, cs, red, work + 2 * md.mat, 60, 1e-14);
+  double *W = work ? work + wstride * blockIdx.x : sm + 2 * n2;
+  double *cs = work ? sm + 2 * n2 : W + jacobi_work(n);
+  const bool ok = jacobi_block(n, A, V, red, W, 60, 1e-14);
   // s^-1/2 on the diagonal of A
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double s = A[i + (size_t)n * i];
@@ -62,8 +64,11 @@ __global__ void __launch_bounds__(BT) batch_orth_kernel(const MolDesc *__restric
   __syncthreads();
   if (threadIdx.x == 0 && !ok) atomicOr(status + blockIdx.x, 2);
   for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) A[idx] = V[idx] * cs[idx / n];
-  __syncthreads();
-  cta_mm<true>(n, n, n, A, V, X + md.mat);
+  const JacobiWork jw(W, n);
+  cta_fix_rows(n, n, A, 1, n, jw.e1, jw.U1);
+  cta_fix_rows(n, n, V, 1, n, jw.e2, jw.U2);
+  double *Xm = X + md.mat;
+  cta_fix_mm(n, n, n, jw.U1, jw.e1, jw.U2, jw.e2, [&](int i, int j, double v) { Xm[i + n * j] = v; });
 }
 
 // F = H + G and E_k = 1/2 sum D (F + H) + E_nuc (getEnr, scf.f90:1122-1152;
@@ -73,7 +78,7 @@ __global__ void __launch_bounds__(BT) batch_energy_kernel(const MolDesc *__restr
                                                           const double *__restrict__ H, const double *__restrict__ G,
                                                           const double *__restrict__ D, const double *__restrict__ enuc,
                                                           double *__restrict__ F, double *__restrict__ Ek) {
-  __shared__ double red[BT / 32];
+  __shared__ double red[32];
   const int m = blockIdx.x;
   if (!active[m]) return;
   const MolDesc md = mols[m];
@@ -98,9 +103,10 @@ __global__ void __launch_bounds__(BT) batch_diis_kernel(const MolDesc *__restric
                                                         const double *__restrict__ D, const double *__restrict__ S,
                                                         double *__restrict__ Fh, double *__restrict__ Eh,
                                                         double *__restrict__ Bm, int2 *__restrict__ state, int ndiis,
-                                                        size_t mat_total, double *__restrict__ Fx) {
+                                                        size_t mat_total, double *__restrict__ Fx,
+                                                        double *__restrict__ work, size_t wstride) {
   extern __shared__ double sm[];
-  __shared__ double red[BT / 32];
+  __shared__ double red[32];
   __shared__ double cvec[DIIS_MAX];
   __shared__ double sys[(DIIS_MAX + 1) * (DIIS_MAX + 2)];
   const int m = blockIdx.x;
@@ -108,18 +114,23 @@ __global__ void __launch_bounds__(BT) batch_diis_kernel(const MolDesc *__restric
   const MolDesc md = mols[m];
   const int n = md.n;
   const size_t n2 = (size_t)n * n;
-  double *T = sm, *U = sm + n2;
+  double *T = sm;
+  const JacobiWork jw(work ? work + wstride * blockIdx.x : sm + (n2 + 1) / 2 * 2, n);
   const int2 st = state[m];
   const int h = st.x, nh = min(st.y + 1, ndiis);
-  cta_mm(n, n, n, F + md.mat, D + md.mat, T);
-  __syncthreads();
-  cta_mm(n, n, n, T, S + md.mat, U);
+  // T = F D, then T <- T S (F, D and S are symmetric: rows are columns)
+  cta_fix_rows(n, n, F + md.mat, n, 1, jw.e1, jw.U1);
+  cta_fix_rows(n, n, D + md.mat, n, 1, jw.e2, jw.U2);
+  cta_fix_mm(n, n, n, jw.U1, jw.e1, jw.U2, jw.e2, [&](int i, int j, double v) { T[i + n * j] = v; });
+  cta_fix_rows(n, n, T, 1, n, jw.e1, jw.U1);
+  cta_fix_rows(n, n, S + md.mat, n, 1, jw.e2, jw.U2);
+  cta_fix_mm(n, n, n, jw.U1, jw.e1, jw.U2, jw.e2, [&](int i, int j, double v) { T[i + n * j] = v; });
   __syncthreads();
   double *Fs = Fh + mat_total * h + md.mat, *Es = Eh + mat_total * h + md.mat;
   for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) {
     const size_t t = (idx % n) * n + idx / n;
     Fs[idx] = F[md.mat + idx];
-    Es[idx] = U[idx] - U[t];
+    Es[idx] = T[idx] - T[t];
   }
   __syncthreads();
   double *B = Bm + (size_t)m * ndiis * ndiis;
@@ -195,23 +206,28 @@ __global__ void __launch_bounds__(BT) batch_density_kernel(
     int guess, const MolDesc *__restrict__ mols, int *__restrict__ active, const double *__restrict__ X,
     const double *__restrict__ Fx, double *__restrict__ D, double *__restrict__ Dn, double *__restrict__ eps,
     int *__restrict__ iters, int *__restrict__ conv, const double *__restrict__ Ek, double *__restrict__ Efin,
-    double thr, int conv_rms, int max_iter, double *__restrict__ work, int *__restrict__ status) {
+    double thr, int conv_rms, int max_iter, double *__restrict__ work, size_t wstride, int *__restrict__ status) {
   extern __shared__ double sm[];
-  __shared__ double red[BT / 32];
+  __shared__ double red[32];
   __shared__ int decision;
   const int m = blockIdx.x;
   if (!guess && !active[m]) return;
   const MolDesc md = mols[m];
   const int n = md.n, nocc = md.nocc;
   const size_t n2 = (size_t)n * n;
-  double *A = sm, *V = sm + n2, *cs = V + n2;
-  int *perm = (int *)(cs + n + 2);
+  double *A = sm, *V = sm + n2;
+  double *W = work ? work + wstride * blockIdx.x : sm + 2 * n2;
+  int *perm = (int *)(work ? sm + 2 * n2 : W + jacobi_work(n));
+  const JacobiWork jw(W, n);
   const double *Xm = X + md.mat;
-  cta_mm(n, n, n, Fx + md.mat, Xm, V);  // T = Fx X
+  // A = X (Fx X) (both symmetric: rows are columns)
+  cta_fix_rows(n, n, Fx + md.mat, n, 1, jw.e1, jw.U1);
+  cta_fix_rows(n, n, Xm, n, 1, jw.e2, jw.U2);
+  cta_fix_mm(n, n, n, jw.U1, jw.e1, jw.U2, jw.e2, [&](int i, int j, double v) { V[i + n * j] = v; });
+  cta_fix_rows(n, n, V, n, 1, jw.e1, jw.U1);
+  cta_fix_mm(n, n, n, jw.U2, jw.e2, jw.U1, jw.e1, [&](int i, int j, double v) { A[i + n * j] = v; });
   __syncthreads();
-  cta_mm(n, n, n, Xm, V, A);  // X T (X symmetric)
-  __syncthreads();
-  const bool ok = jacobi_block(n, A, V, cs, red, work + 2 * md.mat, 60, 1e-14);
+  const bool ok = jacobi_block(n, A, V, red, W, 60, 1e-14);
   if (threadIdx.x == 0 && !ok) atomicOr(status + m, 2);
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const int r = jacobi_rank(n, A, i);
@@ -220,9 +236,14 @@ __global__ void __launch_bounds__(BT) batch_density_kernel(
   }
   __syncthreads();
   // C_occ (n x nocc) into A, D_new
-  cta_mm(n, nocc, n, Xm, V, A, 1.0, perm);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) jw.e2[i] = 1;  // |entries| of an orthogonal matrix < 2
   __syncthreads();
-  cta_mm<true>(n, n, nocc, A, A, Dn + md.mat, 2.0);
+  cta_fix(nocc, n, true, jw.e2, jw.U2, [&](int r, int k) { return V[k + n * perm[r]]; });
+  cta_fix_rows(n, n, Xm, n, 1, jw.e1, jw.U1);
+  cta_fix_mm(n, nocc, n, jw.U1, jw.e1, jw.U2, jw.e2, [&](int i, int j, double v) { A[i + n * j] = v; });
+  cta_fix_rows(n, nocc, A, 1, n, jw.e1, jw.U1);
+  double *Dm = Dn + md.mat;
+  cta_fix_mm(n, n, nocc, jw.U1, jw.e1, jw.U1, jw.e1, [&](int i, int j, double v) { Dm[i + n * j] = 2.0 * v; });
   __syncthreads();
   double dmax = 0.0, dss = 0.0;
   for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) {
@@ -476,8 +497,13 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
   float2 *d_DJ = (float2 *)buf(c, "batch_dsplit", mat * sizeof(float2));
   double *d_Kp = (double *)buf(c, "batch_kslices", tl.size() * (size_t)nmax * sizeof(double));
   double *d_Q = (double *)buf(c, "batch_Q", std::max<size_t>(q, 1) * sizeof(double));
-  double *d_eig = (double *)buf(c, "batch_eig", mat * sizeof(double) * 2);  // the eigensolver's scratch
-  if (!d_eig || !d_XX || !d_mats || !d_vecs || !d_B || !d_ints || !d_DJ || !d_Kp || !d_Q) return MQ_ENOMEM;
+  // scratch of the eigensolver and the products: in shared memory while two
+  // CTAs fit an SM (n <= 58), else in global memory
+  const size_t mat_max = (size_t)nmax * nmax * sizeof(double), work_max = (size_t)jacobi_work(nmax) * sizeof(double);
+  const bool smem_work = 2 * mat_max + work_max + 16 * (size_t)nmax <= 110 * 1024;
+  const size_t eig_stride = jacobi_work(nmax);
+  double *d_eig = smem_work ? nullptr : (double *)buf(c, "batch_eig", eig_stride * M * sizeof(double));
+  if ((!smem_work && !d_eig) || !d_XX || !d_mats || !d_vecs || !d_B || !d_ints || !d_DJ || !d_Kp || !d_Q) return MQ_ENOMEM;
   double *dS = d_mats, *dH = dS + mat, *dX = dH + mat, *dD = dX + mat, *dDn = dD + mat, *dF = dDn + mat,
          *dG = dF + mat, *dFx = dG + mat, *dJ = dFx + mat, *dK = dJ + mat, *dFh = dK + mat,
          *dEh = dFh + mat * (size_t)nd;
@@ -500,14 +526,14 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
   c->d_boys = saved_boys;
   MQ_TRY(rc);
   // ---- S^-1/2 and the core-Hamiltonian guess
-  const size_t smem = (2 * (size_t)nmax * nmax + nmax + 2) * sizeof(double) + nmax * sizeof(int) + 16;
-  const size_t smem_diis = 2 * (size_t)nmax * nmax * sizeof(double);
+  const size_t smem = 2 * mat_max + (smem_work ? work_max : 0) + 16 * (size_t)nmax + 16;
+  const size_t smem_diis = mat_max + (smem_work ? work_max : 0) + 16;
   MQ_CUDA(c, cudaFuncSetAttribute(batch_orth_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   MQ_CUDA(c, cudaFuncSetAttribute(batch_density_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   MQ_CUDA(c, cudaFuncSetAttribute(batch_diis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_diis));
-  batch_orth_kernel<<<M, BT, smem, c->stream>>>(d_md, dS, dX, d_eig, d_status);
+  batch_orth_kernel<<<M, BT, smem, c->stream>>>(d_md, dS, dX, d_eig, eig_stride, d_status);
   batch_density_kernel<<<M, BT, smem, c->stream>>>(1, d_md, d_active, dX, dH, dD, dDn, d_eps, d_it, d_conv, d_Ek,
-                                                   d_Ef, thr, o->conv_rms, max_iter, d_eig, d_status);
+                                                   d_Ef, thr, o->conv_rms, max_iter, d_eig, eig_stride, d_status);
   c->stats.launches += 2;
   c->stats.guesses_taken = 0;
   if (o->D_in) {
@@ -549,11 +575,11 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
     const double *Fuse = dF;
     if (ndiis > 0) {
       batch_diis_kernel<<<M, BT, smem_diis, c->stream>>>(d_md, d_active, dF, dD, dS, dFh, dEh, d_B, d_state, ndiis,
-                                                         mat, dFx);
+                                                         mat, dFx, d_eig, eig_stride);
       Fuse = dFx;
     }
     batch_density_kernel<<<M, BT, smem, c->stream>>>(0, d_md, d_active, dX, Fuse, dD, dDn, d_eps, d_it, d_conv,
-                                                     d_Ek, d_Ef, thr, o->conv_rms, max_iter, d_eig, d_status);
+                                                     d_Ek, d_Ef, thr, o->conv_rms, max_iter, d_eig, eig_stride, d_status);
     MQ_CUDA(c, cudaGetLastError());
     return MQ_OK;
   };

@@ -1,0 +1,237 @@
+// fixmm.cuh -- FP64 matrix products on the tensor cores, as exact integer
+// products of fixed-point operands (the splitting of Ozaki, Ogita, Oishi and
+// Rump, Numer. Algorithms 59, 95 (2012), on FP16 digits).
+//
+// Each row of op(A) and each column of op(B) is scaled by a power of two to
+// |x| < 2^62 and rounded to an integer (every element within 2^9 of the row's
+// largest stays exact), cut into eight digits of eight bits,
+// x = sum_k s_k 256^(7-k), -128 <= s_k <= 127, |s_0| <= 64.  FP16 holds a digit
+// exactly, a digit product is an integer of at most 2^14, and the sum of one
+// level (the products s_k s'_l with k + l = L) over K <= 144 stays below 2^24,
+// so the FP32 accumulators of mma.sync hold every level exactly in any order.
+// The levels L = 0..7 (36 digit products) are combined as integers and rounded
+// to FP64 once.  What is dropped -- the rounding of the operands, 2^-63 of the
+// row's largest element, and levels 8 to 14 -- is about 2^-61 of the largest
+// possible sum, so an element is correct to rounding unless it is 2^-8 of that
+// and less; an FP64 sum rounds after each of its K additions.
+//
+// Why: this GPU issues two FP64 multiply-adds per clock and SM.  36 digit
+// products take the tensor cores a small part of that time; operands of up to a few hundred
+// rows do not fill the larger tiles of tcgen05.mma and would have to be staged
+// in shared memory seven times over, whereas the fragments of mma.sync are
+// built in registers from one 8-byte integer per element: byte k of x + (128 in
+// every byte) is s_k + 128; with 0x64 above it, it is the FP16 number
+// 1024 + s_k + 128, and one subtraction per two elements gives the digits.  Two
+// neighbouring elements' bytes are stored alternating, so that one byte
+// permutation forms the pair of a fragment register.
+#pragma once
+#include <cuda_fp16.h>
+#include <stdint.h>
+
+namespace mq {
+
+constexpr int FX_DIG = 8;
+constexpr int FX_KMAX = 144;  // (6 * 128^2 + 2 * 64 * 128) * 144 < 2^24
+constexpr unsigned long long FX_BIAS = 0x8080808080808080ull;
+constexpr int FX_BITS = 62;
+
+// Position of the pair of elements (2 kp, 2 kp + 1) in row r of fixed-point
+// pairs: within each run of 8 pairs (128 bytes) the rows are permuted so that
+// neither a fragment's 16-byte loads (4 neighbouring pairs of 2 neighbouring
+// rows per quarter warp) nor a quarter warp's stores of one pair of 8
+// neighbouring rows meet a bank conflict.
+__device__ __forceinline__ int fx_pos(int r, int kp) { return kp ^ (((r & 1) << 2) | ((r >> 1) & 3)); }
+
+// x * 2^(FX_BITS - e) rounded to nearest (ties away), biased; |x| < 2^e
+__device__ __forceinline__ unsigned long long fx_fix(double x, int e) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int E = (int)(b >> 52) & 0x7ff;
+  const int sh = e - FX_BITS + 1075 - E;  // > 0: right shift
+  unsigned long long m = (b & 0xfffffffffffffull) | 0x10000000000000ull;
+  if (E == 0 || sh > 54) m = 0;
+  else if (sh > 0) m = (m + (1ull << (sh - 1))) >> sh;
+  else m <<= -sh;
+  return ((long long)b < 0 ? 0ull - m : m) + FX_BIAS;
+}
+// e with |x| < 2^e for every x of exponent field <= E (0 for a zero row)
+__device__ __forceinline__ int fx_exp(int E) { return E == 0 ? -1100 : E - 1022; }
+__device__ __forceinline__ int fx_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// Two biased integers with their bytes alternating, lowest first
+__device__ __forceinline__ uint4 fx_pair(unsigned long long u0, unsigned long long u1) {
+  const unsigned l0 = (unsigned)u0, h0 = (unsigned)(u0 >> 32), l1 = (unsigned)u1, h1 = (unsigned)(u1 >> 32);
+  return make_uint4(__byte_perm(l0, l1, 0x5140), __byte_perm(l0, l1, 0x7362), __byte_perm(h0, h1, 0x5140),
+                    __byte_perm(h0, h1, 0x7362));
+}
+
+// The digits of a pair (k, k + 1) as FP16 pairs
+__device__ __forceinline__ void fx_digits(uint4 u, unsigned (&d)[FX_DIG]) {
+  const unsigned word[4] = {u.x, u.y, u.z, u.w};
+  const __half2 off = __half2half2(__ushort_as_half(0x6480));  // 1024 + 128
+#pragma unroll
+  for (int k = 0; k < FX_DIG; ++k) {
+    const int by = FX_DIG - 1 - k;  // byte of digit k
+    const unsigned w = __byte_perm(word[by >> 1], 0x64646464u, by & 1 ? 0x4342 : 0x4140);
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&w), off);
+    d[k] = *reinterpret_cast<const unsigned *>(&h);
+  }
+}
+
+__device__ __forceinline__ void fx_mma(float (&c)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// sum_L v_L 256^(7-L) * 2^(ea + eb - 2 FX_BITS + 8 * 7), rounded to nearest.
+// Integers throughout: an FP64 instruction would occupy its SM for 16 clocks
+// per warp, and the result of a product needs five of them.
+__device__ __forceinline__ double fx_combine(const float *v, int ea, int eb) {
+  auto four = [](const float *q) {
+    return ((long long)__float2int_rn(q[0]) << 24) + ((long long)__float2int_rn(q[1]) << 16) +
+           ((long long)__float2int_rn(q[2]) << 8) + __float2int_rn(q[3]);
+  };
+  const long long lo = four(v + 4);
+  long long h = four(v) + (lo >> 32);  // the sum is h 2^32 + l, |h| < 2^45, 0 <= l < 2^32
+  unsigned l = (unsigned)lo;
+  const bool neg = h < 0;
+  if (neg) {
+    h = ~h + (l == 0);
+    l = 0u - l;
+  }
+  if (h == 0 && l == 0) return 0.0;
+  // the leading 64 bits: m 2^x with the top bit of m set
+  const int z = h ? __clzll(h) : 64 + __clz(l);
+  const unsigned long long m = z >= 32 ? ((unsigned long long)h << 32 | l) << (z - 32)
+                                       : ((unsigned long long)h << z | l >> (32 - z));
+  // (h 2^32 + l < 2^77, so z >= 19; the sum is m 2^(32 - z))
+  const int e = 32 - z + 63 + ea + eb - 2 * FX_BITS + 56;  // binary exponent of the leading bit
+  const unsigned long long r = (m >> 11) + ((m >> 10) & 1);  // 53 bits, maybe 2^53 after rounding
+  if (e > -1022 && e < 1023) {
+    const long long bits = ((long long)(e + 1022) << 52) + (long long)r;
+    return __longlong_as_double(neg ? bits | (long long)0x8000000000000000ull : bits);
+  }
+  // at the ends of the exponent range: scaled by FP64 products
+  const double x = (double)r * (neg ? -1.0 : 1.0);
+  const int s = e - 52, s1 = max(min(s / 2, 1000), -1000), s2 = max(min(s - s1, 1000), -1000);
+  return x * __hiloint2double((s1 + 1023) << 20, 0) * __hiloint2double((s2 + 1023) << 20, 0);
+}
+
+// A 16 x (8 NT) tile: rows of UA (fragment rows r0 + g, r0 + g + 8; clamped to
+// rows na - 1), columns = rows of UB (c0 + 8 j + g, clamped), K = 16 ksteps.
+// acc[j][level][4].
+template <int NT>
+__device__ __forceinline__ void fx_tile(const uint4 *UA, const uint4 *UB, int ld, int na, int nb, int r0, int c0,
+                                        int ksteps, float (&acc)[NT][FX_DIG][4]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int ra = min(r0 + g, na - 1), rb = min(r0 + g + 8, na - 1);
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int L = 0; L < FX_DIG; ++L)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[j][L][i] = 0.f;
+#pragma unroll 1
+  for (int ks = 0; ks < ksteps; ++ks) {
+    const int k0 = 8 * ks + t;
+    unsigned a[4][FX_DIG];
+    fx_digits(UA[(size_t)ra * ld + fx_pos(ra, k0)], a[0]);
+    fx_digits(UA[(size_t)rb * ld + fx_pos(rb, k0)], a[1]);
+    fx_digits(UA[(size_t)ra * ld + fx_pos(ra, k0 + 4)], a[2]);
+    fx_digits(UA[(size_t)rb * ld + fx_pos(rb, k0 + 4)], a[3]);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      const int cb = min(c0 + 8 * j + g, nb - 1);
+      unsigned b[2][FX_DIG];
+      fx_digits(UB[(size_t)cb * ld + fx_pos(cb, k0)], b[0]);
+      fx_digits(UB[(size_t)cb * ld + fx_pos(cb, k0 + 4)], b[1]);
+#pragma unroll
+      for (int x = 0; x < FX_DIG; ++x)
+#pragma unroll
+        for (int y = 0; y + x < FX_DIG; ++y) {
+          const unsigned av[4] = {a[0][x], a[1][x], a[2][x], a[3][x]};
+          const unsigned bv[2] = {b[0][y], b[1][y]};
+          fx_mma(acc[j][x + y], av, bv);
+        }
+    }
+  }
+}
+
+// ---- One CTA's products.  Row r < nr of a matrix, X(r, k) at x[r rs + k ks],
+// k < nk, becomes fx_ld(nk) fixed-point pairs (zeros behind nk) under the
+// exponent e[r]; neighbouring threads take neighbouring elements of the faster
+// index.  (No barrier inside: e must be visible to all, after one.)
+__host__ __device__ constexpr int fx_ld(int nk) { return (nk + 15) / 16 * 8; }
+
+static __device__ __forceinline__ void cta_row_exp(int nr, int nk, const double *x, int rs, int ks, int *e) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (ks == 1) {  // a warp per row
+    for (int r = w; r < nr; r += nw) {
+      int m = 0;
+      for (int k = lane; k < nk; k += 32) m = max(m, fx_field(x[(size_t)r * rs + k]));
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (lane == 0) e[r] = fx_exp(m);
+    }
+  } else {  // 4 threads per row, 8 neighbouring rows per warp
+    for (int r0 = 8 * w; r0 < nr; r0 += 8 * nw) {
+      const int r = r0 + (lane & 7);
+      int m = 0;
+      if (r < nr)
+        for (int k = lane >> 3; k < nk; k += 4) m = max(m, fx_field(x[(size_t)r * rs + (size_t)k * ks]));
+      m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
+      m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+      if (r < nr && lane < 8) e[r] = fx_exp(m);
+    }
+  }
+}
+// elem(r, k) is X(r, k); `fast_k`: k is the faster index
+template <class Elem>
+static __device__ __forceinline__ void cta_fix(int nr, int nk, bool fast_k, const int *e, uint4 *U, Elem elem) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, ld = fx_ld(nk);
+  auto put = [&](int r, int kp) {
+    const int k = 2 * kp, ex = e[r];
+    const unsigned long long u0 = k < nk ? fx_fix(elem(r, k), ex) : FX_BIAS;
+    const unsigned long long u1 = k + 1 < nk ? fx_fix(elem(r, k + 1), ex) : FX_BIAS;
+    U[(size_t)r * ld + fx_pos(r, kp)] = fx_pair(u0, u1);
+  };
+  if (fast_k) {
+    for (int r = w; r < nr; r += nw)
+      for (int kp = lane; kp < ld; kp += 32) put(r, kp);
+  } else {
+    for (int kp = w; kp < ld; kp += nw)
+      for (int r = lane; r < nr; r += 32) put(r, kp);
+  }
+}
+
+// Both: the rows X(r, k) = x[r rs + k ks] with their exponents, ready for all
+// threads (begins and ends with a barrier)
+static __device__ __forceinline__ void cta_fix_rows(int nr, int nk, const double *x, int rs, int ks, int *e, uint4 *U) {
+  __syncthreads();
+  cta_row_exp(nr, nk, x, rs, ks, e);
+  __syncthreads();
+  cta_fix(nr, nk, ks == 1, e, U, [=](int r, int k) { return x[(size_t)r * rs + (size_t)k * ks]; });
+  __syncthreads();
+}
+
+// store(i, j, value) of the na x nb product of the fixed-point rows UA and UB
+template <class Store>
+static __device__ __forceinline__ void cta_fix_mm(int na, int nb, int nk, const uint4 *UA, const int *ea,
+                                                  const uint4 *UB, const int *eb, Store store) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, g = lane >> 2, t = lane & 3;
+  const int tm = (na + 15) / 16, tn = (nb + 7) / 8;
+  for (int tile = w; tile < tm * tn; tile += nw) {
+    const int tj = tile / tm, ti = tile - tj * tm;
+    float acc[1][FX_DIG][4];
+    fx_tile<1>(UA, UB, fx_ld(nk), na, nb, 16 * ti, 8 * tj, (nk + 15) / 16, acc);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = 16 * ti + g + 8 * (i >> 1), cc = 8 * tj + 2 * t + (i & 1);
+      float v[FX_DIG];
+#pragma unroll
+      for (int L = 0; L < FX_DIG; ++L) v[L] = acc[0][L][i];
+      if (r < na && cc < nb) store(r, cc, fx_combine(v, ea[r], eb[cc]));
+    }
+  }
+}
+
+}  // namespace mq

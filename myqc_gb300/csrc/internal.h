@@ -454,10 +454,6 @@ int syev_large_warm(mq_ctx *c, int n, double *d_A, double *d_w, double *d_V);
 // syev_large_warm: FP32 cluster Jacobi and the FP64 first-order refinement,
 // queued on c->stream with no grid-wide barrier and nothing read back (eigen.cu)
 int syev_large_start(mq_ctx *c, int n, const double *d_A, double *d_V);
-// small FP64 products on all SMs (dgemm.cu); gemm() takes them when they fit
-bool dgemm_small_fits(int m, int n, int k);
-int dgemm_small(mq_ctx *c, char ta, char tb, int m, int n, int k, double alpha, const double *A, int lda,
-                const double *B, int ldb, double beta, double *C, int ldc);
 // any FP64 product, batched over blockIdx.z with strides sA, sB, sC (dgemm.cu)
 int dgemm_batched(mq_ctx *c, char ta, char tb, int m, int n, int k, double alpha, const double *A, int lda,
                   long long sA, const double *B, int ldb, long long sB, double beta, double *C, int ldc,

@@ -9,6 +9,7 @@
 // tol * ||A||_F.  Replaces the eigen step of DSYEV/DSYGV (src/scf/scf.f90:692,
 // 478, 848).
 #pragma once
+#include "fixmm.cuh"
 
 namespace mq {
 
@@ -29,28 +30,35 @@ __device__ __forceinline__ void rr_pair(int np, int r, int k, int &p, int &q) {
   }
 }
 
-// Sum over the block of one value per thread (red: blockDim.x/32 doubles).
-__device__ __forceinline__ double jac_block_sum(double v, double *red) {
+// Sum (largest) over the block of one value per thread, in every thread (red:
+// 32 entries).  One warp adds the warps' sums: each FP64 addition occupies its
+// SM for 16 clocks per warp, so sixteen warps each adding sixteen sums would
+// take 4000.
+template <class T, class Op>
+__device__ __forceinline__ T jac_block_reduce(T v, T *red, T zero, Op op) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
   __syncthreads();
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  double t = 0.0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-  return t;
+  if (threadIdx.x < 32) {
+    T t = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : zero;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t = op(t, __shfl_xor_sync(0xffffffffu, t, o));
+    __syncwarp();
+    if (threadIdx.x == 0) red[0] = t;
+  }
+  __syncthreads();
+  return red[0];
 }
-
-// Largest value of one per thread over the block.
+__device__ __forceinline__ double jac_block_sum(double v, double *red) {
+  return jac_block_reduce(v, red, 0.0, [](double a, double b) { return a + b; });
+}
+__device__ __forceinline__ float jac_block_sum(float v, double *red) {
+  return jac_block_reduce(v, reinterpret_cast<float *>(red), 0.f, [](float a, float b) { return a + b; });
+}
 __device__ __forceinline__ double jac_block_max(double v, double *red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t = fmax(t, red[w]);
-  return t;
+  return jac_block_reduce(v, red, 0.0, [](double a, double b) { return fmax(a, b); });
 }
 
 // pair k of round r as rr_pair gives it (r < np - 1), without integer division
@@ -65,236 +73,283 @@ __device__ __forceinline__ void rr_pair_fast(int np, int r, int k, int &p, int &
   q = max(a, b);
 }
 
-// ---- FP64 products of one CTA, column-major, leading dimension = row count.
-// GB300 issues two FP64 multiply-adds per clock and SM, so the point is to
-// spend FP64 issue slots on nothing else: each thread forms a 2 x 4 block of
-// the product (8 independent chains, 6 loads per 8 multiply-adds), with one
-// integer division per block.
-constexpr int MM_C = 4;
-
-// C (m x n) = f A (m x k) op(B), op(B) = B (k x n) or, TB, the transpose of
-// B (n x k); with `cols` the columns of B are taken in that order
-template <bool TB = false>
-static __device__ __forceinline__ void cta_mm(int m, int n, int k, const double *A, const double *B, double *C,
-                                              double f = 1.0, const int *cols = nullptr) {
-  const size_t sb = TB ? n : 1;
-  const int hi = (m + 1) / 2, nj = (n + MM_C - 1) / MM_C;
-  for (int t = threadIdx.x; t < hi * nj; t += blockDim.x) {
-    const int tj = t / hi, i0 = t - tj * hi, i1 = i0 + hi < m ? i0 + hi : i0, j0 = tj * MM_C;
-    const double *b[MM_C];
-    double s0[MM_C], s1[MM_C];
-#pragma unroll
-    for (int c = 0; c < MM_C; ++c) {
-      const int j = min(j0 + c, n - 1);
-      b[c] = TB ? B + j : B + (size_t)k * (cols ? cols[j] : j);
-      s0[c] = s1[c] = 0.0;
-    }
-#pragma unroll 4
-    for (int l = 0; l < k; ++l) {
-      const double a0 = A[i0 + (size_t)m * l], a1 = A[i1 + (size_t)m * l];
-#pragma unroll
-      for (int c = 0; c < MM_C; ++c) {
-        const double x = b[c][sb * l];
-        s0[c] = fma(a0, x, s0[c]);
-        s1[c] = fma(a1, x, s1[c]);
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < MM_C; ++c)
-      if (j0 + c < n) {
-        C[i0 + (size_t)m * (j0 + c)] = f * s0[c];
-        C[i1 + (size_t)m * (j0 + c)] = f * s1[c];
-      }
-  }
-}
-
-// C (n x n) = A^T B, all n x n.  A thread's rows are the columns i0, i1 of A; its
-// sum starts at row (thread) mod n, so that neighbouring threads read
-// addresses n + 1 apart (no shared-memory bank conflicts).
-static __device__ __forceinline__ void cta_mm_tn(int n, const double *A, const double *B, double *C) {
-  const int hi = (n + 1) / 2, nj = (n + MM_C - 1) / MM_C;
-  for (int t = threadIdx.x; t < hi * nj; t += blockDim.x) {
-    const int tj = t / hi, i0 = t - tj * hi, i1 = i0 + hi < n ? i0 + hi : i0, j0 = tj * MM_C;
-    const double *a0 = A + (size_t)n * i0, *a1 = A + (size_t)n * i1;
-    const double *b[MM_C];
-    double s0[MM_C], s1[MM_C];
-#pragma unroll
-    for (int c = 0; c < MM_C; ++c) {
-      b[c] = B + (size_t)n * min(j0 + c, n - 1);
-      s0[c] = s1[c] = 0.0;
-    }
-    int l = i0;
-#pragma unroll 4
-    for (int s = 0; s < n; ++s) {
-      const double x0 = a0[l], x1 = a1[l];
-#pragma unroll
-      for (int c = 0; c < MM_C; ++c) {
-        const double x = b[c][l];
-        s0[c] = fma(x0, x, s0[c]);
-        s1[c] = fma(x1, x, s1[c]);
-      }
-      l = l + 1 < n ? l + 1 : 0;
-    }
-#pragma unroll
-    for (int c = 0; c < MM_C; ++c)
-      if (j0 + c < n) {
-        C[i0 + (size_t)n * (j0 + c)] = s0[c];
-        C[i1 + (size_t)n * (j0 + c)] = s1[c];
-      }
-  }
-}
-
 // Tangent of the Jacobi angle that annihilates apq, from aqq - app, in FP32
-// with the fast reciprocal and square root (any angle near it converges).
-__device__ __forceinline__ float tangent_f32(float diff, float apq) {
-  const float theta = __fdividef(diff, 2.f * apq), a = fabsf(theta);
-  const float t = a > 1e15f ? __fdividef(0.5f, a) : __fdividef(1.f, a + __fsqrt_rn(fmaf(a, a, 1.f)));
-  return copysignf(t, theta);
+// with the approximate reciprocal and square root (any angle near it
+// converges); apq != 0.
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
-__device__ __forceinline__ float2 rotation_f32(float diff, float apq) {
-  const float t = tangent_f32(diff, apq), c = rsqrtf(fmaf(t, t, 1.f));
-  return make_float2(c, t * c);
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float tangent_f32(float diff, float apq) {
+  // 2 apq / (|diff| + sqrt(diff^2 + 4 apq^2)), signed: one reciprocal
+  const float b = 2.f * apq, t = fabsf(b) * rcp_approx(fabsf(diff) + sqrt_approx(fmaf(diff, diff, b * b)));
+  return copysignf(1.f, diff) * copysignf(1.f, apq) * fminf(t, 1.f);
 }
 
-// FP32 cyclic Jacobi of Af (n x n, destroyed), Vf <- the rotations: the start
-// vectors of jacobi_block.  A round rotates n'/2 disjoint pairs as independent
-// 2 x 2 blocks (rows {p, q} of pair P, columns {u, v} of pair Q), so it needs
-// one barrier after the angles and one after the update; a warp's lanes run
-// over P, whose p and q are runs of consecutive indices (no bank conflicts).
-// Ends at an off-diagonal norm of 1e-6 ||A||_F, near FP32's floor, or when a
-// late sweep no longer halves it.
-static __device__ void jacobi_block_f32(int n, float *Af, float *Vf, float2 *cs, double *red) {
+// FP32 cyclic Jacobi of A0 (n x n, n <= 128, destroyed with its twin A1), Vf <-
+// the rotations: the start vectors of jacobi_block.  A round rotates n'/2
+// disjoint pairs as independent 2 x 2 blocks (rows {p, q} of pair P, columns
+// {u, v} of pair Q).  Every warp computes all the round's angles itself, a pair
+// per lane (the lanes are idle otherwise), and writes the blocks of its pairs Q
+// to the other copy of A, so that a round costs one barrier.  Ends at an
+// off-diagonal norm of 1e-6 ||A||_F, near FP32's floor, or when a late sweep no
+// longer halves it.
+template <int CH>  // pairs per lane: n <= 64 CH
+static __device__ __forceinline__ void jacobi_block_f32(int n, float *A0, float *A1, float *Vf, double *red) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int np = n + (n & 1), half = np / 2;
   float fro = 0.f;
-  for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) fro += Af[idx] * Af[idx];
-  const float stop = 1e-12f * (float)jac_block_sum(fro, red);
+  for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) fro += A0[idx] * A0[idx];
+  const float stop = 1e-12f * jac_block_sum(fro, red);
   float last = INFINITY;
   for (int sweep = 0; sweep < 12; ++sweep) {
     float off = 0.f;
     for (int j = w; j < n; j += nw)
       for (int i = lane; i < n; i += 32)
-        if (i != j) off += Af[i + n * j] * Af[i + n * j];
-    off = (float)jac_block_sum(off, red);
+        if (i != j) off += A0[i + n * j] * A0[i + n * j];
+    off = jac_block_sum(off, red);
     if (!(off > stop) || (sweep > 6 && off > 0.25f * last)) return;
     last = off;
     for (int r = 0; r < np - 1; ++r) {
-      for (int k = threadIdx.x; k < half; k += blockDim.x) {
-        int p, q;
-        rr_pair_fast(np, r, k, p, q);
-        float2 v = make_float2(1.f, 0.f);
-        if (q < n) {
-          const float apq = Af[p + n * q], app = Af[p + n * p], aqq = Af[q + n * q];
+      const float *__restrict__ Ai = A0;
+      float *__restrict__ Ao = A1;
+      float cs[CH], sn[CH];
+      int pp[CH], qq[CH];
+#pragma unroll
+      for (int c = 0; c < CH; ++c) {
+        rr_pair_fast(np, r, min(lane + 32 * c, half - 1), pp[c], qq[c]);
+        cs[c] = 1.f;
+        sn[c] = 0.f;
+        if (qq[c] < n) {
+          const int p = pp[c], q = qq[c];
+          const float apq = Ai[p + n * q], app = Ai[p + n * p], aqq = Ai[q + n * q];
           if (fabsf(apq) > 1e-9f * (fabsf(app) + fabsf(aqq))) {
-            v = rotation_f32(aqq - app, apq);
+            const float t = tangent_f32(aqq - app, apq);
+            asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(cs[c]) : "f"(fmaf(t, t, 1.f)));
+            sn[c] = t * cs[c];
           }
+        } else {  // the dummy index: unit rotation, both copies of the row get the same value
+          qq[c] = pp[c];
         }
-        cs[k] = v;
       }
-      __syncthreads();
       for (int Q = w; Q < half; Q += nw) {
+        const float cq = __shfl_sync(0xffffffffu, CH == 1 || Q < 32 ? cs[0] : cs[CH - 1], Q & 31);
+        const float sq = __shfl_sync(0xffffffffu, CH == 1 || Q < 32 ? sn[0] : sn[CH - 1], Q & 31);
         int u, v;
         rr_pair_fast(np, r, Q, u, v);
-        const float2 cq = cs[Q];
         const bool vv = v < n;
-        float *au = Af + n * u, *av = Af + n * (vv ? v : u);
-        for (int P = lane; P < half; P += 32) {
-          int p, q;
-          rr_pair_fast(np, r, P, p, q);
-          const float2 cp = cs[P];
-          const bool qv = q < n;
-          const float apu = au[p], aqu = qv ? au[q] : 0.f, apv = vv ? av[p] : 0.f, aqv = qv && vv ? av[q] : 0.f;
-          const float bpu = cp.x * apu - cp.y * aqu, bqu = cp.y * apu + cp.x * aqu;
-          const float bpv = cp.x * apv - cp.y * aqv, bqv = cp.y * apv + cp.x * aqv;
-          au[p] = cq.x * bpu - cq.y * bpv;
-          if (qv) au[q] = cq.x * bqu - cq.y * bqv;
-          if (vv) av[p] = cq.y * bpu + cq.x * bpv;
-          if (qv && vv) av[q] = cq.y * bqu + cq.x * bqv;
+        const int cu = n * u, cv = n * (vv ? v : u);
+        float x[2 * CH], y[2 * CH];  // V's columns u and v
+#pragma unroll
+        for (int c = 0; c < 2 * CH; ++c) {
+          const int i = lane + 32 * c;
+          x[c] = i < n ? Vf[cu + i] : 0.f;
+          y[c] = i < n ? Vf[cv + i] : 0.f;
         }
-        if (!vv || cq.y == 0.f) continue;
-        float *vu = Vf + n * u, *v2 = Vf + n * v;
-        for (int i = lane; i < n; i += 32) {
-          const float x = vu[i], y = v2[i];
-          vu[i] = cq.x * x - cq.y * y;
-          v2[i] = cq.y * x + cq.x * y;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+          const int p = pp[c], q = qq[c];
+          const float apu = Ai[cu + p], aqu = Ai[cu + q], apv = Ai[cv + p], aqv = Ai[cv + q];
+          const float bpu = cs[c] * apu - sn[c] * aqu, bqu = sn[c] * apu + cs[c] * aqu;
+          const float bpv = cs[c] * apv - sn[c] * aqv, bqv = sn[c] * apv + cs[c] * aqv;
+          if (lane + 32 * c < half) {
+            Ao[cu + p] = cq * bpu - sq * bpv;
+            Ao[cu + q] = cq * bqu - sq * bqv;
+            if (vv) {
+              Ao[cv + p] = sq * bpu + cq * bpv;
+              Ao[cv + q] = sq * bqu + cq * bqv;
+            }
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 2 * CH; ++c) {
+          const int i = lane + 32 * c;
+          if (i < n && vv) {
+            Vf[cu + i] = cq * x[c] - sq * y[c];
+            Vf[cv + i] = sq * x[c] + cq * y[c];
+          }
         }
       }
+      float *t = A0;
+      A0 = A1;
+      A1 = t;
       __syncthreads();
     }
   }
 }
 
-// Diagonalise A in place (n x n, column-major, shared or global memory of this
-// CTA), V <- its eigenvectors.  cs: n' doubles (a cosine and a sine per pair
-// of a round, n' = n rounded up to even), red: blockDim.x/32 doubles, work:
-// 2 n^2 doubles of this CTA (shared or global memory).  Returns false when
-// max_sweeps did not reach the tolerance ||offdiag||_F <= tol ||A||_F.
+// Scratch of jacobi_block and of the products beside it: two fixed-point copies
+// of an n x n matrix, two exponents per row and a sine and cosine per pair.
+__host__ __device__ constexpr int jacobi_work(int n) {  // doubles, even
+  return 2 * n * 2 * fx_ld(n) + (n + 2 * (n + 1) + 1) / 2 * 2;
+}
+struct JacobiWork {
+  uint4 *U1, *U2;
+  double *cs;
+  int *e1, *e2;
+  __device__ __forceinline__ JacobiWork(double *work, int n)
+      : U1(reinterpret_cast<uint4 *>(work)), U2(U1 + n * fx_ld(n)), cs(reinterpret_cast<double *>(U2 + n * fx_ld(n))),
+        e1(reinterpret_cast<int *>(cs + 2 * ((n + 1) / 2))), e2(e1 + n) {}
+};
+
+// Diagonalise A in place (n x n, n <= 128, column-major, shared or global
+// memory of this CTA), V <- its eigenvectors.  red: 32 doubles, work:
+// jacobi_work(n) doubles of this CTA on a 16-byte boundary (shared or global
+// memory).  Returns false when max_sweeps did not reach the tolerance
+// ||offdiag||_F <= tol ||A||_F, or A is not finite (V is then NaN).
 //
-// Bound by FP64 issue (two multiply-adds per clock and SM): a cold FP64 sweep
-// of A and V costs 6 n^3 and nine were needed.  So the sweeps run in FP32 (64
-// times the rate) for start vectors, which FP64 products make orthonormal to
-// rounding and apply -- V <- V (I - E/2 + 3/8 E^2), E = V^T V - I, then
-// A <- V^T A V (4 n^3 together) -- and the FP64 sweeps that follow start from
-// off-diagonals of 1e-6 ||A||_F: two of 4 n^3 (A's lower blocks and their
-// mirror images) and a check.  An FP64 division or square root takes a warp
-// about a microsecond, so the tangents are FP32's.
-static __device__ bool jacobi_block(int n, double *A, double *V, double *cs, double *red, double *work,
-                                    int max_sweeps, double tol) {
+// A cold FP64 Jacobi is bound by FP64 issue (two multiply-adds per clock and
+// SM): nine sweeps of 6 n^3.  So the sweeps run in FP32 for start vectors, and
+// FP64 work is products on the tensor cores (fixmm.cuh, rounded as FP64 or
+// better):
+//   V <- V (I - E/2 + 3/8 E^2), E = V^T V - I   orthonormal to rounding
+//   A <- V^T A V                                off-diagonals 1e-6 ||A||_F
+//   twice: P = I + E + E^2/2 with the first-order rotations E_ij =
+//     a_ij / (a_jj - a_ii) of the pairs with |E_ij| <= 3e-4 (E is antisymmetric,
+//     so P is orthogonal to E^4/4 < 1e-14, and the second step's E is
+//     quadratically smaller); V <- V P, A <- P^T A P
+// Pairs too close for that (near-degenerate levels) are left to FP64 Jacobi
+// sweeps, which check the stopping rule of a cold solve and skip every rotation
+// below tol ||A||_F / n: usually the check alone.
+static __device__ bool jacobi_block(int n, double *A, double *V, double *red, double *work, int max_sweeps,
+                                    double tol) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
   const int n2 = n * n;
-  double fro = 0.0, big = 0.0;
-  for (int idx = tid; idx < n2; idx += blockDim.x) {
-    fro += A[idx] * A[idx];
-    big = fmax(big, fabs(A[idx]));
-  }
-  fro = jac_block_sum(fro, red);
+  const JacobiWork jw(work, n);
+  uint4 *U1 = jw.U1, *U2 = jw.U2;
+  double *cs = jw.cs;
+  int *e1 = jw.e1, *e2 = jw.e2;
+  double big = 0.0, fro = 0.0;
+  for (int idx = tid; idx < n2; idx += blockDim.x) big = fmax(big, fabs(A[idx]));
   big = jac_block_max(big, red);
-  const double stop2 = tol * tol * fro, skip = tol * sqrt(fro) / n;
-  const int np = n + (n & 1), half = np / 2;
-  // a power of two that brings A into FP32's range
+  // a power of two that brings A into FP32's range and its squares into FP64's
   const double scale = big > 1e-290 && big < 1e290 ? exp2(-(double)ilogb(big)) : 1.0;
-  {  // FP32 start vectors in V's space: the rotations, then the scaled matrix
+  for (int idx = tid; idx < n2; idx += blockDim.x) fro = fma(A[idx] * scale, A[idx] * scale, fro);
+  fro = jac_block_sum(fro, red);
+  if (!isfinite(fro)) {  // infinities or NaN in A
+    for (int idx = tid; idx < n2; idx += blockDim.x) V[idx] = fro - fro;
+    __syncthreads();
+    return false;
+  }
+  const double stop2 = tol * tol * fro, skip = tol * sqrt(fro) / (n * scale);
+  const int np = n + (n & 1), half = np / 2;
+  auto off_norm2 = [&]() {
+    double off = 0.0;
+    for (int j = w; j < n; j += nw)
+      for (int i = j + 1 + lane; i < n; i += 32) {
+        const double x = A[i + (size_t)n * j] * scale;
+        off = fma(x, x, off);
+      }
+    return 2.0 * jac_block_sum(off, red);
+  };
+  auto mirror = [&]() {  // (a congruence is symmetric but for the rounding of its halves)
+    __syncthreads();
+    for (int j = w; j < n; j += nw)
+      for (int i = j + 1 + lane; i < n; i += 32) A[j + (size_t)n * i] = A[i + (size_t)n * j];
+    __syncthreads();
+  };
+  auto col = [&](const double *x) { return [=](int r, int k) { return x[k + (size_t)n * r]; }; };
+  auto row = [&](const double *x) { return [=](int r, int k) { return x[r + (size_t)n * k]; }; };
+  {
     float *Vf = reinterpret_cast<float *>(V), *Af = Vf + n2;
     for (int idx = tid; idx < n2; idx += blockDim.x) {
       Af[idx] = (float)(A[idx] * scale);
       Vf[idx] = idx % (n + 1) == 0 ? 1.f : 0.f;
     }
     __syncthreads();
-    jacobi_block_f32(n, Af, Vf, reinterpret_cast<float2 *>(cs), red);
+    if (n <= 64) jacobi_block_f32<1>(n, Af, reinterpret_cast<float *>(work), Vf, red);
+    else jacobi_block_f32<2>(n, Af, reinterpret_cast<float *>(work), Vf, red);
     __syncthreads();
-    double *W = work + n2;
+    double *W = reinterpret_cast<double *>(U2);
     for (int idx = tid; idx < n2; idx += blockDim.x) W[idx] = (double)Vf[idx];
+    for (int i = tid; i < n; i += blockDim.x) e1[i] = 1;  // |entries| of a rotation < 2
     __syncthreads();
-    cta_mm_tn(n, W, W, work);
+    cta_fix(n, n, true, e1, U1, col(W));
     __syncthreads();
-    // E in FP32 (E is about 1e-6: its square's FP32 rounding is below 1e-19)
-    for (int idx = tid; idx < n2; idx += blockDim.x) Vf[idx] = (float)(work[idx] - (idx % (n + 1) == 0 ? 1.0 : 0.0));
+    cta_fix_mm(n, n, n, U1, e1, U1, e1, [&](int i, int j, double v) { V[i + n * j] = v - (i == j ? 1.0 : 0.0); });
+    __syncthreads();
+    // E is about 1e-6: the FP32 rounding of its square is below 1e-18
+    float *Ef = reinterpret_cast<float *>(U1);
+    for (int idx = tid; idx < n2; idx += blockDim.x) Ef[idx] = (float)V[idx];
     __syncthreads();
     for (int j = w; j < n; j += nw)
       for (int i = lane; i < n; i += 32) {
         float s = 0.f;
-        for (int l = 0; l < n; ++l) s = fmaf(Vf[i + n * l], Vf[l + n * j], s);
-        const double d = i == j ? 1.0 : 0.0;
-        work[i + n * j] = d - 0.5 * (work[i + n * j] - d) + 0.375 * (double)s;
+#pragma unroll 4
+        for (int l = 0; l < n; ++l) s = fmaf(Ef[i + n * l], Ef[l + n * j], s);
+        V[i + (size_t)n * j] = (i == j ? 1.0 : 0.0) - 0.5 * V[i + (size_t)n * j] + 0.375 * (double)s;
       }
     __syncthreads();
-    cta_mm(n, n, n, W, work, V);
+    cta_fix(n, n, false, e1, U1, row(W));
     __syncthreads();
-    cta_mm(n, n, n, A, V, work);
+    cta_fix(n, n, true, e1, U2, col(V));
     __syncthreads();
-    cta_mm_tn(n, V, work, A);
+    cta_fix_mm(n, n, n, U1, e1, U2, e1, [&](int i, int j, double v) { V[i + n * j] = v; });
     __syncthreads();
-    // (V^T A V is symmetric but for the rounding of its two halves)
-    for (int j = w; j < n; j += nw)
-      for (int i = j + 1 + lane; i < n; i += 32) A[j + (size_t)n * i] = A[i + (size_t)n * j];
+    // A <- V^T (A V)
+    for (int i = tid; i < n; i += blockDim.x) e2[i] = 1;
+    cta_row_exp(n, n, A, n, 1, e1);
     __syncthreads();
+    cta_fix(n, n, true, e1, U1, col(A));
+    cta_fix(n, n, true, e2, U2, col(V));
+    __syncthreads();
+    cta_fix_mm(n, n, n, U1, e1, U2, e2, [&](int i, int j, double v) { A[i + n * j] = v; });
+    __syncthreads();
+    cta_row_exp(n, n, A, n, 1, e1);
+    __syncthreads();
+    cta_fix(n, n, true, e1, U1, col(A));
+    __syncthreads();
+    cta_fix_mm(n, n, n, U2, e2, U1, e1, [&](int i, int j, double v) { A[i + n * j] = v; });
+    mirror();
+  }
+  for (int step = 0; step < 2; ++step) {
+    const double off2 = off_norm2();
+    if (off2 <= stop2) return true;
+    constexpr double EMAX = 3e-4;
+    constexpr int EEXP = -11;  // EMAX < 2^EEXP
+    auto E = [&](int i, int j) {
+      const double a = A[i + (size_t)n * j], gap = A[j + (size_t)n * j] - A[i + (size_t)n * i];
+      const float x = (float)(a * scale), g = (float)(gap * scale);
+      return i != j && fabsf(x) <= (float)EMAX * fabsf(g) && g != 0.f ? (double)__fdividef(x, g) : 0.0;
+    };
+    for (int i = tid; i < n; i += blockDim.x) e1[i] = EEXP, e2[i] = 1;
+    __syncthreads();
+    cta_fix(n, n, true, e1, U2, [&](int r, int k) { return E(k, r); });  // the columns of E
+    __syncthreads();
+    double *P = reinterpret_cast<double *>(U1);
+    cta_fix_mm(n, n, n, U2, e1, U2, e1, [&](int i, int j, double v) {  // v = (E^T E)_ij = -(E^2)_ij
+      P[i + n * j] = (i == j ? 1.0 : 0.0) + E(i, j) - 0.5 * v;
+    });
+    __syncthreads();
+    cta_fix(n, n, true, e2, U2, col(P));  // the columns of P
+    __syncthreads();
+    for (int i = tid; i < n; i += blockDim.x) e1[i] = 1;
+    __syncthreads();
+    cta_fix(n, n, false, e1, U1, row(V));
+    __syncthreads();
+    cta_fix_mm(n, n, n, U1, e1, U2, e2, [&](int i, int j, double v) { V[i + n * j] = v; });
+    __syncthreads();
+    cta_row_exp(n, n, A, n, 1, e1);
+    __syncthreads();
+    cta_fix(n, n, true, e1, U1, col(A));
+    __syncthreads();
+    cta_fix_mm(n, n, n, U1, e1, U2, e2, [&](int i, int j, double v) { A[i + n * j] = v; });
+    __syncthreads();
+    cta_row_exp(n, n, A, n, 1, e1);
+    __syncthreads();
+    cta_fix(n, n, true, e1, U1, col(A));
+    __syncthreads();
+    cta_fix_mm(n, n, n, U2, e2, U1, e1, [&](int i, int j, double v) { A[i + n * j] = v; });
+    mirror();
   }
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
-    double off = 0.0;
-    for (int j = w; j < n; j += nw)
-      for (int i = j + 1 + lane; i < n; i += 32) off = fma(A[i + (size_t)n * j], A[i + (size_t)n * j], off);
-    off = 2.0 * jac_block_sum(off, red);
-    if (off <= stop2) return true;
+    if (off_norm2() <= stop2) return true;
     for (int r = 0; r < np - 1; ++r) {
       int any = 0;
       for (int k = tid; k < half; k += blockDim.x) {

@@ -29,12 +29,11 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(int n, double *__re
   const int b = blockIdx.x;
   const size_t n2 = (size_t)n * n;
   double *Ain = Ag + n2 * b, *A = sm, *V = sm + n2;
-  double *W = SMEM ? sm + 2 * n2 : work + 2 * n2 * b;  // 2 n^2 doubles of scratch
-  __shared__ double cs[2 * 512];  // (c, s) per pair of a round, n <= 1024
-  __shared__ double red[JAC_THREADS / 32];
+  double *W = SMEM ? sm + 2 * n2 : work + (size_t)jacobi_work(n) * b;
+  __shared__ double red[32];
   for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) A[idx] = Ain[idx];
   __syncthreads();
-  const bool ok = jacobi_block(n, A, V, cs, red, W, max_sweeps, tol);
+  const bool ok = jacobi_block(n, A, V, red, W, max_sweeps, tol);
   if (threadIdx.x == 0 && !ok) atomicExch(status, 1);
   jacobi_sorted_out(n, A, V, wg + (size_t)n * b, Vg + n2 * b);
 }
@@ -271,12 +270,12 @@ int syev_batched_device(mq_ctx *c, int n, int batch, double *d_A, double *d_w, d
     for (int b = 0; b < batch; ++b) MQ_TRY(syev_large_cold(c, n, d_A + n2 * b, d_w + (size_t)n * b, d_V + n2 * b));
     return MQ_OK;
   }
-  // A, V and the scratch in shared memory while 4 n^2 doubles fit (n <= 80);
-  // above, the scratch in global memory
-  const size_t mat2 = 2 * n2 * sizeof(double);
-  const bool smem_work = 2 * mat2 <= 205 * 1024;
-  const size_t smem = smem_work ? 2 * mat2 : mat2;
-  int *status = (int *)buf(c, "jacobi_work", 64 + (smem_work ? 0 : mat2 * batch));
+  // A, V and the scratch in shared memory while they fit (n <= 80); above, the
+  // scratch in global memory
+  const size_t mat2 = 2 * n2 * sizeof(double), wbytes = jacobi_work(n) * sizeof(double);
+  const bool smem_work = mat2 + wbytes <= 220 * 1024;
+  const size_t smem = smem_work ? mat2 + wbytes : mat2;
+  int *status = (int *)buf(c, "jacobi_work", 64 + (smem_work ? 0 : wbytes * batch));
   if (!status) return MQ_ENOMEM;
   MQ_CUDA(c, cudaMemsetAsync(status, 0, sizeof(int), c->stream));
   const int max_sweeps = 60;
