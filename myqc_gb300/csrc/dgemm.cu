@@ -3,15 +3,19 @@
 //
 // FP64 issue on this GPU is two multiply-adds per clock and SM, so the products
 // are formed on the tensor cores from fixed-point digits (fixmm.cuh), correct to
-// FP64 rounding or better.  A CTA forms a TM x TN tile of C: per chunk of up to
-// 128 of K it reads its rows of op(A) and columns of op(B) into registers,
-// finds their exponents, leaves them in shared memory as fixed-point pairs, and
-// each warp accumulates a 16 x 8 NT block of digit products; the chunk's sums
-// are rounded to FP64 and added over the chunks in FP64, in order.  Bound by
-// integer issue (cutting and recombining digits) and the tensor pipe.
+// FP64 rounding or better: 36 digit products per multiply-add at the 1024 per
+// clock and SM that mma.sync gives, 28 multiply-adds per clock and SM at best.
 //
-// Tiles of 64 x 64 serve products with enough of them to fill the SMs; others
-// take 32 x 32, which spread a product of order ~200 over more SMs.
+// A CTA of 8 warps forms 32 x 32 tiles of C: it reads 32 rows of op(A) and 32
+// columns of op(B) over up to 128 of K into registers, finds their exponents,
+// leaves them in shared memory as fixed-point pairs, and each warp accumulates a
+// 16 x 8 block of digit products.  Sums over more than one chunk of K are
+// rounded to FP64 per chunk and added in order.  Each CTA keeps the 32 columns
+// of the operand with fewer tiles and goes through tiles of the other (X), so
+// that the tall products of the four-index transform cut the small operand once
+// per CTA.  The small tile leaves two CTAs per SM, whose load and digit phases
+// run under each other's products, and spreads a product of order ~200 over
+// many SMs; larger tiles (64 x 64, one CTA per SM) were slower on both.
 //
 // A row or column with an infinity or NaN has no fixed-point form: its elements
 // of C are summed in FP64 from the operands as they are.
@@ -24,127 +28,124 @@ namespace mq {
 
 constexpr int GX_K = 128;          // K chunk (exact up to FX_KMAX)
 constexpr int GX_LD = GX_K / 2;    // pairs per row
+constexpr int GX_T = 32;           // tile
+constexpr int GX_THREADS = 256;
 constexpr int GX_BAD = 4000;       // exponent that marks a row with a non-finite element
 
-// TR rows of an operand's K chunk as fixed-point pairs.  ROWFAST: element (r, k)
-// at x[r + ld k], else at x[k + ld r]; nr rows and kc elements exist.  Leaves
-// the rows' exponents in e (fields: TR ints of scratch).
-template <int TR, bool ROWFAST, int THREADS>
+// The 32 rows of an operand's K chunk as fixed-point pairs.  ROWFAST: element
+// (r, k) at x[r + ld k], else at x[k + ld r]; nr rows and kc elements exist.
+// Leaves the rows' exponents in e (fields: scratch).
+template <bool ROWFAST>
 __device__ __forceinline__ void gx_load(const double *__restrict__ x, size_t ld, int nr, int kc, int *fields, int *e,
                                         uint4 *U) {
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int pairs = (kc + 15) / 16 * 8;
   auto put = [&](int r, int kp, double a, double b, int ex) {
     U[r * GX_LD + fx_pos(r, kp)] =
         ex == GX_BAD ? make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u) : fx_pair(fx_fix(a, ex), fx_fix(b, ex));
   };
   auto exponent = [](int f) { return f == 0x7ff ? GX_BAD : fx_exp(f); };
-  if (ROWFAST) {
-    constexpr int GR = THREADS / TR, PER = GX_K / GR;  // threads per row, elements per thread
-    const int r = tid % TR, k0 = (tid / TR) * PER;
-    if (tid < TR) fields[tid] = 0;
-    double v[PER];
+  if (ROWFAST) {  // lanes over the rows, warps over the pairs
+    constexpr int NW = GX_THREADS / 32, PER = GX_LD / NW;
+    if (tid < GX_T) fields[tid] = 0;
+    double v[PER][2];
     int f = 0;
 #pragma unroll
-    for (int i = 0; i < PER; ++i) v[i] = r < nr && k0 + i < kc ? x[r + ld * (k0 + i)] : 0.0;
+    for (int i = 0; i < PER; ++i) {
+      const int k = 2 * (w + NW * i);
+      v[i][0] = lane < nr && k < kc ? x[lane + ld * k] : 0.0;
+      v[i][1] = lane < nr && k + 1 < kc ? x[lane + ld * (k + 1)] : 0.0;
+    }
 #pragma unroll
-    for (int i = 0; i < PER; ++i) f = max(f, fx_field(v[i]));
+    for (int i = 0; i < PER; ++i) f = max(f, max(fx_field(v[i][0]), fx_field(v[i][1])));
     __syncthreads();
-    if (f) atomicMax(fields + r, f);
+    if (f) atomicMax(fields + lane, f);
     __syncthreads();
-    const int ex = exponent(fields[r]);
-    if (tid < TR) e[tid] = ex;
+    const int ex = exponent(fields[lane]);
+    if (w == 0) e[lane] = ex;
 #pragma unroll
-    for (int i = 0; i < PER; i += 2) put(r, (k0 + i) / 2, v[i], v[i + 1], ex);
-  } else {
-    const int lane = tid & 31, w = tid >> 5;
-    constexpr int NW = THREADS / 32;
-#pragma unroll 4
-    for (int r = w; r < TR; r += NW) {
-      double v[4];
+    for (int i = 0; i < PER; ++i)
+      if (w + NW * i < pairs) put(lane, w + NW * i, v[i][0], v[i][1], ex);
+  } else {  // a warp per row
+    constexpr int PER = GX_T / (GX_THREADS / 32);
+    double v[PER][4];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int r = w * PER + j;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int k = 2 * lane + (i & 1) + 64 * (i >> 1);
-        v[i] = r < nr && k < kc ? x[k + ld * r] : 0.0;
+        v[j][i] = r < nr && k < kc ? x[k + ld * r] : 0.0;
       }
-      const int f = max(max(fx_field(v[0]), fx_field(v[1])), max(fx_field(v[2]), fx_field(v[3])));
+    }
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int r = w * PER + j;
+      const int f = max(max(fx_field(v[j][0]), fx_field(v[j][1])), max(fx_field(v[j][2]), fx_field(v[j][3])));
       const int ex = exponent(__reduce_max_sync(0xffffffffu, f));
       if (lane == 0) e[r] = ex;
-      put(r, lane, v[0], v[1], ex);
-      put(r, lane + 32, v[2], v[3], ex);
+      if (lane < pairs) put(r, lane, v[j][0], v[j][1], ex);
+      if (lane + 32 < pairs) put(r, lane + 32, v[j][2], v[j][3], ex);
     }
   }
 }
 
-template <int TM, int TN, bool TA, bool TB>
-__global__ void __launch_bounds__(TM * 4) dgemm_kernel(int m, int n, int k, double alpha, const double *__restrict__ A,
-                                                       int lda, long long sA, const double *__restrict__ B, int ldb,
-                                                       long long sB, double beta, double *__restrict__ C, int ldc,
-                                                       long long sC) {
-  constexpr int THREADS = TM * 4, WM = TM / 16, WN = THREADS / 32 / WM, NT = TN / WN / 8;
+// C(r, c) at C[r sr + c sc]: rows r < mx of X, columns c < ny of Y
+template <bool XROW, bool YROW>
+__global__ void __launch_bounds__(GX_THREADS, 2) dgemm_kernel(int mx, int ny, int k, double alpha,
+                                                              const double *__restrict__ X, size_t ldx, long long sX,
+                                                              const double *__restrict__ Y, size_t ldy, long long sY,
+                                                              double beta, double *__restrict__ C, size_t sr,
+                                                              size_t sc, long long sC) {
   extern __shared__ __align__(16) unsigned char gx_smem[];
-  uint4 *UA = reinterpret_cast<uint4 *>(gx_smem), *UB = UA + TM * GX_LD;
-  __shared__ int fields[TM + TN], ea[TM], eb[TN];
-  const int tiles_m = (m + TM - 1) / TM;
-  const int r0 = (int)(blockIdx.x % tiles_m) * TM, c0 = (int)(blockIdx.x / tiles_m) * TN;
-  A += sA * blockIdx.z;  // the batch's operands
-  B += sB * blockIdx.z;
+  uint4 *UX = reinterpret_cast<uint4 *>(gx_smem), *UY = UX + GX_T * GX_LD;
+  __shared__ int fields[2 * GX_T], ex[GX_T], ey[GX_T];
+  const int tiles = (mx + GX_T - 1) / GX_T, c0 = blockIdx.y * GX_T;
+  X += sX * blockIdx.z;  // the batch's operands
+  Y += sY * blockIdx.z;
   C += sC * blockIdx.z;
-  const double *Ar = TA ? A + (size_t)lda * r0 : A + r0, *Bc = TB ? B + c0 : B + (size_t)ldb * c0;
+  const double *Yc = Y + (YROW ? (size_t)c0 : ldy * c0);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const int wr = (w % WM) * 16, wc = (w / WM) * (8 * NT);
-  double sum[NT][4];
-  for (int kb = 0; kb < k || kb == 0; kb += GX_K) {
-    const int kc = min(GX_K, k - kb);
-    if (kb) __syncthreads();  // the previous chunk's operands have been read
-    gx_load<TM, !TA, THREADS>(TA ? Ar + kb : Ar + (size_t)lda * kb, lda, min(TM, m - r0), kc, fields, ea, UA);
-    gx_load<TN, TB, THREADS>(TB ? Bc + (size_t)ldb * kb : Bc + kb, ldb, min(TN, n - c0), kc, fields + TM, eb, UB);
-    __syncthreads();
-    float acc[NT][FX_DIG][4];
-    fx_tile<NT>(UA, UB, GX_LD, TM, TN, wr, wc, (kc + 15) / 16, acc);
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
+  const int wr = (w & 1) * 16, wc = (w >> 1) * 8;
+  const bool one = k <= GX_K;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int r0 = tile * GX_T;
+    const double *Xr = X + (XROW ? (size_t)r0 : ldx * r0);
+    double sum[4];
+    for (int kb = 0; kb < k || kb == 0; kb += GX_K) {
+      const int kc = min(GX_K, k - kb);
+      __syncthreads();  // the previous operands have been read
+      gx_load<XROW>(Xr + (XROW ? ldx * kb : (size_t)kb), ldx, min(GX_T, mx - r0), kc, fields, ex, UX);
+      if (!one || tile == (int)blockIdx.x)
+        gx_load<YROW>(Yc + (YROW ? ldy * kb : (size_t)kb), ldy, min(GX_T, ny - c0), kc, fields + GX_T, ey, UY);
+      __syncthreads();
+      float acc[1][FX_DIG][4];
+      fx_tile<1>(UX, UY, GX_LD, GX_T, GX_T, wr, wc, (kc + 15) / 16, acc);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int r = wr + g + 8 * (i >> 1), c = wc + 8 * j + 2 * t + (i & 1);
-        double x;
-        if (ea[r] != GX_BAD && eb[c] != GX_BAD) {
+        const int r = wr + g + 8 * (i >> 1), c = wc + 2 * t + (i & 1);
+        double x = 0.0;
+        if (ex[r] != GX_BAD && ey[c] != GX_BAD) {
           float v[FX_DIG];
 #pragma unroll
-          for (int L = 0; L < FX_DIG; ++L) v[L] = acc[j][L][i];
-          x = fx_combine(v, ea[r], eb[c]);
-        } else {
-          x = 0.0;
-          if (r0 + r < m && c0 + c < n) for (int l = kb; l < kb + kc; ++l)
-            x = fma(TA ? A[l + (size_t)lda * (r0 + r)] : A[r0 + r + (size_t)lda * l],
-                    TB ? B[c0 + c + (size_t)ldb * l] : B[l + (size_t)ldb * (c0 + c)], x);
+          for (int L = 0; L < FX_DIG; ++L) v[L] = acc[0][L][i];
+          x = fx_combine(v, ex[r], ey[c]);
+        } else if (r0 + r < mx && c0 + c < ny) {
+          for (int l = kb; l < kb + kc; ++l)
+            x = fma(Xr[XROW ? r + ldx * l : l + ldx * r], Yc[YROW ? c + ldy * l : l + ldy * c], x);
         }
-        sum[j][i] = kb ? sum[j][i] + x : x;
+        sum[i] = kb ? sum[i] + x : x;
       }
-  }
-#pragma unroll
-  for (int j = 0; j < NT; ++j)
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int r = r0 + wr + g + 8 * (i >> 1), c = c0 + wc + 8 * j + 2 * t + (i & 1);
-      if (r >= m || c >= n) continue;
-      double *cp = C + r + (size_t)ldc * c;
-      const double x = alpha == 1.0 ? sum[j][i] : alpha * sum[j][i];
+      const int r = r0 + wr + g + 8 * (i >> 1), c = c0 + wc + 2 * t + (i & 1);
+      if (r >= mx || c >= ny) continue;
+      double *cp = C + sr * r + sc * c;
+      const double x = alpha == 1.0 ? sum[i] : alpha * sum[i];
       *cp = beta == 0.0 ? x : fma(beta, *cp, x);
     }
-}
-
-template <int TM, int TN>
-static int launch_gemm(mq_ctx *c, bool TA, bool TB, dim3 grid, int m, int n, int k, double alpha, const double *A,
-                       int lda, long long sA, const double *B, int ldb, long long sB, double beta, double *C, int ldc,
-                       long long sC) {
-  const size_t sm = sizeof(uint4) * (TM + TN) * GX_LD;
-  auto kern = TA ? (TB ? dgemm_kernel<TM, TN, true, true> : dgemm_kernel<TM, TN, true, false>)
-                 : (TB ? dgemm_kernel<TM, TN, false, true> : dgemm_kernel<TM, TN, false, false>);
-  MQ_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  kern<<<grid, TM * 4, sm, c->stream>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC);
-  c->stats.launches += 1;
-  MQ_CUDA(c, cudaGetLastError());
-  return MQ_OK;
+  }
 }
 
 int dgemm_batched(mq_ctx *c, char ta, char tb, int m, int n, int k, double alpha, const double *A, int lda,
@@ -155,14 +156,25 @@ int dgemm_batched(mq_ctx *c, char ta, char tb, int m, int n, int k, double alpha
   const bool TA = ta == 'T' || ta == 't', TB = tb == 'T' || tb == 't';
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-  auto tiles = [&](long long tm, long long tn) { return ((m + tm - 1) / tm) * ((n + tn - 1) / tn); };
-  if (tiles(32, 32) > 2147483647LL) return set_err(c, MQ_EINVAL, "dgemm: too many output tiles");
-  const long long t64 = tiles(64, 64);
-  if (n > 32 && t64 * batch >= 2 * sms)
-    return launch_gemm<64, 64>(c, TA, TB, dim3((unsigned)t64, 1, batch), m, n, k, alpha, A, lda, sA, B, ldb, sB, beta,
-                               C, ldc, sC);
-  return launch_gemm<32, 32>(c, TA, TB, dim3((unsigned)tiles(32, 32), 1, batch), m, n, k, alpha, A, lda, sA, B, ldb, sB,
-                             beta, C, ldc, sC);
+  // X: the operand with more tiles
+  const bool swap = n > m;
+  const int mx = swap ? n : m, ny = swap ? m : n;
+  const bool xrow = swap ? TB : !TA, yrow = swap ? !TA : TB;
+  const int xt = (mx + GX_T - 1) / GX_T, yt = (ny + GX_T - 1) / GX_T;
+  if (yt > 65535) return set_err(c, MQ_EINVAL, "dgemm: too many output tiles");
+  // a few waves of two CTAs per SM, each with as many tiles of X as that leaves
+  const long long want = std::max<long long>(1, (8LL * sms + (long long)yt * batch - 1) / ((long long)yt * batch));
+  const dim3 grid((unsigned)std::min<long long>(xt, want), yt, batch);
+  const size_t sm = sizeof(uint4) * 2 * GX_T * GX_LD;
+  auto kern = xrow ? (yrow ? dgemm_kernel<true, true> : dgemm_kernel<true, false>)
+                   : (yrow ? dgemm_kernel<false, true> : dgemm_kernel<false, false>);
+  MQ_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  kern<<<grid, GX_THREADS, sm, c->stream>>>(mx, ny, k, alpha, swap ? B : A, swap ? ldb : lda, swap ? sB : sA,
+                                            swap ? A : B, swap ? lda : ldb, swap ? sA : sB, beta, C, swap ? ldc : 1,
+                                            swap ? 1 : ldc, sC);
+  c->stats.launches += 1;
+  MQ_CUDA(c, cudaGetLastError());
+  return MQ_OK;
 }
 
 }  // namespace mq
