@@ -30,6 +30,8 @@ enum { EPI_BIAS_ACT = 0, EPI_BIAS = 1, EPI_DACT = 2, EPI_F32 = 3 };
 
 struct MlpGemm {
   int M, N, K, batch, ntile, tmem_cols, b_batched;
+  int ntn;                 // column tiles of ntile
+  int vec;                 // N and the leading dimensions allow 16-byte accesses
   const float *bias;       // [N]
   const float *zin;        // EPI_DACT: z of this layer's input, [M][ldz]
   float *zout;             // EPI_BIAS_ACT: z, [M][ldz]
@@ -61,8 +63,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) mlp_gemm_kernel(const __grid_
   uint32_t *tmem_slot = (uint32_t *)(drain + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int mtiles = (g.M + UM - 1) / UM;
-  const long long ntiles = (long long)mtiles * g.batch;
+  const long long ntiles = (long long)mtiles * g.ntn * g.batch;
   const int kchunks = (g.K + UK - 1) / UK;
+  // tile t: column tile fastest (the CTAs of one row tile share its A in L2)
+  auto tile = [&](long long t, int &mt, int &nt, int &bt) {
+    nt = (int)(t % g.ntn);
+    t /= g.ntn;
+    mt = (int)(t % mtiles);
+    bt = (int)(t / mtiles);
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -92,13 +101,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) mlp_gemm_kernel(const __grid_
       uint32_t ph = 1;
       unsigned armed = 0, armed_par = 0;
       for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int mt = (int)(t % mtiles), bt = (int)(t / mtiles);
+        int mt, nt, bt;
+        tile(t, mt, nt, bt);
         for (int kc = 0; kc < kchunks; ++kc) {
           if (!mbar_wait(empty + s, ph, g.err)) goto prod_exit;
           uint8_t *st = smem + s * stage_bytes;
           mbar_expect_tx(full + s, stage_bytes);
           tma_load_3d(st, &maps.a, full + s, kc * UK, mt * UM, bt);
-          tma_load_3d(st + a_bytes, &maps.b, full + s, kc * UK, 0, g.b_batched ? bt : 0);
+          tma_load_3d(st + a_bytes, &maps.b, full + s, kc * UK, nt * ntile, g.b_batched ? bt : 0);
           armed |= 1u << s;
           armed_par = (armed_par & ~(1u << s)) | ((ph ^ 1u) << s);
           if (++s == STAGES) {
@@ -150,7 +160,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) mlp_gemm_kernel(const __grid_
     const int row = q * 32 + lane;
     uint32_t acc_ph = 0;
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-      const int mt = (int)(t % mtiles), bt = (int)(t / mtiles);
+      int mt, nt, bt;
+      tile(t, mt, nt, bt);
       int ok = 0;
       if (lane == 0) ok = mbar_wait(acc_full, acc_ph, g.err);
       ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -162,10 +173,53 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) mlp_gemm_kernel(const __grid_
       for (int c0 = 0; c0 < ntile; c0 += 16) {
         float v[16];
         tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
-        if (!live) continue;
+        const int n0 = nt * ntile + c0;
+        if (!live || n0 >= g.N) continue;
+        if (g.vec) {  // 16 whole columns: 16-byte accesses
+          float z[16];
+          if (EPI == EPI_BIAS_ACT || EPI == EPI_BIAS) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+              const float4 b4 = __ldg(reinterpret_cast<const float4 *>(g.bias + n0 + i));
+              z[i] = v[i] + b4.x, z[i + 1] = v[i + 1] + b4.y, z[i + 2] = v[i + 2] + b4.z, z[i + 3] = v[i + 3] + b4.w;
+            }
+          } else if (EPI == EPI_DACT) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+              const float4 z4 = __ldg(reinterpret_cast<const float4 *>(g.zin + m * g.ldz + n0 + i));
+              z[i] = z4.x, z[i + 1] = z4.y, z[i + 2] = z4.z, z[i + 3] = z4.w;
+            }
+          }
+          if (EPI == EPI_BIAS || EPI == EPI_F32 || EPI == EPI_BIAS_ACT) {
+            float *o = EPI == EPI_BIAS_ACT ? g.zout + m * g.ldz + n0
+                                           : g.out32 + (EPI == EPI_F32 ? (long long)bt * g.s_b : 0) + m * g.ldo + n0;
+#pragma unroll
+            for (int i = 0; i < 16; i += 4)
+              *reinterpret_cast<float4 *>(o + i) = EPI == EPI_F32 ? make_float4(v[i], v[i + 1], v[i + 2], v[i + 3])
+                                                                  : make_float4(z[i], z[i + 1], z[i + 2], z[i + 3]);
+          }
+          if (EPI == EPI_BIAS_ACT || EPI == EPI_DACT) {
+            unsigned p[8];
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              float y[2];
+#pragma unroll
+              for (int k = 0; k < 2; ++k) {
+                const float zz = z[i + k], sg = sigm(zz);
+                y[k] = EPI == EPI_BIAS_ACT ? zz * sg : v[i + k] * sg * (1.0f + zz * (1.0f - sg));
+              }
+              const __nv_bfloat162 b2 = __floats2bfloat162_rn(y[0], y[1]);
+              p[i / 2] = *reinterpret_cast<const unsigned *>(&b2);
+            }
+            uint4 *o = reinterpret_cast<uint4 *>(g.out16 + m * g.ldo + n0);
+            o[0] = make_uint4(p[0], p[1], p[2], p[3]);
+            o[1] = make_uint4(p[4], p[5], p[6], p[7]);
+          }
+          continue;
+        }
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const int n = c0 + i;
+          const int n = n0 + i;
           if (n >= g.N) break;
           if (EPI == EPI_BIAS_ACT) {
             const float z = v[i] + g.bias[n];
@@ -196,21 +250,28 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) mlp_gemm_kernel(const __grid_
 }
 
 // ---------------------------------------------------------------- pointwise
-// src (rows x cols, leading dimension lds) -> dst in chunk-major transposed
-// layout: sample s, column c at (s / kc) * cols * kc + c * kc + s % kc, so that
-// each chunk of kc samples is a contiguous cols x kc K-major operand
-__global__ void transpose_chunked_kernel(const bf16 *__restrict__ src, int rows, int cols, int lds, int kc,
-                                         bf16 *__restrict__ dst) {
+// The six operands of the weight gradients, src (rows x cols, leading dimension
+// lds), in chunk-major transposed layout: sample s, column c at
+// (s / kc) * cols * kc + c * kc + s % kc, so that each chunk of kc samples is a
+// contiguous cols x kc K-major operand.  blockIdx.z: operand.
+struct Transposes {
+  const bf16 *src[6];
+  bf16 *dst[6];
+  int cols[6], lds[6];
+  int rows, kc;
+};
+__global__ void transpose_chunked_kernel(Transposes a) {
   __shared__ bf16 tile[32][33];
-  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+  const int z = blockIdx.z, r0 = blockIdx.y * 32, c0 = blockIdx.x * 32, cols = a.cols[z];
+  if (c0 >= cols) return;
   for (int i = threadIdx.y; i < 32; i += blockDim.y) {
     const int r = r0 + i, c = c0 + threadIdx.x;
-    tile[i][threadIdx.x] = (r < rows && c < cols) ? src[(size_t)r * lds + c] : __float2bfloat16_rn(0.f);
+    tile[i][threadIdx.x] = (r < a.rows && c < cols) ? a.src[z][(size_t)r * a.lds[z] + c] : __float2bfloat16_rn(0.f);
   }
   __syncthreads();
   for (int i = threadIdx.y; i < 32; i += blockDim.y) {
     const int c = c0 + i, r = r0 + threadIdx.x;
-    if (c < cols && r < rows) dst[(size_t)(r / kc) * cols * kc + (size_t)c * kc + r % kc] = tile[threadIdx.x][i];
+    if (c < cols && r < a.rows) a.dst[z][(size_t)(r / a.kc) * cols * a.kc + (size_t)c * a.kc + r % a.kc] = tile[threadIdx.x][i];
   }
 }
 
@@ -227,7 +288,8 @@ __global__ void to_bf16_kernel(const float *__restrict__ src, long long rows, in
 // rows of src picked by idx -> dst (dataset minibatch gather)
 __global__ void gather_rows_kernel(const bf16 *__restrict__ src, const float *__restrict__ t,
                                    const float *__restrict__ w, const int *__restrict__ idx, int rows, int ld_in,
-                                   int nout, bf16 *__restrict__ xb, float *__restrict__ tb, float *__restrict__ wb) {
+                                   int nout, bf16 *__restrict__ xb, float *__restrict__ tb, float *__restrict__ wb,
+                                   double *__restrict__ wrow) {
   const int r = blockIdx.x;
   if (r >= rows) return;
   const long long s = idx[r];
@@ -236,14 +298,43 @@ __global__ void gather_rows_kernel(const bf16 *__restrict__ src, const float *__
     tb[(size_t)r * nout + c] = t[s * nout + c];
     wb[(size_t)r * nout + c] = w[s * nout + c];
   }
+  if (threadIdx.x < 32) {  // the row's loss weight
+    double v = 0.0;
+    for (int c = threadIdx.x; c < nout; c += 32) v += w[s * nout + c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (threadIdx.x == 0) wrow[r] = v;
+  }
+}
+
+// sums of n doubles (one CTA, fixed order): scal[0] <- the sum, at least 0 and 1
+// if it is 0 (a minibatch's weight); or, with the weight in scal[0],
+// scal[1] += sum / scal[0] (its loss)
+__global__ void __launch_bounds__(1024) scalar_sum_kernel(const double *__restrict__ v, int n, int is_loss,
+                                                          double *__restrict__ scal) {
+  __shared__ double red[32];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) s += v[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  s = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (threadIdx.x) return;
+  if (is_loss) scal[1] += s / scal[0];
+  else scal[0] = s > 0.0 ? s : 1.0;
 }
 
 // weighted squared error: loss partials per block; dy = 2 w (y - t) / wsum as
 // BF16 rows of width ldd (zero padded)
 __global__ void loss_kernel(const float *__restrict__ y, const float *__restrict__ t, const float *__restrict__ w,
-                            int rows, int nout, float inv_wsum, bf16 *__restrict__ dy, int ldd,
+                            int rows, int nout, const double *__restrict__ wsum, bf16 *__restrict__ dy, int ldd,
                             double *__restrict__ partial) {
   __shared__ double red[32];
+  const float inv_wsum = (float)(1.0 / wsum[0]);
   double acc = 0.0;
   const long long total = (long long)rows * ldd;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -269,59 +360,76 @@ __global__ void loss_kernel(const float *__restrict__ y, const float *__restrict
   }
 }
 
-// column sums of a BF16 [rows][ld] matrix (bias gradient), one block per column
-__global__ void colsum_kernel(const bf16 *__restrict__ a, int rows, int ld, float *__restrict__ out) {
-  __shared__ float red[32];
-  const int c = blockIdx.x;
+// The three layers' gradients: weight gradients as the sums of their K-chunk
+// partials (fixed order) and bias gradients as the column sums of the
+// chunk-major transposes of dz (rows beyond the batch excluded).  blockIdx.y:
+// layer; the first `wblocks` blocks of a layer serve weights, the others one
+// bias entry each.
+struct GradSums {
+  const float *part[3];
+  float *gW[3], *gb[3];
+  const bf16 *t_dz[3];
+  int nout[3];
+  long long nw[3];
+  int nchunk, kc, rows, wblocks;
+};
+__global__ void __launch_bounds__(256) grad_sum_kernel(GradSums a) {
+  const int l = blockIdx.y;
+  if ((int)blockIdx.x < a.wblocks) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.nw[l]) return;
+    float s = 0.f;
+    for (int b = 0; b < a.nchunk; ++b) s += a.part[l][b * a.nw[l] + i];
+    a.gW[l][i] = s;
+    return;
+  }
+  __shared__ float red[8];
+  const int c = (int)blockIdx.x - a.wblocks;
+  if (c >= a.nout[l]) return;
   float s = 0.f;
-  for (int r = threadIdx.x; r < rows; r += blockDim.x) s += __bfloat162float(a[(size_t)r * ld + c]);
+  for (int r = threadIdx.x; r < a.rows; r += blockDim.x)
+    s += __bfloat162float(a.t_dz[l][((size_t)(r / a.kc) * a.nout[l] + c) * a.kc + r % a.kc]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
     float t = 0.f;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += red[k];
-    out[c] = t;
+    for (int k = 0; k < 8; ++k) t += red[k];
+    a.gb[l][c] = t;
   }
 }
 
-// out[i] = sum_b part[b][i] (fixed order)
-__global__ void chunk_sum_kernel(const float *__restrict__ part, int nchunk, long long stride, long long n,
-                                 float *__restrict__ out) {
+// Adam on the three layers (blockIdx.y): W (nout x nin, FP32 master), b; writes
+// BF16 W [nout][ldw] and W^T [nin][ldt] (zero padding beyond the real sizes is
+// left as set up)
+struct AdamLayers {
+  float *W[3], *mW[3], *vW[3], *b[3], *mb[3], *vb[3];
+  const float *gW[3], *gb[3];
+  bf16 *Wb[3], *Wt[3];
+  int nout[3], nin[3], ldw[3], ldt[3];
+};
+__global__ void adam_kernel(AdamLayers a, float lr, float b1, float b2, float eps, float c1, float c2) {
+  const int l = blockIdx.y;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float s = 0.f;
-  for (int b = 0; b < nchunk; ++b) s += part[b * stride + i];
-  out[i] = s;
-}
-
-// Adam on one layer: W (nout x nin, FP32 master), b; writes BF16 W [nout][ldw]
-// and W^T [nin][ldt] (zero padding beyond the real sizes is left as set up)
-__global__ void adam_kernel(float *__restrict__ W, float *__restrict__ mW, float *__restrict__ vW,
-                            const float *__restrict__ gW, int nout, int nin, float *__restrict__ b,
-                            float *__restrict__ mb, float *__restrict__ vb, const float *__restrict__ gb, float lr,
-                            float b1, float b2, float eps, float c1, float c2, bf16 *__restrict__ Wb, int ldw,
-                            bf16 *__restrict__ Wt, int ldt) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long nw = (long long)nout * nin;
+  const long long nw = (long long)a.nout[l] * a.nin[l];
   if (i < nw) {
-    const float g = gW[i];
-    const float m = b1 * mW[i] + (1.f - b1) * g, v = b2 * vW[i] + (1.f - b2) * g * g;
-    mW[i] = m;
-    vW[i] = v;
-    const float w = W[i] - lr * (m * c1) / (sqrtf(v * c2) + eps);
-    W[i] = w;
-    const int o = (int)(i / nin), k = (int)(i % nin);
-    Wb[(size_t)o * ldw + k] = __float2bfloat16_rn(w);
-    Wt[(size_t)k * ldt + o] = __float2bfloat16_rn(w);
-  } else if (i < nw + nout) {
+    const float g = a.gW[l][i];
+    const float m = b1 * a.mW[l][i] + (1.f - b1) * g, v = b2 * a.vW[l][i] + (1.f - b2) * g * g;
+    a.mW[l][i] = m;
+    a.vW[l][i] = v;
+    const float w = a.W[l][i] - lr * (m * c1) / (sqrtf(v * c2) + eps);
+    a.W[l][i] = w;
+    const int o = (int)(i / a.nin[l]), k = (int)(i % a.nin[l]);
+    a.Wb[l][(size_t)o * a.ldw[l] + k] = __float2bfloat16_rn(w);
+    a.Wt[l][(size_t)k * a.ldt[l] + o] = __float2bfloat16_rn(w);
+  } else if (i < nw + a.nout[l]) {
     const int o = (int)(i - nw);
-    const float g = gb[o];
-    const float m = b1 * mb[o] + (1.f - b1) * g, v = b2 * vb[o] + (1.f - b2) * g * g;
-    mb[o] = m;
-    vb[o] = v;
-    b[o] -= lr * (m * c1) / (sqrtf(v * c2) + eps);
+    const float g = a.gb[l][o];
+    const float m = b1 * a.mb[l][o] + (1.f - b1) * g, v = b2 * a.vb[l][o] + (1.f - b2) * g * g;
+    a.mb[l][o] = m;
+    a.vb[l][o] = v;
+    a.b[l][o] -= lr * (m * c1) / (sqrtf(v * c2) + eps);
   }
 }
 
@@ -367,7 +475,18 @@ template <int EPI>
 static int mlp_gemm(mq_ctx *c, const GemmOperand &A, const GemmOperand &B, MlpGemm g) {
   if (g.N <= 0 || g.M <= 0) return MQ_OK;
   if (g.N > 256) return set_err(c, MQ_EINVAL, "MLP GEMM: N > 256");
+  // Column tiles: the whole width while the row tiles fill the SMs, else 64
+  // columns, so that a minibatch's products (32 row tiles at 4096 samples)
+  // spread over the chip and each epilogue warp has a quarter of the columns.
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+  const long long rowtiles = (long long)((g.M + UM - 1) / UM) * A.batch;
   g.ntile = (g.N + 15) / 16 * 16;
+  if (rowtiles < sms && g.ntile > 64) g.ntile = 64;
+  g.ntn = (g.N + g.ntile - 1) / g.ntile;
+  auto al16 = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
+  g.vec = g.N % 16 == 0 && al16(g.bias) && al16(g.zin) && al16(g.zout) && al16(g.out32) && al16(g.out16) &&
+          g.ldz % 4 == 0 && g.ldo % 8 == 0 && g.s_b % 4 == 0;
   MlpMaps maps;
   MQ_TRY(map_general(c, &maps.a, A.ptr, A.kdim, A.rows, A.row_stride, A.batch, A.batch_stride, UM));
   MQ_TRY(map_general(c, &maps.b, B.ptr, B.kdim, B.rows, B.row_stride, B.batch, B.batch_stride, g.ntile));
@@ -381,10 +500,7 @@ static int mlp_gemm(mq_ctx *c, const GemmOperand &A, const GemmOperand &B, MlpGe
   const size_t limit = 227 * 1024 - 1024 - 256;
   const int stages = limit >= 4 * stage ? 4 : (limit >= 3 * stage ? 3 : 2);
   const size_t smem = stages * stage + 1024 + 256;
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-  const long long tiles = (long long)(g.M + UM - 1) / UM * g.batch;
-  const int grid = (int)std::min<long long>(tiles, sms);
+  const int grid = (int)std::min<long long>(rowtiles * g.ntn, sms);
   auto kern = stages == 4 ? mlp_gemm_kernel<EPI, 4> : (stages == 3 ? mlp_gemm_kernel<EPI, 3> : mlp_gemm_kernel<EPI, 2>);
   MQ_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<grid, GEMM_THREADS, smem, c->stream>>>(maps, g);
@@ -497,10 +613,11 @@ int mlp_get_params(mq_ctx *c, float *h) {
 // (rows rounded up to the split-K chunk, zero beyond `rows`), FP32 z and
 // outputs, and scratch for split-K and loss partials.
 constexpr int KCHUNK = 2048;
+constexpr int LOSS_BLOCKS = 256;
 struct Acts {
   bf16 *x, *y1, *y2, *dy3, *dz2, *dz1, *t_x, *t_y1, *t_y2, *t_dy3, *t_dz2, *t_dz1;
-  float *z1, *z2, *out, *part32;
-  double *loss_part;
+  float *z1, *z2, *out, *part32[3];
+  double *loss_part, *wrow, *scal;  // loss partials (LOSS_BLOCKS), row weights, sums (weight, loss)
   int rows, rp;  // rp: rows rounded up to KCHUNK
   size_t t_elems;
 };
@@ -516,10 +633,10 @@ static int acts_alloc(mq_ctx *c, Mlp *m, int rows, Acts &a) {
   a.t_elems = Rp * (size_t)(d0 + d1 + d2 + d3 + d2 + d1);
   bf16 *b = (bf16 *)buf(c, "mlp_acts16", (rowmajor + a.t_elems) * sizeof(bf16) + 256);
   const size_t nchunk = Rp / KCHUNK;
-  size_t maxw = 0;
-  for (int l = 0; l < 3; ++l) maxw = std::max(maxw, (size_t)m->d[l + 1] * m->d[l]);
-  float *f = (float *)buf(c, "mlp_acts32", (R * (size_t)(d1 + d2 + d3) + nchunk * maxw) * sizeof(float) +
-                                               512 * sizeof(double) + 256);
+  size_t sumw = 0;
+  for (int l = 0; l < 3; ++l) sumw += ((size_t)m->d[l + 1] * m->d[l] + 3) / 4 * 4;
+  float *f = (float *)buf(c, "mlp_acts32", (R * (size_t)(d1 + d2 + d3) + 16 + nchunk * sumw) * sizeof(float) +
+                                               (LOSS_BLOCKS + R + 2) * sizeof(double) + 256);
   if (!b || !f) return MQ_ENOMEM;
   MQ_CUDA(c, cudaMemsetAsync(b, 0, rowmajor * sizeof(bf16), c->stream));  // K padding columns stay zero
   a.x = b;
@@ -538,8 +655,11 @@ static int acts_alloc(mq_ctx *c, Mlp *m, int rows, Acts &a) {
   a.z1 = f;
   a.z2 = a.z1 + R * d1;
   a.out = a.z2 + R * d2;
-  a.loss_part = (double *)(a.out + R * d3 + (R * d3) % 2);
-  a.part32 = (float *)(a.loss_part + 512);
+  a.loss_part = (double *)(a.out + (R * d3 + 3) / 4 * 4);
+  a.wrow = a.loss_part + LOSS_BLOCKS;
+  a.scal = a.wrow + R;
+  a.part32[0] = (float *)(a.scal + 2);
+  for (int l = 1; l < 3; ++l) a.part32[l] = a.part32[l - 1] + nchunk * (((size_t)m->d[l] * m->d[l - 1] + 3) / 4 * 4);
   return MQ_OK;
 }
 
@@ -574,18 +694,9 @@ static int forward(mq_ctx *c, Mlp *m, Acts &a) {
   return MQ_OK;
 }
 
-static int transpose(mq_ctx *c, const bf16 *src, int rows, int cols, int lds, bf16 *dst) {
-  dim3 grid((cols + 31) / 32, (rows + 31) / 32), block(32, 8);
-  transpose_chunked_kernel<<<grid, block, 0, c->stream>>>(src, rows, cols, lds, KCHUNK, dst);
-  c->stats.launches += 1;
-  MQ_CUDA(c, cudaGetLastError());
-  return MQ_OK;
-}
-
 // dW[l] = dZ^T Y (split-K over chunks of KCHUNK samples, one batch entry per
-// chunk of the chunk-major transposes), db[l] = column sums of dZ
-static int weight_grad(mq_ctx *c, Mlp *m, int l, const bf16 *t_dz, const bf16 *t_y, const bf16 *dz, int ld_dz, int R,
-                       int Rp, float *part) {
+// chunk of the chunk-major transposes)
+static int weight_grad(mq_ctx *c, Mlp *m, int l, const bf16 *t_dz, const bf16 *t_y, int Rp, float *part) {
   const int nout = m->d[l + 1], nin = m->d[l];
   const int nchunk = Rp / KCHUNK;
   MlpGemm g{};
@@ -595,26 +706,29 @@ static int weight_grad(mq_ctx *c, Mlp *m, int l, const bf16 *t_dz, const bf16 *t
   g.out32 = part;
   g.ldo = nin;
   g.s_b = (long long)nout * nin;
-  MQ_TRY(mlp_gemm<EPI_F32>(c, {t_dz, KCHUNK, nout, KCHUNK, nchunk, (long long)nout * KCHUNK},
-                           {t_y, KCHUNK, nin, KCHUNK, nchunk, (long long)nin * KCHUNK}, g));
-  const long long n = (long long)nout * nin;
-  chunk_sum_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(part, nchunk, n, n, m->gW[l]);
-  colsum_kernel<<<nout, 256, 0, c->stream>>>(dz, R, ld_dz, m->gb[l]);
-  c->stats.launches += 2;
-  MQ_CUDA(c, cudaGetLastError());
+  return mlp_gemm<EPI_F32>(c, {t_dz, KCHUNK, nout, KCHUNK, nchunk, (long long)nout * KCHUNK},
+                           {t_y, KCHUNK, nin, KCHUNK, nchunk, (long long)nin * KCHUNK}, g);
+}
+
+// Before a series of backward() on one Acts: the samples beyond the batch in the
+// last chunk of the transposes are zero (nothing writes them afterwards), and
+// the summed loss.
+static int backward_begin(mq_ctx *c, Acts &a) {
+  if (a.rows != a.rp) MQ_CUDA(c, cudaMemsetAsync(a.t_x, 0, a.t_elems * sizeof(bf16), c->stream));
+  MQ_CUDA(c, cudaMemsetAsync(a.scal, 0, 2 * sizeof(double), c->stream));
   return MQ_OK;
 }
 
-// forward + loss + backward on the batch in a (x filled); tb, wb: targets and
-// loss weights [R][nout]; gradients into m->gW/gb; loss partials summed on the host
-static int backward(mq_ctx *c, Mlp *m, Acts &a, const float *tb, const float *wb, double wsum, double *loss) {
+// forward + loss + backward on the batch in a (x filled; its loss weight in
+// a.scal[0]); tb, wb: targets and loss weights [R][nout]; gradients into
+// m->gW/gb, the loss is added to a.scal[1].  Nothing waits for the device:
+// backward_end does.
+static int backward(mq_ctx *c, Mlp *m, Acts &a, const float *tb, const float *wb) {
   const int R = a.rows;
   MQ_TRY(forward(c, m, a));
-  const int nb = 256;
-  loss_kernel<<<nb, 256, 0, c->stream>>>(a.out, tb, wb, R, m->d[3], (float)(1.0 / wsum), a.dy3, m->kp[3], a.loss_part);
-  c->stats.launches += 1;
-  std::vector<double> part(nb);
-  MQ_CUDA(c, cudaMemcpyAsync(part.data(), a.loss_part, nb * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  loss_kernel<<<LOSS_BLOCKS, 256, 0, c->stream>>>(a.out, tb, wb, R, m->d[3], a.scal, a.dy3, m->kp[3], a.loss_part);
+  scalar_sum_kernel<<<1, 256, 0, c->stream>>>(a.loss_part, LOSS_BLOCKS, 1, a.scal);
+  c->stats.launches += 2;
   MlpGemm g{};
   g.err = (int *)buf(c, "mlp_err", 64);
   // dz2 = (dy3 W3) * SiLU'(z2)
@@ -632,24 +746,51 @@ static int backward(mq_ctx *c, Mlp *m, Acts &a, const float *tb, const float *wb
   g.out16 = a.dz1;
   g.ldo = m->kp[1];
   MQ_TRY(mlp_gemm<EPI_DACT>(c, {a.dz2, m->kp[2], R, m->kp[2], 1, 0}, {m->Wt[1], m->kp[2], m->d[1], m->kp[2], 1, 0}, g));
-  // chunk-major transposes (zero beyond the batch's rows) and the weight gradients
-  MQ_CUDA(c, cudaMemsetAsync(a.t_x, 0, a.t_elems * sizeof(bf16), c->stream));
-  MQ_TRY(transpose(c, a.x, R, m->d[0], m->kp[0], a.t_x));
-  MQ_TRY(transpose(c, a.y1, R, m->d[1], m->kp[1], a.t_y1));
-  MQ_TRY(transpose(c, a.y2, R, m->d[2], m->kp[2], a.t_y2));
-  MQ_TRY(transpose(c, a.dy3, R, m->d[3], m->kp[3], a.t_dy3));
-  MQ_TRY(transpose(c, a.dz2, R, m->d[2], m->kp[2], a.t_dz2));
-  MQ_TRY(transpose(c, a.dz1, R, m->d[1], m->kp[1], a.t_dz1));
-  MQ_TRY(weight_grad(c, m, 2, a.t_dy3, a.t_y2, a.dy3, m->kp[3], R, a.rp, a.part32));
-  MQ_TRY(weight_grad(c, m, 1, a.t_dz2, a.t_y1, a.dz2, m->kp[2], R, a.rp, a.part32));
-  MQ_TRY(weight_grad(c, m, 0, a.t_dz1, a.t_x, a.dz1, m->kp[1], R, a.rp, a.part32));
-  MQ_CUDA(c, cudaStreamSynchronize(c->stream));
+  // chunk-major transposes, then the weight and bias gradients
+  const Transposes t{{a.x, a.y1, a.y2, a.dy3, a.dz2, a.dz1},
+                     {a.t_x, a.t_y1, a.t_y2, a.t_dy3, a.t_dz2, a.t_dz1},
+                     {m->d[0], m->d[1], m->d[2], m->d[3], m->d[2], m->d[1]},
+                     {m->kp[0], m->kp[1], m->kp[2], m->kp[3], m->kp[2], m->kp[1]},
+                     R, KCHUNK};
+  const int cmax = std::max(std::max(m->d[0], m->d[1]), std::max(m->d[2], m->d[3]));
+  if ((R + 31) / 32 > 65535) return set_err(c, MQ_EINVAL, "MLP gradient: too many rows");
+  transpose_chunked_kernel<<<dim3((cmax + 31) / 32, (R + 31) / 32, 6), dim3(32, 8), 0, c->stream>>>(t);
+  MQ_TRY(weight_grad(c, m, 2, a.t_dy3, a.t_y2, a.rp, a.part32[2]));
+  MQ_TRY(weight_grad(c, m, 1, a.t_dz2, a.t_y1, a.rp, a.part32[1]));
+  MQ_TRY(weight_grad(c, m, 0, a.t_dz1, a.t_x, a.rp, a.part32[0]));
+  GradSums gs{};
+  const bf16 *tdz[3] = {a.t_dz1, a.t_dz2, a.t_dy3};
+  long long nmax = 0;
+  int omax = 0;
+  for (int l = 0; l < 3; ++l) {
+    gs.part[l] = a.part32[l];
+    gs.gW[l] = m->gW[l];
+    gs.gb[l] = m->gb[l];
+    gs.t_dz[l] = tdz[l];
+    gs.nout[l] = m->d[l + 1];
+    gs.nw[l] = (long long)m->d[l + 1] * m->d[l];
+    nmax = std::max(nmax, gs.nw[l]);
+    omax = std::max(omax, gs.nout[l]);
+  }
+  gs.nchunk = a.rp / KCHUNK;
+  gs.kc = KCHUNK;
+  gs.rows = R;
+  gs.wblocks = (int)((nmax + 255) / 256);
+  grad_sum_kernel<<<dim3(gs.wblocks + omax, 3), 256, 0, c->stream>>>(gs);
+  c->stats.launches += 2;
+  MQ_CUDA(c, cudaGetLastError());
+  return MQ_OK;
+}
+
+// waits for the queued work: its time-out flag and the summed loss
+static int backward_end(mq_ctx *c, Acts &a, double *loss) {
+  int *err = (int *)buf(c, "mlp_err", 64);
+  if (!err) return MQ_ENOMEM;
   int herr = 0;
-  MQ_CUDA(c, cudaMemcpy(&herr, g.err, sizeof(int), cudaMemcpyDeviceToHost));
+  MQ_CUDA(c, cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  MQ_CUDA(c, cudaMemcpyAsync(loss, a.scal + 1, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  MQ_CUDA(c, cudaStreamSynchronize(c->stream));
   if (herr) return set_err(c, MQ_ETIMEOUT, "MLP GEMM wait timed out");
-  double s = 0.0;
-  for (double v : part) s += v;
-  *loss = s / wsum;
   return MQ_OK;
 }
 
@@ -657,13 +798,17 @@ static int adam(mq_ctx *c, Mlp *m, float lr) {
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   m->step += 1;
   const float c1 = 1.0f / (1.0f - powf(b1, (float)m->step)), c2 = 1.0f / (1.0f - powf(b2, (float)m->step));
+  AdamLayers p{};
+  long long nmax = 0;
   for (int l = 0; l < 3; ++l) {
-    const long long n = (long long)m->d[l + 1] * m->d[l] + m->d[l + 1];
-    adam_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(
-        m->W[l], m->mW[l], m->vW[l], m->gW[l], m->d[l + 1], m->d[l], m->b[l], m->mb[l], m->vb[l], m->gb[l], lr, b1, b2,
-        eps, c1, c2, m->Wb[l], m->kp[l], m->Wt[l], m->kp[l + 1]);
+    p.W[l] = m->W[l], p.mW[l] = m->mW[l], p.vW[l] = m->vW[l], p.gW[l] = m->gW[l];
+    p.b[l] = m->b[l], p.mb[l] = m->mb[l], p.vb[l] = m->vb[l], p.gb[l] = m->gb[l];
+    p.Wb[l] = m->Wb[l], p.Wt[l] = m->Wt[l];
+    p.nout[l] = m->d[l + 1], p.nin[l] = m->d[l], p.ldw[l] = m->kp[l], p.ldt[l] = m->kp[l + 1];
+    nmax = std::max(nmax, (long long)m->d[l + 1] * m->d[l] + m->d[l + 1]);
   }
-  c->stats.launches += 3;
+  adam_kernel<<<dim3((unsigned)((nmax + 255) / 256), 3), 256, 0, c->stream>>>(p, lr, b1, b2, eps, c1, c2);
+  c->stats.launches += 1;
   MQ_CUDA(c, cudaGetLastError());
   return MQ_OK;
 }
@@ -748,7 +893,11 @@ int mlp_grad(mq_ctx *c, int rows, const float *X, const float *T, const float *W
   MQ_CUDA(c, cudaMemcpyAsync(tw + nt, Wl, nt * sizeof(float), cudaMemcpyHostToDevice, c->stream));
   double wsum = 0.0;
   for (size_t i = 0; i < nt; ++i) wsum += Wl[i];
-  MQ_TRY(backward(c, m, a, tw, tw + nt, wsum > 0 ? wsum : 1.0, loss));
+  MQ_TRY(backward_begin(c, a));
+  if (!(wsum > 0.0)) wsum = 1.0;
+  MQ_CUDA(c, cudaMemcpyAsync(a.scal, &wsum, sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  MQ_TRY(backward(c, m, a, tw, tw + nt));
+  MQ_TRY(backward_end(c, a, loss));
   // packed like the parameters: gW then gb per layer
   float *dst = grads;
   for (int l = 0; l < 3; ++l) {
@@ -802,25 +951,19 @@ int mlp_train_epoch(mq_ctx *c, const int *perm, int batch, float lr, double *los
   float *tb = (float *)buf(c, "mlp_tw", 2 * (size_t)batch * m->d[3] * sizeof(float) + 16);
   if (!tb) return MQ_ENOMEM;
   float *wb = tb + (size_t)batch * m->d[3];
-  double total = 0.0;
+  MQ_TRY(backward_begin(c, a));
   int nb = 0;
-  for (long long r0 = 0; r0 + batch <= n; r0 += batch) {
+  for (long long r0 = 0; r0 + batch <= n; r0 += batch) {  // queued without a wait between minibatches
     gather_rows_kernel<<<batch, 128, 0, c->stream>>>(m->X, m->T, m->Wt8, d_perm + r0, batch, m->kp[0], m->d[3], a.x,
-                                                     tb, wb);
-    c->stats.launches += 1;
-    // the loss is normalised by the minibatch's weight sum (host side, from a device sum)
-    std::vector<float> hw((size_t)batch * m->d[3]);
-    MQ_CUDA(c, cudaMemcpyAsync(hw.data(), wb, hw.size() * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-    MQ_CUDA(c, cudaStreamSynchronize(c->stream));
-    double wsum = 0.0;
-    for (float v : hw) wsum += v;
-    double l = 0.0;
-    MQ_TRY(backward(c, m, a, tb, wb, wsum > 0 ? wsum : 1.0, &l));
+                                                     tb, wb, a.wrow);
+    scalar_sum_kernel<<<1, 1024, 0, c->stream>>>(a.wrow, batch, 0, a.scal);
+    c->stats.launches += 2;
+    MQ_TRY(backward(c, m, a, tb, wb));
     MQ_TRY(adam(c, m, lr));
-    total += l;
     ++nb;
   }
-  MQ_CUDA(c, cudaStreamSynchronize(c->stream));
+  double total = 0.0;
+  MQ_TRY(backward_end(c, a, &total));
   *loss = nb ? total / nb : 0.0;
   return mark_params(c);
 }
