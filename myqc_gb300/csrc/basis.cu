@@ -495,7 +495,7 @@ static void boys_series(long double T, int nm, long double *F) {
   for (int j = m - 1; j >= 0; --j) F[j] = (2.0L * T * F[j + 1] + e) / (2.0L * j + 1.0L);
 }
 
-// [m < 3][577 rows, T step 1/16][8]: F_m(T) as a polynomial of degree 6 in
+// [m < 4][577 rows, T step 1/16][8]: F_m(T) as a polynomial of degree 6 in
 // d = Tk - T, |d| <= 1/32, and Tk.  The Taylor polynomial of degree 8 with its
 // two highest terms economised over the interval: x^8 and x^7 (x = 32 d)
 // replaced through the Chebyshev polynomials T8 = 128 x^8 - 256 x^6 + 160 x^4

@@ -23,7 +23,7 @@
 //   parity: Ft(0:120,0:22) column-major (2783 doubles), then Tk/10 (121)
 //   tight : tab[Tk][m], 361 x 13 row-major (4693 doubles), then Tk/10 (361),
 //           then F_{m+k}(Tk)/k! [m < 5][Tk][k < 9], then the degree-6 rows of
-//           boys_fine [m < 3][577][8]
+//           boys_fine [m < 4][577][8]
 #pragma once
 #include "internal.h"
 
@@ -115,7 +115,7 @@ __device__ __forceinline__ void boys_tight(double T, const double *__restrict__ 
   }
 }
 
-// F_0 .. F_L, L <= 2, for the low-order integral kernels: below 36 each order
+// F_0 .. F_L, L <= 3, for the early-contracted integral kernels: below 36 each order
 // by its own polynomial of degree 6 about the nearest multiple of 1/16 (one row
 // of 64 bytes per order, whose last entry is that multiple).  The row number
 // comes from the low word of T + 1.5 2^48 (whose unit in the last place is

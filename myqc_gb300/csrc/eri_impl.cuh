@@ -249,9 +249,14 @@ __device__ __forceinline__ void boys_any(const EriArgs &g, float T, float (&F)[L
   boys_f32<L>(T, g.boys_f, F);
 }
 
-// What becomes of a quartet's integrals (this thread's share of them).
+// What becomes of a quartet's integrals (this thread's share of them).  ROLE: of
+// a quartet shared by two threads, 1 has the integrals with an s function among
+// a, b, c, 2 the others (0: not shared).
+__host__ __device__ constexpr bool role_has(int role, int a, int b, int c) {
+  return role == 0 || (role == 2) == (a > 0 && b > 0 && c > 0);
+}
 template <int LA, int LB, int LC, int LD, int A0, int A1, int B0, int B1, int C0, int C1, int D0, int D1, int EPI,
-          class RT>
+          int ROLE = 0, class RT>
 __device__ __forceinline__ void eri_epilogue(const EriArgs &g, int P, int Q, size_t n, double *XXout,
                                              const RT (&acc)[A1 - A0][B1 - B0][C1 - C0][D1 - D0], unsigned nprim) {
   const PairTable &t = g.t;
@@ -267,7 +272,7 @@ __device__ __forceinline__ void eri_epilogue(const EriArgs &g, int P, int Q, siz
     atomicMax(g.sch + P, (unsigned long long)__double_as_longlong(sqrt(m)));
     return;
   }
-  if (g.counters && A0 == 0 && B0 == 0 && C0 == 0 && D0 == 0) {  // one atomic pair per warp, not per quartet
+  if (g.counters && A0 == 0 && B0 == 0 && C0 == 0 && D0 == 0 && ROLE != 2) {  // one atomic pair per warp, not per quartet
     const unsigned act = __activemask();
     const unsigned nq_w = __popc(act), np_w = __reduce_add_sync(act, nprim);
     if ((threadIdx.x & 31) == __ffs(act) - 1) {
@@ -285,7 +290,8 @@ __device__ __forceinline__ void eri_epilogue(const EriArgs &g, int P, int Q, siz
         for (int c = C0; c < C1; ++c)
 #pragma unroll
           for (int d = D0; d < D1; ++d)
-            XXout[((a * NB_ + b) * NC_ + c) * ND_ + d] = (double)acc[a - A0][b - B0][c - C0][d - D0];
+            if (role_has(ROLE, a, b, c))
+              XXout[((a * NB_ + b) * NC_ + c) * ND_ + d] = (double)acc[a - A0][b - B0][c - C0][d - D0];
     return;
   }
 #pragma unroll
@@ -296,6 +302,7 @@ __device__ __forceinline__ void eri_epilogue(const EriArgs &g, int P, int Q, siz
       for (int c = C0; c < C1; ++c)
 #pragma unroll
         for (int d = D0; d < D1; ++d) {
+          if (!role_has(ROLE, a, b, c)) continue;
           const int i = i0 + a, j = j0 + b, k = k0 + c, l = l0 + d;
           if (A == B && i < j) continue;
           if (C == D && k < l) continue;
@@ -779,14 +786,6 @@ __global__ void __launch_bounds__(512) eri_shared_kernel(EriArgs g) {
       out += g.mols[m].xx;
     }
   }
-  if constexpr (NSPLIT == 4) {
-    switch (w) {
-      case 0: quartet_shared<LA, LB, LC, LD, 4, 0, 1, 0, 1, EPI>(g, valid, P, Q, n, out, smR, smI); break;
-      case 1: quartet_shared<LA, LB, LC, LD, 4, 1, 2, 0, 1, EPI>(g, valid, P, Q, n, out, smR, smI); break;
-      case 2: quartet_shared<LA, LB, LC, LD, 4, 2, 3, 0, 1, EPI>(g, valid, P, Q, n, out, smR, smI); break;
-      default: quartet_shared<LA, LB, LC, LD, 4, 3, 4, 0, 1, EPI>(g, valid, P, Q, n, out, smR, smI); break;
-    }
-  } else {
 #define MQ_SH16(s)                                                                                            \
   case s:                                                                                                     \
     quartet_shared<LA, LB, LC, LD, 16, (s) / 4, (s) / 4 + 1, (s) % 4, (s) % 4 + 1, EPI>(g, valid, P, Q, n, out, smR, \
@@ -798,7 +797,6 @@ __global__ void __launch_bounds__(512) eri_shared_kernel(EriArgs g) {
       default: quartet_shared<LA, LB, LC, LD, 16, 3, 4, 3, 4, EPI>(g, valid, P, Q, n, out, smR, smI); break;
     }
 #undef MQ_SH16
-  }
 }
 
 }  // namespace mq
@@ -839,7 +837,6 @@ __global__ void __launch_bounds__(256) eri_kernel(EriArgs g) {
     }
     return;
   }
-  constexpr int NSPLIT = NOUT <= 16 ? 1 : (NOUT <= 64 ? 4 : 16);
   const int lane = threadIdx.x & 31;
   if (g.queue) {  // persistent: each warp takes work units from the launch's queue until it is empty
     for (;;) {
@@ -860,7 +857,8 @@ template <int LA, int LB, int LC, int LD, int EPI, class RT>
 __device__ __forceinline__ void eri_unit(const EriArgs &g, long long warp, int lane) {
   constexpr int NA = nfun(LA), NB = nfun(LB);
   constexpr int NOUT = NA * NB * nfun(LC) * nfun(LD);
-  constexpr int NSPLIT = NOUT <= 16 ? 1 : (NOUT <= 64 ? 4 : 16);
+  constexpr bool EARLY = std::is_same<RT, double>::value && (EPI == EPI_XX || EPI == EPI_STORE) && NOUT <= 64;
+  constexpr int NSPLIT = NOUT <= 16 ? 1 : (NOUT <= 64 ? (EARLY ? 2 : 4) : 16);
   const int split = (int)(warp % NSPLIT);
   long long q = (warp / NSPLIT) * 32 + lane;
   int P, Q, m;
@@ -873,8 +871,11 @@ __device__ __forceinline__ void eri_unit(const EriArgs &g, long long warp, int l
   }
   if constexpr (EPI == EPI_STORE) XX = g.store + q * NOUT;
   constexpr int NC = nfun(LC), ND = nfun(LD);
-  if constexpr (NSPLIT == 1 && std::is_same<RT, double>::value && (EPI == EPI_XX || EPI == EPI_STORE)) {
+  if constexpr (EARLY && NSPLIT == 1) {
     quartet_low<LA, LB, LC, LD, EPI>(g, P, Q, n, XX);
+  } else if constexpr (EARLY) {
+    if (split == 0) quartet_mid<1, EPI>(g, P, Q, n, XX);
+    else quartet_mid<2, EPI>(g, P, Q, n, XX);
   } else if (NSPLIT == 1) {
     quartet<LA, LB, LC, LD, 0, NA, 0, NB, 0, NC, 0, ND, EPI, RT>(g, P, Q, n, XX);
   } else if (NSPLIT == 4) {  // (sp sp|sp s): one ket function c per thread, the whole bra
@@ -896,9 +897,11 @@ __device__ __forceinline__ void eri_unit(const EriArgs &g, long long warp, int l
   }
 }
 
-static inline int nsplit_of(int cP, int cQ) {
+// warps that serve the same 32 quartets; `early`: the early-contracted kernels
+// (FP64, EPI_XX and EPI_STORE)
+static inline int nsplit_of(int cP, int cQ, bool early) {
   int nout = (cP == 0 ? 1 : cP == 1 ? 4 : 16) * (cQ == 0 ? 1 : cQ == 1 ? 4 : 16);
-  return nout <= 16 ? 1 : (nout <= 64 ? 4 : 16);
+  return nout <= 16 ? 1 : (nout <= 64 ? (early ? 2 : 4) : 16);
 }
 
 // The launch order of an integral launch sorted by surviving primitive
@@ -911,8 +914,9 @@ int eri_batch_launch(mq_ctx *c, const EriArgs &h, int cP, int cQ);
 // thread-per-quartet kernel (64, 128 or 256; the autotuner's choice)
 template <int EPI, class RT = double>
 static int launch_class(mq_ctx *c, EriArgs g, int cP, int cQ, int block = 128, bool persistent = false) {
+  constexpr bool early = (EPI == EPI_STORE || EPI == EPI_XX) && std::is_same<RT, double>::value;
   // Schwarz: one warp slot per diagonal function pair (ab|ab) of the class
-  const int nsplit = EPI == EPI_SCHWARZ ? (cP == 0 ? 1 : cP == 1 ? 4 : 16) : nsplit_of(cP, cQ);
+  const int nsplit = EPI == EPI_SCHWARZ ? (cP == 0 ? 1 : cP == 1 ? 4 : 16) : nsplit_of(cP, cQ, early);
   const long long warps = (g.nq + 31) / 32 * nsplit;
   const long long threads = warps * 32;
   if (block != 64 && block != 128 && block != 256) return set_err(c, MQ_EINVAL, "integral launch: bad CTA size");
@@ -933,25 +937,17 @@ static int launch_class(mq_ctx *c, EriArgs g, int cP, int cQ, int block = 128, b
   }
   if (grid > 2147483647LL) return set_err(c, MQ_EINVAL, "integral launch too large");
   dim3 gd((unsigned)grid);
-  constexpr bool shared = (EPI == EPI_STORE || EPI == EPI_XX) && std::is_same<RT, double>::value;
-  if constexpr (shared) {
-    if (nsplit > 1) {  // the split classes: per-primitive work shared by the CTA's warps
+  if constexpr (early) {
+    if (nsplit == 16) {  // (sp sp|sp sp): per-primitive work shared by the CTA's warps
       const long long ctas = (g.nq + 31) / 32;
       if (ctas > 2147483647LL) return set_err(c, MQ_EINVAL, "integral launch too large");
-      if (cP == 2 && cQ == 1) {
-        const size_t sm = sizeof(double) * 4 * 32 * nherm(3) + sizeof(int2) * 4 * 32;
-        MQ_CUDA(c, cudaFuncSetAttribute(eri_shared_kernel<1, 1, 1, 0, EPI>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        eri_shared_kernel<1, 1, 1, 0, EPI><<<(unsigned)ctas, 128, sm, c->stream>>>(g);
-      } else {
-        const size_t sm = sizeof(double) * 16 * 32 * nherm(4) + sizeof(int2) * 16 * 32;
-        MQ_CUDA(c, cudaFuncSetAttribute(eri_shared_kernel<1, 1, 1, 1, EPI>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        eri_shared_kernel<1, 1, 1, 1, EPI><<<(unsigned)ctas, 512, sm, c->stream>>>(g);
-      }
+      const size_t sm = sizeof(double) * 16 * 32 * nherm(4) + sizeof(int2) * 16 * 32;
+      MQ_CUDA(c, cudaFuncSetAttribute(eri_shared_kernel<1, 1, 1, 1, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sm));
+      eri_shared_kernel<1, 1, 1, 1, EPI><<<(unsigned)ctas, 512, sm, c->stream>>>(g);
       c->stats.launches += 1;
       MQ_CUDA(c, cudaGetLastError());
-      return sync_check(c, "eri_store");
+      return sync_check(c, "eri_shared");
     }
   }
 #define MQ_LAUNCH(a, b, cc, d) eri_kernel<a, b, cc, d, EPI, RT><<<gd, block, 0, c->stream>>>(g)
@@ -959,9 +955,9 @@ static int launch_class(mq_ctx *c, EriArgs g, int cP, int cQ, int block = 128, b
   else if (cP == 1 && cQ == 0) MQ_LAUNCH(1, 0, 0, 0);
   else if (cP == 1 && cQ == 1) MQ_LAUNCH(1, 0, 1, 0);
   else if (cP == 2 && cQ == 0) MQ_LAUNCH(1, 1, 0, 0);
-  if constexpr (!shared) {
-    if (cP == 2 && cQ == 1) MQ_LAUNCH(1, 1, 1, 0);
-    else if (cP == 2 && cQ == 2) MQ_LAUNCH(1, 1, 1, 1);
+  else if (cP == 2 && cQ == 1) MQ_LAUNCH(1, 1, 1, 0);
+  if constexpr (!early) {
+    if (cP == 2 && cQ == 2) MQ_LAUNCH(1, 1, 1, 1);
   }
 #undef MQ_LAUNCH
   c->stats.launches += 1;

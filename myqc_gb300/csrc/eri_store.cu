@@ -145,9 +145,9 @@ static int run_candidate(mq_ctx *c, const EriArgs &h0, int cP, int cQ, int slot,
 // ran last.
 template <int EPI>
 static int tuned_launch(mq_ctx *c, const EriArgs &h, int cP, int cQ, int combo, int slot) {
-  // the split classes run their CTA-shared kernel: its shape is fixed by the
-  // warp count, only the order is a choice
-  const bool fixed_shape = nsplit_of(cP, cQ) > 1;
+  // (sp sp|sp sp) runs its CTA-shared kernel: its shape is fixed by the warp
+  // count, only the order is a choice
+  const bool fixed_shape = nsplit_of(cP, cQ, true) == 16;
   EriTune def;
   if (c->eri_tune_mode == 0 || h.nq < TUNE_MIN_QUARTETS) return run_candidate<EPI>(c, h, cP, cQ, slot, def);
   const unsigned long long key = tune_key(EPI, combo, h.nq);

@@ -345,6 +345,7 @@ struct PairLaunch {
   const MolDesc *mols;
   const int *active;
   int ntiles, nmol, nmax;
+  long long cols;  // density columns of all molecules (MolDesc::vec counts them)
   int tri;   // DJ carries lower-triangle weights: J sums over l <= k only
   const unsigned char *live;  // slab (i,j) may be nonzero (n x n, single system); null: every slab
   int arith;  // FOCK_ARITH_*: FP64 arrays, float pairs (double-float), or floats (FP32 increments)
@@ -391,7 +392,7 @@ int upload_pairs(mq_ctx *c, const HostPairs &h, std::vector<void *> *allocs, Pai
 void free_pairs(mq_ctx *c);
 void tight_boys_table(std::vector<double> &tab);  // TIGHT_NT x TIGHT_NM, row-major [T][m]
 constexpr int BOYS_SCALED_M = 5;                  // orders with their own Taylor-coefficient table
-constexpr int BOYS_FINE_M = 3, BOYS_FINE_NT = 577;  // orders and rows (T step 1/16) of the degree-6 tables
+constexpr int BOYS_FINE_M = 4, BOYS_FINE_NT = 577;  // orders and rows (T step 1/16) of the degree-6 tables
 // their offset in the device table: behind the values, grid and Taylor tables, on a 64-byte boundary
 constexpr size_t BOYS_FINE_OFF = ((size_t)TIGHT_NT * (TIGHT_NM + 1 + 9 * BOYS_SCALED_M) + 7) / 8 * 8;
 void tight_boys_device_table(std::vector<double> &tab);  // the table, its grid, the scaled tables
