@@ -449,8 +449,8 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
       }
       total[k] = mqo[k][M];
     }
-  // Fock tiles (i, j-run of 2, molecule) and per-molecule row tables
-  const int JC = 2;
+  // Fock tiles (i, j-run of 4, molecule) and per-molecule row tables
+  const int JC = 4;
   std::vector<int4> tl;
   std::vector<int> rf;
   for (int m = 0; m < M; ++m) {
@@ -564,6 +564,7 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
   L.ntiles = (int)tl.size();
   L.nmol = M;
   L.nmax = nmax;
+  L.cols = (long long)vec;
   L.J = dJ;
   L.Kpa = d_Kp;
   L.Qa = d_Q;

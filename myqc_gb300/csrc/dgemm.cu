@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(GX_THREADS, 2) dgemm_kernel(int mx, int ny, in
       if (!one || tile == (int)blockIdx.x)
         gx_load<YROW>(Yc + (YROW ? ldy * kb : (size_t)kb), ldy, min(GX_T, ny - c0), kc, fields + GX_T, ey, UY);
       __syncthreads();
-      float acc[1][FX_DIG][4];
-      fx_tile<1>(UX, UY, GX_LD, GX_T, GX_T, wr, wc, (kc + 15) / 16, acc);
+      float acc[FX_DIG][4];
+      fx_tile(UX, UY, GX_LD, GX_T, GX_T, wr, wc, (kc + 15) / 16, acc);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int r = wr + g + 8 * (i >> 1), c = wc + 2 * t + (i & 1);
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(GX_THREADS, 2) dgemm_kernel(int mx, int ny, in
         if (ex[r] != GX_BAD && ey[c] != GX_BAD) {
           float v[FX_DIG];
 #pragma unroll
-          for (int L = 0; L < FX_DIG; ++L) v[L] = acc[0][L][i];
+          for (int L = 0; L < FX_DIG; ++L) v[L] = acc[L][i];
           x = fx_combine(v, ex[r], ey[c]);
         } else if (r0 + r < mx && c0 + c < ny) {
           for (int l = kb; l < kb + kc; ++l)

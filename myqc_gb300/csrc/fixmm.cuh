@@ -3,14 +3,14 @@
 // Rump, Numer. Algorithms 59, 95 (2012), on FP16 digits).
 //
 // Each row of op(A) and each column of op(B) is scaled by a power of two to
-// |x| < 2^62 and rounded to an integer (every element within 2^9 of the row's
+// |x| < 2^62 and cut to an integer (every element within 2^9 of the row's
 // largest stays exact), cut into eight digits of eight bits,
 // x = sum_k s_k 256^(7-k), -128 <= s_k <= 127, |s_0| <= 64.  FP16 holds a digit
 // exactly, a digit product is an integer of at most 2^14, and the sum of one
 // level (the products s_k s'_l with k + l = L) over K <= 144 stays below 2^24,
 // so the FP32 accumulators of mma.sync hold every level exactly in any order.
 // The levels L = 0..7 (36 digit products) are combined as integers and rounded
-// to FP64 once.  What is dropped -- the rounding of the operands, 2^-63 of the
+// to FP64 once.  What is dropped -- the cutting of the operands, 2^-62 of the
 // row's largest element, and levels 8 to 14 -- is about 2^-61 of the largest
 // possible sum, so an element is correct to rounding unless it is 2^-8 of that
 // and less; an FP64 sum rounds after each of its K additions.
@@ -42,16 +42,16 @@ constexpr int FX_BITS = 62;
 // neighbouring rows meet a bank conflict.
 __device__ __forceinline__ int fx_pos(int r, int kp) { return kp ^ (((r & 1) << 2) | ((r >> 1) & 3)); }
 
-// x * 2^(FX_BITS - e) rounded to nearest (ties away), biased; |x| < 2^e
+// x * 2^(FX_BITS - e) cut to an integer, biased; |x| < 2^e, e = fx_exp(field of
+// the row's largest element)
 __device__ __forceinline__ unsigned long long fx_fix(double x, int e) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int E = (int)(b >> 52) & 0x7ff;
-  const int sh = e - FX_BITS + 1075 - E;  // > 0: right shift
-  unsigned long long m = (b & 0xfffffffffffffull) | 0x10000000000000ull;
-  if (E == 0 || sh > 54) m = 0;
-  else if (sh > 0) m = (m + (1ull << (sh - 1))) >> sh;
-  else m <<= -sh;
-  return ((long long)b < 0 ? 0ull - m : m) + FX_BIAS;
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const int E = (int)(hi >> 20) & 0x7ff;
+  const unsigned h = (hi & 0xfffffu) | 0x100000u;
+  // the significand with its leading bit at 2^61, moved down to the row's scale
+  unsigned long long m = ((unsigned long long)(h << 9 | lo >> 23) << 32 | lo << 9) >> min(e + 1022 - E, 63);
+  if (E == 0) m = 0;
+  return ((int)hi < 0 ? 0ull - m : m) + FX_BIAS;
 }
 // e with |x| < 2^e for every x of exponent field <= E (0 for a zero row)
 __device__ __forceinline__ int fx_exp(int E) { return E == 0 ? -1100 : E - 1022; }
@@ -64,23 +64,41 @@ __device__ __forceinline__ uint4 fx_pair(unsigned long long u0, unsigned long lo
                     __byte_perm(h0, h1, 0x7362));
 }
 
-// The digits of a pair (k, k + 1) as FP16 pairs
-__device__ __forceinline__ void fx_digits(uint4 u, unsigned (&d)[FX_DIG]) {
-  const unsigned word[4] = {u.x, u.y, u.z, u.w};
+// Digit k of a pair of elements as an FP16 pair
+__device__ __forceinline__ unsigned fx_digit(const uint4 &u, int k) {
+  const int by = FX_DIG - 1 - k;  // byte of digit k
+  const unsigned word = (by >> 1) == 0 ? u.x : (by >> 1) == 1 ? u.y : (by >> 1) == 2 ? u.z : u.w;
+  const unsigned w = __byte_perm(word, 0x64646464u, by & 1 ? 0x4342 : 0x4140);
   const __half2 off = __half2half2(__ushort_as_half(0x6480));  // 1024 + 128
-#pragma unroll
-  for (int k = 0; k < FX_DIG; ++k) {
-    const int by = FX_DIG - 1 - k;  // byte of digit k
-    const unsigned w = __byte_perm(word[by >> 1], 0x64646464u, by & 1 ? 0x4342 : 0x4140);
-    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&w), off);
-    d[k] = *reinterpret_cast<const unsigned *>(&h);
-  }
+  const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&w), off);
+  return *reinterpret_cast<const unsigned *>(&h);
 }
 
 __device__ __forceinline__ void fx_mma(float (&c)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// acc[L] += the digit products of level L of a 16 x 16 fragment A (pairs (row g,
+// k), (g + 8, k), (g, k + 8), (g + 8, k + 8)) and a 16 x 8 fragment B.  A's
+// digits are formed as they are used, B's are kept.
+__device__ __forceinline__ void fx_block(float (&acc)[FX_DIG][4], const uint4 (&a)[4], const uint4 (&b)[2]) {
+  unsigned bd[2][FX_DIG];
+#pragma unroll
+  for (int k = 0; k < FX_DIG; ++k) {
+    bd[0][k] = fx_digit(b[0], k);
+    bd[1][k] = fx_digit(b[1], k);
+  }
+#pragma unroll
+  for (int x = 0; x < FX_DIG; ++x) {
+    const unsigned av[4] = {fx_digit(a[0], x), fx_digit(a[1], x), fx_digit(a[2], x), fx_digit(a[3], x)};
+#pragma unroll
+    for (int y = 0; y + x < FX_DIG; ++y) {
+      const unsigned bv[2] = {bd[0][y], bd[1][y]};
+      fx_mma(acc[x + y], av, bv);
+    }
+  }
 }
 
 // sum_L v_L 256^(7-L) * 2^(ea + eb - 2 FX_BITS + 8 * 7), rounded to nearest.
@@ -117,43 +135,23 @@ __device__ __forceinline__ double fx_combine(const float *v, int ea, int eb) {
   return x * __hiloint2double((s1 + 1023) << 20, 0) * __hiloint2double((s2 + 1023) << 20, 0);
 }
 
-// A 16 x (8 NT) tile: rows of UA (fragment rows r0 + g, r0 + g + 8; clamped to
-// rows na - 1), columns = rows of UB (c0 + 8 j + g, clamped), K = 16 ksteps.
-// acc[j][level][4].
-template <int NT>
+// A 16 x 8 tile: rows of UA (fragment rows r0 + g, r0 + g + 8; clamped to
+// na - 1), columns = rows of UB (c0 + g, clamped), K = 16 ksteps.
 __device__ __forceinline__ void fx_tile(const uint4 *UA, const uint4 *UB, int ld, int na, int nb, int r0, int c0,
-                                        int ksteps, float (&acc)[NT][FX_DIG][4]) {
+                                        int ksteps, float (&acc)[FX_DIG][4]) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int ra = min(r0 + g, na - 1), rb = min(r0 + g + 8, na - 1);
+  const int ra = min(r0 + g, na - 1), rb = min(r0 + g + 8, na - 1), cb = min(c0 + g, nb - 1);
 #pragma unroll
-  for (int j = 0; j < NT; ++j)
+  for (int L = 0; L < FX_DIG; ++L)
 #pragma unroll
-    for (int L = 0; L < FX_DIG; ++L)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[j][L][i] = 0.f;
+    for (int i = 0; i < 4; ++i) acc[L][i] = 0.f;
 #pragma unroll 1
   for (int ks = 0; ks < ksteps; ++ks) {
     const int k0 = 8 * ks + t;
-    unsigned a[4][FX_DIG];
-    fx_digits(UA[(size_t)ra * ld + fx_pos(ra, k0)], a[0]);
-    fx_digits(UA[(size_t)rb * ld + fx_pos(rb, k0)], a[1]);
-    fx_digits(UA[(size_t)ra * ld + fx_pos(ra, k0 + 4)], a[2]);
-    fx_digits(UA[(size_t)rb * ld + fx_pos(rb, k0 + 4)], a[3]);
-#pragma unroll
-    for (int j = 0; j < NT; ++j) {
-      const int cb = min(c0 + 8 * j + g, nb - 1);
-      unsigned b[2][FX_DIG];
-      fx_digits(UB[(size_t)cb * ld + fx_pos(cb, k0)], b[0]);
-      fx_digits(UB[(size_t)cb * ld + fx_pos(cb, k0 + 4)], b[1]);
-#pragma unroll
-      for (int x = 0; x < FX_DIG; ++x)
-#pragma unroll
-        for (int y = 0; y + x < FX_DIG; ++y) {
-          const unsigned av[4] = {a[0][x], a[1][x], a[2][x], a[3][x]};
-          const unsigned bv[2] = {b[0][y], b[1][y]};
-          fx_mma(acc[j][x + y], av, bv);
-        }
-    }
+    const uint4 a[4] = {UA[(size_t)ra * ld + fx_pos(ra, k0)], UA[(size_t)rb * ld + fx_pos(rb, k0)],
+                        UA[(size_t)ra * ld + fx_pos(ra, k0 + 4)], UA[(size_t)rb * ld + fx_pos(rb, k0 + 4)]};
+    const uint4 b[2] = {UB[(size_t)cb * ld + fx_pos(cb, k0)], UB[(size_t)cb * ld + fx_pos(cb, k0 + 4)]};
+    fx_block(acc, a, b);
   }
 }
 
@@ -221,14 +219,14 @@ static __device__ __forceinline__ void cta_fix_mm(int na, int nb, int nk, const 
   const int tm = (na + 15) / 16, tn = (nb + 7) / 8;
   for (int tile = w; tile < tm * tn; tile += nw) {
     const int tj = tile / tm, ti = tile - tj * tm;
-    float acc[1][FX_DIG][4];
-    fx_tile<1>(UA, UB, fx_ld(nk), na, nb, 16 * ti, 8 * tj, (nk + 15) / 16, acc);
+    float acc[FX_DIG][4];
+    fx_tile(UA, UB, fx_ld(nk), na, nb, 16 * ti, 8 * tj, (nk + 15) / 16, acc);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = 16 * ti + g + 8 * (i >> 1), cc = 8 * tj + 2 * t + (i & 1);
       float v[FX_DIG];
 #pragma unroll
-      for (int L = 0; L < FX_DIG; ++L) v[L] = acc[0][L][i];
+      for (int L = 0; L < FX_DIG; ++L) v[L] = acc[L][i];
       if (r < na && cc < nb) store(r, cc, fx_combine(v, ea[r], eb[cc]));
     }
   }

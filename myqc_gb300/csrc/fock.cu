@@ -19,6 +19,7 @@
 #include <string>
 
 #include "df32.cuh"
+#include "fixmm.cuh"
 #include "internal.h"
 
 namespace mq {
@@ -273,10 +274,9 @@ __global__ void __launch_bounds__(PAIR_MAX_THREADS) fock_pair_kernel(
   for (int jj = 0; jj < JC; ++jj)
     if (jj < nj && (!live || live[i + N * (j0 + jj)])) lvm |= 1u << jj;
   const double *S0 = XX + n2 * ((size_t)i + N * j0);
-  // FP64 (the reference's arithmetic, the plain path) and the largest orders
-  // (R = 4) interleave loads and arithmetic; the FP32-pipe arithmetics batch
-  // the loads of several columns (below).
-  constexpr bool BATCH = !std::is_same<P, ArithF64>::value && R <= 2;
+  // The largest orders (R = 4) interleave loads and arithmetic; the others
+  // batch the loads of several columns (below).
+  constexpr bool BATCH = R <= 2;
   if constexpr (!BATCH) {
 #pragma unroll 2
     for (int l = 0; lvm && l < n; ++l) {
@@ -401,6 +401,201 @@ __global__ void __launch_bounds__(PAIR_MAX_THREADS) fock_pair_kernel(
   }
 }
 
+// ---- The same digestion in FP64 accuracy on the tensor cores.  FP64 issue is
+// two multiply-adds per clock and SM, and a slab element needs two of them for
+// K of one spin (S . D(:,j) and S . D(:,i)); as a fixed-point product (fixmm.cuh)
+// with the columns D(:,j), D(:,i) of both spins as the eight columns of one
+// mma.sync fragment, a 16 x 16 block of S takes 36 of them, 72 clocks of the
+// tensor pipe for 256 elements whatever the number of spins.  J_ij = <S, Dt>
+// stays on the FP64 pipe, beside it: S is symmetric, so only the blocks on and
+// below the diagonal are summed (half a multiply-add per element).
+//
+// One warp per 16 rows k of a slab (the units of a tile's slabs are dealt to the
+// CTA's warps, so that small molecules keep them all busy); it reads its rows
+// twice, once for their exponents (over up to 128 columns) and once, from L1,
+// for the digits.
+// Columns of D come as fixed-point pairs from fock_cols_kernel.  Outputs as
+// fock_pair_kernel's.  A row or column with an infinity or NaN is summed in
+// FP64 as it is.
+constexpr int FXF_THREADS = 256;
+constexpr int FXF_BAD = 4000;  // exponent of a row with a non-finite element
+constexpr int FXF_JC = 4;      // slabs per tile at most
+
+// Column j (blockIdx.x) of molecule blockIdx.y, spin blockIdx.z, as fixed-point
+// pairs U[(spin cols + vec + j) ld + kp] and its exponent
+__global__ void __launch_bounds__(32) fock_cols_kernel(const double *__restrict__ Da, const double *__restrict__ Db,
+                                                       const MolDesc *__restrict__ mols,
+                                                       const int *__restrict__ active, long long cols, int ld,
+                                                       uint4 *__restrict__ U, int *__restrict__ e) {
+  const int m = blockIdx.y, j = blockIdx.x, lane = threadIdx.x;
+  if (active && !active[m]) return;
+  const MolDesc md = mols[m];
+  const int n = md.n;
+  if (j >= n) return;
+  const double *x = (blockIdx.z ? Db : Da) + md.mat + (size_t)n * j;
+  const long long c = blockIdx.z * cols + md.vec + j;
+  int f = 0;
+  for (int l = lane; l < n; l += 32) f = max(f, fx_field(x[l]));
+  f = __reduce_max_sync(0xffffffffu, f);
+  const int ex = f == 0x7ff ? FXF_BAD : fx_exp(f);
+  if (lane == 0) e[c] = ex;
+  if (ex == FXF_BAD) return;
+  for (int kp = lane; kp < fx_ld(n); kp += 32) {
+    const int l = 2 * kp;
+    U[c * ld + kp] = fx_pair(l < n ? fx_fix(x[l], ex) : FX_BIAS, l + 1 < n ? fx_fix(x[l + 1], ex) : FX_BIAS);
+  }
+}
+
+template <bool UHF>
+__global__ void __launch_bounds__(FXF_THREADS, 2) fock_fx_kernel(
+    const double *__restrict__ XX, const double *__restrict__ DJ, const double *__restrict__ DKa,
+    const double *__restrict__ DKb, const uint4 *__restrict__ U, const int *__restrict__ eD, long long cols, int ld,
+    const int4 *__restrict__ tiles, const MolDesc *__restrict__ mols, const int *__restrict__ active, int kp_stride,
+    int tri, const unsigned char *__restrict__ live, double *__restrict__ J, double *__restrict__ Kpa,
+    double *__restrict__ Kpb, double *__restrict__ Qa, double *__restrict__ Qb) {
+  __shared__ double jp[FXF_JC][FXF_THREADS];
+  extern __shared__ double kpart[];  // [slab][spin][row]: the slabs' parts of K(:, i)
+  const int4 tile = tiles[blockIdx.x];
+  if (active && !active[tile.w]) return;
+  const MolDesc md = mols[tile.w];
+  const int i = tile.x, j0 = tile.y, nj = tile.z - tile.y, n = md.n;
+  const size_t N = n, n2 = N * N;
+  XX += md.xx;
+  DJ += md.mat;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5, g = lane >> 2, t = lane & 3;
+  for (int jj = 0; jj < nj; ++jj) jp[jj][tid] = 0.0;
+  const bool vec2 = ((md.xx | n) & 1) == 0;  // 16-byte loads of XX
+  // the fragment column g: Da(:,j), Da(:,i), Db(:,j), Db(:,i), none
+  const bool has = g < (UHF ? 4 : 2);
+  const long long spin = g >= 2 ? cols : 0;
+  constexpr int NS = UHF ? 2 : 1;
+  const int nrb = (n + 15) / 16;
+  for (int unit = w; unit < nrb * nj; unit += nw) {
+    const int jj = unit / nrb, rb = unit - jj * nrb;
+    const int ra = min(16 * rb + g, n - 1), rc = min(16 * rb + g + 8, n - 1);
+    {
+      const int j = j0 + jj;
+      const bool zero = live && !live[i + N * j];  // every quartet of the slab screened out
+      double kj[2] = {0.0, 0.0}, ks[2] = {0.0, 0.0}, js = 0.0;
+      if (!zero) {
+        const double *S = XX + n2 * ((size_t)i + N * j);
+        const double *Sa = S + N * ra, *Sc = S + N * rc;
+        const long long cg = spin + md.vec + (g & 1 ? i : j);
+        for (int cb = 0; cb < n; cb += 128) {
+          const int cw = min(128, n - cb), ksteps = (cw + 15) / 16;
+          auto pair = [&](const double *p, int l) {
+            double2 v = make_double2(0.0, 0.0);
+            if (l + 1 < n) {
+              if (vec2) v = __ldg(reinterpret_cast<const double2 *>(p + l));
+              else v = make_double2(__ldg(p + l), __ldg(p + l + 1));
+            } else if (l < n) {
+              v.x = __ldg(p + l);
+            }
+            return v;
+          };
+          int fa = 0, fc = 0;
+#pragma unroll 4
+          for (int ks8 = 0; ks8 < 2 * ksteps; ++ks8) {
+            const int l = cb + 8 * ks8 + 2 * t;
+            const double2 a = pair(Sa, l), c = pair(Sc, l);
+            fa = max(fa, max(fx_field(a.x), fx_field(a.y)));
+            fc = max(fc, max(fx_field(c.x), fx_field(c.y)));
+          }
+#pragma unroll
+          for (int o = 1; o < 4; o <<= 1) {
+            fa = max(fa, __shfl_xor_sync(0xffffffffu, fa, o));
+            fc = max(fc, __shfl_xor_sync(0xffffffffu, fc, o));
+          }
+          const int ea = fx_exp(fa), ec = fx_exp(fc);
+          float acc[FX_DIG][4];
+#pragma unroll
+          for (int L = 0; L < FX_DIG; ++L)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) acc[L][x] = 0.f;
+#pragma unroll 1
+          for (int ks1 = 0; ks1 < ksteps; ++ks1) {
+            const int l = cb + 16 * ks1 + 2 * t, l0 = cb + 16 * ks1;
+            const double2 a0 = pair(Sa, l), a1 = pair(Sc, l), a2 = pair(Sa, l + 8), a3 = pair(Sc, l + 8);
+            if (l0 <= 16 * rb) {  // J: the blocks on and below the diagonal
+              const double wgt = !tri && l0 < 16 * rb ? 2.0 : 1.0;
+              double jb = 0.0;
+#pragma unroll
+              for (int x = 0; x < 2; ++x) {
+                const int k = x ? 16 * rb + g + 8 : 16 * rb + g;
+                if (k >= n) continue;
+                const double2 s0 = x ? a1 : a0, s1 = x ? a3 : a2;
+                // (DJ is symmetric, or lower-triangular with row k >= column l)
+                if (l < n) jb = fma(s0.x, DJ[k + N * l], jb);
+                if (l + 1 < n) jb = fma(s0.y, DJ[k + N * (l + 1)], jb);
+                if (l + 8 < n) jb = fma(s1.x, DJ[k + N * (l + 8)], jb);
+                if (l + 9 < n) jb = fma(s1.y, DJ[k + N * (l + 9)], jb);
+              }
+              js = fma(wgt, jb, js);
+            }
+            const uint4 none = make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);
+            const uint4 *uc = U + cg * ld + l0 / 2 + t;
+            const uint4 bv[2] = {has ? __ldg(uc) : none, has ? __ldg(uc + 4) : none};
+            const uint4 av[4] = {fx_pair(fx_fix(a0.x, ea), fx_fix(a0.y, ea)), fx_pair(fx_fix(a1.x, ec), fx_fix(a1.y, ec)),
+                                 fx_pair(fx_fix(a2.x, ea), fx_fix(a2.y, ea)), fx_pair(fx_fix(a3.x, ec), fx_fix(a3.y, ec))};
+            fx_block(acc, av, bv);
+          }
+          if (t < (UHF ? 2 : 1)) {  // lanes t: columns 2t = D(:,j), 2t + 1 = D(:,i) of spin t
+            const long long c0 = t * cols + md.vec;
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+              const int ed = eD[c0 + (x & 1 ? i : j)], es = x < 2 ? ea : ec, fs = x < 2 ? fa : fc;
+              double v;
+              if (fs != 0x7ff && ed != FXF_BAD) {
+                float lv[FX_DIG];
+#pragma unroll
+                for (int L = 0; L < FX_DIG; ++L) lv[L] = acc[L][x];
+                v = fx_combine(lv, es, ed);
+              } else {
+                const double *D = (t ? DKb : DKa) + md.mat + N * (x & 1 ? i : j), *Sr = x < 2 ? Sa : Sc;
+                v = 0.0;
+                for (int l = cb; l < cb + cw; ++l) v = fma(Sr[l], D[l], v);
+              }
+              if (x & 1) ks[x >> 1] += v;
+              else kj[x >> 1] += v;
+            }
+          }
+        }
+      }
+      jp[jj][tid] += js;
+      if (t < NS) {
+        double *kp = kpart + (size_t)(jj * NS + t) * n;
+        double *Q = j > i ? (t ? Qb : Qa) + md.q + N * i + n2 * j : nullptr;
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const int k = 16 * rb + g + 8 * x;
+          if (k >= n) continue;
+          kp[k] = kj[x];
+          if (Q) Q[k] = ks[x];
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int x = tid; x < NS * n; x += blockDim.x) {
+    const int s = x / n, k = x - s * n;
+    double v = kpart[x];
+    for (int jj = 1; jj < nj; ++jj) v += kpart[(size_t)jj * NS * n + x];
+    (s ? Kpb : Kpa)[(size_t)kp_stride * blockIdx.x + k] = v;
+  }
+  // J_ij: one warp per slab adds the threads' parts in a fixed order
+  for (int jj = w; jj < nj; jj += nw) {
+    double v = 0.0;
+    for (int k = lane; k < (int)blockDim.x; k += 32) v += jp[jj][k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) {
+      double *Jm = J + md.mat;
+      Jm[i + N * (j0 + jj)] = v;
+      Jm[j0 + jj + N * i] = v;
+    }
+  }
+}
+
 // K(k, j) = sum over row j's tiles of their slices + sum_{i<j} Q(k, i, j);
 // blockIdx.y is the molecule
 __global__ void fock_pair_assemble_kernel(const double *__restrict__ Kp, const double *__restrict__ Q,
@@ -475,6 +670,32 @@ static int launch_pair_r(mq_ctx *c, int Rp, int jc, const PairLaunch &L, int thr
   }
 }
 
+// The FP64 digestion: the densities' columns as fixed-point pairs, then the slabs
+static int launch_fx(mq_ctx *c, const PairLaunch &L, bool uhf) {
+  const int ns = uhf ? 2 : 1, ld = fx_ld(L.nmax);
+  const size_t cols = (size_t)L.cols, ub = sizeof(uint4) * cols * ns * ld;
+  char *w = (char *)buf(c, "fock_cols", ub + sizeof(int) * cols * ns);
+  if (!w) return MQ_ENOMEM;
+  uint4 *U = (uint4 *)w;
+  int *e = (int *)(w + ub);
+  const double *DJ = (const double *)L.DJ, *DKa = (const double *)L.DKa, *DKb = (const double *)L.DKb;
+  fock_cols_kernel<<<dim3(L.nmax, L.nmol, ns), 32, 0, c->stream>>>(DKa, DKb, L.mols, L.active, L.cols, ld, U, e);
+  const int threads = 32 * std::min(FXF_THREADS / 32, (L.nmax + 15) / 16);
+  const size_t sm = sizeof(double) * FXF_JC * ns * L.nmax;
+  MQ_CUDA(c, cudaFuncSetAttribute(fock_fx_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  MQ_CUDA(c, cudaFuncSetAttribute(fock_fx_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  if (uhf)
+    fock_fx_kernel<true><<<L.ntiles, threads, sm, c->stream>>>(L.XX, DJ, DKa, DKb, U, e, L.cols, ld, L.tiles, L.mols,
+                                                              L.active, L.nmax, L.tri, L.live, L.J, L.Kpa, L.Kpb,
+                                                              L.Qa, L.Qb);
+  else
+    fock_fx_kernel<false><<<L.ntiles, threads, sm, c->stream>>>(L.XX, DJ, DKa, nullptr, U, e, L.cols, ld, L.tiles,
+                                                               L.mols, L.active, L.nmax, L.tri, L.live, L.J, L.Kpa,
+                                                               nullptr, L.Qa, nullptr);
+  c->stats.launches += 1;
+  return MQ_OK;
+}
+
 void pair_tiles_host(int n, int JC, int mol, std::vector<int4> &tl, std::vector<int> &rf) {
   for (int i = 0; i < n; ++i) {
     rf.push_back((int)tl.size());
@@ -515,6 +736,7 @@ static int pair_tiles(mq_ctx *c, int n, int JC, PairLaunch &L) {
   L.ntiles = ft.ntiles;
   L.nmol = 1;
   L.nmax = n;
+  L.cols = n;
   L.active = nullptr;
   return MQ_OK;
 }
@@ -529,7 +751,7 @@ int pair_digest(mq_ctx *c, int JC, bool uhf, const PairLaunch &L, double *d_Ga, 
   if (timed) c->t_fock_kernel.start(c->stream);
   if (L.arith == FOCK_ARITH_DF32) MQ_TRY(launch_pair_r<ArithDF32>(c, Rp, JC, L, T, uhf));
   else if (L.arith == FOCK_ARITH_F32) MQ_TRY(launch_pair_r<ArithF32>(c, Rp, JC, L, T, uhf));
-  else MQ_TRY(launch_pair_r<ArithF64>(c, Rp, JC, L, T, uhf));
+  else MQ_TRY(launch_fx(c, L, uhf));
   if (timed) {
     c->t_fock_kernel.stop(c->stream);
     c->stats.fock_kernel_launches += 1;
