@@ -12,7 +12,7 @@
 //           = 2X_k - X_k^2 otherwise
 // until the idempotency error tr(X - X^2) vanishes; convergence is quadratic
 // once the occupied and virtual eigenvalues have separated.  Each step is one
-// FP64 GEMM (cuBLAS) and one fused select/update kernel; no host round trip
+// FP64 GEMM and one fused select/update kernel; no host round trip
 // except a convergence poll every few steps.  The SCF fixed point does not
 // change: at a gapped spectrum P is exactly the aufbau projector.  Without a
 // gap (degenerate frontier levels) the error stalls and the caller falls back
@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "df32.cuh"
+#include "fixmm.cuh"
 #include "gridsync.cuh"
 #include "internal.h"
 
@@ -31,15 +32,38 @@ namespace mq {
 
 constexpr int PUR_THREADS = 1024;
 
-__device__ __forceinline__ double block_sum(double v, double *red) {
+// sums over the block of two values per thread, in every thread (red: 64); one
+// warp adds the warps' sums (each FP64 addition occupies the SM for 16 clocks
+// per warp that executes it)
+__device__ __forceinline__ void block_sum2(double &v, double &u, double *red) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 16; o > 0; o >>= 1) {
+    v += __shfl_xor_sync(0xffffffffu, v, o);
+    u += __shfl_xor_sync(0xffffffffu, u, o);
+  }
   __syncthreads();  // red may still be read from a previous call
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    red[w] = v;
+    red[32 + w] = u;
+  }
   __syncthreads();
-  double t = 0.0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-  return t;
+  if (threadIdx.x < 32) {
+    double a = threadIdx.x < nw ? red[threadIdx.x] : 0.0, c = threadIdx.x < nw ? red[32 + threadIdx.x] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      c += __shfl_xor_sync(0xffffffffu, c, o);
+    }
+    __syncwarp();
+    if (threadIdx.x == 0) {
+      red[0] = a;
+      red[32] = c;
+    }
+  }
+  __syncthreads();
+  v = red[0];
+  u = red[32];
 }
 
 __device__ __forceinline__ double block_min(double v, double *red) {
@@ -129,8 +153,7 @@ __global__ void purify_step_kernel(const double *__restrict__ X, const double *_
     tx += X[r + N * r];
     tt += T[r + N * r];
   }
-  tx = block_sum(tx, red);
-  tt = block_sum(tt, red);
+  block_sum2(tx, tt, red);
   const bool square = fabs(tt - nocc) < fabs(2.0 * tx - tt - nocc);
   if (blockIdx.x == 0 && threadIdx.x == 0) err[k] = tx - tt;
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n2; idx += (size_t)gridDim.x * blockDim.x) {
@@ -149,7 +172,11 @@ __global__ void identity_kernel(double *__restrict__ A, int n) {
 // CTA b owns the lower-triangle 16x16 tiles b, b + grid, ... of X^2.  X is
 // symmetric, so (X^2)_ij = sum_k X_ki X_kj: the tile's 16 + 16 columns are
 // staged in shared memory and each thread forms one element.  F64 = true
-// (the default): FP64 products and sums.  F64 = false (contexts whose Fock
+// (the default): the columns as fixed-point pairs (|X_ij| <= 1, so with one
+// exponent) and the product on the tensor cores, correct to FP64 rounding
+// (fixmm.cuh): two 16 x 8 fragments, each with its K range shared by four warps,
+// whose sums are added in order; on the FP64 pipe the 16 x 16 x 224 products of a
+// step took 15 us of its 25.  F64 = false (contexts whose Fock
 // digestion is double-float, mq_set_fock_precision(MQ_FOCK_DF32)): the columns
 // as double-float pairs and the products and sums in double-float on the FP32
 // pipes, which issue many times faster than FP64 on this GPU.  X itself, the
@@ -176,8 +203,7 @@ __device__ __forceinline__ void tile_of(int t, int &I, int &J) {
 // partial sums of one tile of X (lower triangle): [0] diagonal, [1] squares
 // weighted by 2 off the diagonal tiles; written to part[2 * tile + 0/1]
 __device__ __forceinline__ void tile_partials(double tr, double sq, double *red, double *part, int tile) {
-  tr = block_sum(tr, red);
-  sq = block_sum(sq, red);
+  block_sum2(tr, sq, red);
   if (threadIdx.x == 0) {
     part[2 * tile] = tr;
     part[2 * tile + 1] = sq;
@@ -189,12 +215,15 @@ __global__ void __launch_bounds__(256) purify_persist_kernel(int n, double nocc,
                                                              double *X1, double *part,
                                                              double *__restrict__ err, int *__restrict__ info,
                                                              GridSync gs) {
-  // [2][16][ld] doubles or double-float pairs (8 bytes either way), ld = n | 1:
-  // a warp's 16 columns hit 16 bank pairs
-  typedef typename std::conditional<F64, double, float2>::type Col;
+  // F64: [2][16][fx_ld(n)] fixed-point pairs, then [4][256] sums; else
+  // [2][16][ld] double-float pairs, ld = n | 1: a warp's 16 columns hit 16 bank
+  // pairs
+  typedef float2 Col;
   extern __shared__ __align__(16) unsigned char cols_raw[];
   Col *cols = (Col *)cols_raw;
-  __shared__ double red[32];
+  uint4 *U = (uint4 *)cols_raw;
+  double *ksum = (double *)(cols_raw + sizeof(uint4) * 2 * PUR_TILE * fx_ld(n));
+  __shared__ double red[64];
   const int nt = (n + PUR_TILE - 1) / PUR_TILE, ntiles = nt * (nt + 1) / 2;
   const int tid = threadIdx.x, ti = tid % PUR_TILE, tj = tid / PUR_TILE;
   const int ld = n | 1;
@@ -222,8 +251,9 @@ __global__ void __launch_bounds__(256) purify_persist_kernel(int n, double nocc,
       tr += pk[2 * t];
       sq += pk[2 * t + 1];
     }
-    const double tx = block_sum(tr, red), tt = block_sum(sq, red);
-    const double e = tx - tt;
+    block_sum2(tr, sq, red);
+    const double tx = tr, tt = sq, e = tx - tt;
+    if (!isfinite(e)) break;  // a non-finite F
     if (blockIdx.x == 0 && tid == 0) err[k] = e;
     if (settled_at < 0 && fabs(e) < PUR_SETTLED) settled_at = k;
     if (settled_at >= 0 && k >= settled_at + 2) break;
@@ -235,48 +265,74 @@ __global__ void __launch_bounds__(256) purify_persist_kernel(int n, double nocc,
       int I, J;
       tile_of(tile, I, J);
       __syncthreads();  // the previous tile's columns are no longer read
-      // 32 columns of n values, warp w staging columns w, w + 8, ..: lane e
-      // loads rows e, e + 32, .. (8 loads in flight per batch), no division
-      for (int cc = tid >> 5; cc < 2 * PUR_TILE; cc += blockDim.x >> 5) {
-        const int col = cc < PUR_TILE ? I * PUR_TILE + cc : J * PUR_TILE + cc - PUR_TILE;
-        Col *dst = cols + (size_t)cc * ld;
-        const double *src = X + N * col;
-        for (int r0 = tid & 31; r0 < n; r0 += 8 * 32) {
-          double v[8];
+      const int i = I * PUR_TILE + ti, j = J * PUR_TILE + tj;
+      double t;
+      if constexpr (F64) {
+        const int lane = tid & 31, w = tid >> 5, ldu = fx_ld(n);
+        for (int cc = w; cc < 2 * PUR_TILE; cc += blockDim.x >> 5) {
+          const int col = cc < PUR_TILE ? I * PUR_TILE + cc : J * PUR_TILE + cc - PUR_TILE;
+          const double *src = X + N * col;
+          for (int kp0 = lane; kp0 < ldu; kp0 += 4 * 32) {
+            double v[4][2];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int r = r0 + 32 * u;
-            v[u] = (col < n && r < n) ? src[r] : 0.0;
-          }
+            for (int u = 0; u < 4; ++u) {
+              const int r = 2 * (kp0 + 32 * u);
+              v[u][0] = (col < n && r < n) ? src[r] : 0.0;
+              v[u][1] = (col < n && r + 1 < n) ? src[r + 1] : 0.0;
+            }
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int r = r0 + 32 * u;
-            if (r < n) {
-              if constexpr (F64) dst[r] = v[u];
-              else dst[r] = split_f64(v[u]);
+            for (int u = 0; u < 4; ++u) {
+              const int kp = kp0 + 32 * u;
+              if (kp < ldu) U[cc * ldu + fx_pos(cc, kp)] = fx_pair(fx_fix(v[u][0], 1), fx_fix(v[u][1], 1));
             }
           }
         }
-      }
-      __syncthreads();
-      const int i = I * PUR_TILE + ti, j = J * PUR_TILE + tj;
-      const double xij = (i < n && j < n) ? X[i + N * j] : 0.0;
-      const Col *ci = cols + (size_t)ti * ld, *cj = cols + (size_t)(PUR_TILE + tj) * ld;
-      double t;
-      if constexpr (F64) {  // (X^2)_ij in FP64, four interleaved sums
-        double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
-        int r = 0;
-        for (; r + 3 < n; r += 4) {
-          t0 = fma(ci[r], cj[r], t0);
-          t1 = fma(ci[r + 1], cj[r + 1], t1);
-          t2 = fma(ci[r + 2], cj[r + 2], t2);
-          t3 = fma(ci[r + 3], cj[r + 3], t3);
+        __syncthreads();
+        // warp w: columns 8 (w & 1) .. of the tile, quarter w >> 1 of the K steps
+        const int half = 8 * (w & 1), q = w >> 1, ks = (n + 15) / 16, per = (ks + 3) / 4;
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int k0 = q * per; k0 < min(ks, (q + 1) * per); k0 += FX_KMAX / 16) {
+          float acc[FX_DIG][4];
+          fx_tile(U + 8 * k0, U + PUR_TILE * ldu + 8 * k0, ldu, PUR_TILE, PUR_TILE, 0, half,
+                  min(FX_KMAX / 16, min(ks, (q + 1) * per) - k0), acc);
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            float v[FX_DIG];
+#pragma unroll
+            for (int L = 0; L < FX_DIG; ++L) v[L] = acc[L][x];
+            s[x] += fx_combine(v, 1, 1);
+          }
         }
-        for (; r < n; ++r) t0 = fma(ci[r], cj[r], t0);
-        t = (t0 + t1) + (t2 + t3);
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+          ksum[256 * q + (lane >> 2) + 8 * (x >> 1) + PUR_TILE * (half + 2 * (lane & 3) + (x & 1))] = s[x];
+        __syncthreads();
+        t = (ksum[tid] + ksum[256 + tid]) + (ksum[512 + tid] + ksum[768 + tid]);
       } else {
+        // 32 columns of n values, warp w staging columns w, w + 8, ..: lane e
+        // loads rows e, e + 32, .. (8 loads in flight per batch), no division
+        for (int cc = tid >> 5; cc < 2 * PUR_TILE; cc += blockDim.x >> 5) {
+          const int col = cc < PUR_TILE ? I * PUR_TILE + cc : J * PUR_TILE + cc - PUR_TILE;
+          Col *dst = cols + (size_t)cc * ld;
+          const double *src = X + N * col;
+          for (int r0 = tid & 31; r0 < n; r0 += 8 * 32) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              const int r = r0 + 32 * u;
+              v[u] = (col < n && r < n) ? src[r] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              const int r = r0 + 32 * u;
+              if (r < n) dst[r] = split_f64(v[u]);
+            }
+          }
+        }
+        __syncthreads();
         // (X^2)_ij in double-float on the FP32 pipes (about 2^-48 relative per
         // product), four interleaved sums
+        const Col *ci = cols + (size_t)ti * ld, *cj = cols + (size_t)(PUR_TILE + tj) * ld;
         float2 t0 = make_float2(0.f, 0.f), t1 = t0, t2 = t0, t3 = t0;
         int r = 0;
         for (; r + 3 < n; r += 4) {
@@ -288,6 +344,7 @@ __global__ void __launch_bounds__(256) purify_persist_kernel(int n, double nocc,
         for (; r < n; ++r) dfma(t0, ci[r], cj[r]);
         t = (df_val(t0) + df_val(t1)) + (df_val(t2) + df_val(t3));
       }
+      const double xij = (i < n && j < n) ? X[i + N * j] : 0.0;
       double ptr = 0.0, psq = 0.0;
       if (i < n && j < n) {
         const double y = square ? t : 2.0 * xij - t;
@@ -309,7 +366,8 @@ __global__ void __launch_bounds__(256) purify_persist_kernel(int n, double nocc,
 static int purify_persistent(mq_ctx *c, int n, int nocc, double *d_P, double *d_W, double *d_err, int *steps) {
   const size_t n2 = (size_t)n * n;
   const int nt = (n + PUR_TILE - 1) / PUR_TILE, ntiles = nt * (nt + 1) / 2;
-  const size_t smem = (size_t)2 * PUR_TILE * (n | 1) * sizeof(double);
+  const size_t smem = c->fock_df32 ? (size_t)2 * PUR_TILE * (n | 1) * sizeof(double)
+                                   : (size_t)2 * PUR_TILE * fx_ld(n) * sizeof(uint4) + 4 * 256 * sizeof(double);
   const void *kfn = c->fock_df32 ? (const void *)purify_persist_kernel<false> : (const void *)purify_persist_kernel<true>;
   char *ws = (char *)buf(c, "purify_persist", 256 + 64 + sizeof(double) * 4 * ntiles);
   if (!ws) return MQ_ENOMEM;
@@ -411,7 +469,7 @@ int purify_projector(mq_ctx *c, int n, int nocc, const double *d_Fp, double *d_P
 // T = 1.5 I - 0.5 A (A = Z Y); err[k] = ||I - A||_F^2 (block 0)
 __global__ void ns_step_kernel(const double *__restrict__ A, int n, double *__restrict__ T, double *__restrict__ err,
                                int k) {
-  __shared__ double red[32];
+  __shared__ double red[64];
   const size_t N = n, n2 = N * N;
   double e = 0.0;
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n2; idx += (size_t)gridDim.x * blockDim.x) {
@@ -419,7 +477,8 @@ __global__ void ns_step_kernel(const double *__restrict__ A, int n, double *__re
     e += d * d;
     T[idx] = 0.5 * d + ((idx % (N + 1) == 0) ? 1.0 : 0.0);
   }
-  e = block_sum(e, red);
+  double unused = 0.0;
+  block_sum2(e, unused, red);
   if (threadIdx.x == 0) atomicAdd(err + k, e);
 }
 
