@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "jacobi.cuh"
 
 namespace mq {
 
@@ -76,10 +77,11 @@ __global__ void __launch_bounds__(RED_THREADS) energy_part_kernel(const double *
 }
 // out[2 slot] = 1/2 sum of the partials
 __global__ void energy_final_kernel(const double *__restrict__ part, int nb, double *__restrict__ out, int slot) {
-  if (threadIdx.x != 0) return;
-  double e = 0.0;
-  for (int b = 0; b < nb; ++b) e += part[b];
-  out[2 * slot] = 0.5 * e;
+  double e = 0.0;  // one warp
+  for (int b = threadIdx.x; b < nb; b += 32) e += part[b];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+  if (threadIdx.x == 0) out[2 * slot] = 0.5 * e;
 }
 
 // part[2b], part[2b+1] = partial max |Dn - Do| and sum (Dn - Do)^2
@@ -102,12 +104,17 @@ __global__ void __launch_bounds__(RED_THREADS) diff_part_kernel(const double *__
 }
 // out[0] = max |Dn - Do|, out[1] = RMS over all spin blocks
 __global__ void diff_final_kernel(const double *__restrict__ part, int nb, size_t n2, double *__restrict__ out) {
-  if (threadIdx.x != 0) return;
-  double m = 0.0, s2 = 0.0;
-  for (int b = 0; b < nb; ++b) {
+  double m = 0.0, s2 = 0.0;  // one warp
+  for (int b = threadIdx.x; b < nb; b += 32) {
     m = fmax(m, part[2 * b]);
     s2 += part[2 * b + 1];
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  }
+  if (threadIdx.x) return;
   out[0] = m;
   out[1] = sqrt(s2 / (double)n2);
 }
@@ -148,13 +155,95 @@ __global__ void __launch_bounds__(RED_THREADS) dots_part_kernel(const double *__
     if (threadIdx.x == 0) part[16 * blockIdx.x + j] = t;
   }
 }
-// B[j] = sum over CTAs of the partials, j < m
+// B[j] = sum over CTAs of the partials, j < m: one warp per j
 __global__ void dots_final_kernel(const double *__restrict__ part, int nb, int m, double *__restrict__ B) {
-  const int j = threadIdx.x;
+  const int j = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (j >= m) return;
   double t = 0.0;
-  for (int b = 0; b < nb; ++b) t += part[16 * b + j];
-  B[j] = t;
+  for (int b = lane; b < nb; b += 32) t += part[16 * b + j];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) B[j] = t;
+}
+
+// ---- Small systems (n <= SMALL_MAX, no purification): an iteration is bound by
+// its launches, so the steps around the Fock build and DIIS are one launch each,
+// one CTA per spin (grid: spins).
+constexpr int SMALL_MAX = 64;
+constexpr int SMALL_THREADS = 512;
+
+// F = H + G and out[2 s] = 1/2 sum D (F + H)
+__global__ void __launch_bounds__(SMALL_THREADS) small_fock_kernel(int n, const double *__restrict__ H,
+                                                                   const double *__restrict__ G,
+                                                                   const double *__restrict__ D, double *__restrict__ F,
+                                                                   double *__restrict__ out) {
+  __shared__ double red[32];
+  const size_t n2 = (size_t)n * n, o = n2 * blockIdx.x;
+  double e = 0.0;
+  for (size_t i = threadIdx.x; i < n2; i += blockDim.x) {
+    const double f = H[i] + G[o + i];
+    F[o + i] = f;
+    e = fma(D[o + i], f + H[i], e);
+  }
+  e = jac_block_sum(e, red);
+  if (threadIdx.x == 0) out[2 * blockIdx.x] = 0.5 * e;
+}
+
+// The density step: F' = X F X, its eigenvectors (jacobi.cuh; each with its
+// largest component positive), eps ascending, C = X V, Dn = occf C_occ C_occ^T;
+// out[3 s ..] = max |Dn - D|, sum (Dn - D)^2, 1 if the eigensolver failed.
+// The same products and eigensolver as the separate launches it replaces.
+__global__ void __launch_bounds__(SMALL_THREADS) small_density_kernel(
+    int n, const double *__restrict__ X, const double *__restrict__ F, int nocc0, int nocc1, double occf,
+    const double *__restrict__ D, double *__restrict__ C, double *__restrict__ eps, double *__restrict__ Dn,
+    double *__restrict__ out) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ double red[32];
+  const int s = blockIdx.x, nocc = s ? nocc1 : nocc0;
+  const size_t n2 = (size_t)n * n;
+  F += n2 * s, D += n2 * s, C += n2 * s, Dn += n2 * s, eps += (size_t)n * s;
+  double *A = sm, *V = sm + n2, *W = sm + 2 * n2, *sign = W + jacobi_work(n);
+  int *perm = (int *)(sign + n);
+  const JacobiWork jw(W, n);
+  cta_fix_rows(n, n, F, n, 1, jw.e1, jw.U1);  // F and X are symmetric: rows are columns
+  cta_fix_rows(n, n, X, n, 1, jw.e2, jw.U2);
+  cta_fix_mm(n, n, n, jw.U1, jw.e1, jw.U2, jw.e2, [&](int i, int j, double v) { V[i + n * j] = v; });
+  cta_fix_rows(n, n, V, n, 1, jw.e1, jw.U1);
+  cta_fix_mm(n, n, n, jw.U2, jw.e2, jw.U1, jw.e1, [&](int i, int j, double v) { A[i + n * j] = v; });
+  __syncthreads();
+  const bool ok = jacobi_block(n, A, V, red, W, 60, 1e-14);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int r = jacobi_rank(n, A, i);
+    perm[r] = i;
+    eps[r] = A[i + (size_t)n * i];
+    double big = 0.0;
+    for (int k = 0; k < n; ++k)
+      if (fabs(V[k + (size_t)n * i]) > fabs(big)) big = V[k + (size_t)n * i];
+    sign[r] = big < 0 ? -1.0 : 1.0;
+    jw.e2[i] = 1;  // |entries| of an orthogonal matrix < 2
+  }
+  __syncthreads();
+  cta_fix(n, n, true, jw.e2, jw.U2, [&](int r, int k) { return sign[r] * V[k + (size_t)n * perm[r]]; });
+  cta_fix_rows(n, n, X, n, 1, jw.e1, jw.U1);
+  cta_fix_mm(n, n, n, jw.U1, jw.e1, jw.U2, jw.e2, [&](int i, int j, double v) {
+    A[i + n * j] = v;
+    C[i + n * j] = v;
+  });
+  cta_fix_rows(n, nocc, A, 1, n, jw.e1, jw.U1);
+  double m = 0.0, s2 = 0.0;
+  cta_fix_mm(n, n, nocc, jw.U1, jw.e1, jw.U1, jw.e1, [&](int i, int j, double v) {
+    const double x = occf * v, d = x - D[i + n * j];
+    Dn[i + n * j] = x;
+    m = fmax(m, fabs(d));
+    s2 = fma(d, d, s2);
+  });
+  m = jac_block_max(m, red);
+  s2 = jac_block_sum(s2, red);
+  if (threadIdx.x == 0) {
+    out[3 * s] = m;
+    out[3 * s + 1] = s2;
+    out[3 * s + 2] = ok ? 0.0 : 1.0;
+  }
 }
 
 __global__ void lincomb_kernel(const double *F, size_t stride, const double *coef, int m, double *out, size_t n2) {
@@ -441,6 +530,11 @@ int scf_device(mq_ctx *c, const double *S, const double *H, const mq_scf_opts *o
     for (int s = 0; s < ns; ++s) MQ_TRY(density_device(c, n, nocc[s], dC + n2 * s, occf, dD + n2 * s));
   }
 
+  // small systems: the launches around the Fock build fused
+  const bool small = !purify && n <= SMALL_MAX;
+  const size_t small_smem = sizeof(double) * (2 * n2 + jacobi_work(n) + n) + sizeof(int) * n;
+  if (small)
+    MQ_CUDA(c, cudaFuncSetAttribute(small_density_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem));
   const double enuc = nuclear_repulsion(c);
   StageTimer t_fock, t_diag, t_all, t_full;  // t_full: the full builds of a screened-increment SCF
   c->t_fock_kernel.collect();
@@ -518,8 +612,9 @@ int scf_device(mq_ctx *c, const double *S, const double *H, const mq_scf_opts *o
       have_prev_g = true;
     }
     t_fock.stop(c->stream);
-    for (int s = 0; s < ns; ++s) add_kernel<<<blocks(n2), 256, 0, c->stream>>>(dH, dG + n2 * s, dF + n2 * s, n2);
-    for (int s = 0; s < ns; ++s) {
+    if (small) small_fock_kernel<<<ns, SMALL_THREADS, 0, c->stream>>>(n, dH, dG, dD, dF, dScal);
+    for (int s = 0; s < ns && !small; ++s) add_kernel<<<blocks(n2), 256, 0, c->stream>>>(dH, dG + n2 * s, dF + n2 * s, n2);
+    for (int s = 0; s < ns && !small; ++s) {
       energy_part_kernel<<<RED_BLOCKS, RED_THREADS, 0, c->stream>>>(dD + n2 * s, dF + n2 * s, dH, n2, dRed);
       energy_final_kernel<<<1, 32, 0, c->stream>>>(dRed, RED_BLOCKS, dScal, s);
     }
@@ -539,7 +634,7 @@ int scf_device(mq_ctx *c, const double *S, const double *H, const mq_scf_opts *o
       std::vector<double> row(ndiis, 0.0);
       for (int s = 0; s < ns; ++s) {
         dots_part_kernel<<<RED_BLOCKS, RED_THREADS, 0, c->stream>>>(dEh + n2 * s, n2, head, nh, n2 * ns, dRed);
-        dots_final_kernel<<<1, 32, 0, c->stream>>>(dRed, RED_BLOCKS, nh, dScal + 16 + 16 * s);
+        dots_final_kernel<<<1, 32 * 16, 0, c->stream>>>(dRed, RED_BLOCKS, nh, dScal + 16 + 16 * s);
       }
       std::vector<double> hrow(32);
       MQ_CUDA(c, cudaMemcpyAsync(hrow.data(), dScal + 16, 32 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -568,15 +663,29 @@ int scf_device(mq_ctx *c, const double *S, const double *H, const mq_scf_opts *o
       early_done = true;
     }
     t_diag.start(c->stream);
-    MQ_TRY(density_step(Fdiag, dDn));
+    if (small) {
+      small_density_kernel<<<ns, n <= 16 ? 128 : (n <= 32 ? 256 : SMALL_THREADS), small_smem, c->stream>>>(n, dX, Fdiag, nocc[0], nocc[1], occf, dD, dC,
+                                                                         dEps, dDn, dScal + 8);
+      MQ_CUDA(c, cudaGetLastError());
+      c->stats.diag_calls += 1;
+    } else {
+      MQ_TRY(density_step(Fdiag, dDn));
+    }
     t_diag.stop(c->stream);
     lastF = Fdiag;
-    diff_part_kernel<<<RED_BLOCKS, RED_THREADS, 0, c->stream>>>(dDn, dD, n2 * ns, dRed);
-    diff_final_kernel<<<1, 32, 0, c->stream>>>(dRed, RED_BLOCKS, n2 * ns, dScal + 8);
-    c->stats.launches += 2 + 2 * ns;
-    double hs[10];
-    MQ_CUDA(c, cudaMemcpyAsync(hs, dScal, 10 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    if (!small) {
+      diff_part_kernel<<<RED_BLOCKS, RED_THREADS, 0, c->stream>>>(dDn, dD, n2 * ns, dRed);
+      diff_final_kernel<<<1, 32, 0, c->stream>>>(dRed, RED_BLOCKS, n2 * ns, dScal + 8);
+    }
+    c->stats.launches += small ? 2 : 2 + 2 * ns;
+    double hs[14];
+    MQ_CUDA(c, cudaMemcpyAsync(hs, dScal, 14 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     MQ_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (small) {  // per spin: max, sum of squares, failure
+      if (hs[10] != 0.0 || (uhf && hs[13] != 0.0)) return set_err(c, MQ_ENOCONV, "Jacobi eigensolver did not converge");
+      hs[8] = uhf ? std::max(hs[8], hs[11]) : hs[8];
+      hs[9] = std::sqrt((hs[9] + (uhf ? hs[12] : 0.0)) / (double)(n2 * ns));
+    }
     t_fock.collect();
     t_full.collect();
     t_diag.collect();
