@@ -165,6 +165,11 @@ int mq_free(mq_ctx *c) {
   if (c->pin) cudaFreeHost(c->pin);
   cudaStreamDestroy(c->stream);
   if (c->side) cudaStreamDestroy(c->side);
+  for (int k = 0; k < 5; ++k) {
+    if (c->fork[k]) cudaStreamDestroy(c->fork[k]);
+    if (c->ev_join[k]) cudaEventDestroy(c->ev_join[k]);
+  }
+  if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->aux) cudaStreamDestroy(c->aux);
   if (c->ev_params) cudaEventDestroy(c->ev_params);
   if (c->ev_early) cudaEventDestroy(c->ev_early);

@@ -108,44 +108,91 @@ static int compact_quartets(mq_ctx *c, EriArgs &h, int slot) {
   return MQ_OK;
 }
 
+// The class combinations write different integrals, so they may run side by
+// side: a small molecule's launches are one wave or less, each as long as its
+// slowest thread (0.2-0.9 ms at (H2O)8), and on forked streams the pass takes
+// the longest of them instead of their sum.  Larger passes fill the GPU one by
+// one.
+constexpr long long FORK_MAX_QUARTETS = 1 << 18;
+
+static int ensure_fork(mq_ctx *c) {
+  if (c->ev_fork) return MQ_OK;
+  int lo = 0, hi = 0;
+  MQ_CUDA(c, cudaDeviceGetStreamPriorityRange(&lo, &hi));
+  for (int k = 0; k < 5; ++k) {
+    if (!c->fork[k]) MQ_CUDA(c, cudaStreamCreateWithPriority(&c->fork[k], cudaStreamNonBlocking, hi));
+    if (!c->ev_join[k]) MQ_CUDA(c, cudaEventCreateWithFlags(&c->ev_join[k], cudaEventDisableTiming));
+  }
+  MQ_CUDA(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+  return MQ_OK;
+}
+
+template <int EPI>
+static int run_combo(mq_ctx *c, const EriArgs &g, int cP, int cQ);
+
 template <int EPI>
 static int run_all(mq_ctx *c, EriArgs g) {
-  const int *off = c->pt.class_off;
-  for (int cP = 0; cP < 3; ++cP)
-    for (int cQ = 0; cQ <= cP; ++cQ) {
-      const int nP = off[cP + 1] - off[cP], nQ = off[cQ + 1] - off[cQ];
-      if (nP == 0 || nQ == 0) continue;
-      EriArgs h = g;
-      h.pOff = off[cP];
-      h.nP = nP;
-      h.qOff = off[cQ];
-      h.nQ = nQ;
-      h.tri = cP == cQ;
-      h.diag = 0;
-      h.nq = h.tri ? (long long)nP * (nP + 1) / 2 : (long long)nP * nQ;
-      h.list = nullptr;
-      h.list_n = nullptr;
-      const int slot = cP * (cP + 1) / 2 + cQ;
-      if constexpr (EPI == EPI_XX) {
-        if (g.boys_f && c->eri_f32_tau > h.thr) {
-          // mixed precision: bounds >= tau in FP64, [thr, tau) in FP32
-          EriArgs h64 = h, h32 = h;
-          h64.thr = c->eri_f32_tau;
-          h64.thr_hi = 0.0;
-          MQ_TRY(compact_quartets(c, h64, slot));
-          MQ_TRY(launch_class<EPI>(c, h64, cP, cQ));
-          h32.thr = std::max(h.thr, 1e-300);
-          h32.thr_hi = c->eri_f32_tau;
-          h32.counters = h.counters ? h.counters + 2 : nullptr;
-          MQ_TRY(compact_quartets(c, h32, slot + 8));
-          MQ_TRY((launch_class<EPI, float>(c, h32, cP, cQ)));
-          continue;
-        }
+  const long long np = c->pt.npairs;
+  const bool fork = EPI == EPI_XX && np * (np + 1) / 2 <= FORK_MAX_QUARTETS;
+  if (fork) {
+    MQ_TRY(ensure_fork(c));
+    MQ_CUDA(c, cudaEventRecord(c->ev_fork, c->stream));
+  }
+  int k = 0;
+  // the heaviest combination first, on the context's own stream
+  for (int cP = 2; cP >= 0; --cP)
+    for (int cQ = cP; cQ >= 0; --cQ, ++k) {
+      if (!fork || k == 0) {
+        MQ_TRY(run_combo<EPI>(c, g, cP, cQ));
+        continue;
       }
-      if (h.thr > 0.0) MQ_TRY(compact_quartets(c, h, slot));
-      MQ_TRY(launch_class<EPI>(c, h, cP, cQ));
+      cudaStream_t main = c->stream, s = c->fork[k - 1];
+      MQ_CUDA(c, cudaStreamWaitEvent(s, c->ev_fork, 0));
+      c->stream = s;
+      const int rc = run_combo<EPI>(c, g, cP, cQ);
+      c->stream = main;
+      // joined whatever was queued
+      MQ_CUDA(c, cudaEventRecord(c->ev_join[k - 1], s));
+      MQ_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join[k - 1], 0));
+      MQ_TRY(rc);
     }
   return MQ_OK;
+}
+
+template <int EPI>
+static int run_combo(mq_ctx *c, const EriArgs &g, int cP, int cQ) {
+  const int *off = c->pt.class_off;
+  const int nP = off[cP + 1] - off[cP], nQ = off[cQ + 1] - off[cQ];
+  if (nP == 0 || nQ == 0) return MQ_OK;
+  EriArgs h = g;
+  h.pOff = off[cP];
+  h.nP = nP;
+  h.qOff = off[cQ];
+  h.nQ = nQ;
+  h.tri = cP == cQ;
+  h.diag = 0;
+  h.nq = h.tri ? (long long)nP * (nP + 1) / 2 : (long long)nP * nQ;
+  h.list = nullptr;
+  h.list_n = nullptr;
+  const int slot = cP * (cP + 1) / 2 + cQ;
+  if constexpr (EPI == EPI_XX) {
+    if (g.boys_f && c->eri_f32_tau > h.thr) {
+      // mixed precision: bounds >= tau in FP64, [thr, tau) in FP32
+      EriArgs h64 = h, h32 = h;
+      h64.thr = c->eri_f32_tau;
+      h64.thr_hi = 0.0;
+      MQ_TRY(compact_quartets(c, h64, slot));
+      MQ_TRY(launch_class<EPI>(c, h64, cP, cQ));
+      h32.thr = std::max(h.thr, 1e-300);
+      h32.thr_hi = c->eri_f32_tau;
+      h32.counters = h.counters ? h.counters + 2 : nullptr;
+      MQ_TRY(compact_quartets(c, h32, slot + 8));
+      MQ_TRY((launch_class<EPI, float>(c, h32, cP, cQ)));
+      return MQ_OK;
+    }
+  }
+  if (h.thr > 0.0) MQ_TRY(compact_quartets(c, h, slot));
+  return launch_class<EPI>(c, h, cP, cQ);
 }
 
 int eri_schwarz(mq_ctx *c) {

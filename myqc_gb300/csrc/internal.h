@@ -232,6 +232,9 @@ struct mq_ctx {
   // stream; ev_params marks the last write of the network's parameters
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_params = nullptr;
+  // streams of an integral pass whose class combinations run side by side (eri.cu)
+  cudaStream_t fork[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  cudaEvent_t ev_fork = nullptr, ev_join[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   cudaEvent_t ev_early = nullptr;  // the SCF's early eigensolve on the aux stream
   int ao2mo_prefetch = 0;  // planes (2, 3) to slice XX into ahead of the transform; 0: off
   int xx_sliced = 0;       // the slice buffers hold XX cut into this many planes (0: not)
