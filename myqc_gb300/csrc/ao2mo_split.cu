@@ -268,30 +268,39 @@ __device__ __forceinline__ int exp_field(double x) {
   return (int)((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ff;
 }
 __device__ __forceinline__ int exp_field(float x) { return (__float_as_int(x) >> 23) & 0xff; }
-// value = mant * 2^(ex) with mant the full integer significand (implicit bit set)
-__device__ __forceinline__ void decompose(double x, long long &mant, int &ex) {
+// y with round(y) = round(x 2^(8 S - 1 - erow)), halves up, for |x| < 2^erow (a row's exponent).
+template <int S>
+__device__ __forceinline__ float row_scaled(double x, int erow, float) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int E = (int)(b >> 52) & 0x7ff;
-  if (E == 0) {  // zero (subnormals are far below any slice)
-    mant = 0;
-    ex = 0;
-    return;
-  }
-  mant = (long long)((b & 0xfffffffffffffull) | 0x10000000000000ull);
-  if (b >> 63) mant = -mant;
-  ex = E - 1075;
+  const int E = (int)(b >> 52) & 0x7ff, sh = erow - E + 1076 - 8 * S;  // sh >= 1
+  if (E == 0 || sh >= 62) return 0.f;  // (subnormals are far below any slice)
+  const long long m = (long long)((b & 0xfffffffffffffull) | 0x10000000000000ull);
+  return (float)(int)(((b >> 63 ? -m : m) + (1ll << (sh - 1))) >> sh);
 }
-__device__ __forceinline__ void decompose(float x, long long &mant, int &ex) {
-  const unsigned b = (unsigned)__float_as_int(x);
-  const int E = (int)(b >> 23) & 0xff;
-  if (E == 0) {
-    mant = 0;
-    ex = 0;
-    return;
+template <int S>
+__device__ __forceinline__ float row_scaled(float x, int, float scale) {
+  return x * scale;
+}
+// The balanced digits of q = floor(y + 1/2), |y| <= 2^(8 S - 1): q = sum d[i] 256^(S - 1 - i),
+// d in [-128, 127] but for d[0] = 128.  FP32 additions and multiply-adds alone: the integer form
+// (shifts, masks, bytes: half their rate) bound the slicing, not memory.  A sum
+// with 1.5 2^23 rounded down is the floor of the other term.
+__device__ __forceinline__ float floor_of(float x, float f) {
+  return __fmaf_rd(x, f, 12582912.f) - 12582912.f;
+}
+template <int S>
+__device__ __forceinline__ void row_digits(float y, float (&d)[S]) {
+  // floor((q + 128) / 256) = floor((y + 128.5) / 256), whatever the sum loses below its last bit
+  float hi = floor_of(__fadd_rd(y, 128.5f), 0.00390625f);
+  const float lo = fmaf(hi, -256.f, y);  // exact
+  d[S - 1] = floor_of(__fadd_rd(lo, 0.5f), 1.f);
+#pragma unroll
+  for (int i = S - 2; i > 0; --i) {
+    const float up = floor_of(hi + 128.f, 0.00390625f);
+    d[i] = fmaf(up, -256.f, hi);
+    hi = up;
   }
-  mant = (long long)((b & 0x7fffffu) | 0x800000u);
-  if (b >> 31) mant = -mant;
-  ex = E - 150;
+  d[0] = hi;
 }
 
 // One warp per row: the r-th row at in + r*ld (kvalid values) becomes S planes
@@ -335,8 +344,7 @@ __device__ __forceinline__ void load_chunk(const T *__restrict__ x, int k0, int 
 //   ROW_SYMM   row (v, jb) of the pair-packed Y2: element u is
 //              in[jb * npairs + pidx(min(u, v), max(u, v))], pidx(u, v) = u + v (v + 1) / 2.
 //   ROW_TRANS  row (b, p) of the [p][l][b] array the store's first quarter
-//              writes: element l at in[(p n + l) nb + b]; the rows are visited
-//              with b fastest, so the warps reading one p share its sectors
+//              writes: element l at in[(p n + l) nb + b]
 enum { ROW_PLAIN = 0, ROW_PAIRS = 1, ROW_SYMM = 2, ROW_TRANS = 3 };
 struct StoreView {
   const double *X;
@@ -349,6 +357,7 @@ struct StoreView {
   const double *pbound;  // Schwarz bound of each pair
   const double *qmax;    // per shell: the largest bound of a pair containing it
   const int *partners;   // per shell S: the shells D by the bound of the pair (D, S), descending
+  const int4 *plist;     // the same as records: the bound's bits, the rank, a0 << 16 | na << 8 | class << 2 | flags
   double thr;            // the store's threshold
 };
 struct RowSrc {
@@ -367,15 +376,30 @@ __device__ __forceinline__ void slice_row_regs(T (&v)[H][8], long long r, int nc
                                                bf16 *__restrict__ out, int *__restrict__ e) {
   const int lane = threadIdx.x & 31;
   int emax = 0;
+  float amax = 0.f;
 #pragma unroll
   for (int h = 0; h < H; ++h)
     if (lane + 32 * h < nchunk)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) emax = max(emax, exp_field(v[h][j]));
+      for (int j = 0; j < 8; ++j)
+        if (sizeof(T) == 8) emax = max(emax, exp_field(v[h][j]));
+        else amax = fmaxf(amax, fabsf((float)v[h][j]));
+  if (sizeof(T) == 4) emax = exp_field(amax);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
   // |x| < 2^erow with erow = unbiased exponent of the largest element + 1
   const int erow = emax == 0 ? -200 : emax - (sizeof(T) == 8 ? 1022 : 126);
+  float scale = 0.f;
+  if (sizeof(T) == 4) {
+    // 2^(8 S - 1 - erow), a normal number for |x| down to 2^-100; smaller rows are scaled up first
+    const int up = erow < -100 ? 64 : 0;
+    if (up)
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[h][j] = emax ? v[h][j] * (T)18446744073709551616.0 : (T)0;
+    scale = __int_as_float((max(127 + 8 * S - 1 - erow - up, 1) & 0xff) << 23);
+  }
   if (lane == 0) e[r] = erow;
 #pragma unroll
   for (int h = 0; h < H; ++h) {
@@ -384,29 +408,12 @@ __device__ __forceinline__ void slice_row_regs(T (&v)[H][8], long long r, int nc
     unsigned packed[S][4];
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {
-      float dig[2][S];
+      float f0[S], f1[S];
+      row_digits<S>(row_scaled<S>(v[h][j], erow, scale), f0);
+      row_digits<S>(row_scaled<S>(v[h][j + 1], erow, scale), f1);
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        long long mant;
-        int ex;
-        decompose(v[h][j + t], mant, ex);
-        // q = round(mant * 2^(ex + 8S - 1 - erow)); the shift is negative for every nonzero x
-        const int sh = -(ex + 8 * S - 1 - erow);
-        int q = 0;
-        if (mant != 0 && sh < 62) q = (int)(sh > 0 ? ((mant + (1ll << (sh - 1))) >> sh) : (mant << -sh));
-#pragma unroll
-        for (int d = S - 1; d > 0; --d) {
-          const int hi = (q + 128) >> 8;  // balanced digit: q = hi*256 + lo, lo in [-128, 127]
-          dig[t][d] = (float)(q - hi * 256);
-          q = hi;
-        }
-        dig[t][0] = (float)q;
-      }
-#pragma unroll
-      for (int d = 0; d < S; ++d) {
-        const __nv_bfloat162 b2 = __floats2bfloat162_rn(dig[0][d], dig[1][d]);
-        packed[d][j >> 1] = *reinterpret_cast<const unsigned *>(&b2);
-      }
+      for (int d = 0; d < S; ++d)  // at most 8 bits: the upper half is the BF16
+        packed[d][j >> 1] = __byte_perm(__float_as_uint(f0[d]), __float_as_uint(f1[d]), 0x7632u);
     }
 #pragma unroll
     for (int d = 0; d < S; ++d)
@@ -423,43 +430,77 @@ __global__ void __launch_bounds__(256, 4) slice_rows_kernel(const T *__restrict_
   const int lane = threadIdx.x & 31;
   const int nchunk = Kp >> 3;
   for (long long ri = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); ri < rows; ri += warps) {
-    long long r = ri;
-    const T *x = in + r * ld;
-    long long jb = 0;
-    int vrow = 0;
-    if (MODE == ROW_TRANS) {
-      const long long p = ri / rs.nb, b = ri - p * rs.nb;
-      r = b * rs.npairs + p;
-      x = in + p * rs.n * rs.nb + b;
-    } else if (MODE == ROW_PAIRS) {
-      const long long pidx = r / rs.n;
+    const T *x = in + ri * ld;
+    if (MODE == ROW_PAIRS) {
+      const long long pidx = ri / rs.n;
       const int2 uv = rs.pairs[pidx];
-      x = in + ((r - pidx * rs.n) + rs.n * (uv.x + rs.n * (long long)uv.y)) * ld;
-    } else if (MODE == ROW_SYMM) {
-      jb = r / rs.n;
-      vrow = (int)(r - jb * rs.n);
-      x = in + jb * rs.npairs;
+      x = in + ((ri - pidx * rs.n) + rs.n * (uv.x + rs.n * (long long)uv.y)) * ld;
     }
     T v[H][8];
 #pragma unroll
+    for (int h = 0; h < H; ++h)
+      if (lane + 32 * h < nchunk) load_chunk(x, 8 * (lane + 32 * h), kvalid, vec != 0, v[h]);
+    slice_row_regs<S, T, H>(v, ri, nchunk, Kp, plane, out, e);
+  }
+}
+
+// The same for rows whose elements are not contiguous (ROW_SYMM, ROW_TRANS):
+// read one by one, each warp load touched 28 lines and the kernels were bound by L1's
+// lookups.  A CTA takes 32 rows through shared memory: loads run along the source's contiguous index (b; v for u > v, u for
+// u <= v), element k of row i lies at i * ldp + k + k / 8 with ldp odd, so that
+// both these stores and the lanes' 8-element chunks are free of conflicts.
+// With the digits in FP32 (row_digits), (H2O)32, n = 224: 1.62 -> 1.14 ms (2.3M
+// rows, ROW_SYMM) and 1.30 -> 1.12 ms (1.6M rows, ROW_TRANS).
+constexpr int TILE_ROWS = 32;
+static __host__ __device__ __forceinline__ int tile_ldp(int nchunk) { return (9 * nchunk) | 1; }
+template <int S, int H, int MODE>
+__global__ void __launch_bounds__(256) slice_tile_kernel(const float *__restrict__ in, long long rows, int n, int Kp,
+                                                         long long plane, bf16 *__restrict__ out, int *__restrict__ e,
+                                                         RowSrc rs) {
+  extern __shared__ float ts[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int nchunk = Kp >> 3, ldp = tile_ldp(nchunk);
+  long long ri, r;  // the lane's row of the tile, as it is visited and as it is written
+  int nrow;
+  if (MODE == ROW_TRANS) {  // 32 consecutive (p, b), b fastest
+    const long long r0 = (long long)blockIdx.x * TILE_ROWS;
+    nrow = (int)min((long long)TILE_ROWS, rows - r0);
+    ri = r0 + lane;
+    const long long p = ri / rs.nb, b = ri - p * rs.nb;
+    r = b * rs.npairs + p;
+    const float *x = in + p * n * rs.nb + b;
+    if (lane < nrow)
+#pragma unroll 8
+      for (int k = w; k < n; k += nw) ts[lane * ldp + k + (k >> 3)] = __ldg(x + k * rs.nb);
+  } else {  // 32 consecutive v of one jb
+    const int nt = (n + TILE_ROWS - 1) / TILE_ROWS;
+    const long long jb = blockIdx.x / nt;
+    const int v0 = (int)(blockIdx.x - jb * nt) * TILE_ROWS;
+    nrow = min(TILE_ROWS, n - v0);
+    r = jb * n + v0 + lane;
+    const float *x = in + jb * rs.npairs;
+    for (int i = w; i < nrow; i += nw) {
+      const int v = v0 + i;
+      const float *xv = x + (long long)v * (v + 1) / 2;
+#pragma unroll 4
+      for (int u = lane; u <= v; u += 32) ts[i * ldp + u + (u >> 3)] = __ldg(xv + u);
+    }
+    const int v = v0 + lane;
+    if (lane < nrow)
+#pragma unroll 4
+      for (int u = v0 + 1 + w; u < n; u += nw)
+        if (u > v) ts[lane * ldp + u + (u >> 3)] = __ldg(x + v + (long long)u * (u + 1) / 2);
+  }
+  __syncthreads();
+  for (int i = w; i < nrow; i += nw) {
+    float v[H][8];
+#pragma unroll
     for (int h = 0; h < H; ++h) {
       const int c = lane + 32 * h;
-      if (c < nchunk) {
-        if (MODE == ROW_SYMM) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int u = 8 * c + j, lo = min(u, vrow), hi = max(u, vrow);
-            v[h][j] = u < kvalid ? __ldg(x + lo + (long long)hi * (hi + 1) / 2) : (T)0;
-          }
-        } else if (MODE == ROW_TRANS) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[h][j] = 8 * c + j < kvalid ? __ldg(x + (8 * c + j) * rs.nb) : (T)0;
-        } else {
-          load_chunk(x, 8 * c, kvalid, vec != 0, v[h]);
-        }
-      }
+      for (int j = 0; j < 8; ++j) v[h][j] = 8 * c + j < n ? ts[i * ldp + 9 * c + j] : 0.f;
     }
-    slice_row_regs<S, T, H>(v, r, nchunk, Kp, plane, out, e);
+    slice_row_regs<S, float, H>(v, __shfl_sync(0xffffffffu, r, i), nchunk, Kp, plane, out, e);
   }
 }
 
@@ -473,33 +514,14 @@ struct LiveBlock {
   long long off;  // the block in the store
   int a0;         // first AO of D
   int flags;      // bit0: (D, L) stored as (L, D); bit1: D = L; bit2: (D, L) is the bra; bit3: (D, L) = (U, V);
-                  // bits 4, 5, 6: 4 functions in the block's second, third, fourth shell; bits 8-11: AOs of D
+                  // bits 8-11: AOs of D
 };
 
-// the store offset of the element (d l|u v) of a listed block; (i2, f2) and
-// (j2, g2): the AOs of (u, v) and their function indices, in the stored
-// orientation of (U, V)
-__device__ __forceinline__ long long live_offset(const LiveBlock &b, int d, int fd, int l, int fl, int i2, int f2,
-                                                 int j2, int g2, int n) {
-  int i1 = d, fi1 = fd, j1 = l, fj1 = fl;
-  if (b.flags & 1) {
-    i1 = l, fi1 = fl, j1 = d, fj1 = fd;
-  }
-  if ((b.flags & 2) && i1 < j1) {  // A = B: the canonical element has i >= j
-    const int t = i1, ft = fi1;
-    i1 = j1, fi1 = fj1, j1 = t, fj1 = ft;
-  }
-  const bool bra1 = b.flags & 4;
-  int ia = bra1 ? i1 : i2, fa = bra1 ? fi1 : f2, ja = bra1 ? j1 : j2, fb = bra1 ? fj1 : g2;
-  int ka = bra1 ? i2 : i1, fc = bra1 ? f2 : fi1, la = bra1 ? j2 : j1, fdd = bra1 ? g2 : fj1;
-  if ((b.flags & 8) && (long long)ia * n + ja < (long long)ka * n + la) {  // P = Q: ij >= kl
-    int t = fa;
-    fa = fc, fc = t;
-    t = fb;
-    fb = fdd, fdd = t;
-  }
-  const int NB = (b.flags & 16) ? 4 : 1, NC = (b.flags & 32) ? 4 : 1, ND = (b.flags & 64) ? 4 : 1;
-  return b.off + ((fa * NB + fb) * NC + fc) * ND + fdd;
+// place of the functions (f, g) of the shells F, G in their pair's block: stored
+// as (G, F) with `swap`; one shell with itself holds f >= g
+__device__ __forceinline__ int pair_place(int f, int nf, int g, int ng, bool swap, bool same) {
+  if (same) return max(f, g) * ng + min(f, g);
+  return swap ? g * nf + f : f * ng + g;
 }
 
 // ---- The first quarter transform straight from the quartet store.
@@ -516,9 +538,18 @@ __device__ __forceinline__ long long live_offset(const LiveBlock &b, int d, int 
 // columns b = k + 32 j, and each gathered element is one shared-memory
 // broadcast for KB multiply-adds per lane.  Every lane is busy whatever the
 // row count, and only stored elements are visited.
+//
+// The groups are small (5 rows by 25 AOs on average for (H2O)32), so the time is
+// the latency of their listing and of the gather's addresses, and instruction
+// fetches.  Hence: one record per partner in place of four dependent
+// tables (fq_partner_kernel); a lane gathers for one row of the pass, whose place
+// in the blocks is found once; groups taken from a counter by CTAs that all reside
+// (four per SM, C through L1; two with C in shared memory: 3.8 ms), four
+// shells L at a time (16: 3.2 ms, 8: 2.8).  (H2O)32, n = 224, 64 columns, 36.5M stored
+// elements: 5.96 -> 2.7 ms (1.44 GB of Y1 written: 0.2 ms).
 constexpr int FQ_ROWS = 8;
 constexpr int FQ_KCHUNK = 64;  // listed AOs gathered at a time
-constexpr int FQ_LCH = 16;      // shells L per group
+constexpr int FQ_LCH = 4;      // shells L per group
 constexpr int FQ_GATHER = 2;    // gathered elements in flight per lane
 
 // row f of a group: AO pair (u, v) number f / nl of the shells U <= V (u <= v),
@@ -539,59 +570,47 @@ __device__ __forceinline__ void fq_row(int f, int nl, int u0, int nu, int v0, in
 }
 
 // rows f0 .. f0 + nr - 1 of the group (nr <= R; the others of the pass are zeros, not written).
-// Not inlined: the three pass widths would otherwise triple the kernel's code,
-// and its instruction fetches were a leading stall.
 template <int KB, int R>
-__device__ __noinline__ void fq_pass(const StoreView &sv, int n, int Kp, const float *Cf, int nvb,
-                                        float *__restrict__ Y1, long long np, const int *dl, const LiveBlock *tab,
-                                        int nd, float *Vs, int f0, int nr, int nl, int l0, int u0, int nu, int v0,
-                                        int nv, bool same, int4 e2) {
-  const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void fq_pass(const double *__restrict__ X, int n, const float *__restrict__ Cf, int nvb,
+                                     float *__restrict__ Y1, const int *dl, const LiveBlock *tab, int nd, float *Vs,
+                                     int f0, int nr, int nl, int l0, int u0, int nu, int v0, int nv, bool same,
+                                     bool swap2) {
+  const int lane = threadIdx.x & 31, rr = lane % R;
+  // the lane's row in the gather
+  int gu, gv, fl;
+  fq_row(f0 + min(rr, nr - 1), nl, u0, nu, v0, nv, same, gu, gv, fl);
+  const int c2 = pair_place(gu - u0, nu, gv - v0, nv, swap2, same), n2 = nu * nv;
   float acc[R][KB];
 #pragma unroll
-  for (int rr = 0; rr < R; ++rr)
+  for (int i = 0; i < R; ++i)
 #pragma unroll
-    for (int j = 0; j < KB; ++j) acc[rr][j] = 0.f;
+    for (int j = 0; j < KB; ++j) acc[i][j] = 0.f;
   // the listed AOs in chunks of FQ_KCHUNK: gather the chunk's elements, then
   // its products
   for (int kc = 0; kc < nd; kc += FQ_KCHUNK) {
     const int kn = min(FQ_KCHUNK, nd - kc);
-    // gather: element (k, rr) by lane (k * R + rr) mod 32; FQ_GATHER
-    // elements per lane at a time -- their offsets first, then every load in
-    // flight together, then the shared-memory stores
-    for (int base = 0; base < kn * R; base += 32 * FQ_GATHER) {
-      long long off[FQ_GATHER];
-#pragma unroll
-      for (int t = 0; t < FQ_GATHER; ++t) {
-        off[t] = -1;
-        const int idx = base + lane + 32 * t;
-        if (idx >= kn * R) continue;
-        const int k = idx / R, rr = idx - k * R;
-        if (rr >= nr) continue;
-        int u, v, l;
-        fq_row(f0 + rr, nl, u0, nu, v0, nv, same, u, v, l);
-        int i2 = u, f2 = u - u0, j2 = v, g2 = v - v0;
-        if (e2.w & 1) {
-          i2 = v, f2 = v - v0, j2 = u, g2 = u - u0;
-        }
-        if ((e2.w & 2) && i2 < j2) {
-          const int tt = i2, ft = f2;
-          i2 = j2, f2 = g2, j2 = tt, g2 = ft;
-        }
-        const int e = dl[kc + k], d = e & 0xffff;
-        const LiveBlock b = tab[e >> 16];
-        off[t] = live_offset(b, d, d - b.a0, l0 + l, l, i2, f2, j2, g2, n);
-      }
+    // gather: row rr by the lanes rr + R i, FQ_GATHER elements per lane at a
+    // time -- their loads in flight together, then the shared-memory stores
+    for (int k0 = lane / R; k0 < kn; k0 += 32 / R * FQ_GATHER) {
       double x[FQ_GATHER];
 #pragma unroll
-      for (int t = 0; t < FQ_GATHER; ++t) x[t] = off[t] >= 0 ? __ldg(sv.X + off[t]) : 0.0;
+      for (int t = 0; t < FQ_GATHER; ++t) {
+        const int k = k0 + 32 / R * t;
+        x[t] = 0.0;
+        if (k < kn && rr < nr) {
+          const int e = dl[kc + k];
+          const LiveBlock b = tab[e >> 16];
+          const int nd1 = (b.flags >> 8) & 15;
+          const int c1 = pair_place((e & 0xffff) - b.a0, nd1, fl, nl, b.flags & 1, b.flags & 2);
+          int o = b.flags & 4 ? c1 * n2 + c2 : c2 * (nd1 * nl) + c1;
+          if (b.flags & 8) o = max(c1, c2) * n2 + min(c1, c2);  // one pair with itself holds ij >= kl
+          x[t] = __ldg(X + b.off + o);
+        }
+      }
 #pragma unroll
       for (int t = 0; t < FQ_GATHER; ++t) {
-        const int idx = base + lane + 32 * t;
-        if (idx < kn * R) {
-          const int k = idx / R, rr = idx - k * R;
-          Vs[k * FQ_ROWS + rr] = (float)x[t];
-        }
+        const int k = k0 + 32 / R * t;
+        if (k < kn) Vs[k * FQ_ROWS + rr] = (float)x[t];
       }
     }
     __syncwarp();
@@ -616,45 +635,38 @@ __device__ __noinline__ void fq_pass(const StoreView &sv, int n, int Kp, const f
         }
       } else {
 #pragma unroll
-        for (int rr = 0; rr < R; ++rr)
+        for (int i = 0; i < R; ++i)
 #pragma unroll
-          for (int j = 0; j < KB; ++j) acc[rr][j] = fmaf(cv[j], x[rr], acc[rr][j]);
+          for (int j = 0; j < KB; ++j) acc[i][j] = fmaf(cv[j], x[i], acc[i][j]);
       }
     }
     __syncwarp();  // Vs is read before the next chunk's gather
   }
 #pragma unroll
-  for (int rr = 0; rr < R; ++rr) {
-    if (rr >= nr) break;
+  for (int i = 0; i < R; ++i) {
+    if (i >= nr) break;
     int u, v, l;
-    fq_row(f0 + rr, nl, u0, nu, v0, nv, same, u, v, l);
+    fq_row(f0 + i, nl, u0, nu, v0, nv, same, u, v, l);
     const long long p = (long long)u + (long long)v * (v + 1) / 2;
 #pragma unroll
     for (int j = 0; j < KB; ++j) {
       const int bb = lane + 32 * j;
-      if (bb < nvb) Y1[((size_t)p * n + l0 + l) * nvb + bb] = acc[rr][j];
+      if (bb < nvb) Y1[((size_t)p * n + l0 + l) * nvb + bb] = acc[i][j];
     }
   }
 }
 
 template <int KB>
-__global__ void __launch_bounds__(256, 2) store_first_quarter_kernel(const StoreView sv, int n, int Kp,
-                                                                   const float *Cf, int nvb, int cs_floats,
-                                                                   float *__restrict__ Y1, long long np,
-                                                                   long long ngroups) {
+__global__ void __launch_bounds__(256, KB <= 2 ? 4 : 2) store_first_quarter_kernel(const StoreView sv, int n,
+                                                                   const float *__restrict__ Cf, int nvb,
+                                                                   float *__restrict__ Y1, long long ngroups,
+                                                                   int *next) {
   extern __shared__ __align__(16) unsigned char fq_sm_raw[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int nsh = sv.nsh;
-  // C in shared memory when it fits (cs_floats > 0), then per warp: gathered
-  // elements [FQ_KCHUNK][FQ_ROWS] floats, listed blocks [nsh], listed AOs [n]
-  float *Cs = reinterpret_cast<float *>(fq_sm_raw);
-  if (cs_floats > 0) {
-    for (int i = threadIdx.x; i < cs_floats; i += blockDim.x) Cs[i] = __ldg(Cf + i);
-    __syncthreads();
-    Cf = Cs;
-  }
-  // (the per-warp regions start on a 16-byte boundary: Vs is read as float4)
-  unsigned char *fq_sm = fq_sm_raw + (size_t)((cs_floats + 3) & ~3) * sizeof(float);
+  // per warp: gathered elements [FQ_KCHUNK][FQ_ROWS] floats, listed blocks [nsh],
+  // listed AOs [n]; C comes through L1, which leaves room for four CTAs per SM
+  unsigned char *fq_sm = fq_sm_raw;
   constexpr int VSZ = FQ_KCHUNK * FQ_ROWS;
   float *Vs = reinterpret_cast<float *>(fq_sm) + (size_t)w * VSZ;
   LiveBlock *tab = reinterpret_cast<LiveBlock *>(reinterpret_cast<float *>(fq_sm) + (size_t)nw * VSZ) +
@@ -663,12 +675,15 @@ __global__ void __launch_bounds__(256, 2) store_first_quarter_kernel(const Store
                                                                   (size_t)nw * VSZ) +
                                     (size_t)nw * nsh) +
             (size_t)w * n;
-  const long long warps = (long long)gridDim.x * nw;
   // group g: shell pair q = U + V (V + 1) / 2 (U <= V) and the chunk of FQ_LCH
-  // consecutive shells L; the warp's rows then cover whole runs of l for each
-  // (u, v), so the sectors of Y1 it writes are completed while in L2
+  // consecutive shells L
   const int nch = (nsh + FQ_LCH - 1) / FQ_LCH;
-  for (long long g = (long long)blockIdx.x * nw + w; g < ngroups; g += warps) {
+  // (the groups' work differs widely: each warp takes the next one when it is done)
+  for (;;) {
+    int g = 0;
+    if (lane == 0) g = atomicAdd(next, 1);
+    g = __shfl_sync(0xffffffffu, g, 0);
+    if (g >= ngroups) break;
     const long long q = g / nch;
     const int Lc = (int)(g - q * nch);
     int V1 = (int)((sqrt(8.0 * (double)q + 1.0) - 1.0) * 0.5);
@@ -685,26 +700,26 @@ __global__ void __launch_bounds__(256, 2) store_first_quarter_kernel(const Store
     // the stored blocks of the group, then their AOs d
     int cnt = 0;
     if (sv.qmax[L] * quv >= sv.thr) {
-      const int *ptn = sv.partners + (size_t)L * nsh;
+      const int4 *ptn = sv.plist + (size_t)L * nsh;
       for (int base = 0; base < nsh; base += 32) {
         const int k = base + lane;
         bool ok = false, live = false;
         LiveBlock b{};
         if (k < nsh) {
-          const int D = ptn[k];
-          const int4 e1 = sv.pinfo[D * nsh + L];
-          ok = sv.pbound[e1.x] * quv >= sv.thr;
+          const int4 rec = __ldg(ptn + k);
+          ok = __hiloint2double(rec.y, rec.x) * quv >= sv.thr;
           if (ok) {
-            const bool first_bra = e1.y > e2.y || (e1.y == e2.y && e1.z >= e2.z);
-            const int4 eb = first_bra ? e1 : e2, ek = first_bra ? e2 : e1;
-            const int K = eb.y * (eb.y + 1) / 2 + ek.y;
-            live = ek.z < sv.len[K][eb.z];
-            const int NB = sv_nfb(eb.y), NC = sv_nfa(ek.y), ND = sv_nfb(ek.y), NOUT = sv_nfa(eb.y) * NB * NC * ND;
-            const int a0 = sv.ao0[D], a1 = D + 1 < nsh ? sv.ao0[D + 1] : n;
-            b.off = sv.base[K] + (sv.off[K][eb.z] + ek.z) * NOUT;
-            b.a0 = a0;
-            b.flags = (e1.w & 3) | (first_bra ? 4 : 0) | (eb.x == ek.x ? 8 : 0) | (NB == 4 ? 16 : 0) |
-                      (NC == 4 ? 32 : 0) | (ND == 4 ? 64 : 0) | ((a1 - a0) << 8);
+            const int c1 = (rec.w >> 2) & 3, r1 = rec.z;
+            const bool first_bra = c1 > e2.y || (c1 == e2.y && r1 >= e2.z);
+            const int cb = first_bra ? c1 : e2.y, ck = first_bra ? e2.y : c1;
+            const int rb = first_bra ? r1 : e2.z, rk = first_bra ? e2.z : r1;
+            const int K = cb * (cb + 1) / 2 + ck;
+            live = rk < sv.len[K][rb];
+            const int NOUT = sv_nfa(cb) * sv_nfb(cb) * sv_nfa(ck) * sv_nfb(ck);
+            b.off = sv.base[K] + (sv.off[K][rb] + rk) * NOUT;
+            b.a0 = (unsigned)rec.w >> 16;
+            b.flags = (rec.w & 3) | (first_bra ? 4 : 0) | (cb == ck && rb == rk ? 8 : 0) |
+                      (rec.w & 0xf00);
           }
         }
         const unsigned lv = __ballot_sync(0xffffffffu, live);
@@ -734,20 +749,32 @@ __global__ void __launch_bounds__(256, 2) store_first_quarter_kernel(const Store
       const int left = rows - f0;
       if (left >= 5 && KB <= 2) {
         const int nr = min(left, 8);
-        fq_pass<KB, 8>(sv, n, Kp, Cf, nvb, Y1, np, dl, tab, nd, Vs, f0, nr, nl, l0, u0, nu, v0, nv, same, e2);
+        fq_pass<KB, 8>(sv.X, n, Cf, nvb, Y1, dl, tab, nd, Vs, f0, nr, nl, l0, u0, nu, v0, nv, same, e2.w & 1);
         f0 += nr;
       } else if (left >= 2) {
         const int nr = min(left, 4);
-        fq_pass<KB, 4>(sv, n, Kp, Cf, nvb, Y1, np, dl, tab, nd, Vs, f0, nr, nl, l0, u0, nu, v0, nv, same, e2);
+        fq_pass<KB, 4>(sv.X, n, Cf, nvb, Y1, dl, tab, nd, Vs, f0, nr, nl, l0, u0, nu, v0, nv, same, e2.w & 1);
         f0 += nr;
       } else {
-        fq_pass<KB, 1>(sv, n, Kp, Cf, nvb, Y1, np, dl, tab, nd, Vs, f0, 1, nl, l0, u0, nu, v0, nv, same, e2);
+        fq_pass<KB, 1>(sv.X, n, Cf, nvb, Y1, dl, tab, nd, Vs, f0, 1, nl, l0, u0, nu, v0, nv, same, e2.w & 1);
         f0 += 1;
       }
     }
     __syncwarp();  // the tables are read before the next shell L's
     }
   }
+}
+
+// sv.plist
+__global__ void fq_partner_kernel(StoreView sv, int n, int4 *__restrict__ out) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x, L = blockIdx.y;
+  if (k >= sv.nsh) return;
+  const int D = sv.partners[(size_t)L * sv.nsh + k];
+  const int4 e = sv.pinfo[D * sv.nsh + L];
+  const double b = sv.pbound[e.x];
+  const int a0 = sv.ao0[D], a1 = D + 1 < sv.nsh ? sv.ao0[D + 1] : n;
+  out[(size_t)L * sv.nsh + k] = make_int4(__double2loint(b), __double2hiint(b), e.z,
+                                          (int)((unsigned)a0 << 16 | (a1 - a0) << 8 | e.y << 2 | (e.w & 3)));
 }
 
 // C(d, b) as FP32, b fastest
@@ -813,8 +840,7 @@ static int slice_rows(mq_ctx *c, const T *in, long long rows, int kvalid, long l
   const int tb = 256;
   const long long blocks = std::max<long long>(1, std::min<long long>((rows + 7) / 8, 1 << 20));
   const int per16 = 16 / (int)sizeof(T);
-  const int vec = MODE != ROW_SYMM && MODE != ROW_TRANS && ((uintptr_t)in % 16 == 0) && (ld % per16 == 0) &&
-                  (kvalid % per16 == 0);
+  const int vec = ((uintptr_t)in % 16 == 0) && (ld % per16 == 0) && (kvalid % per16 == 0);
   if (Kp <= 256)
     slice_rows_kernel<S, T, 1, MODE><<<(unsigned)blocks, tb, 0, c->stream>>>(in, rows, kvalid, ld, Kp, o.plane,
                                                                              o.base, o.e, vec, rs);
@@ -824,6 +850,22 @@ static int slice_rows(mq_ctx *c, const T *in, long long rows, int kvalid, long l
   c->stats.launches += 1;
   MQ_CUDA(c, cudaGetLastError());
   return sync_check(c, "slice_rows");
+}
+
+template <int S, int MODE>
+static int slice_tiles(mq_ctx *c, const float *in, long long rows, int n, int Kp, Sliced o, RowSrc rs) {
+  if (Kp % 8 || Kp > 512) return set_err(c, MQ_EINVAL, "slice_tiles: Kp must be a multiple of 8 up to 512");
+  const long long tiles = MODE == ROW_TRANS ? (rows + TILE_ROWS - 1) / TILE_ROWS
+                                            : rows / n * ((n + TILE_ROWS - 1) / TILE_ROWS);
+  if (tiles > 2147483647LL) return set_err(c, MQ_EINVAL, "slice_tiles: too many rows");
+  if (tiles <= 0) return MQ_OK;
+  const size_t sm = (size_t)TILE_ROWS * tile_ldp(Kp >> 3) * sizeof(float);
+  auto kern = Kp <= 256 ? slice_tile_kernel<S, 1, MODE> : slice_tile_kernel<S, 2, MODE>;
+  MQ_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  kern<<<(unsigned)tiles, 256, sm, c->stream>>>(in, rows, n, Kp, o.plane, o.base, o.e, rs);
+  c->stats.launches += 1;
+  MQ_CUDA(c, cudaGetLastError());
+  return sync_check(c, "slice_tiles");
 }
 
 // (u, v) of every AO pair u <= v at p = u + v (v + 1) / 2
@@ -875,17 +917,19 @@ static int slice_xx(mq_ctx *c, long long n, int Kp, Sliced A, const int2 *pairs)
 }
 
 // Y1[p][l][b] from the quartet store and C(:, b), b < nvb
-static int store_first_quarter(mq_ctx *c, long long n, int Kp, const double *Cb, int nvb, float *y1, long long np) {
+// (*next: zero)
+static int store_first_quarter(mq_ctx *c, long long n, const double *Cb, int nvb, float *y1, int *next) {
   const int nsh = c->nshell, nw = 256 / 32;
   float *Cf = (float *)buf(c, "fq_coef", sizeof(float) * (size_t)n * std::max(nvb, 1));
-  if (!Cf) return MQ_ENOMEM;
+  int4 *plist = (int4 *)buf(c, "fq_partners", sizeof(int4) * (size_t)nsh * nsh);
+  if (!Cf || !plist) return MQ_ENOMEM;
+  StoreView sv = store_view(c);
+  sv.plist = plist;
+  fq_partner_kernel<<<dim3((nsh + 127) / 128, nsh), 128, 0, c->stream>>>(sv, (int)n, plist);
   coef_f32_kernel<<<(unsigned)((n * nvb + 255) / 256), 256, 0, c->stream>>>(Cb, (int)n, nvb, Cf);
   const long long groups = (long long)nsh * (nsh + 1) / 2 * ((nsh + FQ_LCH - 1) / FQ_LCH);
-  size_t sm = (size_t)nw * ((size_t)FQ_KCHUNK * FQ_ROWS * sizeof(float) + (size_t)n * sizeof(int) +
+  const size_t sm = (size_t)nw * ((size_t)FQ_KCHUNK * FQ_ROWS * sizeof(float) + (size_t)n * sizeof(int) +
                             (size_t)nsh * sizeof(LiveBlock));
-  // C in shared memory when the CTA still fits twice per SM
-  const int cs_floats = sm + (size_t)n * nvb * sizeof(float) <= 110 * 1024 ? (int)(n * nvb) : 0;
-  sm += (size_t)((cs_floats + 3) & ~3) * sizeof(float);
   if (sm > 200 * 1024) return set_err(c, MQ_EINVAL, "split transform: too many shells for the store transform");
   if (n > 0xffff || nsh > 0xffff) return set_err(c, MQ_EINVAL, "split transform: too many AOs for the store transform");
   auto kern = nvb <= 32 ? store_first_quarter_kernel<1>
@@ -893,11 +937,12 @@ static int store_first_quarter(mq_ctx *c, long long n, int Kp, const double *Cb,
                                      : (nvb <= 128 ? store_first_quarter_kernel<4> : store_first_quarter_kernel<8>));
   // (with KB >= 4, passes of at most 4 rows keep the accumulators in registers)
   MQ_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  int sms = 0;
+  int sms = 0, occ = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-  const long long blocks = std::max<long long>(1, std::min<long long>((groups + nw - 1) / nw, (long long)sms * 16));
-  kern<<<(unsigned)blocks, 256, sm, c->stream>>>(store_view(c), (int)n, Kp, Cf, nvb, cs_floats, y1, np, groups);
-  c->stats.launches += 2;
+  MQ_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 256, sm));
+  const long long blocks = std::min<long long>((groups + nw - 1) / nw, (long long)sms * std::max(occ, 1));
+  kern<<<(unsigned)blocks, 256, sm, c->stream>>>(sv, (int)n, Cf, nvb, y1, groups, next);
+  c->stats.launches += 3;
   MQ_CUDA(c, cudaGetLastError());
   return sync_check(c, "store_first_quarter");
 }
@@ -929,7 +974,7 @@ static int ao2mo_slices(mq_ctx *c, const double *Ci, int no1, const double *Ca, 
   float *y2 = (float *)buf(c, "slice_y2", r2 * Kp * sizeof(float));
   int *err = (int *)buf(c, "split_err", 64);
   if (!pa || !ea || !pb || !eb || !y1 || !y2 || !err) return MQ_ENOMEM;
-  MQ_CUDA(c, cudaMemsetAsync(err, 0, sizeof(int), c->stream));
+  MQ_CUDA(c, cudaMemsetAsync(err, 0, 2 * sizeof(int), c->stream));
   // the padding columns Kp > n of the intermediates are never read: slicing reads n values per row
   // coefficient blocks: column p of C (n contiguous) becomes row p of B (K-major)
   const long long plB = rB * Kp;
@@ -957,7 +1002,7 @@ static int ao2mo_slices(mq_ctx *c, const double *Ci, int no1, const double *Ca, 
   if (from_store) {
     StageTimer t1;
     t1.start(c->stream);
-    MQ_TRY(store_first_quarter(c, n, Kp, Cb, nv2, y1, np));
+    MQ_TRY(store_first_quarter(c, n, Cb, nv2, y1, err + 1));
     t1.stop(c->stream);
     t1.collect_sync();
     c->stats.ms_ao2mo_first = t1.total;
@@ -977,7 +1022,7 @@ static int ao2mo_slices(mq_ctx *c, const double *Ci, int no1, const double *Ca, 
   const long long r1p = (long long)nv2 * np;
   A = Sliced{pa, r1p * Kp, ea};
   if (from_store)  // Y1 as [p][l][b]
-    MQ_TRY((slice_rows<S, ROW_TRANS>(c, y1, r1p, (int)n, 0, Kp, A, RowSrc{nullptr, n, np, nv2})));
+    MQ_TRY((slice_tiles<S, ROW_TRANS>(c, y1, r1p, (int)n, Kp, A, RowSrc{nullptr, n, np, nv2})));
   else
     MQ_TRY(slice_rows<S>(c, y1, r1p, (int)n, Kp, Kp, A));
   g.out32 = y2;
@@ -989,7 +1034,7 @@ static int ao2mo_slices(mq_ctx *c, const double *Ci, int no1, const double *Ca, 
   MQ_TRY(slice_gemm<S>(c, A, np, nv2, np * Kp, Bj, no2, Kp, g));
   // 3: batch (j + no2*b); rows v, K = u (gathered from the packed pairs) -> Y3[a + nv1*(j + no2*b)][v]
   A = Sliced{pa, r2 * Kp, ea};
-  MQ_TRY((slice_rows<S, ROW_SYMM>(c, y2, r2, (int)n, 0, Kp, A, rs)));
+  MQ_TRY((slice_tiles<S, ROW_SYMM>(c, y2, r2, (int)n, Kp, A, rs)));
   g.out32 = y1;  // Y1 is dead
   g.mdiv = 1ll << 62;
   g.s_m0 = 1;
