@@ -113,129 +113,129 @@ int build_shells(mq_ctx *c, int nnuc, const int *Z, const double *xyz, const dou
 }
 
 void free_pairs(mq_ctx *c) {
-  for (void *p : c->pair_allocs) cudaFree(p);
-  c->pair_allocs.clear();
   c->pt = PairTable{};
   c->schwarz_valid = 0;
 }
 
 // Shell pairs of one molecule, in class order (ss), (sp,s), (sp,sp), with
-// their surviving primitive pairs.
+// their surviving primitive pairs.  The host finds what survives and its order;
+// everything else of a pair is formed on the device (pair_fill_kernel).
 void pairs_host(const std::vector<HostShell> &shells, const std::vector<double> &xyz, HostPairs &h) {
   h = HostPairs{};
   const int ns = (int)shells.size();
-  std::vector<std::pair<int, int>> pl[3];
+  h.shells.resize(ns);
+  for (int s = 0; s < ns; ++s) {
+    const HostShell &sh = shells[s];
+    PairShell &d = h.shells[s];
+    d = PairShell{};
+    for (int k = 0; k < 3; ++k) d.x[k] = xyz[3 * sh.atom + k];
+    for (int i = 0; i < sh.nprim; ++i) d.alpha[i] = sh.alpha[i], d.cs[i] = sh.cs[i], d.cp[i] = sh.cp[i];
+    d.ao0 = sh.ao0;
+  }
+  struct Cand {
+    int A, B, n, first;
+  };
+  std::vector<Cand> pl[3];
+  std::vector<double> K;
+  std::vector<int> ij;
+  const size_t np = (size_t)ns * (ns + 1) / 2;
+  K.reserve(9 * np);
+  ij.reserve(9 * np);
   for (int a = 0; a < ns; ++a)
     for (int b = 0; b <= a; ++b) {
-      int A = a, B = b;
-      const HostShell &sa = shells[a], &sb = shells[b];
-      if (sb.type > sa.type) std::swap(A, B);
-      pl[sa.type + sb.type].push_back({A, B});
-    }
-  // within a class, pairs with more primitive pairs first: neighbouring quartets
-  // of an integral launch (one warp) then loop over similar primitive counts
-  auto live = [&](const std::pair<int, int> &ab) {
-    const HostShell &A = shells[ab.first], &B = shells[ab.second];
-    const double *xa = &xyz[3 * A.atom], *xb = &xyz[3 * B.atom];
-    double AB2 = 0;
-    for (int k = 0; k < 3; ++k) AB2 += (xa[k] - xb[k]) * (xa[k] - xb[k]);
-    int cnt = 0;
-    for (int i = 0; i < A.nprim; ++i)
-      for (int j = 0; j < B.nprim; ++j) {
-        const double a = A.alpha[i], b = B.alpha[j];
-        cnt += std::exp(-a * b * AB2 / (a + b)) >= 1.0e-14;
-      }
-    return cnt;
-  };
-  for (int cl = 0; cl < 3; ++cl) {
-    std::vector<std::pair<int, std::pair<int, int>>> keyed;
-    for (auto &ab : pl[cl]) keyed.push_back({live(ab), ab});
-    std::stable_sort(keyed.begin(), keyed.end(),
-                     [](const auto &x, const auto &y) { return x.first > y.first; });
-    for (size_t k = 0; k < keyed.size(); ++k) pl[cl][k] = keyed[k].second;
-  }
-  int idx = 0;
-  for (int cl = 0; cl < 3; ++cl) {
-    h.class_off[cl] = idx;
-    for (auto &ab : pl[cl]) {
-      const HostShell &A = shells[ab.first], &B = shells[ab.second];
+      int iA = a, iB = b;
+      if (shells[b].type > shells[a].type) std::swap(iA, iB);
+      const HostShell &A = shells[iA], &B = shells[iB];
       const double *xa = &xyz[3 * A.atom], *xb = &xyz[3 * B.atom];
       double AB2 = 0;
       for (int k = 0; k < 3; ++k) AB2 += (xa[k] - xb[k]) * (xa[k] - xb[k]);
-      h.shA.push_back(ab.first);
-      h.shB.push_back(ab.second);
-      h.aoA.push_back(A.ao0);
-      h.aoB.push_back(B.ao0);
-      h.mol.push_back(0);
-      for (int k = 0; k < 3; ++k) h.geom.push_back(xa[k]);
-      for (int k = 0; k < 3; ++k) h.geom.push_back(xb[k] - xa[k]);
-      h.off.push_back((int)h.p.size());
-      // the surviving primitive pairs, K descending (stable: ties keep the
-      // (i, j) order): the pairs of a ket passing the screen against one bra
-      // primitive are then a prefix of the ket's list, and the integral
-      // kernels visit exactly the surviving primitive quartets
-      std::vector<std::pair<double, std::pair<int, int>>> live_pp;
+      // the surviving primitive pairs, K descending (ties keep the (i, j)
+      // order): the pairs of a ket passing the screen against one bra primitive
+      // are then a prefix of the ket's list, and the integral kernels visit
+      // exactly the surviving primitive quartets
+      double Kp[KMAX * KMAX];
+      int ip[KMAX * KMAX], n = 0;
       for (int i = 0; i < A.nprim; ++i)
         for (int j = 0; j < B.nprim; ++j) {
-          const double a = A.alpha[i], b = B.alpha[j];
-          const double Kab = std::exp(-a * b * AB2 / (a + b));
+          const double a1 = A.alpha[i], b1 = B.alpha[j];
+          const double Kab = std::exp(-a1 * b1 * AB2 / (a1 + b1));
           // a primitive pair whose EIJ is below 1e-14 fails the reference's
           // screen EIJ*EGH < 1e-14 (int2e.f90:257; int1e.f90:238) for any
           // partner, since EGH <= 1
-          if (Kab >= 1.0e-14) live_pp.push_back({Kab, {i, j}});
+          if (!(Kab >= 1.0e-14)) continue;
+          int t = n++;
+          for (; t > 0 && Kp[t - 1] < Kab; --t) Kp[t] = Kp[t - 1], ip[t] = ip[t - 1];
+          Kp[t] = Kab;
+          ip[t] = i | j << 8;
         }
-      std::stable_sort(live_pp.begin(), live_pp.end(),
-                       [](const auto &x, const auto &y) { return x.first > y.first; });
-      for (const auto &lp : live_pp) {
-        const int i = lp.second.first, j = lp.second.second;
-        double a = A.alpha[i], b = B.alpha[j], pp = a + b;
-        double Kab = lp.first;
-        double P[3], PA[3], PB[3];
-        for (int k = 0; k < 3; ++k) {
-          P[k] = (a * xa[k] + b * xb[k]) / pp;
-          PA[k] = P[k] - xa[k];
-          PB[k] = P[k] - xb[k];
-        }
-        h.p.push_back(pp);
-        h.inv2p.push_back(1.0 / (2.0 * pp));
-        h.beta.push_back(b);
-        h.Px.push_back(P[0]); h.Py.push_back(P[1]); h.Pz.push_back(P[2]);
-        h.PAx.push_back(PA[0]); h.PAy.push_back(PA[1]); h.PAz.push_back(PA[2]);
-        h.PBx.push_back(PB[0]); h.PBy.push_back(PB[1]); h.PBz.push_back(PB[2]);
-        h.K.push_back(Kab);
-        double ca[2] = {A.cs[i], A.cp[i]}, cb[2] = {B.cs[j], B.cp[j]};
-        for (int la = 0; la < 2; ++la)
-          for (int lb = 0; lb < 2; ++lb) h.c4.push_back(Kab * ca[la] * cb[lb]);
-      }
-      ++idx;
+      pl[A.type + B.type].push_back({iA, iB, n, (int)K.size()});
+      K.insert(K.end(), Kp, Kp + n);
+      ij.insert(ij.end(), ip, ip + n);
+    }
+  h.shA.reserve(np);
+  h.shB.reserve(np);
+  h.off.reserve(np + 1);
+  h.K.reserve(K.size());
+  h.ij.reserve(K.size());
+  for (int cl = 0; cl < 3; ++cl) {
+    h.class_off[cl] = (int)h.shA.size();
+    // within a class, pairs with more primitive pairs first: neighbouring quartets
+    // of an integral launch (one warp) then loop over similar primitive counts
+    std::stable_sort(pl[cl].begin(), pl[cl].end(), [](const Cand &x, const Cand &y) { return x.n > y.n; });
+    for (const Cand &q : pl[cl]) {
+      h.shA.push_back(q.A);
+      h.shB.push_back(q.B);
+      h.off.push_back((int)h.K.size());
+      h.K.insert(h.K.end(), K.begin() + q.first, K.begin() + q.first + q.n);
+      h.ij.insert(h.ij.end(), ij.begin() + q.first, ij.begin() + q.first + q.n);
     }
   }
-  h.class_off[3] = idx;
-  h.off.push_back((int)h.p.size());
+  h.class_off[3] = (int)h.shA.size();
+  h.off.push_back((int)h.K.size());
 }
 
-// Append the class-cl pairs of one molecule's table to a batch table (whose
-// pairs are ordered class first, then molecule), tagging them with `mol`.
-void append_pairs_class(HostPairs &dst, const HostPairs &src, int cl, int mol) {
-  if (dst.off.empty()) dst.off.push_back(0);
-  for (int P = src.class_off[cl]; P < src.class_off[cl + 1]; ++P) {
-    dst.shA.push_back(src.shA[P]);
-    dst.shB.push_back(src.shB[P]);
-    dst.aoA.push_back(src.aoA[P]);
-    dst.aoB.push_back(src.aoB[P]);
-    dst.mol.push_back(mol);
-    dst.geom.insert(dst.geom.end(), src.geom.begin() + 6 * (size_t)P, src.geom.begin() + 6 * (size_t)P + 6);
-    for (int q = src.off[P]; q < src.off[P + 1]; ++q) {
-      dst.p.push_back(src.p[q]);
-      dst.inv2p.push_back(src.inv2p[q]);
-      dst.beta.push_back(src.beta[q]);
-      dst.Px.push_back(src.Px[q]); dst.Py.push_back(src.Py[q]); dst.Pz.push_back(src.Pz[q]);
-      dst.PAx.push_back(src.PAx[q]); dst.PAy.push_back(src.PAy[q]); dst.PAz.push_back(src.PAz[q]);
-      dst.PBx.push_back(src.PBx[q]); dst.PBy.push_back(src.PBy[q]); dst.PBz.push_back(src.PBz[q]);
-      dst.K.push_back(src.K[q]);
-      for (int k = 0; k < 4; ++k) dst.c4.push_back(src.c4[4 * q + k]);
+// The table's other fields from the shells, one warp per pair; ij: the primitives of each pair.
+__global__ void pair_fill_kernel(PairTable t, const PairShell *__restrict__ shells, const int *__restrict__ shell0,
+                                 const int *__restrict__ ij) {
+  const int P = blockIdx.x, m = t.mol[P];
+  const PairShell &A = shells[shell0[m] + t.shA[P]], &B = shells[shell0[m] + t.shB[P]];
+  if (threadIdx.x == 0) {
+    t.aoA[P] = A.ao0;
+    t.aoB[P] = B.ao0;
+    t.schwarz[P] = 1.0e300;
+  }
+  if (threadIdx.x < 3) {
+    t.geom[6 * (size_t)P + threadIdx.x] = A.x[threadIdx.x];
+    t.geom[6 * (size_t)P + 3 + threadIdx.x] = B.x[threadIdx.x] - A.x[threadIdx.x];
+  }
+  for (int q = t.pp_off[P] + threadIdx.x; q < t.pp_off[P + 1]; q += blockDim.x) {
+    const int i = ij[q] & 255, j = ij[q] >> 8;
+    const double a = A.alpha[i], b = B.alpha[j], pp = a + b, K = t.K[q];
+    double X[3], PA[3], PB[3], c4[4];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      X[k] = (a * A.x[k] + b * B.x[k]) / pp;
+      PA[k] = X[k] - A.x[k];
+      PB[k] = X[k] - B.x[k];
     }
-    dst.off.push_back((int)dst.p.size());  // end of this pair's primitives = start of the next
+    const double i2p = 1.0 / (2.0 * pp);
+    c4[0] = K * A.cs[i] * B.cs[j];
+    c4[1] = K * A.cs[i] * B.cp[j];
+    c4[2] = K * A.cp[i] * B.cs[j];
+    c4[3] = K * A.cp[i] * B.cp[j];
+    t.p[q] = pp;
+    t.inv2p[q] = i2p;
+    t.beta[q] = b;
+    t.Px[q] = X[0], t.Py[q] = X[1], t.Pz[q] = X[2];
+    t.PAx[q] = PA[0], t.PAy[q] = PA[1], t.PAz[q] = PA[2];
+    t.PBx[q] = PB[0], t.PBy[q] = PB[1], t.PBz[q] = PB[2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) t.c4[4 * (size_t)q + k] = c4[k];
+    float4 *f = t.pf + 4 * (size_t)q;
+    f[0] = make_float4((float)pp, (float)i2p, (float)K, (float)X[0]);
+    f[1] = make_float4((float)X[1], (float)X[2], (float)PA[0], (float)PA[1]);
+    f[2] = make_float4((float)PA[2], (float)PB[0], (float)PB[1], (float)PB[2]);
+    f[3] = make_float4((float)c4[0], (float)c4[1], (float)c4[2], (float)c4[3]);
   }
 }
 
@@ -343,73 +343,49 @@ static int pair_records(mq_ctx *c, PairTable &t, int mode) {
   return MQ_OK;
 }
 
-// All arrays of the table in one device block (256-byte aligned pieces),
-// staged through one pinned host buffer and one copy.  allocs != null: a new
-// block recorded there (batches); null: the context's reusable "pair_table"
-// buffer, after the work queued on the stream (which may read the previous
-// table) has finished.
-int upload_pairs(mq_ctx *c, const HostPairs &h, std::vector<void *> *allocs, PairTable &t, int mode) {
+// The table of M molecules, class first, then molecule, in one device block
+// (256-byte aligned pieces; the context's buffer `name`, once the work queued on the
+// stream, which may read the previous table, has finished).  Only what pairs_host
+// found is staged, through one pinned host buffer and one copy.
+int upload_pairs(mq_ctx *c, const HostPairs *const *mols, int M, const char *name, PairTable &t, int mode) {
   t = PairTable{};
-  for (int k = 0; k < 4; ++k) t.class_off[k] = h.class_off[k];
-  t.npairs = (int)h.shA.size();
-  t.npp = (int)h.p.size();
-  std::vector<double> ones(h.shA.size(), 1.0e300);
-  std::vector<float4> pf(4 * h.p.size());
-  for (size_t i = 0; i < h.p.size(); ++i) {
-    pf[4 * i] = make_float4((float)h.p[i], (float)h.inv2p[i], (float)h.K[i], (float)h.Px[i]);
-    pf[4 * i + 1] = make_float4((float)h.Py[i], (float)h.Pz[i], (float)h.PAx[i], (float)h.PAy[i]);
-    pf[4 * i + 2] = make_float4((float)h.PAz[i], (float)h.PBx[i], (float)h.PBy[i], (float)h.PBz[i]);
-    pf[4 * i + 3] = make_float4((float)h.c4[4 * i], (float)h.c4[4 * i + 1], (float)h.c4[4 * i + 2],
-                                (float)h.c4[4 * i + 3]);
-  }
-  struct Item {
-    void **dst;
-    const void *src;
-    size_t bytes, off;
-  };
-  std::vector<Item> items;
+  size_t npairs = 0, npp = 0, nsh = 0;
+  for (int m = 0; m < M; ++m) npairs += mols[m]->shA.size(), npp += mols[m]->K.size(), nsh += mols[m]->shells.size();
+  if (npairs > 2147483646ull || npp > 2147483646ull) return set_err(c, MQ_EINVAL, "pair table too large");
+  t.npairs = (int)npairs;
+  t.npp = (int)npp;
   size_t total = 0;
-  auto add = [&](auto *&dst, const auto &src) {
-    using T = typename std::decay<decltype(src)>::type::value_type;
-    const size_t bytes = src.size() * sizeof(T);
-    items.push_back({(void **)&dst, (const void *)src.data(), bytes, total});
-    total += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+  std::vector<std::pair<void **, size_t>> items;
+  auto room = [&](auto *&dst, size_t count) {
+    items.push_back({(void **)&dst, total});
+    total += (std::max<size_t>(count, 1) * sizeof(*dst) + 255) / 256 * 256;
   };
-  add(t.shA, h.shA);
-  add(t.shB, h.shB);
-  add(t.pp_off, h.off);
-  add(t.aoA, h.aoA);
-  add(t.aoB, h.aoB);
-  add(t.mol, h.mol);
-  add(t.schwarz, ones);
-  add(t.p, h.p);
-  add(t.inv2p, h.inv2p);
-  add(t.beta, h.beta);
-  add(t.Px, h.Px); add(t.Py, h.Py); add(t.Pz, h.Pz);
-  add(t.PAx, h.PAx); add(t.PAy, h.PAy); add(t.PAz, h.PAz);
-  add(t.PBx, h.PBx); add(t.PBy, h.PBy); add(t.PBz, h.PBz);
-  add(t.K, h.K);
-  add(t.c4, h.c4);
-  add(t.pf, pf);
-  add(t.geom, h.geom);
+  PairShell *shells = nullptr;
+  int *shell0 = nullptr, *ij = nullptr;
+  room(shells, nsh);
+  room(shell0, M);
+  room(t.shA, npairs);
+  room(t.shB, npairs);
+  room(t.pp_off, npairs + 1);
+  room(t.mol, npairs);
+  room(t.K, npp);
+  room(ij, npp);
   const size_t copied = total;  // behind it: what the device forms itself
-  auto room = [&](auto *&dst, size_t bytes) {
-    items.push_back({(void **)&dst, nullptr, 0, total});
-    total += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
-  };
-  room(t.rec, sizeof(double) * PP_REC * h.p.size());
-  room(t.pid, sizeof(int) * h.p.size());
-  room(t.pq, sizeof(double2) * PQ_MAX * PQ_MAX);
-  room(t.pq_n, sizeof(int));
-  char *dev = nullptr;
+  room(t.aoA, npairs);
+  room(t.aoB, npairs);
+  room(t.schwarz, npairs);
+  room(t.geom, 6 * npairs);
+  for (double **v : {&t.p, &t.inv2p, &t.beta, &t.Px, &t.Py, &t.Pz, &t.PAx, &t.PAy, &t.PAz, &t.PBx, &t.PBy, &t.PBz})
+    room(*v, npp);
+  room(t.c4, 4 * npp);
+  room(t.pf, 4 * npp);
+  room(t.rec, PP_REC * npp);
+  room(t.pid, npp);
+  room(t.pq, (size_t)PQ_MAX * PQ_MAX);
+  room(t.pq_n, 1);
   MQ_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (allocs) {
-    if (cudaMalloc((void **)&dev, total) != cudaSuccess) return set_err(c, MQ_ENOMEM, "cudaMalloc pair table");
-    allocs->push_back(dev);
-  } else {
-    dev = (char *)buf(c, "pair_table", total);
-    if (!dev) return MQ_ENOMEM;
-  }
+  char *dev = (char *)buf(c, name, total);
+  if (!dev) return MQ_ENOMEM;
   if (c->pin_bytes < copied) {
     if (c->pin) cudaFreeHost(c->pin);
     c->pin = nullptr;
@@ -417,12 +393,37 @@ int upload_pairs(mq_ctx *c, const HostPairs &h, std::vector<void *> *allocs, Pai
     MQ_CUDA(c, cudaHostAlloc(&c->pin, copied, cudaHostAllocDefault));
     c->pin_bytes = copied;
   }
-  char *st = (char *)c->pin;
-  for (const Item &it : items) {
-    if (it.bytes) memcpy(st + it.off, it.src, it.bytes);
-    *it.dst = dev + it.off;
+  for (auto &it : items) *it.first = (char *)c->pin + it.second;  // (the staged pieces first, as host pointers)
+  size_t P = 0, q = 0, s = 0;
+  for (int m = 0; m < M; ++m) {
+    shell0[m] = (int)s;
+    std::copy(mols[m]->shells.begin(), mols[m]->shells.end(), shells + s);
+    s += mols[m]->shells.size();
   }
-  MQ_CUDA(c, cudaMemcpyAsync(dev, st, copied, cudaMemcpyHostToDevice, c->stream));
+  for (int cl = 0; cl < 3; ++cl) {
+    t.class_off[cl] = (int)P;
+    for (int m = 0; m < M; ++m) {
+      const HostPairs &h = *mols[m];
+      const int P0 = h.class_off[cl], P1 = h.class_off[cl + 1], q0 = h.off[P0], q1 = h.off[P1];
+      std::copy(h.shA.begin() + P0, h.shA.begin() + P1, t.shA + P);
+      std::copy(h.shB.begin() + P0, h.shB.begin() + P1, t.shB + P);
+      std::fill(t.mol + P, t.mol + P + (P1 - P0), m);
+      for (int k = P0; k < P1; ++k) t.pp_off[P + (k - P0)] = (int)q + h.off[k] - q0;
+      std::copy(h.K.begin() + q0, h.K.begin() + q1, t.K + q);
+      std::copy(h.ij.begin() + q0, h.ij.begin() + q1, ij + q);
+      P += P1 - P0;
+      q += q1 - q0;
+    }
+  }
+  t.class_off[3] = (int)P;
+  t.pp_off[P] = (int)q;
+  for (auto &it : items) *it.first = dev + it.second;
+  MQ_CUDA(c, cudaMemcpyAsync(dev, c->pin, copied, cudaMemcpyHostToDevice, c->stream));
+  if (npairs > 0) {
+    pair_fill_kernel<<<(unsigned)npairs, 32, 0, c->stream>>>(t, shells, shell0, ij);
+    c->stats.launches += 1;
+    MQ_CUDA(c, cudaGetLastError());
+  }
   MQ_CUDA(c, cudaStreamSynchronize(c->stream));  // the staging buffer is reused by the next upload
   return pair_records(c, t, mode);
 }
@@ -431,13 +432,18 @@ int build_pairs(mq_ctx *c) {
   free_pairs(c);
   HostPairs h;
   pairs_host(c->shells, c->xyz, h);
-  MQ_TRY(upload_pairs(c, h, nullptr, c->pt, c->mode));
+  const HostPairs *hp = &h;
+  MQ_TRY(upload_pairs(c, &hp, 1, "pair_table", c->pt, c->mode));
   c->pair_class_count = {h.class_off[1] - h.class_off[0], h.class_off[2] - h.class_off[1],
                          h.class_off[3] - h.class_off[2]};
   c->hp_shA = h.shA;
   c->hp_shB = h.shB;
-  c->hp_aoA = h.aoA;
-  c->hp_aoB = h.aoB;
+  c->hp_aoA.resize(h.shA.size());
+  c->hp_aoB.resize(h.shA.size());
+  for (size_t P = 0; P < h.shA.size(); ++P) {
+    c->hp_aoA[P] = c->shells[h.shA[P]].ao0;
+    c->hp_aoB[P] = c->shells[h.shB[P]].ao0;
+  }
   for (int k = 0; k < 4; ++k) c->hp_class_off[k] = h.class_off[k];
   c->qs.valid = 0;
   c->qs.tables_valid = 0;

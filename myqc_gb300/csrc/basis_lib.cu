@@ -72,7 +72,7 @@ int basis_build(mq_ctx *c, int nnuc, const int *Z, std::vector<double> &bas, std
   for (int i = 0; i < nnuc; ++i) {
     if (Z[i] < 1 || Z[i] > 10) return set_err(c, MQ_EINVAL, "basis library: element out of range");
     size_t q = p;
-    while (q < rows.size() && (rows[q].empty() || rows[q][0].substr(0, 8) != ELEMENT_NAME[Z[i] - 1])) ++q;
+    while (q < rows.size() && (rows[q].empty() || rows[q][0].compare(0, 8, ELEMENT_NAME[Z[i] - 1]) != 0)) ++q;
     if (q + 1 >= rows.size() || rows[q + 1].size() < 3)
       return set_err(c, MQ_EINVAL, std::string("basis library: no ") + ELEMENT_NAME[Z[i] - 1]);
     int sec, orb, nset;

@@ -346,14 +346,8 @@ static double nuc_rep(const std::vector<double> &nuc) {
   return E;
 }
 
-static void free_batch_pairs(mq_ctx *c) {
-  for (void *p : c->batch_allocs) cudaFree(p);
-  c->batch_allocs.clear();
-}
-
 int batch_clear(mq_ctx *c) {
   c->bmols.clear();
-  free_batch_pairs(c);
   return MQ_OK;
 }
 
@@ -424,18 +418,15 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
     nmax = std::max(nmax, (int)n);
   }
   // ---- batch pair table (class-major, then molecule)
-  HostPairs bh;
+  std::vector<const HostPairs *> mp(M);
   std::vector<int> pstart(3 * (size_t)M), pcount(3 * (size_t)M);
-  for (int cl = 0; cl < 3; ++cl) {
-    bh.class_off[cl] = (int)bh.shA.size();
+  for (int m = 0; m < M; ++m) mp[m] = &mols[m].pairs;
+  for (int cl = 0, P = 0; cl < 3; ++cl)
     for (int m = 0; m < M; ++m) {
-      pstart[3 * m + cl] = (int)bh.shA.size();
-      append_pairs_class(bh, mols[m].pairs, cl, m);
-      pcount[3 * m + cl] = (int)bh.shA.size() - pstart[3 * m + cl];
+      pstart[3 * m + cl] = P;
+      pcount[3 * m + cl] = mp[m]->class_off[cl + 1] - mp[m]->class_off[cl];
+      P += pcount[3 * m + cl];
     }
-  }
-  bh.class_off[3] = (int)bh.shA.size();
-  if (bh.off.empty()) bh.off.push_back(0);
   // quartet-count prefixes per class combination
   std::vector<long long> mqo[6];
   long long total[6];
@@ -470,9 +461,8 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
     MQ_CUDA(c, cudaMalloc((void **)&c->d_boys_tight, tab.size() * sizeof(double)));
     MQ_CUDA(c, cudaMemcpy(c->d_boys_tight, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice));
   }
-  free_batch_pairs(c);
   PairTable bpt;
-  MQ_TRY(upload_pairs(c, bh, &c->batch_allocs, bpt, MQ_MODE_TIGHT));
+  MQ_TRY(upload_pairs(c, mp.data(), M, "batch_pairs", bpt, MQ_MODE_TIGHT));
   MolDesc *d_md = upload_vec(c, "batch_mols", md);
   double *d_nuc = upload_vec(c, "batch_nuc", nuc);
   double *d_en = upload_vec(c, "batch_enuc", en);

@@ -61,13 +61,19 @@ struct PairTable {
 constexpr int PP_REC = 14;
 constexpr int PQ_MAX = 512;
 
-// Host copy of a pair table (same fields as PairTable), built per molecule
-// and concatenated for batches.
+// A shell as the device forms the pair tables from it.
+struct PairShell {
+  double x[3], alpha[KMAX], cs[KMAX], cp[KMAX];
+  int ao0;
+};
+
+// What the host finds of one molecule's pair table: per pair its shells, per
+// surviving primitive pair K and the primitives i | j << 8.
 struct HostPairs {
   int class_off[4] = {0, 0, 0, 0};
-  std::vector<int> shA, shB, off, aoA, aoB, mol;
-  std::vector<double> p, inv2p, beta, Px, Py, Pz, PAx, PAy, PAz, PBx, PBy, PBz, K, c4;
-  std::vector<double> geom;  // 6 per pair: A, B - A
+  std::vector<int> shA, shB, off, ij;
+  std::vector<double> K;
+  std::vector<PairShell> shells;
 };
 
 // One molecule added to a batch: host pair table, nuclei (x, y, z, Z) and
@@ -254,7 +260,6 @@ struct mq_ctx {
   double eri_f32_tau = 0.0;     // quartets with a Schwarz bound below this are computed in FP32 (0: off)
   double *d_nuc = nullptr;   // nnuc x 4: x, y, z, Z
   mq::PairTable pt{};
-  std::vector<void *> pair_allocs;
   void *pin = nullptr;  // pinned staging buffer of the pair-table uploads
   size_t pin_bytes = 0;
   int boys_loaded = -1;  // mode whose Boys table d_boys holds (-1: none; reference tables are always reloaded)
@@ -263,7 +268,6 @@ struct mq_ctx {
   int xx_valid = 0;          // d_XX holds the current system's integrals (mq_eri_store / mq_eri_upload)
   // batch of independent closed-shell molecules (mq_batch_*)
   std::vector<mq::BatchMol> bmols;
-  std::vector<void *> batch_allocs;  // batch pair table
   double *d_boys_tight = nullptr;    // the tight Boys table, for batches
   void *mlp = nullptr;               // the learned guess's network (mlp.cu)
   mq::StageTimer t_fock_kernel;
@@ -390,8 +394,7 @@ int build_shells(mq_ctx *c, int nnuc, const int *Z, const double *xyz, const dou
                  const int *basinfo, const int *setinfo);
 int build_pairs(mq_ctx *c);
 void pairs_host(const std::vector<HostShell> &shells, const std::vector<double> &xyz, HostPairs &h);
-void append_pairs_class(HostPairs &dst, const HostPairs &src, int cl, int mol);
-int upload_pairs(mq_ctx *c, const HostPairs &h, std::vector<void *> *allocs, PairTable &t, int mode);
+int upload_pairs(mq_ctx *c, const HostPairs *const *mols, int M, const char *name, PairTable &t, int mode);
 void free_pairs(mq_ctx *c);
 void tight_boys_table(std::vector<double> &tab);  // TIGHT_NT x TIGHT_NM, row-major [T][m]
 constexpr int BOYS_SCALED_M = 5;                  // orders with their own Taylor-coefficient table

@@ -104,7 +104,9 @@ class Context:
         nnuc = np.array([len(s.atoms) for s in systems], dtype=np.int32)
         Z = np.ascontiguousarray(np.concatenate([np.asarray(s.atoms) for s in systems]), dtype=np.int32)
         xyz = f64(np.concatenate([np.asarray(s.xyz, dtype=float).reshape(-1, 3) for s in systems]))
-        sizes = [int(sum(1 if z <= 2 else 5 for z in s.atoms)) for s in systems]
+        ao = np.concatenate([[0], np.cumsum(np.where(Z <= 2, 1, 5))])  # functions before each atom
+        at = np.concatenate([[0], np.cumsum(nnuc)])
+        sizes = np.diff(ao[at]).tolist()
         D = np.zeros(sum(n * n for n in sizes))
         self._check(self.L.mq_guess_predict(self.h, len(systems), ptr(nnuc), ptr(Z), ptr(xyz), ptr(D)))
         out, o = [], 0
