@@ -127,6 +127,22 @@ static int ensure_fork(mq_ctx *c) {
   return MQ_OK;
 }
 
+// Everything queued on the context's stream so far comes before what is queued
+// on the fork streams next, and that before what follows join_streams (once all is queued).
+int fork_streams(mq_ctx *c) {
+  MQ_TRY(ensure_fork(c));
+  MQ_CUDA(c, cudaEventRecord(c->ev_fork, c->stream));
+  for (int k = 0; k < 5; ++k) MQ_CUDA(c, cudaStreamWaitEvent(c->fork[k], c->ev_fork, 0));
+  return MQ_OK;
+}
+int join_streams(mq_ctx *c) {
+  for (int k = 0; k < 5; ++k) {
+    MQ_CUDA(c, cudaEventRecord(c->ev_join[k], c->fork[k]));
+    MQ_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join[k], 0));
+  }
+  return MQ_OK;
+}
+
 template <int EPI>
 static int run_combo(mq_ctx *c, const EriArgs &g, int cP, int cQ);
 
@@ -134,29 +150,18 @@ template <int EPI>
 static int run_all(mq_ctx *c, EriArgs g) {
   const long long np = c->pt.npairs;
   const bool fork = EPI == EPI_XX && np * (np + 1) / 2 <= FORK_MAX_QUARTETS;
-  if (fork) {
-    MQ_TRY(ensure_fork(c));
-    MQ_CUDA(c, cudaEventRecord(c->ev_fork, c->stream));
-  }
-  int k = 0;
+  if (fork) MQ_TRY(fork_streams(c));
+  const cudaStream_t main = c->stream;
+  int k = 0, rc = MQ_OK;
   // the heaviest combination first, on the context's own stream
-  for (int cP = 2; cP >= 0; --cP)
-    for (int cQ = cP; cQ >= 0; --cQ, ++k) {
-      if (!fork || k == 0) {
-        MQ_TRY(run_combo<EPI>(c, g, cP, cQ));
-        continue;
-      }
-      cudaStream_t main = c->stream, s = c->fork[k - 1];
-      MQ_CUDA(c, cudaStreamWaitEvent(s, c->ev_fork, 0));
-      c->stream = s;
-      const int rc = run_combo<EPI>(c, g, cP, cQ);
+  for (int cP = 2; cP >= 0 && rc == MQ_OK; --cP)
+    for (int cQ = cP; cQ >= 0 && rc == MQ_OK; --cQ, ++k) {
+      if (fork && k > 0) c->stream = c->fork[k - 1];
+      rc = run_combo<EPI>(c, g, cP, cQ);
       c->stream = main;
-      // joined whatever was queued
-      MQ_CUDA(c, cudaEventRecord(c->ev_join[k - 1], s));
-      MQ_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join[k - 1], 0));
-      MQ_TRY(rc);
     }
-  return MQ_OK;
+  if (fork) MQ_TRY(join_streams(c));  // (whatever was queued)
+  return rc;
 }
 
 template <int EPI>

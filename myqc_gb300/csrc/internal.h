@@ -427,6 +427,8 @@ int fock_direct_store_rhf(mq_ctx *c, const double *d_D, double *d_G);
 int ensure_xx_full(mq_ctx *c);
 int ensure_xx_alloc(mq_ctx *c);  // the n^4 device array of the current order (capi.cu)
 int eri_schwarz(mq_ctx *c);
+int fork_streams(mq_ctx *c);
+int join_streams(mq_ctx *c);
 int ensure_schwarz(mq_ctx *c);  // eri_schwarz unless the current system's bounds are there
 int fock_direct_device(mq_ctx *c, const double *d_Da, const double *d_Db, double *d_J, double *d_Ka, double *d_Kb);
 // G = sym(J) - f sym(K) from the direct kernel's half-sums (f = 1/2 RHF, 1 UHF)

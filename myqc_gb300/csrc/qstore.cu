@@ -27,14 +27,21 @@
 // with six FP64 multiply-adds per unique integral that passes the screen.
 // The constant factors 4 and 2 are applied once, in the assembly.
 //
-// Row pass: one CTA per bra pair P = (A,B) and one thread per shell s.
-// Thread s walks the kets Q of P's staircase rows in which s is the first
+// Row pass: per bra pair P = (A,B) one thread per AO column of a shell s.
+// The thread walks the kets Q of P's staircase rows in which s is the first
 // shell C (adding Kh[i,k], Kh[j,k] and the row part of Jh[i,j]) or the second
 // shell D (Kh[i,l], Kh[j,l]).  It alone owns the columns of s in P's partial
 // rows Kh[A u B, :], so nothing is shared and nothing is atomic.  Column
 // pass: one CTA per ket pair Q, Jh[k,l] over the bra pairs that reach Q.
 // Assembly sums each shell's partial rows over the pairs that contain it in a
 // fixed order.  The result is deterministic.
+//
+// What bounds it is the FP64 pipe (six multiply-adds per stored integral: 0.38 ms of the
+// 1.5 ms for (H2O)32, n = 224, 36.5M integrals): the row pass keeps it 60-70 % busy, with 17
+// to 19 of 32 lanes active, because a warp's columns have lists of
+// different length.  Columns ordered by the number of strong pairs, CTAs of two
+// warps, (sp,sp) kets read two elements at a time and the six passes side by side:
+// 1.63 -> 1.49 ms.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -49,7 +56,7 @@ __host__ __device__ constexpr int nfa(int cls) { return cls >= 1 ? 4 : 1; }
 __host__ __device__ constexpr int nfb(int cls) { return cls == 2 ? 4 : 1; }
 __host__ __device__ constexpr int combo_index(int cP, int cQ) { return cP * (cP + 1) / 2 + cQ; }
 
-constexpr int QS_THREADS = 256;      // row pass: AO columns (x shares) per CTA
+constexpr int QS_THREADS = 64;       // row pass: AO columns per CTA
 constexpr int QS_COL_THREADS = 256;  // column pass
 constexpr int QS_SHARES[3] = {1, 2, 4};  // row-pass CTAs per bra pair, by bra class
 constexpr int QS_MAX_SHARES = 4;
@@ -84,14 +91,15 @@ struct QsArgs {
   const int4 *lst;
   const int4 *rinfo;  // by class offset + rank: pair, A | B << 16, i0 | j0 << 16
   const int *thr_ao;
-  int nshare[3];  // row-pass shares (CTAs per bra pair) by bra class
+  int nshare[3];  // row-pass shares (CTAs per bra pair and column group) by bra class
+  int ngroup;     // row-pass column groups
   const int2 *ksh;
   const int *ksh_off;
   const int *shell_ao0;
   int nshell, n, npairs;
   const double *D;
   double *Kpart;  // [pair][8 rows][n]
-  double *Jrow;   // [pair][16]
+  double *Jrow;   // [share, group][pair][16]
   double *Jcol;   // [pair][16]
   double *Jh, *Kh;
   // screened increments: the kets (and, in the column pass, the bras) of a
@@ -118,7 +126,38 @@ template <int NA, int NB, int NC, int ND, int ROLE, bool DEGEN>
 __device__ __forceinline__ void row_block(const double *__restrict__ Xb, const double *__restrict__ D, size_t n,
                                           int A, int B, int C, int Dsh, int P, int Q, int i0, int j0, int k0, int l0,
                                           int f, double (&KA)[4], double (&KB)[4], double (&Jr)[4][4]) {
-  if (ROLE == 0) {  // column k = k0 + f: Kh[i,k] += x D[j,l], Kh[j,k] += x D[i,l], Jh[i,j] += x D[k,l]
+  if constexpr (ROLE == 0 && ND == 4) {
+    // the same for two l at a time: with d outermost each sector of the block was
+    // read four times, and L1 does not hold a CTA's blocks (all four l at once spill)
+#pragma unroll 1
+    for (int d0 = 0; d0 < 4; d0 += 2) {
+      double Dbd[NB][2], Dcd[2];
+#pragma unroll
+      for (int d = 0; d < 2; ++d) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) Dbd[b][d] = D[(j0 + b) + n * (l0 + d0 + d)];
+        Dcd[d] = D[(k0 + f) + n * (l0 + d0 + d)];
+      }
+#pragma unroll
+      for (int a = 0; a < NA; ++a) {
+        double Dad[2];
+#pragma unroll
+        for (int d = 0; d < 2; ++d) Dad[d] = D[(i0 + a) + n * (l0 + d0 + d)];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          const double2 x2 = __ldg(reinterpret_cast<const double2 *>(Xb + ((a * NB + b) * NC + f) * 4 + d0));
+          double x[2] = {x2.x, x2.y};
+#pragma unroll
+          for (int d = 0; d < 2; ++d) {
+            if (DEGEN) x[d] *= canon_weight(A, B, C, Dsh, P, Q, i0 + a, j0 + b, k0 + f, l0 + d0 + d, (int)n);
+            KA[a] = fma(x[d], Dbd[b][d], KA[a]);
+            KB[b] = fma(x[d], Dad[d], KB[b]);
+            Jr[a][b] = fma(x[d], Dcd[d], Jr[a][b]);
+          }
+        }
+      }
+    }
+  } else if (ROLE == 0) {  // column k = k0 + f: Kh[i,k] += x D[j,l], Kh[j,k] += x D[i,l], Jh[i,j] += x D[k,l]
 #pragma unroll 1
     for (int d = 0; d < ND; ++d) {
       double Dbd[NB], Dad[NA];
@@ -174,10 +213,12 @@ __device__ __forceinline__ void row_role(const QsArgs &g, int r, int P, int A, i
   const size_t n = g.n;
   const double *D = g.D;
   const double kq = g.kscreen > 0.0 ? g.kscreen / g.sch[P] : 0.0;  // smallest ket bound kept
+  int4 qn = lo + k < hi ? g.lst[lo + k] : make_int4(0, 0, 0, 0);
 #pragma unroll 1
   for (int e = lo + k; e < hi; e += S) {
-    const int4 q = g.lst[e];  // rank, pair, shells C | D << 16, AOs k0 | l0 << 16
-    if (q.x >= lenr) break;   // ranks ascend: the rest lie beyond the staircase
+    const int4 q = qn;       // rank, pair, shells C | D << 16, AOs k0 | l0 << 16
+    if (e + S < hi) qn = g.lst[e + S];
+    if (q.x >= lenr) break;  // ranks ascend: the rest lie beyond the staircase
     if (kq > 0.0 && g.sch[q.y] < kq) break;  // and their bounds fall: the rest are screened out too
     const int Q = q.y, C = q.z & 0xffff, Dsh = q.z >> 16, k0 = q.w & 0xffff, l0 = q.w >> 16;
     const double *Xb = Xc + (size_t)q.x * NOUT;
@@ -226,17 +267,17 @@ __device__ __forceinline__ void row_column(const QsArgs &g, int r, int P, int A,
   }
 }
 
-// Row pass for the bra pairs of class CP: CTA (bra rank, share k of S), thread
+// Row pass for the bra pairs of class CP: CTA (bra rank, share k of S, column group z), thread
 // = one AO column (the four AOs of each sp shell first, padded to whole
 // warps, then the s shells: warps never mix the two code paths).  Share k
-// takes every S-th ket of each list; its partial rows and row part of Jh go to
-// its own slice (the assembly adds the S slices in order), so the result does
+// takes every S-th ket of each list; its partial rows and row part of Jh (the latter
+// per column group) go to its own slice (the assembly adds the S slices in order), so the result does
 // not depend on timing.
 template <int CP>
-__global__ void __launch_bounds__(QS_THREADS) qs_row_kernel(QsArgs g) {
+__global__ void __launch_bounds__(QS_THREADS, 8) qs_row_kernel(QsArgs g) {
   constexpr int NA = nfa(CP), NB = nfb(CP);
   __shared__ double red[QS_THREADS / 32][NA * NB];
-  const int r = blockIdx.x, k = blockIdx.y, S = gridDim.y;
+  const int r = blockIdx.x, k = blockIdx.y, S = gridDim.y, z = blockIdx.z;
   const int P = g.perm[g.cls_off[CP] + r];
   const int A = g.shA[P], B = g.shB[P], i0 = g.aoA[P], j0 = g.aoB[P];
   const size_t n = g.n;
@@ -246,10 +287,10 @@ __global__ void __launch_bounds__(QS_THREADS) qs_row_kernel(QsArgs g) {
 #pragma unroll
     for (int b = 0; b < 4; ++b) Jr[a][b] = 0.0;
   double *kp0 = g.Kpart + ((size_t)k * g.npairs + P) * 8 * n;
-  for (int t = threadIdx.x; t < g.nthr; t += blockDim.x) {
+  const int t = z * QS_THREADS + threadIdx.x;
+  if (t < g.nthr && g.thr_shell[t] >= 0) {
     double KA[4] = {0.0, 0.0, 0.0, 0.0}, KB[4] = {0.0, 0.0, 0.0, 0.0};
     row_column<CP>(g, r, P, A, B, i0, j0, t, k, S, KA, KB, Jr);
-    if (g.thr_shell[t] < 0) continue;
     double *kp = kp0 + g.thr_ao[t];  // this column of P's partial rows: A's rows, then B's
 #pragma unroll
     for (int a = 0; a < NA; ++a) kp[(size_t)a * n] = KA[a];
@@ -271,7 +312,7 @@ __global__ void __launch_bounds__(QS_THREADS) qs_row_kernel(QsArgs g) {
   if (threadIdx.x < NA * NB) {
     double v = 0.0;
     for (int q = 0; q < (int)(blockDim.x >> 5); ++q) v += red[q][threadIdx.x];
-    g.Jrow[((size_t)k * g.npairs + P) * 16 + threadIdx.x] = v;
+    g.Jrow[(((size_t)k * gridDim.z + z) * g.npairs + P) * 16 + threadIdx.x] = v;
   }
 }
 
@@ -378,7 +419,7 @@ __global__ void qs_jhat_kernel(QsArgs g) {
   for (int a = 0; a < NA; ++a)
     for (int b = 0; b < NB; ++b) {
       double v = 0.0;
-      for (int k = 0; k < g.nshare[cls]; ++k) v += g.Jrow[((size_t)k * g.npairs + P) * 16 + a * NB + b];
+      for (int k = 0; k < g.nshare[cls] * g.ngroup; ++k) v += g.Jrow[((size_t)k * g.npairs + P) * 16 + a * NB + b];
       g.Jh[(i0 + a) + n * (j0 + b)] = 4.0 * (v + g.Jcol[(size_t)P * 16 + a * NB + b]);
     }
 }
@@ -480,7 +521,7 @@ int qstore_build(mq_ctx *c) {
   }
   Blob blob;
   size_t o_off[6], o_len[6], o_rcol[6];
-  long long base = 0;
+  long long base = 0, elems = 0;
   double quartets = 0, unique = 0;
   for (int cP = 0; cP < 3; ++cP)
     for (int cQ = 0; cQ <= cP; ++cQ) {
@@ -522,8 +563,9 @@ int qstore_build(mq_ctx *c) {
         rcol[s] = lo;
       }
       cb.total = off[cb.nP];
-      cb.base = base;
-      base += cb.total * cb.nout;
+      cb.base = base;  // (a sector: the row pass reads pairs of elements)
+      base += (cb.total * cb.nout + 3) / 4 * 4;
+      elems += cb.total * cb.nout;
       quartets += (double)cb.total;
       // canonical unique integrals of the combination: degenerate blocks
       // (A = B, C = D, P = Q) hold fewer than NA NB NC ND
@@ -558,7 +600,19 @@ int qstore_build(mq_ctx *c) {
   // row-pass threads, one per AO column: the four AOs of each sp shell
   // (padded to a warp multiple), then the s shells' AOs (padded)
   std::vector<int> thr_shell, thr_ao;
-  for (int s = 0; s < nsh; ++s)
+  // The shells with more strong pairs first: a warp's lanes walk lists of similar
+  // length (an FP64 instruction costs the same with one lane as with 32; in the
+  // order of the atoms 17 to 19 of 32 were active).  Strong: a quartet of two
+  // such pairs just passes.
+  std::vector<int> strong(nsh, 0), order(nsh);
+  for (int p = 0; p < np; ++p)
+    if (sch[p] * sch[p] >= thr) {
+      ++strong[c->hp_shA[p]];
+      ++strong[c->hp_shB[p]];
+    }
+  for (int s = 0; s < nsh; ++s) order[s] = s;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return strong[a] > strong[b]; });
+  for (int s : order)
     if (c->shells[s].type == 1)
       for (int f = 0; f < 4; ++f) {
         thr_shell.push_back(s);
@@ -569,7 +623,7 @@ int qstore_build(mq_ctx *c) {
     thr_ao.push_back(0);
   }
   const int nsp_pad = (int)thr_shell.size();
-  for (int s = 0; s < nsh; ++s)
+  for (int s : order)
     if (c->shells[s].type == 0) {
       thr_shell.push_back(s);
       thr_ao.push_back(c->shells[s].ao0);
@@ -688,8 +742,8 @@ int qstore_build(mq_ctx *c) {
   qs.shell_qmax = (double *)(d + o_qm);
   qs.pinfo = (int4 *)(d + o_pi);
   qs.partners = (int *)(d + o_ptn);
-  qs.X_elems = (size_t)base;
-  qs.X = (double *)buf(c, "qstore_X", sizeof(double) * std::max<size_t>(qs.X_elems, 1));
+  qs.X_elems = (size_t)elems;
+  qs.X = (double *)buf(c, "qstore_X", sizeof(double) * std::max<size_t>((size_t)base, 1));
   if (!qs.X) return MQ_ENOMEM;
   qs.quartets = quartets;
   qs.unique = unique;
@@ -755,8 +809,9 @@ int qstore_fock_rhf(mq_ctx *c, const double *d_D, double *d_G, const double *d_G
   const int n = c->nao, np = c->pt.npairs;
   const size_t N = n, n2 = N * N;
   const size_t SH = QS_MAX_SHARES;
+  const size_t NG = (qs.nthr + QS_THREADS - 1) / QS_THREADS;
   double *w = (double *)buf(c, "qstore_fock",
-                            sizeof(double) * (SH * np * 8 * N + SH * np * 16 + (size_t)np * 16 + 2 * n2));
+                            sizeof(double) * (SH * np * 8 * N + SH * NG * np * 16 + (size_t)np * 16 + 2 * n2));
   if (!w) return MQ_ENOMEM;
   QsArgs g = qs_args(c);
   g.D = d_D;
@@ -764,7 +819,8 @@ int qstore_fock_rhf(mq_ctx *c, const double *d_D, double *d_G, const double *d_G
   g.kscreen = kscreen;
   g.Kpart = w;
   g.Jrow = w + SH * np * 8 * N;
-  g.Jcol = g.Jrow + SH * np * 16;
+  g.Jcol = g.Jrow + SH * NG * np * 16;
+  g.ngroup = (int)NG;
   g.Jh = g.Jcol + (size_t)np * 16;
   g.Kh = g.Jh + n2;
   // pairs that are no bra (or no ket) of any stored quartet still get their
@@ -774,13 +830,19 @@ int qstore_fock_rhf(mq_ctx *c, const double *d_D, double *d_G, const double *d_G
   g.nshare[0] = QS_SHARES[0];
   g.nshare[1] = QS_SHARES[1];
   g.nshare[2] = QS_SHARES[2];
-  const int rt = std::min(QS_THREADS, qs.nthr);
-  if (qs.ncls[0]) qs_row_kernel<0><<<dim3(qs.ncls[0], g.nshare[0]), rt, 0, c->stream>>>(g);
-  if (qs.ncls[1]) qs_row_kernel<1><<<dim3(qs.ncls[1], g.nshare[1]), rt, 0, c->stream>>>(g);
-  if (qs.ncls[2]) qs_row_kernel<2><<<dim3(qs.ncls[2], g.nshare[2]), rt, 0, c->stream>>>(g);
-  if (qs.ncls[0]) qs_col_kernel<0><<<qs.ncls[0], QS_COL_THREADS, 0, c->stream>>>(g);
-  if (qs.ncls[1]) qs_col_kernel<1><<<qs.ncls[1], QS_COL_THREADS, 0, c->stream>>>(g);
-  if (qs.ncls[2]) qs_col_kernel<2><<<qs.ncls[2], QS_COL_THREADS, 0, c->stream>>>(g);
+  const int rt = QS_THREADS;
+  const unsigned ng = (unsigned)NG;
+  // the six passes are independent, and each is a few waves of CTAs that wait on
+  // memory: side by side, the longest first, on the context's own stream
+  cudaStream_t main = c->stream;
+  MQ_TRY(fork_streams(c));
+  if (qs.ncls[2]) qs_row_kernel<2><<<dim3(qs.ncls[2], g.nshare[2], ng), rt, 0, main>>>(g);
+  if (qs.ncls[1]) qs_row_kernel<1><<<dim3(qs.ncls[1], g.nshare[1], ng), rt, 0, c->fork[0]>>>(g);
+  if (qs.ncls[0]) qs_col_kernel<0><<<qs.ncls[0], QS_COL_THREADS, 0, c->fork[1]>>>(g);
+  if (qs.ncls[1]) qs_col_kernel<1><<<qs.ncls[1], QS_COL_THREADS, 0, c->fork[2]>>>(g);
+  if (qs.ncls[2]) qs_col_kernel<2><<<qs.ncls[2], QS_COL_THREADS, 0, c->fork[3]>>>(g);
+  if (qs.ncls[0]) qs_row_kernel<0><<<dim3(qs.ncls[0], g.nshare[0], ng), rt, 0, c->fork[4]>>>(g);
+  MQ_TRY(join_streams(c));
   qs_khat_kernel<<<dim3(c->nshell, (4 * n + QS_COL_THREADS - 1) / QS_COL_THREADS), QS_COL_THREADS, 0, c->stream>>>(g);
   qs_jhat_kernel<<<(np + 127) / 128, 128, 0, c->stream>>>(g);
   qs_combine_kernel<<<(unsigned)((n2 + 255) / 256), 256, 0, c->stream>>>(g.Jh, g.Kh, n, 0.5, d_Gprev, d_G);
