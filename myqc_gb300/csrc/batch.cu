@@ -574,7 +574,7 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
     MQ_CUDA(c, cudaGetLastError());
     return MQ_OK;
   };
-  const int per_iter = 4 + (ndiis > 0 ? 1 : 0) + 3;  // split, digest (3), energy, diis, density
+  const int per_iter = 4 + (ndiis > 0 ? 1 : 0) + 3;  // digest (columns or split, tiles, 2), energy, diis, density
   StageTimer t_all;
   t_all.start(c->stream);
   MQ_TRY(iteration());  // eager: sets kernel attributes outside any capture

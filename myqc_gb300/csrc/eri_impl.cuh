@@ -26,10 +26,13 @@
 // Work decomposition: one thread per contracted shell quartet.  Shell pairs
 // are kept in three classes (s,s), (sp,s), (sp,sp); a kernel instance serves
 // one (bra class, ket class) combination, so every thread of a launch runs the
-// same fully unrolled register code.  Quartets with more than 16 integrals
-// ((sp sp|sp s): 64, (sp sp|sp sp): 256) are split over 4 or 16 threads by
-// ket function c or ket pair (c, d), each thread forming the whole bra; the
-// split index is constant per warp (warp w serves split w % nsplit for 32
+// same fully unrolled register code.  In FP64 the stored epilogues (EPI_XX,
+// EPI_STORE) of every class but (sp sp|sp sp) take the early-contracted kernels of
+// eri_low.cuh, and (sp sp|sp sp) the shared form below (quartet_shared).
+// Otherwise quartets with more than 16 integrals ((sp sp|sp s): 64,
+// (sp sp|sp sp): 256) are split over 4 or 16 threads by ket function c or ket
+// pair (c, d), each thread forming the whole bra.  A split index is
+// constant per warp (warp w serves split w % nsplit for 32
 // consecutive quartets), so no lane diverges.  The Schwarz launches split a
 // diagonal quartet (P|P) the same way into one thread per diagonal integral
 // (ab|ab).
@@ -594,8 +597,7 @@ __device__ __forceinline__ bool next_survivor(const PairTable &t, int p1, int q0
   return false;
 }
 
-// FP64 pass of the split classes ((sp sp|sp s): 4 warps, one ket
-// function c each; (sp sp|sp sp): 16 warps, one ket pair (c, d) each), with
+// FP64 pass of (sp sp|sp sp): 16 warps, one ket pair (c, d) each, with
 // the per-primitive-quartet work shared.  The CTA's warps serve the same 32
 // quartets (lane = quartet), so every one of them needs the same Boys values
 // and Hermite integrals R_tuv of each primitive quartet.  A lane's surviving
@@ -762,11 +764,11 @@ __device__ __forceinline__ void quartet_shared(const EriArgs &g, bool valid, int
   eri_epilogue<LA, LB, LC, LD, 0, NA, 0, NB, C0, C1, D0, D1, EPI>(h, P, Q, n, XXout, acc, 0u);
 }
 
-// A split class: one CTA of NSPLIT warps per 32 quartets.
+// (sp sp|sp sp): one CTA of 16 warps per 32 quartets.
 template <int LA, int LB, int LC, int LD, int EPI>
 __global__ void __launch_bounds__(512) eri_shared_kernel(EriArgs g) {
   constexpr int NOUT = nfun(LA) * nfun(LB) * nfun(LC) * nfun(LD);
-  constexpr int NSPLIT = NOUT <= 64 ? 4 : 16;
+  constexpr int NSPLIT = 16;
   constexpr int NR = nherm(LA + LB + LC + LD);
   extern __shared__ double sm_shared[];  // R of the round's survivors [NSPLIT][32][NR], then their (bra, ket) pairs
   double *smR = sm_shared;

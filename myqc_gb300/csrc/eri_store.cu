@@ -1,6 +1,7 @@
 // eri_store.cu -- the quartet store's integral pass (qstore.cu builds its
 // tables): one launch per class combination over the staircase of surviving
-// quartets; the split classes share their per-primitive work across warps.
+// quartets, early-contracted but for (sp sp|sp sp), whose warps share their
+// per-primitive work.
 // Also the launch-order binning of the integral launches and the autotuner
 // that picks, per class combination and size, whether to bin, whether the
 // warps take their quartets from a persistent work queue, and the CTA size.

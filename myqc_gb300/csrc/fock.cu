@@ -26,8 +26,9 @@ namespace mq {
 
 constexpr int FOCK_THREADS = 256;
 
-// Arithmetic of the digestion.  ArithF64 is plain FP64, the reference's
-// arithmetic (the default).  ArithDF32 keeps each integral as a float pair and
+// Arithmetic of the digestion.  FP64 builds, the default, run fock_fx_kernel
+// (FP64 products on the tensor cores); ArithF64 is plain FP64, for the build that allocates
+// nothing.  ArithDF32 keeps each integral as a float pair and
 // the row sums as double-float on the FP32 pipes (opt-in, mq_set_fock_precision):
 // about 2^-48 relative per product, below 1e-12 relative on G.  Either way
 // the sums over slabs and the assembly are FP64.

@@ -2,10 +2,11 @@
 // device routines shared by the batched eigensolver kernel (linalg.cu) and the
 // per-molecule SCF kernels of the batch engine (batch.cu).
 //
-// Each sweep runs the n'-1 rounds of a round-robin tournament (n' = n rounded
-// up to even); a round rotates n'/2 disjoint index pairs at once: rotation
-// angles, then rows, then columns of A and V, with a block barrier between
-// phases.  Converges when the off-diagonal Frobenius norm falls below
+// An FP32 Jacobi gives start vectors, products on the tensor cores refine them to
+// FP64, and a cyclic FP64 Jacobi finishes where that leaves something.  Each sweep runs
+// the n'-1 rounds of a round-robin tournament (n' = n rounded
+// up to even); a round rotates n'/2 disjoint index pairs at once.
+// Converges when the off-diagonal Frobenius norm falls below
 // tol * ||A||_F.  Replaces the eigen step of DSYEV/DSYGV (src/scf/scf.f90:692,
 // 478, 848).
 #pragma once

@@ -1,15 +1,10 @@
 // linalg.cu -- FP64 dense kernels for the SCF: batched cyclic Jacobi
 // eigensolver (replaces LAPACK DSYEV/DSYGV's eigen step, src/scf/scf.f90:692,
-// 478, 848), density matrix (src/dens/dens.f90:115-124, 213-228), and GEMM
-// wrappers (plain library GEMMs go to cuBLAS).
+// 478, 848) and density matrix (src/dens/dens.f90:115-124, 213-228).
 //
-// Jacobi: one CTA per matrix.  Each sweep runs the n'-1 rounds of a
-// round-robin tournament (n' = n rounded up to even); a round rotates n'/2
-// disjoint index pairs at once: rotation angles, then rows, then columns of
-// A and V, with a block barrier between phases.  The matrix and the
-// eigenvectors live in shared memory when 2 n^2 doubles fit, else in a
-// global workspace.  Converges when the off-diagonal Frobenius norm falls
-// below tol * ||A||_F; the result is sorted ascending.
+// Jacobi: one CTA per matrix (jacobi.cuh).  The matrix and the
+// eigenvectors live in shared memory when 2 n^2 doubles and the working set
+// fit, else in a global workspace; the result is sorted ascending.
 
 #include <string>
 
