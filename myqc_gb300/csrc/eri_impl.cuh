@@ -94,6 +94,7 @@ struct EriArgs {
   // they last; units = warp slots of the launch (quartets / 32 x split)
   unsigned long long *queue;
   long long units;
+  int lg;  // eri_shared_kernel: 2^lg lanes per quartet
 };
 
 __host__ __device__ constexpr int fl(int f, int axis) { return f == axis + 1 ? 1 : 0; }  // f: 0 s, 1 px, 2 py, 3 pz
@@ -610,6 +611,13 @@ __device__ __forceinline__ bool next_survivor(const PairTable &t, int p1, int q0
 // outputs.  The round count is the warp's largest S (every warp of the CTA
 // computes the same S per lane), so the barriers are reached by every thread,
 // and a round has idle producers only at the end of a lane's list.
+//
+// A CTA keeps its SM's FP64 pipe busy (89 %), so a launch of fewer CTAs than SMs, or with
+// few heavy ones, takes as long as its heaviest CTA: 1.44 ms for (H2O)16's 85 CTAs, whose
+// SMs were active 21 % of it, and as long for one quartet.  Small launches
+// therefore give a quartet 2^lg lanes (lane = quartet << lg | part): part i
+// takes the survivors k = i mod 2^lg, and the parts' sums are added across
+// the lanes at the end.  Integrals of H2O+ 1.44 -> 0.34 ms, of (H2O)8 1.51 -> 0.95 ms.
 template <int LA, int LB, int LC, int LD, int NSPLIT, int C0, int C1, int D0, int D1, int EPI>
 __device__ __forceinline__ void quartet_shared(const EriArgs &g, bool valid, int P, int Q, size_t n, double *XXout,
                                                double *smR, int2 *smI) {
@@ -640,12 +648,14 @@ __device__ __forceinline__ void quartet_shared(const EriArgs &g, bool valid, int
       S += m;
     }
   }
-  const int rounds = (__reduce_max_sync(0xffffffffu, S) + NSPLIT - 1) / NSPLIT;
-  // this warp's producer position: survivor w, then NSPLIT further each round
+  const int lg = g.lg, part = lane & ((1 << lg) - 1);
+  const int mine = (S - part + (1 << lg) - 1) >> lg;  // survivors of this lane (<= 0: none)
+  const int rounds = (__reduce_max_sync(0xffffffffu, mine) + NSPLIT - 1) / NSPLIT;
+  // this warp's producer position: the lane's survivor w, then NSPLIT further each round
   int ip = p0, iq = q0 - 1;
   double Kab = valid && p0 < p1 ? t.K[p0] : 0.0;
-  bool live = S > 0;
-  for (int k = 0; k <= w && live; ++k) live = next_survivor(t, p1, q0, q1, ip, iq, Kab);
+  bool live = w < mine;
+  for (int k = 0; k <= (w << lg) + part && live; ++k) live = next_survivor(t, p1, q0, q1, ip, iq, Kab);
   const bool parity = g.mode == MQ_MODE_REFERENCE;
   const double pref0 = parity ? 2.0 * 17.493419544621675 : 2.0 * 17.493418327624862;  // 2 pi^2.5
   unsigned nprim = 0;
@@ -681,7 +691,8 @@ __device__ __forceinline__ void quartet_shared(const EriArgs &g, bool valid, int
 #pragma unroll
             for (int z = 0; z <= LT; ++z)
               if (x + y + z <= LT) dst[ridx(LT, x, y, z)] = R[x][y][z];
-        for (int k = 0; k < NSPLIT && live; ++k) live = next_survivor(t, p1, q0, q1, ip, iq, Kab);
+        live = (r + 1) * NSPLIT + w < mine;
+        for (int k = 0; k < NSPLIT << lg && live; ++k) live = next_survivor(t, p1, q0, q1, ip, iq, Kab);
       }
       smI[w * 32 + lane] = id;
     }
@@ -752,19 +763,28 @@ __device__ __forceinline__ void quartet_shared(const EriArgs &g, bool valid, int
   }
   if (g.counters) {  // quartets by warp 0, the primitive quartets each warp formed
     const unsigned np_w = __reduce_add_sync(0xffffffffu, nprim);
-    const unsigned nq_w = __popc(__ballot_sync(0xffffffffu, valid));
+    const unsigned nq_w = __popc(__ballot_sync(0xffffffffu, valid && part == 0));
     if (lane == 0) {
       if (w == 0) atomicAdd(g.counters, (unsigned long long)nq_w);
       atomicAdd(g.counters + 1, (unsigned long long)np_w);
     }
   }
-  if (!valid) return;
+  for (int o = 1; o < 1 << lg; o <<= 1)
+#pragma unroll
+    for (int a = 0; a < NA; ++a)
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int c = 0; c < C1 - C0; ++c)
+#pragma unroll
+          for (int d = 0; d < D1 - D0; ++d) acc[a][b][c][d] += __shfl_xor_sync(0xffffffffu, acc[a][b][c][d], o);
+  if (!valid || part != 0) return;
   EriArgs h = g;
   h.counters = nullptr;  // counted above
   eri_epilogue<LA, LB, LC, LD, 0, NA, 0, NB, C0, C1, D0, D1, EPI>(h, P, Q, n, XXout, acc, 0u);
 }
 
-// (sp sp|sp sp): one CTA of 16 warps per 32 quartets.
+// (sp sp|sp sp): one CTA of 16 warps per 32 >> lg quartets.
 template <int LA, int LB, int LC, int LD, int EPI>
 __global__ void __launch_bounds__(512) eri_shared_kernel(EriArgs g) {
   constexpr int NOUT = nfun(LA) * nfun(LB) * nfun(LC) * nfun(LD);
@@ -774,7 +794,7 @@ __global__ void __launch_bounds__(512) eri_shared_kernel(EriArgs g) {
   double *smR = sm_shared;
   int2 *smI = reinterpret_cast<int2 *>(sm_shared + NSPLIT * 32 * NR);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  long long q = (long long)blockIdx.x * 32 + lane;
+  long long q = ((long long)blockIdx.x * 32 + lane) >> g.lg;
   int P = 0, Q = 0, m = 0;
   const bool valid = decode(g, q, P, Q, m);
   size_t n = (size_t)g.n;
@@ -912,6 +932,10 @@ int bin_quartets(mq_ctx *c, EriArgs &h, int slot);
 // the batch's integral launch of one class combination, in its autotuned shape (eri_store.cu)
 int eri_batch_launch(mq_ctx *c, const EriArgs &h, int cP, int cQ);
 
+// eri_shared_kernel gives quartets more lanes up to this many waves of CTAs: for (H2O)8
+// (666 quartets) 0.95 ms of integrals with 2, 1.12 with 4 and 1.00 with 8; (H2O)24 7.58, 7.67, 7.89
+constexpr int SHARED_WAVES = 2;
+
 // One class combination's integral launch; `block` is the CTA size of the
 // thread-per-quartet kernel (64, 128 or 256; the autotuner's choice)
 template <int EPI, class RT = double>
@@ -941,7 +965,12 @@ static int launch_class(mq_ctx *c, EriArgs g, int cP, int cQ, int block = 128, b
   dim3 gd((unsigned)grid);
   if constexpr (early) {
     if (nsplit == 16) {  // (sp sp|sp sp): per-primitive work shared by the CTA's warps
-      const long long ctas = (g.nq + 31) / 32;
+      int sms = 0;
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+      // up to 32 lanes per quartet while that makes fewer than SHARED_WAVES waves of CTAs
+      g.lg = 0;
+      while (g.lg < 5 && (g.nq << g.lg) < 32LL * SHARED_WAVES * sms) ++g.lg;
+      const long long ctas = ((g.nq << g.lg) + 31) / 32;
       if (ctas > 2147483647LL) return set_err(c, MQ_EINVAL, "integral launch too large");
       const size_t sm = sizeof(double) * 16 * 32 * nherm(4) + sizeof(int2) * 16 * 32;
       MQ_CUDA(c, cudaFuncSetAttribute(eri_shared_kernel<1, 1, 1, 1, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
