@@ -32,10 +32,11 @@ namespace mq {
 
 constexpr int PUR_THREADS = 1024;
 
-// sums over the block of two values per thread, in every thread (red: 64); one
+// sums over the block of two values per thread, in every thread; one
 // warp adds the warps' sums (each FP64 addition occupies the SM for 16 clocks
-// per warp that executes it)
-__device__ __forceinline__ void block_sum2(double &v, double &u, double *red) {
+// per warp that executes it).  red holds two sums of up to 32 warps: taken as an
+// array of that length, so that a shorter one does not compile.
+__device__ __forceinline__ void block_sum2(double &v, double &u, double (&red)[64]) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -146,7 +147,7 @@ static int gershgorin(mq_ctx *c, const double *F, int n, int sym, double *lohi) 
 // same choice; CTA 0 records the idempotency error tr X - tr T of step k.
 __global__ void purify_step_kernel(const double *__restrict__ X, const double *__restrict__ T, int n, double nocc,
                                    double *__restrict__ Xn, double *__restrict__ err, int k) {
-  __shared__ double red[32];
+  __shared__ double red[64];
   const size_t N = n, n2 = N * N;
   double tx = 0.0, tt = 0.0;
   for (int r = threadIdx.x; r < n; r += blockDim.x) {
@@ -202,7 +203,7 @@ __device__ __forceinline__ void tile_of(int t, int &I, int &J) {
 
 // partial sums of one tile of X (lower triangle): [0] diagonal, [1] squares
 // weighted by 2 off the diagonal tiles; written to part[2 * tile + 0/1]
-__device__ __forceinline__ void tile_partials(double tr, double sq, double *red, double *part, int tile) {
+__device__ __forceinline__ void tile_partials(double tr, double sq, double (&red)[64], double *part, int tile) {
   block_sum2(tr, sq, red);
   if (threadIdx.x == 0) {
     part[2 * tile] = tr;
