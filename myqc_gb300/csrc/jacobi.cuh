@@ -436,13 +436,20 @@ static __device__ bool jacobi_block(int n, double *A, double *V, double *red, do
   return false;
 }
 
-// Rank of eigenvalue i among the diagonal of A (ascending, ties by index).
+// Rank of eigenvalue i among the diagonal of A (ascending, ties by index): the
+// ranks are a permutation of 0 .. n - 1 whatever the diagonal holds, since
+// callers place i at its rank.  The bit patterns, ordered as the numbers are,
+// give NaN a place too.
 __device__ __forceinline__ int jacobi_rank(int n, const double *A, int i) {
-  const double wi = A[i + (size_t)n * i];
+  auto key = [&](int j) {
+    const long long b = __double_as_longlong(A[j + (size_t)n * j]);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+  };
+  const long long ki = key(i);
   int rank = 0;
   for (int j = 0; j < n; ++j) {
-    const double wj = A[j + (size_t)n * j];
-    rank += (wj < wi) || (wj == wi && j < i);
+    const long long kj = key(j);
+    rank += kj < ki || (kj == ki && j < i);
   }
   return rank;
 }
