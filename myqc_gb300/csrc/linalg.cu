@@ -37,13 +37,16 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(int n, double *__re
 // Multi-CTA Jacobi for one large matrix (n > JAC_SMEM_MAX).  Each round of the
 // tournament applies A <- J^T A J as independent 2x2 block transforms
 // A[P,Q] <- J_P^T A[P,Q] J_Q over index pairs P >= Q (the mirror block is the
-// transpose), and V <- V J row by row; no element is touched by two threads,
-// so a round needs a single grid barrier.  Every CTA recomputes the round's
-// rotation angles from the diagonal it reads after the barrier.  The barrier
+// transpose), and V <- V J row by row; no element is written by two threads.
+// Every CTA recomputes the round's rotation angles from the matrix it reads after
+// the barrier, so a round reads one copy of A and writes the other: with one copy, a
+// CTA that was late with its angles met the elements that a faster one had
+// already rotated, took other angles, or found none left and skipped the barrier
+// the others waited at.  So a round needs a single grid barrier.  The barrier
 // (gridsync.cuh) raises an error flag on time-out and every CTA leaves.
 // Launched cooperatively so that all CTAs are resident.
 constexpr int JG_THREADS = 256;
-__global__ void __launch_bounds__(JG_THREADS) jacobi_grid_kernel(int n, double *__restrict__ A,
+__global__ void __launch_bounds__(JG_THREADS) jacobi_grid_kernel(int n, double *A, double *B,
                                                                   double *__restrict__ V, double *__restrict__ w,
                                                                   double *__restrict__ Vout, double *part,
                                                                   GridSync gs, int max_sweeps, double tol,
@@ -116,8 +119,8 @@ __global__ void __launch_bounds__(JG_THREADS) jacobi_grid_kernel(int n, double *
         cs[2 * k] = c;
         cs[2 * k + 1] = s;
       }
-      // every CTA reads the same A, so all skip a round without rotations
-      // together, barrier included
+      // every CTA reads the same A, which nothing writes in this round, so all skip a
+      // round without rotations together, barrier included
       if (!__syncthreads_or(active)) continue;
       // blocks (P, Q) with P >= Q, and V rows
       const long long nblk = (long long)half * (half + 1) / 2;
@@ -133,13 +136,16 @@ __global__ void __launch_bounds__(JG_THREADS) jacobi_grid_kernel(int n, double *
           const double cP = cs[2 * P], sP = cs[2 * P + 1], cQ = cs[2 * Q], sQ = cs[2 * Q + 1];
           const bool qv = q < n, vv = v < n;
           if (P == Q) {
-            if (!qv) continue;
+            if (!qv) {  // the index without a partner
+              B[p + N * p] = A[p + N * p];
+              continue;
+            }
             const double app = A[p + N * p], aqq = A[q + N * q], apq = A[p + N * q];
             // diagonalised 2x2 block
-            A[p + N * p] = cP * cP * app - 2 * cP * sP * apq + sP * sP * aqq;
-            A[q + N * q] = sP * sP * app + 2 * cP * sP * apq + cP * cP * aqq;
-            A[p + N * q] = 0.0;
-            A[q + N * p] = 0.0;
+            B[p + N * p] = cP * cP * app - 2 * cP * sP * apq + sP * sP * aqq;
+            B[q + N * q] = sP * sP * app + 2 * cP * sP * apq + cP * cP * aqq;
+            B[p + N * q] = 0.0;
+            B[q + N * p] = 0.0;
             continue;
           }
           // rows {p,q} x cols {u,v}
@@ -151,19 +157,19 @@ __global__ void __launch_bounds__(JG_THREADS) jacobi_grid_kernel(int n, double *
           // J_Q (columns)
           const double n_pu = cQ * b_pu - sQ * b_pv, n_pv = sQ * b_pu + cQ * b_pv;
           const double n_qu = cQ * b_qu - sQ * b_qv, n_qv = sQ * b_qu + cQ * b_qv;
-          A[p + N * u] = n_pu;
-          A[u + N * p] = n_pu;
+          B[p + N * u] = n_pu;
+          B[u + N * p] = n_pu;
           if (qv) {
-            A[q + N * u] = n_qu;
-            A[u + N * q] = n_qu;
+            B[q + N * u] = n_qu;
+            B[u + N * q] = n_qu;
           }
           if (vv) {
-            A[p + N * v] = n_pv;
-            A[v + N * p] = n_pv;
+            B[p + N * v] = n_pv;
+            B[v + N * p] = n_pv;
           }
           if (qv && vv) {
-            A[q + N * v] = n_qv;
-            A[v + N * q] = n_qv;
+            B[q + N * v] = n_qv;
+            B[v + N * q] = n_qv;
           }
         } else {
           const long long t = idx - nblk;
@@ -178,6 +184,9 @@ __global__ void __launch_bounds__(JG_THREADS) jacobi_grid_kernel(int n, double *
         }
       }
       if (!grid_barrier(gs, nb)) return;
+      double *x = A;
+      A = B;
+      B = x;
     }
   }
   if (sweep >= max_sweeps && blockIdx.x == 0 && tid == 0) atomicExch(gs.err, 1);
@@ -215,10 +224,10 @@ int syev_large_device(mq_ctx *c, int n, double *d_A, const double *d_V0, double 
   const int half = (n + 1) / 2;
   int nblocks = std::min(sms * std::max(per_sm, 1), std::max(1, (half * (half + 1) / 2 + JG_THREADS - 1) / JG_THREADS));
   nblocks = std::max(1, std::min(nblocks, sms));
-  char *ws = (char *)buf(c, "jacobi_grid", 256 + sizeof(double) * (n2 + nblocks));
+  char *ws = (char *)buf(c, "jacobi_grid", 256 + sizeof(double) * (2 * n2 + nblocks));
   if (!ws) return MQ_ENOMEM;
   GridSync gs{(unsigned *)ws, (unsigned *)(ws + 64), (int *)(ws + 128)};
-  double *V = (double *)(ws + 256), *part = V + n2;
+  double *V = (double *)(ws + 256), *B = V + n2, *part = B + n2;
   MQ_CUDA(c, cudaMemsetAsync(ws, 0, 256, c->stream));
   if (d_V0) {
     MQ_CUDA(c, cudaMemcpyAsync(V, d_V0, n2 * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
@@ -229,7 +238,7 @@ int syev_large_device(mq_ctx *c, int n, double *d_A, const double *d_V0, double 
   int max_sweeps = 40;
   double tol = 1e-14;  // ||offdiag||_F / ||A||_F at stop; eigenvalue error ~ tol^2 ||A|| / gap
   int *info = (int *)(ws + 192);
-  void *args[] = {&n, &d_A, &V, &d_w, &d_V, &part, &gs, &max_sweeps, &tol, &info};
+  void *args[] = {&n, &d_A, &B, &V, &d_w, &d_V, &part, &gs, &max_sweeps, &tol, &info};
   // every CTA of a grid-barrier kernel must be resident at once: nothing of
   // the side stream (the transform's XX slicing) runs beside it
   if (c->stream != c->side) MQ_TRY(join_side(c));
