@@ -236,7 +236,8 @@ __global__ void __launch_bounds__(BT) batch_density_kernel(
   }
   __syncthreads();
   // C_occ (n x nocc) into A, D_new
-  for (int i = threadIdx.x; i < n; i += blockDim.x) jw.e2[i] = 1;  // |entries| of an orthogonal matrix < 2
+  // |entries| of an orthogonal matrix < 2; V is NaN throughout if A was not finite
+  for (int i = threadIdx.x; i < n; i += blockDim.x) jw.e2[i] = isfinite(V[0]) ? 1 : FX_BAD;
   __syncthreads();
   cta_fix(nocc, n, true, jw.e2, jw.U2, [&](int r, int k) { return V[k + n * perm[r]]; });
   cta_fix_rows(n, n, Xm, n, 1, jw.e1, jw.U1);
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(BT) batch_density_kernel(
     if (!guess) {
       const int it = iters[m];
       const double diff = conv_rms ? sqrt(dss / (double)n2) : dmax;
-      const bool cv = it > 0 && diff < thr;
+      const bool cv = it > 0 && diff < thr && isfinite(dss);  // (the largest difference skips NaN)
       iters[m] = it + 1;
       if (cv || it + 1 >= max_iter) {
         active[m] = 0;

@@ -30,7 +30,6 @@ constexpr int GX_K = 128;          // K chunk (exact up to FX_KMAX)
 constexpr int GX_LD = GX_K / 2;    // pairs per row
 constexpr int GX_T = 32;           // tile
 constexpr int GX_THREADS = 256;
-constexpr int GX_BAD = 4000;       // exponent that marks a row with a non-finite element
 
 // The 32 rows of an operand's K chunk as fixed-point pairs.  ROWFAST: element
 // (r, k) at x[r + ld k], else at x[k + ld r]; nr rows and kc elements exist.
@@ -42,9 +41,8 @@ __device__ __forceinline__ void gx_load(const double *__restrict__ x, size_t ld,
   const int pairs = (kc + 15) / 16 * 8;
   auto put = [&](int r, int kp, double a, double b, int ex) {
     U[r * GX_LD + fx_pos(r, kp)] =
-        ex == GX_BAD ? make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u) : fx_pair(fx_fix(a, ex), fx_fix(b, ex));
+        ex == FX_BAD ? make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u) : fx_pair(fx_fix(a, ex), fx_fix(b, ex));
   };
-  auto exponent = [](int f) { return f == 0x7ff ? GX_BAD : fx_exp(f); };
   if (ROWFAST) {  // lanes over the rows, warps over the pairs
     constexpr int NW = GX_THREADS / 32, PER = GX_LD / NW;
     if (tid < GX_T) fields[tid] = 0;
@@ -61,7 +59,7 @@ __device__ __forceinline__ void gx_load(const double *__restrict__ x, size_t ld,
     __syncthreads();
     if (f) atomicMax(fields + lane, f);
     __syncthreads();
-    const int ex = exponent(fields[lane]);
+    const int ex = fx_row_exp(fields[lane]);
     if (w == 0) e[lane] = ex;
 #pragma unroll
     for (int i = 0; i < PER; ++i)
@@ -82,7 +80,7 @@ __device__ __forceinline__ void gx_load(const double *__restrict__ x, size_t ld,
     for (int j = 0; j < PER; ++j) {
       const int r = w * PER + j;
       const int f = max(max(fx_field(v[j][0]), fx_field(v[j][1])), max(fx_field(v[j][2]), fx_field(v[j][3])));
-      const int ex = exponent(__reduce_max_sync(0xffffffffu, f));
+      const int ex = fx_row_exp(__reduce_max_sync(0xffffffffu, f));
       if (lane == 0) e[r] = ex;
       if (lane < pairs) put(r, lane, v[j][0], v[j][1], ex);
       if (lane + 32 < pairs) put(r, lane + 32, v[j][2], v[j][3], ex);
@@ -125,7 +123,7 @@ __global__ void __launch_bounds__(GX_THREADS, 2) dgemm_kernel(int mx, int ny, in
       for (int i = 0; i < 4; ++i) {
         const int r = wr + g + 8 * (i >> 1), c = wc + 2 * t + (i & 1);
         double x = 0.0;
-        if (ex[r] != GX_BAD && ey[c] != GX_BAD) {
+        if (ex[r] != FX_BAD && ey[c] != FX_BAD) {
           float v[FX_DIG];
 #pragma unroll
           for (int L = 0; L < FX_DIG; ++L) v[L] = acc[L][i];

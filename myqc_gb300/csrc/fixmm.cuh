@@ -49,13 +49,20 @@ __device__ __forceinline__ unsigned long long fx_fix(double x, int e) {
   const int E = (int)(hi >> 20) & 0x7ff;
   const unsigned h = (hi & 0xfffffu) | 0x100000u;
   // the significand with its leading bit at 2^61, moved down to the row's scale
-  unsigned long long m = ((unsigned long long)(h << 9 | lo >> 23) << 32 | lo << 9) >> min(e + 1022 - E, 63);
+  // (unsigned: an element above its row's scale, an infinity or NaN under a fixed
+  // exponent, is cut to 0)
+  unsigned long long m = ((unsigned long long)(h << 9 | lo >> 23) << 32 | lo << 9) >> min((unsigned)(e + 1022 - E), 63u);
   if (E == 0) m = 0;
   return ((int)hi < 0 ? 0ull - m : m) + FX_BIAS;
 }
 // e with |x| < 2^e for every x of exponent field <= E (0 for a zero row)
 __device__ __forceinline__ int fx_exp(int E) { return E == 0 ? -1100 : E - 1022; }
 __device__ __forceinline__ int fx_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+// The exponent of a row with an infinity or NaN, which has no fixed-point form:
+// the products with it are NaN, or summed in FP64 from the operands as they are
+// where those are at hand (dgemm.cu, fock.cu).
+constexpr int FX_BAD = 4000;
+__device__ __forceinline__ int fx_row_exp(int E) { return E == 0x7ff ? FX_BAD : fx_exp(E); }
 
 // Two biased integers with their bytes alternating, lowest first
 __device__ __forceinline__ uint4 fx_pair(unsigned long long u0, unsigned long long u1) {
@@ -168,7 +175,7 @@ static __device__ __forceinline__ void cta_row_exp(int nr, int nk, const double 
       int m = 0;
       for (int k = lane; k < nk; k += 32) m = max(m, fx_field(x[(size_t)r * rs + k]));
       m = __reduce_max_sync(0xffffffffu, m);
-      if (lane == 0) e[r] = fx_exp(m);
+      if (lane == 0) e[r] = fx_row_exp(m);
     }
   } else {  // 4 threads per row, 8 neighbouring rows per warp
     for (int r0 = 8 * w; r0 < nr; r0 += 8 * nw) {
@@ -178,7 +185,7 @@ static __device__ __forceinline__ void cta_row_exp(int nr, int nk, const double 
         for (int k = lane >> 3; k < nk; k += 4) m = max(m, fx_field(x[(size_t)r * rs + (size_t)k * ks]));
       m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
       m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
-      if (r < nr && lane < 8) e[r] = fx_exp(m);
+      if (r < nr && lane < 8) e[r] = fx_row_exp(m);
     }
   }
 }
@@ -211,7 +218,8 @@ static __device__ __forceinline__ void cta_fix_rows(int nr, int nk, const double
   __syncthreads();
 }
 
-// store(i, j, value) of the na x nb product of the fixed-point rows UA and UB
+// store(i, j, value) of the na x nb product of the fixed-point rows UA and UB;
+// NaN where a row's exponent is FX_BAD
 template <class Store>
 static __device__ __forceinline__ void cta_fix_mm(int na, int nb, int nk, const uint4 *UA, const int *ea,
                                                   const uint4 *UB, const int *eb, Store store) {
@@ -227,7 +235,10 @@ static __device__ __forceinline__ void cta_fix_mm(int na, int nb, int nk, const 
       float v[FX_DIG];
 #pragma unroll
       for (int L = 0; L < FX_DIG; ++L) v[L] = acc[L][i];
-      if (r < na && cc < nb) store(r, cc, fx_combine(v, ea[r], eb[cc]));
+      if (r < na && cc < nb) {
+        const int xa = ea[r], xb = eb[cc];
+        store(r, cc, xa == FX_BAD || xb == FX_BAD ? __longlong_as_double(0x7ff8000000000000ll) : fx_combine(v, xa, xb));
+      }
     }
   }
 }

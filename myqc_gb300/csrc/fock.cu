@@ -419,7 +419,6 @@ __global__ void __launch_bounds__(PAIR_MAX_THREADS) fock_pair_kernel(
 // fock_pair_kernel's.  A row or column with an infinity or NaN is summed in
 // FP64 as it is.
 constexpr int FXF_THREADS = 256;
-constexpr int FXF_BAD = 4000;  // exponent of a row with a non-finite element
 constexpr int FXF_JC = 4;      // slabs per tile at most
 
 // Column j (blockIdx.x) of molecule blockIdx.y, spin blockIdx.z, as fixed-point
@@ -438,9 +437,9 @@ __global__ void __launch_bounds__(32) fock_cols_kernel(const double *__restrict_
   int f = 0;
   for (int l = lane; l < n; l += 32) f = max(f, fx_field(x[l]));
   f = __reduce_max_sync(0xffffffffu, f);
-  const int ex = f == 0x7ff ? FXF_BAD : fx_exp(f);
+  const int ex = fx_row_exp(f);
   if (lane == 0) e[c] = ex;
-  if (ex == FXF_BAD) return;
+  if (ex == FX_BAD) return;
   for (int kp = lane; kp < fx_ld(n); kp += 32) {
     const int l = 2 * kp;
     U[c * ld + kp] = fx_pair(l < n ? fx_fix(x[l], ex) : FX_BIAS, l + 1 < n ? fx_fix(x[l + 1], ex) : FX_BIAS);
@@ -546,7 +545,7 @@ __global__ void __launch_bounds__(FXF_THREADS, 2) fock_fx_kernel(
             for (int x = 0; x < 4; ++x) {
               const int ed = eD[c0 + (x & 1 ? i : j)], es = x < 2 ? ea : ec, fs = x < 2 ? fa : fc;
               double v;
-              if (fs != 0x7ff && ed != FXF_BAD) {
+              if (fs != 0x7ff && ed != FX_BAD) {
                 float lv[FX_DIG];
 #pragma unroll
                 for (int L = 0; L < FX_DIG; ++L) lv[L] = acc[L][x];

@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_density_kernel(
     for (int k = 0; k < n; ++k)
       if (fabs(V[k + (size_t)n * i]) > fabs(big)) big = V[k + (size_t)n * i];
     sign[r] = big < 0 ? -1.0 : 1.0;
-    jw.e2[i] = 1;  // |entries| of an orthogonal matrix < 2
+    jw.e2[i] = isfinite(V[0]) ? 1 : FX_BAD;  // |entries| of an orthogonal matrix < 2 (NaN throughout: A was not finite)
   }
   __syncthreads();
   cta_fix(n, n, true, jw.e2, jw.U2, [&](int r, int k) { return sign[r] * V[k + (size_t)n * perm[r]]; });
