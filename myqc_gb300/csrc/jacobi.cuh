@@ -61,6 +61,37 @@ __device__ __forceinline__ float jac_block_sum(float v, double *red) {
 __device__ __forceinline__ double jac_block_max(double v, double *red) {
   return jac_block_reduce(v, red, 0.0, [](double a, double b) { return fmax(a, b); });
 }
+__device__ __forceinline__ float jac_block_max(float v, double *red) {
+  return jac_block_reduce(v, reinterpret_cast<float *>(red), 0.f, [](float a, float b) { return fmaxf(a, b); });
+}
+
+// Largest column sum of |f(i, j)|, i, j < n: a bound of the norm of a symmetric or
+// antisymmetric matrix.
+template <class F>
+__device__ __forceinline__ float jac_norm_bound(int n, double *red, F f) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  float r = 0.f;
+  for (int j = w; j < n; j += nw) {
+    float s = 0.f;
+    for (int i = lane; i < n; i += 32) s += fabsf(f(i, j));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    r = fmaxf(r, s);
+  }
+  return jac_block_max(r, red);
+}
+// acc(i, j, (X Y)_ij) of two n x n FP32 matrices
+template <class Acc>
+__device__ __forceinline__ void jac_mm_f32(int n, const float *X, const float *Y, Acc acc) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int j = w; j < n; j += nw)
+    for (int i = lane; i < n; i += 32) {
+      float s = 0.f;
+#pragma unroll 4
+      for (int l = 0; l < n; ++l) s = fmaf(X[i + n * l], Y[l + n * j], s);
+      acc(i, j, s);
+    }
+}
 
 // pair k of round r as rr_pair gives it (r < np - 1), without integer division
 __device__ __forceinline__ void rr_pair_fast(int np, int r, int k, int &p, int &q) {
@@ -209,15 +240,25 @@ struct JacobiWork {
 // SM): nine sweeps of 6 n^3.  So the sweeps run in FP32 for start vectors, and
 // FP64 work is products on the tensor cores (fixmm.cuh, rounded as FP64 or
 // better):
-//   V <- V (I - E/2 + 3/8 E^2), E = V^T V - I   orthonormal to rounding
+//   V <- V (I - E/2 + 3/8 E^2 [- 5/16 E^3]), E = V^T V - I   orthonormal to rounding
 //   A <- V^T A V                                off-diagonals 1e-6 ||A||_F
-//   twice: P = I + E + E^2/2 with the first-order rotations E_ij =
-//     a_ij / (a_jj - a_ii) of the pairs with |E_ij| <= 3e-4 (E is antisymmetric,
-//     so P is orthogonal to E^4/4 < 1e-14, and the second step's E is
-//     quadratically smaller); V <- V P, A <- P^T A P
-// Pairs too close for that (near-degenerate levels) are left to FP64 Jacobi
-// sweeps, which check the stopping rule of a cold solve and skip every rotation
-// below tol ||A||_F / n: usually the check alone.
+//   twice: P = I + E + E^2/2 [+ E^3/8] with the first-order rotations E_ij =
+//     a_ij / (a_jj - a_ii) of the pairs with |E_ij| <= 3e-4; V <- V P, A <- P^T A P
+//     (the second step's E is quadratically smaller)
+// What is left of either series is a power of ||E||, and nothing after it restores
+// orthogonality, so the terms in brackets are taken by a bound of that norm,
+// the largest column sum r of |E|:
+//   the start vectors' rounding leaves r = 1.7e-5 at n = 56 and 4e-5 at 110, and the
+//   quadratic polynomial 5/16 E^3: 4e-16 and 7e-15; the cubic term above 2e-5;
+//   E is antisymmetric, so P^T P - I = E^4/4 without and -E^6/64 with the cubic term,
+//   which is taken above r = 2.5e-4 (1e-15).  Levels spaced 1e-5 to 5e-4 of the norm
+//   give ||E|| = 1e-3 to 2e-3 (r up to 9e-3): max |V^T V - I| 1.5e-12 at n = 110
+//   without it, 2e-14 with it, as a cold FP64 Jacobi.  Above r = 6e-3 (7e-16) only
+//   the pairs with |E_ij| <= 6e-3 / n are rotated, which keeps r below that.
+// Pairs that this leaves (near-degenerate levels) go to FP64 Jacobi sweeps, which
+// check the stopping rule of a cold solve and skip every rotation below
+// tol ||A||_F / n: none where all levels are 1e-2 of the norm apart, two or three
+// where they are closer.
 static __device__ bool jacobi_block(int n, double *A, double *V, double *red, double *work, int max_sweeps,
                                     double tol) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
@@ -275,17 +316,19 @@ static __device__ bool jacobi_block(int n, double *A, double *V, double *red, do
     __syncthreads();
     cta_fix_mm(n, n, n, U1, e1, U1, e1, [&](int i, int j, double v) { V[i + n * j] = v - (i == j ? 1.0 : 0.0); });
     __syncthreads();
-    // E is about 1e-6: the FP32 rounding of its square is below 1e-18
-    float *Ef = reinterpret_cast<float *>(U1);
+    // ||E|| is below 1e-4: the FP32 rounding of its square and cube is below 1e-15 of 1
+    const bool cubic = jac_norm_bound(n, red, [&](int i, int j) { return (float)V[i + n * j]; }) > 2e-5f;
+    float *Ef = reinterpret_cast<float *>(U1), *Qf = Ef + n2;
     for (int idx = tid; idx < n2; idx += blockDim.x) Ef[idx] = (float)V[idx];
     __syncthreads();
-    for (int j = w; j < n; j += nw)
-      for (int i = lane; i < n; i += 32) {
-        float s = 0.f;
-#pragma unroll 4
-        for (int l = 0; l < n; ++l) s = fmaf(Ef[i + n * l], Ef[l + n * j], s);
-        V[i + (size_t)n * j] = (i == j ? 1.0 : 0.0) - 0.5 * V[i + (size_t)n * j] + 0.375 * (double)s;
-      }
+    if (cubic) {  // 3/8 E^2 - 5/16 E^3 = E (3/8 E - 5/16 E^2)
+      jac_mm_f32(n, Ef, Ef, [&](int i, int j, float s) { Qf[i + n * j] = 0.375f * Ef[i + n * j] - 0.3125f * s; });
+      __syncthreads();
+    }
+    const double c2 = cubic ? 1.0 : 0.375;
+    jac_mm_f32(n, Ef, cubic ? Qf : Ef, [&](int i, int j, float s) {
+      V[i + (size_t)n * j] = (i == j ? 1.0 : 0.0) - 0.5 * V[i + (size_t)n * j] + c2 * (double)s;
+    });
     __syncthreads();
     cta_fix(n, n, false, e1, U1, row(W));
     __syncthreads();
@@ -312,22 +355,37 @@ static __device__ bool jacobi_block(int n, double *A, double *V, double *red, do
   for (int step = 0; step < 2; ++step) {
     const double off2 = off_norm2();
     if (off2 <= stop2) return true;
-    constexpr double EMAX = 3e-4;
+    constexpr float EMAX = 3e-4f, RCUBIC = 2.5e-4f, RMAX = 6e-3f;
     constexpr int EEXP = -11;  // EMAX < 2^EEXP
+    float emax = EMAX;
     auto E = [&](int i, int j) {
       const double a = A[i + (size_t)n * j], gap = A[j + (size_t)n * j] - A[i + (size_t)n * i];
       const float x = (float)(a * scale), g = (float)(gap * scale);
-      return i != j && fabsf(x) <= (float)EMAX * fabsf(g) && g != 0.f ? (double)__fdividef(x, g) : 0.0;
+      return i != j && fabsf(x) <= emax * fabsf(g) && g != 0.f ? __fdividef(x, g) : 0.f;
     };
+    const float r = jac_norm_bound(n, red, E);
+    if (r > RMAX) emax = fminf(EMAX, RMAX / n);
     for (int i = tid; i < n; i += blockDim.x) e1[i] = EEXP, e2[i] = 1;
     __syncthreads();
-    cta_fix(n, n, true, e1, U2, [&](int r, int k) { return E(k, r); });  // the columns of E
+    cta_fix(n, n, true, e1, U2, [&](int r, int k) { return (double)E(k, r); });  // the columns of E
     __syncthreads();
     double *P = reinterpret_cast<double *>(U1);
     cta_fix_mm(n, n, n, U2, e1, U2, e1, [&](int i, int j, double v) {  // v = (E^T E)_ij = -(E^2)_ij
-      P[i + n * j] = (i == j ? 1.0 : 0.0) + E(i, j) - 0.5 * v;
+      P[i + n * j] = (i == j ? 1.0 : 0.0) + (double)E(i, j) - 0.5 * v;
     });
     __syncthreads();
+    if (r > RCUBIC) {  // E^3/8 is below 3e-8: FP32
+      float *Ef = reinterpret_cast<float *>(U2), *Qf = Ef + n2;
+      for (int j = w; j < n; j += nw)
+        for (int i = lane; i < n; i += 32) {
+          const float e = E(i, j);
+          Ef[i + n * j] = e;
+          Qf[i + n * j] = (float)(2.0 * (P[i + n * j] - (i == j ? 1.0 : 0.0) - (double)e));  // (E^2)_ij
+        }
+      __syncthreads();
+      jac_mm_f32(n, Ef, Qf, [&](int i, int j, float s) { P[i + n * j] += 0.125 * (double)s; });
+      __syncthreads();
+    }
     cta_fix(n, n, true, e2, U2, col(P));  // the columns of P
     __syncthreads();
     for (int i = tid; i < n; i += blockDim.x) e1[i] = 1;
