@@ -291,8 +291,9 @@ int mq_syev_batched(mq_ctx *ctx, int n, int batch, double *A, double *w, double 
 
 /* C = alpha op(A) op(B) + beta C on the device, host arrays column-major
  * (BLAS DGEMM semantics; transa/transb 'N' or 'T'), e.g. the DGEMM products of
- * the reference's SCF (src/scf/scf.f90:1306-1307).  Orders up to ~1000 run
- * on the library's own FP64 kernel spread over all SMs. */
+ * the reference's SCF (src/scf/scf.f90:1306-1307).  Each element is within the
+ * bound of an FP64 sum, about k 2^-53 sum |a||b|, whatever the sizes in its row and
+ * column; infinities, NaN and subnormals as in FP64. */
 int mq_dgemm(mq_ctx *ctx, char transa, char transb, int m, int n, int k, double alpha, const double *A, int lda,
              const double *B, int ldb, double beta, double *C, int ldc);
 

@@ -596,7 +596,7 @@ int mq_dgemm(mq_ctx *c, char transa, char transb, int m, int n, int k, double al
   const size_t na = (size_t)lda * (ta ? m : k), nb = (size_t)ldb * (tb ? k : n), nc = (size_t)ldc * n;
   double *dA = to_dev(c, "dgemm_A", A, na), *dB = to_dev(c, "dgemm_B", B, nb), *dC = to_dev(c, "dgemm_C", C, nc);
   if (!dA || !dB || !dC) return MQ_ENOMEM;
-  MQ_TRY(gemm(c, transa, transb, m, n, k, alpha, dA, lda, dB, ldb, beta, dC, ldc));
+  MQ_TRY(dgemm_batched(c, transa, transb, m, n, k, alpha, dA, lda, 0, dB, ldb, 0, beta, dC, ldc, 0, 1, true));
   MQ_CUDA(c, cudaMemcpyAsync(C, dC, nc * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   MQ_CUDA(c, cudaStreamSynchronize(c->stream));
   return MQ_OK;

@@ -2,9 +2,17 @@
 // column-major, as BLAS DGEMM, optionally strided-batched (blockIdx.z).
 //
 // FP64 issue on this GPU is two multiply-adds per clock and SM, so the products
-// are formed on the tensor cores from fixed-point digits (fixmm.cuh), correct to
-// FP64 rounding or better: 36 digit products per multiply-add at the 1024 per
-// clock and SM that mma.sync gives, 28 multiply-adds per clock and SM at best.
+// are formed on the tensor cores from fixed-point digits (fixmm.cuh): 36 digit
+// products per multiply-add at the 1024 per clock and SM that mma.sync gives, 28
+// multiply-adds per clock and SM at best.  Their error is bounded by the largest
+// elements of the row and the column, which is what the library's own steps need
+// (energies, projectors, eigenvectors).  mq_dgemm promises BLAS's DGEMM, whose error is
+// bounded by sum |a||b| of each element (GRADED): there the magnitudes are multiplied
+// too (one more digit product), and an element whose sum falls below 2^-5 of 2^(ea + eb),
+// the fixed point's unit, is summed in FP64 from the operands, in four interleaved sums
+// (K/4 roundings).  At that line the digits' bound is K 2^-53.8 sum |a||b|.  Order 512:
+// 53 us with random elements, 302 us with every element summed in FP64 (232 us of FP64
+// issue); order 224: 18 and 76 us.
 //
 // A CTA of 8 warps forms 32 x 32 tiles of C: it reads 32 rows of op(A) and 32
 // columns of op(B) over up to 128 of K into registers, finds their exponents,
@@ -17,9 +25,10 @@
 // run under each other's products, and spreads a product of order ~200 over
 // many SMs; larger tiles (64 x 64, one CTA per SM) were slower on both.
 //
-// A row or column with an infinity or NaN has no fixed-point form: its elements
-// of C are summed in FP64 from the operands as they are.
+// A row or column with an infinity or NaN has no fixed-point form either: its elements
+// of C are summed in FP64 as well.
 #include <algorithm>
+#include <type_traits>
 
 #include "fixmm.cuh"
 #include "internal.h"
@@ -89,7 +98,7 @@ __device__ __forceinline__ void gx_load(const double *__restrict__ x, size_t ld,
 }
 
 // C(r, c) at C[r sr + c sc]: rows r < mx of X, columns c < ny of Y
-template <bool XROW, bool YROW>
+template <bool XROW, bool YROW, bool GRADED>
 __global__ void __launch_bounds__(GX_THREADS, 2) dgemm_kernel(int mx, int ny, int k, double alpha,
                                                               const double *__restrict__ X, size_t ldx, long long sX,
                                                               const double *__restrict__ Y, size_t ldy, long long sY,
@@ -117,20 +126,28 @@ __global__ void __launch_bounds__(GX_THREADS, 2) dgemm_kernel(int mx, int ny, in
       if (!one || tile == (int)blockIdx.x)
         gx_load<YROW>(Yc + (YROW ? ldy * kb : (size_t)kb), ldy, min(GX_T, ny - c0), kc, fields + GX_T, ey, UY);
       __syncthreads();
-      float acc[FX_DIG][4];
-      fx_tile(UX, UY, GX_LD, GX_T, GX_T, wr, wc, (kc + 15) / 16, acc);
+      float acc[FX_DIG][4], mag[4];
+      fx_tile<GRADED>(UX, UY, GX_LD, GX_T, GX_T, wr, wc, (kc + 15) / 16, acc, &mag);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int r = wr + g + 8 * (i >> 1), c = wc + 2 * t + (i & 1);
         double x = 0.0;
-        if (ex[r] != FX_BAD && ey[c] != FX_BAD) {
+        if (ex[r] != FX_BAD && ey[c] != FX_BAD && (!GRADED || mag[i] >= 0x1p23f)) {
           float v[FX_DIG];
 #pragma unroll
           for (int L = 0; L < FX_DIG; ++L) v[L] = acc[L][i];
           x = fx_combine(v, ex[r], ey[c]);
         } else if (r0 + r < mx && c0 + c < ny) {
-          for (int l = kb; l < kb + kc; ++l)
-            x = fma(Xr[XROW ? r + ldx * l : l + ldx * r], Yc[YROW ? c + ldy * l : l + ldy * c], x);
+          double x4[4] = {0.0, 0.0, 0.0, 0.0};
+          auto term = [&](int l, double s) {
+            return fma(Xr[XROW ? r + ldx * l : l + ldx * r], Yc[YROW ? c + ldy * l : l + ldy * c], s);
+          };
+          int l = kb;
+          for (; l + 3 < kb + kc; l += 4)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x4[u] = term(l + u, x4[u]);
+          for (; l < kb + kc; ++l) x4[0] = term(l, x4[0]);
+          x = (x4[0] + x4[1]) + (x4[2] + x4[3]);
         }
         sum[i] = kb ? sum[i] + x : x;
       }
@@ -148,7 +165,7 @@ __global__ void __launch_bounds__(GX_THREADS, 2) dgemm_kernel(int mx, int ny, in
 
 int dgemm_batched(mq_ctx *c, char ta, char tb, int m, int n, int k, double alpha, const double *A, int lda,
                   long long sA, const double *B, int ldb, long long sB, double beta, double *C, int ldc,
-                  long long sC, int batch) {
+                  long long sC, int batch, bool graded) {
   if (m <= 0 || n <= 0 || batch <= 0) return MQ_OK;
   if (batch > 65535) return set_err(c, MQ_EINVAL, "dgemm: more than 65535 batched products");
   const bool TA = ta == 'T' || ta == 't', TB = tb == 'T' || tb == 't';
@@ -164,8 +181,12 @@ int dgemm_batched(mq_ctx *c, char ta, char tb, int m, int n, int k, double alpha
   const long long want = std::max<long long>(1, (8LL * sms + (long long)yt * batch - 1) / ((long long)yt * batch));
   const dim3 grid((unsigned)std::min<long long>(xt, want), yt, batch);
   const size_t sm = sizeof(uint4) * 2 * GX_T * GX_LD;
-  auto kern = xrow ? (yrow ? dgemm_kernel<true, true> : dgemm_kernel<true, false>)
-                   : (yrow ? dgemm_kernel<false, true> : dgemm_kernel<false, false>);
+  auto pick = [&](auto g) {
+    constexpr bool G = decltype(g)::value;
+    return xrow ? (yrow ? dgemm_kernel<true, true, G> : dgemm_kernel<true, false, G>)
+                : (yrow ? dgemm_kernel<false, true, G> : dgemm_kernel<false, false, G>);
+  };
+  auto kern = graded ? pick(std::true_type{}) : pick(std::false_type{});
   MQ_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   kern<<<grid, GX_THREADS, sm, c->stream>>>(mx, ny, k, alpha, swap ? B : A, swap ? ldb : lda, swap ? sB : sA,
                                             swap ? A : B, swap ? lda : ldb, swap ? sA : sB, beta, C, swap ? ldc : 1,

@@ -10,10 +10,17 @@
 // level (the products s_k s'_l with k + l = L) over K <= 144 stays below 2^24,
 // so the FP32 accumulators of mma.sync hold every level exactly in any order.
 // The levels L = 0..7 (36 digit products) are combined as integers and rounded
-// to FP64 once.  What is dropped -- the cutting of the operands, 2^-62 of the
-// row's largest element, and levels 8 to 14 -- is about 2^-61 of the largest
-// possible sum, so an element is correct to rounding unless it is 2^-8 of that
-// and less; an FP64 sum rounds after each of its K additions.
+// to FP64 once.  What is dropped, in units of 2^(ea + eb), a row's and a column's
+// power of two (up to four times the product of their largest elements):
+//   the cutting of both operands                       at most K 2^-61
+//   levels 8 to 14 (level 8: 7 products of 2^14 2^48 in 2^124)   K 2^-59.2
+// together at most K 2^-58.8, sqrt(K) 2^-62 for digits without a pattern.  So the error is
+// bounded by the rows' norms, not element by element: an element of C is correct to
+// rounding down to about K 2^-6 of 2^(ea + eb), below that it keeps fewer bits, and an
+// operand's element 2^-62 below its row's largest is lost, as are subnormals.
+// An FP64 sum rounds after each of its K additions, by 2^-53 sum |a||b| each.  Where that
+// bound has to hold for every element (dgemm.cu, mq_dgemm), sum |a||b| is formed
+// beside the product from the leading digits (fx_tile<true>).
 //
 // Why: this GPU issues two FP64 multiply-adds per clock and SM.  36 digit
 // products take the tensor cores a small part of that time; operands of up to a few hundred
@@ -142,16 +149,29 @@ __device__ __forceinline__ double fx_combine(const float *v, int ea, int eb) {
   return x * __hiloint2double((s1 + 1023) << 20, 0) * __hiloint2double((s2 + 1023) << 20, 0);
 }
 
+// The magnitudes of a pair in units of 2^(e - 14), to 2^-11 of themselves or one half
+__device__ __forceinline__ unsigned fx_mag(const uint4 &u) {
+  const unsigned d0 = fx_digit(u, 0), d1 = fx_digit(u, 1);
+  const __half2 h = __habs2(__hfma2(*reinterpret_cast<const __half2 *>(&d0), __half2half2(__ushort_as_half(0x5c00)),
+                                    *reinterpret_cast<const __half2 *>(&d1)));  // 256 s_0 + s_1
+  return *reinterpret_cast<const unsigned *>(&h);
+}
+
 // A 16 x 8 tile: rows of UA (fragment rows r0 + g, r0 + g + 8; clamped to
 // na - 1), columns = rows of UB (c0 + g, clamped), K = 16 ksteps.
+// MAG: mag = sum |a||b| in units of 2^(ea + eb - 28).
+template <bool MAG = false>
 __device__ __forceinline__ void fx_tile(const uint4 *UA, const uint4 *UB, int ld, int na, int nb, int r0, int c0,
-                                        int ksteps, float (&acc)[FX_DIG][4]) {
+                                        int ksteps, float (&acc)[FX_DIG][4], float (*mag)[4] = nullptr) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int ra = min(r0 + g, na - 1), rb = min(r0 + g + 8, na - 1), cb = min(c0 + g, nb - 1);
 #pragma unroll
   for (int L = 0; L < FX_DIG; ++L)
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[L][i] = 0.f;
+  if constexpr (MAG)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) (*mag)[i] = 0.f;
 #pragma unroll 1
   for (int ks = 0; ks < ksteps; ++ks) {
     const int k0 = 8 * ks + t;
@@ -159,6 +179,10 @@ __device__ __forceinline__ void fx_tile(const uint4 *UA, const uint4 *UB, int ld
                         UA[(size_t)ra * ld + fx_pos(ra, k0 + 4)], UA[(size_t)rb * ld + fx_pos(rb, k0 + 4)]};
     const uint4 b[2] = {UB[(size_t)cb * ld + fx_pos(cb, k0)], UB[(size_t)cb * ld + fx_pos(cb, k0 + 4)]};
     fx_block(acc, a, b);
+    if constexpr (MAG) {
+      const unsigned am[4] = {fx_mag(a[0]), fx_mag(a[1]), fx_mag(a[2]), fx_mag(a[3])}, bm[2] = {fx_mag(b[0]), fx_mag(b[1])};
+      fx_mma(*mag, am, bm);
+    }
   }
 }
 

@@ -463,10 +463,11 @@ int syev_large_warm(mq_ctx *c, int n, double *d_A, double *d_w, double *d_V);
 // syev_large_warm: FP32 cluster Jacobi and the FP64 first-order refinement,
 // queued on c->stream with no grid-wide barrier and nothing read back (eigen.cu)
 int syev_large_start(mq_ctx *c, int n, const double *d_A, double *d_V);
-// any FP64 product, batched over blockIdx.z with strides sA, sB, sC (dgemm.cu)
+// any FP64 product, batched over blockIdx.z with strides sA, sB, sC; graded: every
+// element within FP64's own bound, sum |a||b|, not the rows' norms (dgemm.cu)
 int dgemm_batched(mq_ctx *c, char ta, char tb, int m, int n, int k, double alpha, const double *A, int lda,
                   long long sA, const double *B, int ldb, long long sB, double beta, double *C, int ldc,
-                  long long sC, int batch);
+                  long long sC, int batch, bool graded = false);
 int gemm(mq_ctx *c, char ta, char tb, int m, int n, int k, double alpha, const double *A, int lda, const double *B,
          int ldb, double beta, double *C, int ldc);
 int gemm_strided_batched(mq_ctx *c, char ta, char tb, int m, int n, int k, double alpha, const double *A, int lda,
