@@ -25,6 +25,12 @@
 // run under each other's products, and spreads a product of order ~200 over
 // many SMs; larger tiles (64 x 64, one CTA per SM) were slower on both.
 //
+// A chunk of K takes a CTA 8.5 us, most of it latency, so a single product of few
+// tiles and more than three chunks splits K over the SMs; the parts go to a workspace
+// and are added in order: 32 x 32 x 512 37 -> 15 us, 32 x 32 x 100000 6635 -> 91,
+// 200 x 200 x 4096 255 -> 82.  (The library's own products have K up to their order, and at
+// four chunks more tiles than SMs.)
+//
 // A row or column with an infinity or NaN has no fixed-point form either: its elements
 // of C are summed in FP64 as well.
 #include <algorithm>
@@ -103,24 +109,29 @@ __global__ void __launch_bounds__(GX_THREADS, 2) dgemm_kernel(int mx, int ny, in
                                                               const double *__restrict__ X, size_t ldx, long long sX,
                                                               const double *__restrict__ Y, size_t ldy, long long sY,
                                                               double beta, double *__restrict__ C, size_t sr,
-                                                              size_t sc, long long sC) {
+                                                              size_t sc, long long sC, int kper,
+                                                              double *__restrict__ W) {
   extern __shared__ __align__(16) unsigned char gx_smem[];
   uint4 *UX = reinterpret_cast<uint4 *>(gx_smem), *UY = UX + GX_T * GX_LD;
   __shared__ int fields[2 * GX_T], ex[GX_T], ey[GX_T];
   const int tiles = (mx + GX_T - 1) / GX_T, c0 = blockIdx.y * GX_T;
-  X += sX * blockIdx.z;  // the batch's operands
-  Y += sY * blockIdx.z;
-  C += sC * blockIdx.z;
+  // blockIdx.z: the part of K whose sums go to W, or the member of the batch
+  const int kbeg = W ? blockIdx.z * kper : 0, kend = W ? min(k, kbeg + kper) : k;
+  if (!W) {
+    X += sX * blockIdx.z;
+    Y += sY * blockIdx.z;
+    C += sC * blockIdx.z;
+  }
   const double *Yc = Y + (YROW ? (size_t)c0 : ldy * c0);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int wr = (w & 1) * 16, wc = (w >> 1) * 8;
-  const bool one = k <= GX_K;
+  const bool one = kend - kbeg <= GX_K;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int r0 = tile * GX_T;
     const double *Xr = X + (XROW ? (size_t)r0 : ldx * r0);
     double sum[4];
-    for (int kb = 0; kb < k || kb == 0; kb += GX_K) {
-      const int kc = min(GX_K, k - kb);
+    for (int kb = kbeg; kb < kend || kb == kbeg; kb += GX_K) {
+      const int kc = min(GX_K, kend - kb);
       __syncthreads();  // the previous operands have been read
       gx_load<XROW>(Xr + (XROW ? ldx * kb : (size_t)kb), ldx, min(GX_T, mx - r0), kc, fields, ex, UX);
       if (!one || tile == (int)blockIdx.x)
@@ -149,18 +160,34 @@ __global__ void __launch_bounds__(GX_THREADS, 2) dgemm_kernel(int mx, int ny, in
           for (; l < kb + kc; ++l) x4[0] = term(l, x4[0]);
           x = (x4[0] + x4[1]) + (x4[2] + x4[3]);
         }
-        sum[i] = kb ? sum[i] + x : x;
+        sum[i] = kb > kbeg ? sum[i] + x : x;
       }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = r0 + wr + g + 8 * (i >> 1), c = c0 + wc + 2 * t + (i & 1);
       if (r >= mx || c >= ny) continue;
+      if (W) {
+        W[(size_t)mx * ny * blockIdx.z + r + (size_t)mx * c] = sum[i];
+        continue;
+      }
       double *cp = C + sr * r + sc * c;
       const double x = alpha == 1.0 ? sum[i] : alpha * sum[i];
       *cp = beta == 0.0 ? x : fma(beta, *cp, x);
     }
   }
+}
+
+// C = alpha (sum of the parts, in order) + beta C; elements as dgemm_kernel's
+__global__ void dgemm_parts_kernel(int mx, int ny, int parts, double alpha, const double *__restrict__ W, double beta,
+                                   double *__restrict__ C, size_t sr, size_t sc) {
+  const size_t mn = (size_t)mx * ny, idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= mn) return;
+  double t = W[idx];
+  for (int p = 1; p < parts; ++p) t += W[mn * p + idx];
+  double *cp = C + sr * (idx % mx) + sc * (idx / mx);
+  const double x = alpha == 1.0 ? t : alpha * t;
+  *cp = beta == 0.0 ? x : fma(beta, *cp, x);
 }
 
 int dgemm_batched(mq_ctx *c, char ta, char tb, int m, int n, int k, double alpha, const double *A, int lda,
@@ -179,7 +206,21 @@ int dgemm_batched(mq_ctx *c, char ta, char tb, int m, int n, int k, double alpha
   if (yt > 65535) return set_err(c, MQ_EINVAL, "dgemm: too many output tiles");
   // a few waves of two CTAs per SM, each with as many tiles of X as that leaves
   const long long want = std::max<long long>(1, (8LL * sms + (long long)yt * batch - 1) / ((long long)yt * batch));
-  const dim3 grid((unsigned)std::min<long long>(xt, want), yt, batch);
+  const long long tiles = (long long)xt * yt;
+  const int chunks = (k + GX_K - 1) / GX_K;
+  int parts = 1, kper = 0;
+  double *W = nullptr;
+  if (batch == 1 && chunks > 3 && tiles < sms) {
+    const int most = std::min(chunks, (int)(2 * sms / tiles)), per = (chunks + most - 1) / most;
+    parts = (chunks + per - 1) / per;
+    kper = per * GX_K;
+    // (products queued on the aux stream have sums of their own)
+    W = (double *)buf(c, c->aux && c->stream == c->aux ? "dgemm_parts_aux" : "dgemm_parts",
+                      sizeof(double) * parts * (size_t)mx * ny);
+    if (!W) return MQ_ENOMEM;
+  }
+  const size_t sr = swap ? ldc : 1, sc = swap ? 1 : ldc;
+  const dim3 grid((unsigned)std::min<long long>(xt, want), yt, W ? parts : batch);
   const size_t sm = sizeof(uint4) * 2 * GX_T * GX_LD;
   auto pick = [&](auto g) {
     constexpr bool G = decltype(g)::value;
@@ -189,9 +230,14 @@ int dgemm_batched(mq_ctx *c, char ta, char tb, int m, int n, int k, double alpha
   auto kern = graded ? pick(std::true_type{}) : pick(std::false_type{});
   MQ_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   kern<<<grid, GX_THREADS, sm, c->stream>>>(mx, ny, k, alpha, swap ? B : A, swap ? ldb : lda, swap ? sB : sA,
-                                            swap ? A : B, swap ? lda : ldb, swap ? sA : sB, beta, C, swap ? ldc : 1,
-                                            swap ? 1 : ldc, sC);
+                                            swap ? A : B, swap ? lda : ldb, swap ? sA : sB, beta, C, sr, sc, sC, kper,
+                                            W);
   c->stats.launches += 1;
+  if (W) {
+    dgemm_parts_kernel<<<(unsigned)(((size_t)mx * ny + 255) / 256), 256, 0, c->stream>>>(mx, ny, parts, alpha, W, beta,
+                                                                                       C, sr, sc);
+    c->stats.launches += 1;
+  }
   MQ_CUDA(c, cudaGetLastError());
   return MQ_OK;
 }
