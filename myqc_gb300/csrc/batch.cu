@@ -322,6 +322,16 @@ __global__ void batch_guess_kernel(const MolDesc *__restrict__ mols, const doubl
   for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x) D[md.mat + idx] = G[idx];
 }
 
+// out <- (D + D^T) / 2
+__global__ void batch_sym_kernel(const MolDesc *__restrict__ mols, const double *__restrict__ D,
+                                 double *__restrict__ out) {
+  const MolDesc md = mols[blockIdx.x];
+  const size_t n = md.n, n2 = n * n;
+  const double *Dm = D + md.mat;
+  for (size_t idx = threadIdx.x; idx < n2; idx += blockDim.x)
+    out[md.mat + idx] = 0.5 * (Dm[idx] + Dm[idx % n * n + idx / n]);
+}
+
 __global__ void batch_count_kernel(const int *__restrict__ active, int nmol, int *__restrict__ out) {
   __shared__ int s;
   if (threadIdx.x == 0) s = 0;
@@ -578,7 +588,15 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
   const int per_iter = 4 + (ndiis > 0 ? 1 : 0) + 3;  // digest (columns or split, tiles, 2), energy, diis, density
   StageTimer t_all;
   t_all.start(c->stream);
+  // the FP64 digestion sums J over one triangle of a symmetric density, which a
+  // caller's guess need not be
+  if (o->D_in && !L.arith) {
+    batch_sym_kernel<<<M, BT, 0, c->stream>>>(d_md, dD, (double *)d_DJ);
+    c->stats.launches += 1;
+    L.DJ = d_DJ;
+  }
   MQ_TRY(iteration());  // eager: sets kernel attributes outside any capture
+  if (!L.arith) L.DJ = dD;
   c->stats.launches += per_iter;
   int done_iters = 1;
   cudaGraphExec_t exec = nullptr;
