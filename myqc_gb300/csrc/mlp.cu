@@ -402,14 +402,17 @@ __global__ void __launch_bounds__(256) grad_sum_kernel(GradSums a) {
 
 // Adam on the three layers (blockIdx.y): W (nout x nin, FP32 master), b; writes
 // BF16 W [nout][ldw] and W^T [nin][ldt] (zero padding beyond the real sizes is
-// left as set up)
+// left as set up).  Nothing is updated once a GEMM's wait has run out (*err): its
+// gradients are not whole, and the host learns of it at the end of the epoch.
 struct AdamLayers {
   float *W[3], *mW[3], *vW[3], *b[3], *mb[3], *vb[3];
   const float *gW[3], *gb[3];
   bf16 *Wb[3], *Wt[3];
   int nout[3], nin[3], ldw[3], ldt[3];
 };
-__global__ void adam_kernel(AdamLayers a, float lr, float b1, float b2, float eps, float c1, float c2) {
+__global__ void adam_kernel(AdamLayers a, float lr, float b1, float b2, float eps, float c1, float c2,
+                            const int *__restrict__ err) {
+  if (*err) return;
   const int l = blockIdx.y;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nw = (long long)a.nout[l] * a.nin[l];
@@ -798,6 +801,8 @@ static int adam(mq_ctx *c, Mlp *m, float lr) {
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   m->step += 1;
   const float c1 = 1.0f / (1.0f - powf(b1, (float)m->step)), c2 = 1.0f / (1.0f - powf(b2, (float)m->step));
+  const int *err = (const int *)buf(c, "mlp_err", 64);
+  if (!err) return MQ_ENOMEM;
   AdamLayers p{};
   long long nmax = 0;
   for (int l = 0; l < 3; ++l) {
@@ -807,7 +812,7 @@ static int adam(mq_ctx *c, Mlp *m, float lr) {
     p.nout[l] = m->d[l + 1], p.nin[l] = m->d[l], p.ldw[l] = m->kp[l], p.ldt[l] = m->kp[l + 1];
     nmax = std::max(nmax, (long long)m->d[l + 1] * m->d[l] + m->d[l + 1]);
   }
-  adam_kernel<<<dim3((unsigned)((nmax + 255) / 256), 3), 256, 0, c->stream>>>(p, lr, b1, b2, eps, c1, c2);
+  adam_kernel<<<dim3((unsigned)((nmax + 255) / 256), 3), 256, 0, c->stream>>>(p, lr, b1, b2, eps, c1, c2, err);
   c->stats.launches += 1;
   MQ_CUDA(c, cudaGetLastError());
   return MQ_OK;
