@@ -44,7 +44,7 @@ __device__ __forceinline__ double bmax(double v, double *red) { return jac_block
 __global__ void __launch_bounds__(BT) batch_orth_kernel(const MolDesc *__restrict__ mols,
                                                         const double *__restrict__ S, double *__restrict__ X,
                                                         double *__restrict__ work, size_t wstride, int *__restrict__ status) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   __shared__ double red[32];
   const MolDesc md = mols[blockIdx.x];
   const int n = md.n;
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(BT) batch_diis_kernel(const MolDesc *__restric
                                                         double *__restrict__ Bm, int2 *__restrict__ state, int ndiis,
                                                         size_t mat_total, double *__restrict__ Fx,
                                                         double *__restrict__ work, size_t wstride) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   __shared__ double red[32];
   __shared__ double cvec[DIIS_MAX];
   __shared__ double sys[(DIIS_MAX + 1) * (DIIS_MAX + 2)];
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(BT) batch_density_kernel(
     const double *__restrict__ Fx, double *__restrict__ D, double *__restrict__ Dn, double *__restrict__ eps,
     int *__restrict__ iters, int *__restrict__ conv, const double *__restrict__ Ek, double *__restrict__ Efin,
     double thr, int conv_rms, int max_iter, double *__restrict__ work, size_t wstride, int *__restrict__ status) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   __shared__ double red[32];
   __shared__ int decision;
   const int m = blockIdx.x;

@@ -20,7 +20,7 @@ template <bool SMEM>
 __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(int n, double *__restrict__ Ag, double *__restrict__ wg,
                                                              double *__restrict__ Vg, double *__restrict__ work,
                                                              int max_sweeps, double tol, int *__restrict__ status) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   const int b = blockIdx.x;
   const size_t n2 = (size_t)n * n;
   double *Ain = Ag + n2 * b, *A = sm, *V = sm + n2;
