@@ -61,25 +61,7 @@ __device__ __forceinline__ float jac_block_sum(float v, double *red) {
 __device__ __forceinline__ double jac_block_max(double v, double *red) {
   return jac_block_reduce(v, red, 0.0, [](double a, double b) { return fmax(a, b); });
 }
-__device__ __forceinline__ float jac_block_max(float v, double *red) {
-  return jac_block_reduce(v, reinterpret_cast<float *>(red), 0.f, [](float a, float b) { return fmaxf(a, b); });
-}
 
-// Largest column sum of |f(i, j)|, i, j < n: a bound of the norm of a symmetric or
-// antisymmetric matrix.
-template <class F>
-__device__ __forceinline__ float jac_norm_bound(int n, double *red, F f) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  float r = 0.f;
-  for (int j = w; j < n; j += nw) {
-    float s = 0.f;
-    for (int i = lane; i < n; i += 32) s += fabsf(f(i, j));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    r = fmaxf(r, s);
-  }
-  return jac_block_max(r, red);
-}
 // acc(i, j, (X Y)_ij) of two n x n FP32 matrices
 template <class Acc>
 __device__ __forceinline__ void jac_mm_f32(int n, const float *X, const float *Y, Acc acc) {
@@ -238,23 +220,24 @@ struct JacobiWork {
 //
 // A cold FP64 Jacobi is bound by FP64 issue (two multiply-adds per clock and
 // SM): nine sweeps of 6 n^3.  So the sweeps run in FP32 for start vectors, and
-// FP64 work is products on the tensor cores (fixmm.cuh, rounded as FP64 or
-// better):
+// FP64 work is products on the tensor cores (fixmm.cuh: within rounding of the rows'
+// norms, as the whole solve is of ||A||):
 //   V <- V (I - E/2 + 3/8 E^2 [- 5/16 E^3]), E = V^T V - I   orthonormal to rounding
+//     (||E|| grows with n to 5e-5; without the cubic term max |V^T V - I| is 5e-16 at
+//     n = 15, 5e-15 at 56 and 1e-14 at 64, with it 1e-15 to 2e-15: taken above 64)
 //   A <- V^T A V                                off-diagonals 1e-6 ||A||_F
 //   twice: P = I + E + E^2/2 [+ E^3/8] with the first-order rotations E_ij =
 //     a_ij / (a_jj - a_ii) of the pairs with |E_ij| <= 3e-4; V <- V P, A <- P^T A P
 //     (the second step's E is quadratically smaller)
-// What is left of either series is a power of ||E||, and nothing after it restores
-// orthogonality, so the terms in brackets are taken by a bound of that norm,
-// the largest column sum r of |E|:
-//   the start vectors' rounding leaves r = 1.7e-5 at n = 56 and 4e-5 at 110, and the
-//   quadratic polynomial 5/16 E^3: 4e-16 and 7e-15; the cubic term above 2e-5;
-//   E is antisymmetric, so P^T P - I = E^4/4 without and -E^6/64 with the cubic term,
-//   which is taken above r = 2.5e-4 (1e-15).  Levels spaced 1e-5 to 5e-4 of the norm
-//   give ||E|| = 1e-3 to 2e-3 (r up to 9e-3): max |V^T V - I| 1.5e-12 at n = 110
-//   without it, 2e-14 with it, as a cold FP64 Jacobi.  Above r = 6e-3 (7e-16) only
-//   the pairs with |E_ij| <= 6e-3 / n are rotated, which keeps r below that.
+// Nothing after the steps restores orthogonality, and what they leave of it is a power of
+// the norm of E, not of its largest entry: E is antisymmetric, so P^T P - I = E^4/4
+// without and -E^6/64 with the cubic term.  The norm is bounded by r = ||E||_F / sqrt(2)
+// (singular values come in pairs; a dense E has r two to four times the norm), and the
+// term taken above r = 4e-4 (6e-15, some 2e-16).  Fock matrices of an SCF of (H2O)8 have r
+// around 3e-4.  Levels spaced 1e-5 to 5e-4 of the norm give ||E|| = 1e-3 to 2e-3 (r up to
+// 1e-2): max |V^T V - I| 1.5e-12 at n = 110 without the term, 2e-14 with it, as a cold
+// FP64 Jacobi.  Above r = 6e-3 (7e-16) only the pairs with |E_ij| <= 6e-3 / n are
+// rotated, whose norm is below that.
 // Pairs that this leaves (near-degenerate levels) go to FP64 Jacobi sweeps, which
 // check the stopping rule of a cold solve and skip every rotation below
 // tol ||A||_F / n: none where all levels are 1e-2 of the norm apart, two or three
@@ -316,11 +299,11 @@ static __device__ bool jacobi_block(int n, double *A, double *V, double *red, do
     __syncthreads();
     cta_fix_mm(n, n, n, U1, e1, U1, e1, [&](int i, int j, double v) { V[i + n * j] = v - (i == j ? 1.0 : 0.0); });
     __syncthreads();
-    // ||E|| is below 1e-4: the FP32 rounding of its square and cube is below 1e-15 of 1
-    const bool cubic = jac_norm_bound(n, red, [&](int i, int j) { return (float)V[i + n * j]; }) > 2e-5f;
+    // ||E|| is below 1e-4: the FP32 rounding of its square and cube is below 1e-15
     float *Ef = reinterpret_cast<float *>(U1), *Qf = Ef + n2;
     for (int idx = tid; idx < n2; idx += blockDim.x) Ef[idx] = (float)V[idx];
     __syncthreads();
+    const bool cubic = n > 64;
     if (cubic) {  // 3/8 E^2 - 5/16 E^3 = E (3/8 E - 5/16 E^2)
       jac_mm_f32(n, Ef, Ef, [&](int i, int j, float s) { Qf[i + n * j] = 0.375f * Ef[i + n * j] - 0.3125f * s; });
       __syncthreads();
@@ -355,20 +338,32 @@ static __device__ bool jacobi_block(int n, double *A, double *V, double *red, do
   for (int step = 0; step < 2; ++step) {
     const double off2 = off_norm2();
     if (off2 <= stop2) return true;
-    constexpr float EMAX = 3e-4f, RCUBIC = 2.5e-4f, RMAX = 6e-3f;
+    constexpr float EMAX = 3e-4f, RCUBIC = 4e-4f, RMAX = 6e-3f;
     constexpr int EEXP = -11;  // EMAX < 2^EEXP
     float emax = EMAX;
     auto E = [&](int i, int j) {
       const double a = A[i + (size_t)n * j], gap = A[j + (size_t)n * j] - A[i + (size_t)n * i];
       const float x = (float)(a * scale), g = (float)(gap * scale);
-      return i != j && fabsf(x) <= emax * fabsf(g) && g != 0.f ? __fdividef(x, g) : 0.f;
+      const float e = __fdividef(x, g);
+      return i != j && fabsf(e) <= emax ? e : 0.f;  // (x / 0 is not taken)
     };
-    const float r = jac_norm_bound(n, red, E);
-    if (r > RMAX) emax = fminf(EMAX, RMAX / n);
     for (int i = tid; i < n; i += blockDim.x) e1[i] = EEXP, e2[i] = 1;
     __syncthreads();
-    cta_fix(n, n, true, e1, U2, [&](int r, int k) { return (double)E(k, r); });  // the columns of E
-    __syncthreads();
+    float f2 = 0.f;
+    auto columns = [&]() {  // of E
+      cta_fix(n, n, true, e1, U2, [&](int c, int k) {
+        const float e = E(k, c);
+        f2 = fmaf(e, e, f2);
+        return (double)e;
+      });
+    };
+    columns();
+    const float r = sqrtf(0.5f * jac_block_sum(f2, red));
+    if (r > RMAX) {
+      emax = RMAX / n;
+      columns();
+      __syncthreads();
+    }
     double *P = reinterpret_cast<double *>(U1);
     cta_fix_mm(n, n, n, U2, e1, U2, e1, [&](int i, int j, double v) {  // v = (E^T E)_ij = -(E^2)_ij
       P[i + n * j] = (i == j ? 1.0 : 0.0) + (double)E(i, j) - 0.5 * v;
