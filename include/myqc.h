@@ -283,9 +283,10 @@ int mq_mp2_uhf(mq_ctx *ctx, const double *CA, const double *CB, const double *eA
 int mq_mp2_pairs(mq_ctx *ctx, const double *iajb, int no1, int nv1, int no2, int nv2, const double *e1,
                  const double *e2, int same_spin, double *e_out);
 
-/* Batched symmetric eigensolver (FP64 Jacobi): `batch` matrices of order n,
- * A (n*n each, column-major, overwritten) -> eigenvalues w (ascending, n each)
- * and eigenvectors V (n*n each).  Replaces DSYEV/DSYGV's eigen step
+/* Batched symmetric eigensolver: `batch` matrices of order n <= 1024, A (n*n each,
+ * column-major, overwritten) -> eigenvalues w (ascending, n each) and eigenvectors
+ * V (n*n each).  FP32 Jacobi start vectors (up to order 512), refined and finished in
+ * FP64: residual, eigenvalues and orthogonality to rounding of ||A||, as LAPACK's.  Replaces DSYEV/DSYGV's eigen step
  * (src/scf/scf.f90:692,848). */
 int mq_syev_batched(mq_ctx *ctx, int n, int batch, double *A, double *w, double *V);
 

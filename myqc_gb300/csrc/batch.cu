@@ -451,7 +451,9 @@ int batch_scf(mq_ctx *c, const mq_batch_opts *o, double *energy, int *iters, int
       }
       total[k] = mqo[k][M];
     }
-  // Fock tiles (i, j-run of 4, molecule) and per-molecule row tables
+  // Fock tiles (i, j-run of 4, molecule) and per-molecule row tables.  Runs of 1, 2 and
+  // 4: 1024 molecules 156, 143 and 134 ms of SCF, 24 molecules 24.2, 24.0 and 24.0,
+  // five clusters of 8 to 16 waters 173, 171 and 170.
   const int JC = 4;
   std::vector<int4> tl;
   std::vector<int> rf;

@@ -407,9 +407,12 @@ __global__ void __launch_bounds__(PAIR_MAX_THREADS) fock_pair_kernel(
 // K of one spin (S . D(:,j) and S . D(:,i)); as a fixed-point product (fixmm.cuh)
 // with the columns D(:,j), D(:,i) of both spins as the eight columns of one
 // mma.sync fragment, a 16 x 16 block of S takes 36 of them, 72 clocks of the
-// tensor pipe for 256 elements whatever the number of spins.  J_ij = <S, Dt>
+// tensor pipe for 256 elements whatever the number of spins; its error is bounded by
+// the largest elements of the slab's row and the density column, over 128 of l.  J_ij = <S, Dt>
 // stays on the FP64 pipe, beside it: S is symmetric, so only the blocks on and
-// below the diagonal are summed (half a multiply-add per element).
+// below the diagonal are summed (half a multiply-add per element).  (H2O)16 UHF 0.765 ->
+// 0.446 ms; on the counters no pipe is above 37 % (ALU: the conversion), and 13 warps an
+// SM wait for the slab rows.
 //
 // One warp per 16 rows k of a slab (the units of a tile's slabs are dealt to the
 // CTA's warps, so that small molecules keep them all busy); it reads its rows

@@ -174,8 +174,8 @@ __global__ void identity_kernel(double *__restrict__ A, int n) {
 // symmetric, so (X^2)_ij = sum_k X_ki X_kj: the tile's 16 + 16 columns are
 // staged in shared memory and each thread forms one element.  F64 = true
 // (the default): the columns as fixed-point pairs (|X_ij| <= 1, so with one
-// exponent) and the product on the tensor cores, correct to FP64 rounding
-// (fixmm.cuh): two 16 x 8 fragments, each with its K range shared by four warps,
+// exponent: an element is cut at 2^-61, absolutely) and the product on the tensor
+// cores, within n 2^-56.8 (fixmm.cuh): two 16 x 8 fragments, each with its K range shared by four warps,
 // whose sums are added in order; on the FP64 pipe the 16 x 16 x 224 products of a
 // step took 15 us of its 25.  F64 = false (contexts whose Fock
 // digestion is double-float, mq_set_fock_precision(MQ_FOCK_DF32)): the columns
